@@ -274,14 +274,23 @@ def prepare(case, seed):
         s["net"] = Surrogate(MODEL_ROW, N_STATS, ensemble=MEMBERS, seed=seed)
         rows, theta = _screen_rows(rng, 8192)
         stats = _screen_stats(theta, rng)
-        s["net"].train(rows, stats, epochs=4, batch=2048)
+        s["net"].train(rows, stats, epochs=40, batch=2048, lr=2e-3)
         # observed genes: the statistics of ordinary draws (both rates of switching and
         # expression near the middle of the prior), with 5 % noise
         G = case["genes"]
         near = theta.copy()[:G] * 0.3
         d = _screen_stats(near, rng)
         s["data"], s["se"] = d, 0.1 * np.abs(d) * rng.lognormal(0.0, 0.5, d.shape)
-        s["thr"] = np.full(G, 2.0)
+        # thresholds and the disagreement bound as the pipeline calibrates them on simulated
+        # draws: each gene keeps a few per cent of the prior, the bound passes 99 %
+        d_rows = torch.as_tensor(rows, device="cuda")
+        keep = torch.empty(8192, device="cuda", dtype=torch.uint8)
+        low = np.zeros((8192, G))
+        s["thr"], s["disagree"] = np.zeros(G), float(np.quantile(s["net"].predict(rows)[2], 0.99))
+        torch.cuda.synchronize()
+        s["net"].screen_device(d_rows.data_ptr(), MODEL_ROW, 8192, s["data"], s["se"], s["thr"], 0.0, s["disagree"],
+                               keep.data_ptr(), err_out=low, z=1.0)
+        s["thr"] = np.quantile(low, 0.06 / G ** 0.5, axis=0)
         fresh, _ = _screen_rows(rng, case["particles"])
         s["rows"] = fresh[:case["predict"]].copy()
         s["d_rows"] = torch.as_tensor(fresh, device="cuda")
@@ -344,8 +353,8 @@ def run(s):
         loss = s["net"].train(s["rows"], s["stats"], epochs=case["epochs"], batch=case["batch"])
         return {"loss": loss, "params": s["net"].params()}
     n = case["particles"]
-    kept = s["net"].screen_device(s["d_rows"].data_ptr(), MODEL_ROW, n, s["data"], s["se"], s["thr"], 0.0, 3.0,
-                                  s["keep"].data_ptr(), z=1.0)
+    kept = s["net"].screen_device(s["d_rows"].data_ptr(), MODEL_ROW, n, s["data"], s["se"], s["thr"], 0.0,
+                                  s["disagree"], s["keep"].data_ptr(), z=1.0)
     m = s["net"].compact_device(s["keep"].data_ptr(), s["d_rows"].data_ptr(), MODEL_ROW, n, s["out"].data_ptr(),
                                 s["idx"].data_ptr())
     mean, var, dis = s["net"].predict(s["rows"])
