@@ -416,7 +416,7 @@ static int prepare_simulate(abc_ctx* c, int64_t P, bool want_cells, int64_t* chu
   CK(c->d_rec.ensure(chunk));
   CK(c->d_recf.ensure(chunk));
   CK(c->d_order.ensure(chunk));
-  CK(c->d_ohist.ensure(128));
+  CK(c->d_ohist.ensure(kOrderWords));
   CK(c->d_counts.ensure((size_t)chunk * C));
   if (want_cells) {
     CK(c->d_captured.ensure((size_t)chunk * C));
@@ -456,7 +456,7 @@ static int enqueue_simulate(abc_ctx* c, int model, const int32_t* d_models, cons
     sa.fp32 = fp64 ? 0 : 1;
     CK(prof_mark(c));
     CK(launch_setup(sa, c->stream));
-    CK(launch_work_order(c->d_rec.p, n, c->d_ohist.p, c->d_order.p, c->stream));
+    CK(launch_work_order(c->d_rec.p, n, c->d_ohist.p, c->d_order.p, C, c->sms, std::max(1, bps), c->stream));
     SsaArgs ss;
     ss.cfg = sa.cfg;
     ss.rec = c->d_rec.p;
@@ -481,7 +481,13 @@ static int enqueue_simulate(abc_ctx* c, int model, const int32_t* d_models, cons
     if (!fp64) CK(launch_init_states(ss, c->sms, c->stream));
     CK(prof_mark(c));
     CK(cudaMemsetAsync(c->d_misc.p, 0, sizeof(unsigned long long), c->stream));
-    const int64_t warps_needed = (ss.n_items + 31) / 32;
+    // Few items: spread over one warp per scheduler (4 per SM), which then holds
+    // fewer trajectories; its lanes' breakpoints interrupt each other less
+    // (2,000 trajectories: 0.21 ms with 4 lanes in 500 warps, 0.27 with 32 in 63).
+    const int64_t warps1 = (int64_t)4 * c->sms;
+    if (!fp64 && ss.n_items <= 32 * warps1) ss.lanes = (int)((ss.n_items + warps1 - 1) / warps1);
+    if (!fp64) ss.plan = reinterpret_cast<const WorkPlan*>(c->d_ohist.p);
+    const int64_t warps_needed = (ss.n_items + ss.lanes - 1) / ss.lanes;
     int64_t grid = (int64_t)std::max(1, bps) * c->sms;
     grid = std::min<int64_t>(grid, (warps_needed + 3) / 4);
     grid = std::max<int64_t>(grid, 1);

@@ -244,8 +244,13 @@ cudaError_t launch_dist_screen(const float* mu, const float* var, const float* s
                                int64_t G, int K, const float* X, float z, int mode, uint8_t* keep, float* err_out,
                                cudaStream_t s);
 
-// particles ordered by expected trajectory cost, descending (hist128: 128 scratch words)
-cudaError_t launch_work_order(const PRec* rec, int64_t P, unsigned int* hist128, uint32_t* order, cudaStream_t s);
+// particles ordered by expected trajectory cost, descending; scratch
+// (kOrderWords words) starts with the batch's WorkPlan for n_cells cells on
+// sms multiprocessors with at most blocks_per_sm blocks each
+constexpr int kOrderHist = (int)(sizeof(WorkPlan) / sizeof(unsigned int));
+constexpr int kOrderWords = kOrderHist + 128;
+cudaError_t launch_work_order(const PRec* rec, int64_t P, unsigned int* scratch, uint32_t* order, int64_t n_cells,
+                              int sms, int blocks_per_sm, cudaStream_t s);
 int ssa_blocks_per_sm_fp64();
 int ssa_blocks_per_sm_fp32(int variant = 0);
 

@@ -36,6 +36,15 @@ enum : uint32_t { CH_ON = 0, CH_OFF = 1, CH_TXU = 2, CH_TXL = 3, CH_DEGU = 4, CH
 // status word bits
 enum : int { STF_EVENT_CAP = 1, STF_OVERFLOW = 2, STF_NONFINITE = 4 };
 
+// Work estimates of a batch of particles (launch_work_order): expected
+// iterations of the longest trajectory and their sum over the particles, and
+// the blocks of the production kernel that run.
+struct WorkPlan {
+  unsigned int max_cost;  // bits of a non-negative float
+  unsigned int blocks;
+  unsigned long long sum_cost;
+};
+
 struct SsaArgs {
   DevCfg cfg;
   const PRec* rec;
@@ -56,6 +65,16 @@ struct SsaArgs {
   int* status;
   int want_hash;
   int chunk = 1;             // production kernel: consecutive items a lane takes per pull
+  int lanes = 32;            // production kernel: lanes of a warp that take work
+  const WorkPlan* plan = nullptr;  // production kernel: which blocks run, NULL = all
+  // Production kernel: how long lanes may wait at a breakpoint.  The special
+  // section costs about one trip of the whole warp however many lanes it
+  // serves, so it runs once the lanes waiting have together idled that much
+  // (10^9 iterations/s with 0, 1, 2, 3, 6, 10 trips, 38 particles x 2,000
+  // cells: 62,000 iterations per trajectory 345, 347, 345, 341, 332, 325;
+  // 3,300 iterations 191, 225, 222, 221, 211, 203).  An argument, not a
+  // constant: the loop compiles to a third faster code for a lone warp.
+  int wait = 1;
   uint32_t rk[20];           // Philox round keys (seed + r * Weyl), filled by the FP32 launcher
 };
 

@@ -5,12 +5,13 @@
 // kernel (ssa.cuh); what changes is how the work maps to the GB300:
 //   * trips: all lanes of a warp run in lockstep, two SSA iterations per
 //     trip, both fed by one Philox4x32-10 block of the lane's stream (words
-//     x, y for the first iteration, z, w for the second).  A lane that
-//     reaches a breakpoint in the first iteration leaves the second one's
-//     words unused, so the stream a trajectory consumes depends only on the
-//     trajectory itself (reproducible, independent of scheduling).  The
-//     counter words that are constant for a trajectory (stream, cell,
-//     particle) are folded into the first Philox round once per trajectory;
+//     x, y for the first iteration, z, w for the second), computed one trip
+//     ahead.  A lane that reaches a breakpoint in the first iteration leaves
+//     the second one's words unused, so the stream a trajectory consumes
+//     depends only on the trajectory itself (reproducible, independent of
+//     scheduling).  The counter words that are constant for a trajectory
+//     (stream, cell, particle) are folded into the first Philox round once
+//     per trajectory;
 //   * clock: within an interval (between two breakpoints, at most one age
 //     step long) the elapsed time is an FP32 Kahan-compensated sum; the
 //     interval start is an integer number of grid quanta (or FP64 when the
@@ -23,23 +24,31 @@
 //     the switch toggles G and a proposal landing at the top by rounding is a
 //     rejection.  Transcription alpha size(t)^s is thinned against its value
 //     at the interval end (linear in time for s in {0, 1}: at0 + at1 t).
-//     The channel is taken from 0/1 step values of the cumulative thresholds
-//     and the counts and G are updated with FP32 arithmetic on them, which
-//     runs on the full-rate FMA pipe instead of compare/select/predicate
-//     instructions on the half-rate ALU pipe (the limit of this kernel);
-//   * the hot loop (a trip) has no divergent control flow: breakpoints,
+//     The channel is taken from one compare per cumulative threshold, whose
+//     predicates guard FP32 additions to the counts and G: full-rate FMA-pipe
+//     work, with the half-rate ALU pipe left to the compares;
+//   * the hot loop (two trips) has no divergent control flow: breakpoints,
 //     divisions, finished trajectories, refills and the event cap are handled
-//     behind one warp-uniform test; events and rejections are counted in FP32
-//     and flushed to integers at breakpoints;
-//   * division: the lanes of the warp that divide in the same trip are
-//     served one after another by the whole warp: each lane popcounts 1/32
-//     of the Bin(n, 1/2) bits (stream ST_AUX, blocks cycle << 24 + i, the
-//     bits of the FP64 mode's sampler layout in 128-bit blocks), summed with
-//     a warp reduction;
+//     behind one warp-uniform test, for several waiting lanes at a time;
+//     iterations and events are counted in FP32 and flushed to integers there;
+//   * division: Bin(n, 1/2) is the popcount of n random bits (stream ST_AUX,
+//     blocks cycle << 24 + i, the bits of the FP64 mode's sampler layout in
+//     128-bit blocks).  Lanes with small counts halve theirs side by side;
+//     large counts are served one lane after another by the whole warp, each
+//     lane taking 1/32 of the bits, summed with a warp reduction;
 //   * molecule counts are FP32 integers (exact below 2^24; a count reaching
 //     2^23 at a breakpoint is reported as ABC_ERR_NONFINITE);
 //   * work: each lane pulls `chunk` consecutive (particle, cell) items per
-//     warp-aggregated atomic from the LPT-ordered particle list.
+//     warp-aggregated atomic from the LPT-ordered particle list; the number
+//     of blocks per SM that run follows from the batch's work estimates
+//     (planned_blocks).
+// The loop is bound by instruction issue and dispatch: about 63 instructions
+// per iteration of a warp (19 of them on the half-rate ALU pipe), 398 x 10^9
+// iterations/s over the GPU with eight blocks per SM on a particle of 62,000
+// iterations per trajectory; 81 instructions and 321 x 10^9 before the
+// compares replaced arithmetic on 0/1 step values and the breakpoints were
+// gathered.  A lone warp per scheduler, where the chain of one trajectory
+// counts, takes 76 ns per iteration (113 before the Philox block moved ahead).
 // Results are a different (equally valid) realisation than the FP64 mode.
 #pragma once
 #include <limits.h>
@@ -72,7 +81,7 @@ struct LaneF {
   T tobs;                // observation time (the cell's age)
   T cs;                  // start of the current cycle
   float el, comp;        // elapsed time in the interval, Kahan compensation
-  float len;             // interval length
+  float len;             // interval length; -1 once its end is reached
   float at0, at1;        // transcription rate at0 + at1 x (elapsed time), exponent s in {0, 1}
   float amax;            // its value at the interval end: the thinning bound
   float lamc;            // labelling probability in this interval
@@ -81,11 +90,11 @@ struct LaneF {
   float alp, scal;       // transcription rate of the step and size exponent (general exponent only)
   float uu, lu, us, ls;  // molecule counts (exact integers in FP32)
   float G;               // gene state, 0 or 1
-  float evf, rejf;       // iterations that were not breakpoints, and rejections among them, since the last flush
+  float evf, firedf;     // iterations that were not breakpoints, and events fired among them, since the last flush
   int k, lab, cyc;
   int ev;                // flushed iteration count of this trajectory
   int rej;               // flushed thinning rejections
-  uint32_t block;        // next Philox block of the main stream
+  uint32_t block;        // Philox block of the first trip since the last flush
   uint32_t r1x, r1y, r1z;  // first Philox round: the trajectory's constant counter words folded in
   int plocal, ci;
 };
@@ -181,19 +190,34 @@ __device__ __forceinline__ void set_interval(LaneF<GRID>& s, typename LaneF<GRID
   }
 }
 
-// 1 where the channel uniform r has passed threshold c, else 0
-__device__ __forceinline__ float past(float r, float c) { return r >= c ? 1.0f : 0.0f; }
+// log2 and reciprocal approximations that treat subnormals as zero: the
+// operands here are not subnormal (U in [2^-23, 1]; a total propensity below
+// 2^-126 gives an infinite waiting time, one above 2^126 a zero one)
+__device__ __forceinline__ float log2_fast(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
-// One SSA iteration from two random words.  Returns true when the interval
-// end (len) comes before the next reaction: a breakpoint, with the lane's
-// state unchanged.  Otherwise applies the event or the thinning rejection.
-// The channel is found from 0/1 step values of the cumulative thresholds and
-// every update is FP32 arithmetic on them (FMA pipe), not selects: for
-// thresholds h1 <= h2 <= ... each channel's indicator is a difference of
-// neighbouring steps.  G is 0.0 or 1.0, so G x (rate) selects exactly.
+// One SSA iteration from two random words.  When the interval end (len)
+// comes before the next reaction the lane's counts and gene state stay as
+// they are and len becomes -1, so that every further iteration does nothing
+// until the breakpoint is handled.  Otherwise applies the event or the
+// thinning rejection.  The thresholds of the channels are nested, so one
+// compare each tells r's channel by the difference of neighbouring outcomes;
+// the compares' predicates guard FP32 additions of the threshold's change to
+// the counts (FMA pipe).  Measured against 0/1 step values combined
+// arithmetically: 63 instead of 73 instructions per iteration of a warp, 19
+// instead of 26 of them on the half-rate ALU pipe (a chain in which each
+// compare also excludes the ones before costs an ALU instruction per link).
+// G is 0.0 or 1.0, so G x (rate) selects exactly.
 template <bool SPLICE, bool GENSCAL, bool GRID>
-__device__ __forceinline__ bool ev_step(LaneF<GRID>& s, float koff, float beta, float invT, float len, uint32_t wt,
-                                        uint32_t wc) {
+__device__ __forceinline__ void ev_step(LaneF<GRID>& s, float koff, float beta, float invT, uint32_t wt, uint32_t wc) {
   const float G = s.G;
   const float sw = fmaf(G, koff, fmaf(-G, s.kon, s.kon));  // k_off if on, k_on if off (exact)
   float c2, c3 = 0.0f, c4 = 0.0f, top;
@@ -210,18 +234,13 @@ __device__ __forceinline__ bool ev_step(LaneF<GRID>& s, float koff, float beta, 
   // waiting time: U1 in (0, 1] from the low 23 bits of wt (mantissa fill);
   // the rates are in log2 units, so -log2(U1) / a0 is the time
   const float U1 = 2.0f - __uint_as_float(0x3F800000u | (wt & 0x7FFFFFu));
-  const float tau = __fdividef(-__log2f(U1), a0);  // a0 = 0 gives inf or NaN: a breakpoint
-  const float y = tau - s.comp;
+  // (a0 = 0 gives inf or NaN: a breakpoint), less the compensation of the clock
+  const float y = fmaf(-log2_fast(U1), rcp_fast(a0), -s.comp);
   const float tt = s.el + y;
-  // no branch: at a breakpoint (ok = 0) every update of the counts, G and the
-  // counters below is multiplied by zero, so the lane's state is unchanged;
-  // the clock (el, comp) may advance past the interval, since the breakpoint
-  // that follows starts a new interval at el = comp = 0
-  const bool ok = tt < len;
-  const float okf = ok ? 1.0f : 0.0f;
+  // no branch: the clock (el, comp) may advance past the interval, since the
+  // breakpoint that follows starts a new interval at el = comp = 0
   s.comp = (tt - s.el) - y;
   s.el = tt;
-  s.evf += okf;
   // channel: 32-bit uniform times a0
   const float r = __uint2float_rn(wc) * (a0 * 2.3283064365386963e-10f);
   float at;
@@ -231,21 +250,64 @@ __device__ __forceinline__ bool ev_step(LaneF<GRID>& s, float koff, float beta, 
     at = s.alp * exp2f(s.scal * __log2f(fmaf(s.ph0 + tt, invT, 1.0f)));
   at = at * G;  // no transcription while off
   // [switch | ... | labelled tx | unlabelled tx | rejection] above top
-  const float hs = past(r, sw), h2 = past(r, c2), ht = past(r, top);
-  const float hl = past(r, fmaf(at, s.lamc, top)), ha = past(r, top + at);
-  s.G = fmaf(okf - okf * hs, fmaf(-2.0f, G, 1.0f), G);  // r < sw: switch
-  if (!SPLICE) {
-    s.uu = fmaf(okf, (hl - ha) - (hs - h2), s.uu);  // unlabelled transcription - decay of u
-    s.lu = fmaf(okf, (ht - hl) - (h2 - ht), s.lu);  // labelled transcription - decay of l
-  } else {
-    const float h3 = past(r, c3), h4 = past(r, c4);
-    s.uu = fmaf(okf, (hl - ha) - (hs - h2), s.uu);  // transcription - splicing
-    s.us = fmaf(okf, (hs - h2) - (h3 - h4), s.us);  // splicing - decay
-    s.lu = fmaf(okf, (ht - hl) - (h2 - h3), s.lu);
-    s.ls = fmaf(okf, (h2 - h3) - (h4 - ht), s.ls);
-  }
-  s.rejf = fmaf(okf, ha, s.rejf);  // thinning rejection (or a proposal that rounding put at the top)
-  return !ok;
+  const float tl = fmaf(at, s.lamc, top), ta = top + at;
+  if (!SPLICE)
+    asm("{\n\t"
+        ".reg .pred k, p0, p1, p2, p3, p4;\n\t"
+        "setp.lt.f32 k, %6, %4;\n\t"
+        "setp.lt.and.f32 p0, %7, %8, k;\n\t"
+        "setp.lt.and.f32 p1, %7, %9, k;\n\t"
+        "setp.lt.and.f32 p2, %7, %10, k;\n\t"
+        "setp.lt.and.f32 p3, %7, %11, k;\n\t"
+        "setp.lt.and.f32 p4, %7, %12, k;\n\t"
+        "selp.f32 %4, %4, 0fBF800000, k;\n\t"
+        "@p0 sub.f32 %0, 0f3F800000, %0;\n\t"   // [0, sw): switch
+        "@p1 add.f32 %1, %1, 0fBF800000;\n\t"   // [sw, c2): decay of u
+        "@p0 add.f32 %1, %1, 0f3F800000;\n\t"
+        "@p2 add.f32 %2, %2, 0fC0000000;\n\t"   // [c2, top): decay of l
+        "@p1 add.f32 %2, %2, 0f3F800000;\n\t"
+        "@p3 add.f32 %2, %2, 0f3F800000;\n\t"   // [top, tl): labelled transcription
+        "@p3 add.f32 %1, %1, 0fBF800000;\n\t"
+        "@p4 add.f32 %1, %1, 0f3F800000;\n\t"   // [tl, ta): unlabelled transcription
+        "@p4 add.f32 %3, %3, 0f3F800000;\n\t"
+        "@k add.f32 %5, %5, 0f3F800000;\n\t"
+        "}"
+        : "+f"(s.G), "+f"(s.uu), "+f"(s.lu), "+f"(s.firedf), "+f"(s.len), "+f"(s.evf)
+        : "f"(tt), "f"(r), "f"(sw), "f"(c2), "f"(top), "f"(tl), "f"(ta));
+  else
+    asm("{\n\t"
+        ".reg .pred k, p0, p1, p2, p3, p4, p5, p6;\n\t"
+        "setp.lt.f32 k, %8, %6;\n\t"
+        "setp.lt.and.f32 p0, %9, %10, k;\n\t"
+        "setp.lt.and.f32 p1, %9, %11, k;\n\t"
+        "setp.lt.and.f32 p2, %9, %12, k;\n\t"
+        "setp.lt.and.f32 p3, %9, %13, k;\n\t"
+        "setp.lt.and.f32 p4, %9, %14, k;\n\t"
+        "setp.lt.and.f32 p5, %9, %15, k;\n\t"
+        "setp.lt.and.f32 p6, %9, %16, k;\n\t"
+        "selp.f32 %6, %6, 0fBF800000, k;\n\t"
+        "@p0 sub.f32 %0, 0f3F800000, %0;\n\t"   // [0, sw): switch
+        "@p1 add.f32 %1, %1, 0fBF800000;\n\t"   // [sw, c2): splicing of unlabelled
+        "@p0 add.f32 %1, %1, 0f3F800000;\n\t"
+        "@p1 add.f32 %3, %3, 0f3F800000;\n\t"
+        "@p0 add.f32 %3, %3, 0fBF800000;\n\t"
+        "@p2 add.f32 %2, %2, 0fBF800000;\n\t"   // [c2, c3): splicing of labelled
+        "@p1 add.f32 %2, %2, 0f3F800000;\n\t"
+        "@p2 add.f32 %4, %4, 0f3F800000;\n\t"
+        "@p1 add.f32 %4, %4, 0fBF800000;\n\t"
+        "@p3 add.f32 %3, %3, 0fBF800000;\n\t"   // [c3, c4): decay of unlabelled spliced
+        "@p2 add.f32 %3, %3, 0f3F800000;\n\t"
+        "@p4 add.f32 %4, %4, 0fBF800000;\n\t"   // [c4, top): decay of labelled spliced
+        "@p3 add.f32 %4, %4, 0f3F800000;\n\t"
+        "@p5 add.f32 %2, %2, 0f3F800000;\n\t"   // [top, tl): labelled transcription
+        "@p4 add.f32 %2, %2, 0fBF800000;\n\t"
+        "@p6 add.f32 %1, %1, 0f3F800000;\n\t"   // [tl, ta): unlabelled transcription
+        "@p5 add.f32 %1, %1, 0fBF800000;\n\t"
+        "@p6 add.f32 %5, %5, 0f3F800000;\n\t"
+        "@k add.f32 %7, %7, 0f3F800000;\n\t"
+        "}"
+        : "+f"(s.G), "+f"(s.uu), "+f"(s.lu), "+f"(s.us), "+f"(s.ls), "+f"(s.firedf), "+f"(s.len), "+f"(s.evf)
+        : "f"(tt), "f"(r), "f"(sw), "f"(c2), "f"(c3), "f"(c4), "f"(top), "f"(tl), "f"(ta));
 }
 
 // Breakpoint at s.te (reached): labelling state, age step, cycle (division
@@ -312,29 +374,49 @@ __device__ __forceinline__ int warp_halve(int n, uint32_t& blk, uint32_t cell, u
   return (int)__reduce_add_sync(0xffffffffu, (unsigned)k);
 }
 
-// Events and rejections counted in FP32 since the last flush: flushed to the
-// integer counts at breakpoints and when the count reaches this (exact below 2^24)
-constexpr float kFlushF = 4194304.0f;  // 2^22
-
-template <bool GRID>
-__device__ __forceinline__ void flush_counts(LaneF<GRID>& s) {
-  s.ev += (int)s.evf;
-  s.rej += (int)s.rejf;
-  s.evf = 0.0f;
-  s.rejf = 0.0f;
+// The same count computed by one lane alone, for small n (a block or two):
+// when several lanes divide together they do so side by side.
+__device__ __forceinline__ int lane_halve(int n, uint32_t& blk, uint32_t cell, uint32_t particle, const uint32_t* rk) {
+  int k = 0;
+  for (int m = n; m > 0; m -= 128) {
+    U4 c;
+    c.x = blk++;
+    c.y = ST_AUX << 30;
+    c.z = cell;
+    c.w = particle;
+    const U4 o = philox_rk(c, rk);
+    const uint64_t lo = ((uint64_t)o.y << 32) | o.x, hi = ((uint64_t)o.w << 32) | o.z;
+    const uint64_t mlo = m >= 64 ? ~(uint64_t)0 : (((uint64_t)1) << m) - 1;
+    const uint64_t mhi = m >= 128 ? ~(uint64_t)0 : m > 64 ? (((uint64_t)1) << (m - 64)) - 1 : 0;
+    k += __popcll(lo & mlo) + __popcll(hi & mhi);
+  }
+  return k;
 }
+
+// counts halved by the lane itself up to this size (three Philox blocks)
+constexpr float kLaneHalveMax = 384.0f;
+
+// Trips between flushes of the FP32 counts (at most two per trip: exact below 2^24)
+constexpr int kFlushTrips = 1 << 21;
 
 // MINB: resident 128-thread blocks per SM the register allocation targets
 // (chosen at run time by the autotuner, abc_autotune).  GENSCAL: a general
 // size exponent (the scaling column of theta) instead of s in {0, 1}.
 //
-// Loop shape: the hot part is one trip (a Philox block and two iterations)
-// with no divergent control flow; everything rare -- breakpoints, divisions,
-// finished trajectories, refills, the event cap -- is handled behind one
-// warp-uniform test, for the lanes that need it.
+// Loop shape: the hot part is two trips (four iterations) with no divergent
+// control flow.  The Philox block of the next trip is computed during this
+// one: it does not depend on the events, so its ten dependent rounds leave
+// the chain of the trajectory, which is what bounds a warp that has its
+// scheduler nearly to itself.  Everything rare -- breakpoints, divisions,
+// finished trajectories, refills, the event cap -- is the special section
+// behind one warp-uniform test.  A lane at a breakpoint waits there until the
+// section runs for several lanes at once; it then continues with the block
+// after the one that held the breakpoint, so its stream depends neither on
+// the wait nor on the trips that passed meanwhile.
 template <bool SPLICE, int MINB, bool GRID, bool GENSCAL>
 __global__ void __launch_bounds__(128, MINB) ssa_kernel_f32(SsaArgs A) {
   using T = typename LaneF<GRID>::T;
+  if (A.plan && blockIdx.x >= A.plan->blocks) return;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const DevCfg& cfg = A.cfg;
@@ -349,23 +431,38 @@ __global__ void __launch_bounds__(128, MINB) ssa_kernel_f32(SsaArgs A) {
   s.r1x = s.r1y = s.r1z = 0;
   s.len = -1.0f;  // no trajectory: every iteration is a breakpoint, which an inactive lane ignores
   s.el = s.comp = 0.0f;
-  s.evf = s.rejf = 0.0f;
+  s.at0 = s.at1 = s.amax = s.lamc = s.kon = s.gam = s.G = 0.0f;
+  s.uu = s.lu = s.us = s.ls = s.evf = s.firedf = 0.0f;
+  if (GENSCAL) s.ph0 = s.alp = s.scal = 0.0f;
   float koff = 0.f, beta = 0.f;
-  bool active = false, done = false;
+  // lanes beyond A.lanes take no work: a launch with few items spreads them
+  // over more warps instead of filling the lanes of a few
+  bool active = false, done = lane >= A.lanes;
   // work cursor: the launch keeps n_items below 2^31 (the host splits larger batches)
   uint32_t inext = 0;
   int left = 0;  // items left in this lane's pulled chunk
   int err = 0;
-  bool bp = false, special = true;
+  unsigned act = 0, waiting = 0;  // lanes with a trajectory, and those of them at a breakpoint
+  int trips = 0, due = 0;         // trips since the special section, and when it runs again
+  U4 w = {0u, 0u, 0u, 0u};        // random words of the next trip
   while (true) {
-    if (__any_sync(FULL, special)) {
-      // ---- breakpoints (divergent, short); divisions are flagged for the warp
+    if (trips >= due) {
+      // ---- breakpoints (divergent, short); divisions are flagged
       bool fin = false, div = false;
-      if (active && bp) {
-        flush_counts(s);
-        fin = on_breakpoint<GRID, GENSCAL>(s, cfg, A.recf, invT, div);
+      const bool bp = active && s.len < 0.0f;
+      if (bp) fin = on_breakpoint<GRID, GENSCAL>(s, cfg, A.recf, invT, div);
+      // ---- divisions: small counts by their lanes side by side, large ones
+      // one lane after another by the whole warp
+      const float most = fmaxf(fmaxf(s.uu, s.lu), fmaxf(s.us, s.ls));
+      if (div && most <= kLaneHalveMax) {
+        const uint32_t cL = s.r1y * kPhiloxM1Inv, pL = s.r1z ^ A.rk[1];
+        uint32_t blk = (uint32_t)s.cyc << 24;
+        s.uu = (float)lane_halve((int)s.uu, blk, cL, pL, A.rk);
+        if (SPLICE) s.us = (float)lane_halve((int)s.us, blk, cL, pL, A.rk);
+        s.lu = (float)lane_halve((int)s.lu, blk, cL, pL, A.rk);
+        if (SPLICE) s.ls = (float)lane_halve((int)s.ls, blk, cL, pL, A.rk);
+        div = false;
       }
-      // ---- divisions of this trip, one lane after another, by the whole warp
       unsigned dm = __ballot_sync(FULL, div);
       while (dm) {
         const int L = __ffs(dm) - 1;
@@ -388,18 +485,23 @@ __global__ void __launch_bounds__(128, MINB) ssa_kernel_f32(SsaArgs A) {
         }
       }
       if (active) {
+        // two iterations per trip; a breakpoint ends its trip
+        const int done_it = (int)s.evf;
+        s.block += (uint32_t)(done_it >> 1) + (bp ? 1u : 0u);
+        s.ev += done_it;
+        s.rej += done_it - (int)s.firedf;
+        s.evf = 0.0f;
+        s.firedf = 0.0f;
         if (bp && !fin &&
             (!(s.uu < kCountLimitF) || !(s.lu < kCountLimitF) || !(s.us < kCountLimitF) || !(s.ls < kCountLimitF))) {
           err |= STF_OVERFLOW;
           fin = true;
         }
-        if (!bp && s.evf >= kFlushF) flush_counts(s);
         if (s.ev - s.rej > cap) {
           err |= STF_EVENT_CAP;
           fin = true;
         }
         if (fin) {
-          flush_counts(s);
           const int64_t out = (int64_t)s.plocal * A.n_cells + s.ci;
           A.counts[out] = make_int2((int)(s.uu + s.us), (int)(s.lu + s.ls));
           if (A.events) A.events[out] = s.ev - s.rej;
@@ -477,7 +579,7 @@ __global__ void __launch_bounds__(128, MINB) ssa_kernel_f32(SsaArgs A) {
             s.ev = 0;
             s.rej = 0;
             s.evf = 0.0f;
-            s.rejf = 0.0f;
+            s.firedf = 0.0f;
             set_interval<GRID, GENSCAL>(s, t0, cfg, F, invT);
             if (!(s.uu < kCountLimitF) || !(s.us < kCountLimitF)) err |= STF_OVERFLOW;
             active = true;
@@ -485,15 +587,27 @@ __global__ void __launch_bounds__(128, MINB) ssa_kernel_f32(SsaArgs A) {
         }
         if (__all_sync(FULL, done)) break;
       }
+      act = __ballot_sync(FULL, active);
+      waiting = 0;
+      trips = 0;
+      due = act ? kFlushTrips : 0;
+      w = main_block(s.block, s.r1x, s.r1y, s.r1z, A.rk);
     }
 
-    // ---- one trip: one Philox block, two iterations (the second sees a
-    // negative interval, i.e. does nothing, once the first reached a breakpoint)
-    const U4 w = main_block(s.block, s.r1x, s.r1y, s.r1z, A.rk);
-    bp = ev_step<SPLICE, GENSCAL, GRID>(s, koff, beta, invT, s.len, w.x, w.y);
-    bp = ev_step<SPLICE, GENSCAL, GRID>(s, koff, beta, invT, bp ? -1.0f : s.len, w.z, w.w) || bp;
-    s.block++;
-    special = active && (bp || s.evf >= kFlushF);
+    // ---- two trips of two iterations, each beside the next trip's Philox block
+    const U4 v = main_block(s.block + (uint32_t)trips + 1u, s.r1x, s.r1y, s.r1z, A.rk);
+    ev_step<SPLICE, GENSCAL, GRID>(s, koff, beta, invT, w.x, w.y);
+    ev_step<SPLICE, GENSCAL, GRID>(s, koff, beta, invT, w.z, w.w);
+    trips += 2;
+    w = main_block(s.block + (uint32_t)trips, s.r1x, s.r1y, s.r1z, A.rk);
+    ev_step<SPLICE, GENSCAL, GRID>(s, koff, beta, invT, v.x, v.y);
+    ev_step<SPLICE, GENSCAL, GRID>(s, koff, beta, invT, v.z, v.w);
+    const unsigned at_bp = __ballot_sync(FULL, s.len < 0.0f) & act;
+    if (at_bp != waiting) {
+      waiting = at_bp;
+      const int n = __popc(at_bp), na = __popc(act);
+      due = n == na ? trips : min(due, trips + A.wait * na / n);
+    }
   }
   for (int o = 16; o > 0; o >>= 1) err |= __shfl_xor_sync(FULL, err, o);
   if (lane == 0 && err) atomicOr(A.status, err);
