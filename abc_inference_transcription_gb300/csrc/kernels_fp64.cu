@@ -62,52 +62,240 @@ cudaError_t launch_prior(const PriorArgs& a, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// theta -> rates, thinning bounds and initial state; one thread per particle.
+// theta -> rates, thinning bounds and initial state, eight lanes per particle
+// (model.cuh has the formulas; every operation and its order are the
+// oracle's, so the record is bit-identical).  One thread per particle ran
+// six dependent passes over a cycle's 80 sub-steps, 0.69 ms for one particle
+// and for 10,000 alike; this takes 0.10 and 0.6 ms, bound by the FP64 pipe.  Here lane k holds age step k; the sub-steps' rates and
+// sources, which depend on E G alone, are computed side by side and only the
+// four recurrences stay serial, the passes from different start values on
+// different lanes.  8 lanes rather than 32: the serial parts then occupy
+// the narrow FP64 pipe once for four particles.
 // ---------------------------------------------------------------------------
-__global__ void setup_kernel(SetupArgs A) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= A.n_particles) return;
+constexpr int kSetupLanes = 8;
+static_assert(kSetupLanes >= kMaxSteps, "lane k holds age step k");
+constexpr int kSetupParticles = 32 / kSetupLanes;  // per block (one warp)
+constexpr int kMaxSub = kMaxSteps * kIcSub;
+
+struct SetupShared {
   PRec R;
-  const int model = A.models ? A.models[p] : A.model;
-  int st = (model >= 1 && model <= 5) ? parse_theta(A.cfg, model, A.theta + p * A.ld_theta, R) : -1;
-  if (st) {
-    atomicOr(A.status, STF_NONFINITE);
-    // a harmless record: the trajectory sees no reactions
-    for (int k = 0; k < kMaxSteps; ++k) R.kon[k] = R.alp[k] = R.gam[k] = R.amax[k] = 0.0;
-    R.koff = R.lam = R.beta = R.scal = R.g0 = R.u0 = R.s0 = R.c0 = R.v0 = 0.0;
-    R.cost = 1.0;
+  double ginf[kMaxSteps], eG[kMaxSteps], phG[kMaxSteps], em[kMaxSteps], phm[kMaxSteps];
+  double ec[kMaxSteps], phc[kMaxSteps], ev[kMaxSteps], phv[kMaxSteps];
+  double g[kMaxSub];  // E G at the start of each sub-step, then 2 alpha
+  double aG[kMaxSub], sm[kMaxSub], sc[kMaxSub];  // alpha E G, sources of E u and Cov(G, u)
+};
+
+// initial_moments (model.cuh) by the particle's lanes; lane 0 writes the record
+__device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) {
+  const int S = cfg.n_steps, N = S * kIcSub;
+  const double T = cfg.cycle;
+  const double h = (T / (double)S) / (double)kIcSub;
+  if (r < S) {
+    const double kG = W.R.kon[r] + W.R.koff, gam = W.R.gam[r];
+    W.ginf[r] = W.R.kon[r] / kG;
+    phi_pair(kG * h, W.eG[r], W.phG[r]);
+    phi_pair(gam * h, W.em[r], W.phm[r]);
+    phi_pair((kG + gam) * h, W.ec[r], W.phc[r]);
+    phi_pair((2.0 * gam) * h, W.ev[r], W.phv[r]);
   }
-  A.rec[p] = R;
+  __syncwarp();
+  // E G over one cycle from 0 (even lanes) and from 1 (odd lanes): its fixed point
+  double g = (double)(r & 1);
+  for (int k = 0; k < S; ++k) {
+    const double gi = W.ginf[k], eG = W.eG[k];
+    for (int i = 0; i < kIcSub; ++i) g = gi + (g - gi) * eG;
+  }
+  const double z0 = __shfl_sync(0xffffffffu, g, 0, kSetupLanes), e0 = __shfl_sync(0xffffffffu, g, 1, kSetupLanes);
+  double g0 = z0 / (1.0 - (e0 - z0));
+  if (!(g0 > 0.0)) g0 = 0.0;
+  if (g0 > 1.0) g0 = 1.0;
+  g = g0;
+  for (int k = 0; k < S; ++k) {
+    const double gi = W.ginf[k], eG = W.eG[k];
+    for (int i = 0; i < kIcSub; ++i) {
+      if (r == 0) W.g[k * kIcSub + i] = g;
+      g = gi + (g - gi) * eG;
+    }
+  }
+  __syncwarp();
+  for (int q = r; q < N; q += kSetupLanes) {
+    const int k = q / kIcSub;
+    const double ph = ((double)q + 0.5) * h;
+    const double a = W.R.alp[k] * xpow(1.0 + ph / T, W.R.scal);
+    const double gi = W.ginf[k];
+    const double Gavg = gi + (W.g[q] - gi) * W.phG[k];
+    W.sm[q] = ((a * Gavg) * h) * W.phm[k];
+    W.sc[q] = ((a * (Gavg * (1.0 - Gavg))) * h) * W.phc[k];
+    W.aG[q] = a * Gavg;
+    W.g[q] = 2.0 * a;
+  }
+  __syncwarp();
+  // the cycle map of (E u, Cov, Var u) from 0, (1, 0, 0), (0, 1, 0), (0, 0, 1) on lanes 0..3
+  double m = r == 1 ? 1.0 : 0.0, c = r == 2 ? 1.0 : 0.0, v = r == 3 ? 1.0 : 0.0;
+  for (int k = 0; k < S; ++k) {
+    const double gam = W.R.gam[k], em = W.em[k], ec = W.ec[k], ev = W.ev[k], phv = W.phv[k];
+    for (int i = 0; i < kIcSub; ++i) {
+      const int q = k * kIcSub + i;
+      const double mn = m * em + W.sm[q];
+      const double cn = c * ec + W.sc[q];
+      const double src = (W.aG[q] + gam * (0.5 * (m + mn))) + W.g[q] * (0.5 * (c + cn));
+      v = v * ev + (src * h) * phv;
+      m = mn;
+      c = cn;
+    }
+  }
+  v = v * 0.25 + m * 0.25;
+  m = m * 0.5;
+  c = c * 0.5;
+  const unsigned F = 0xffffffffu;
+  const double b1 = __shfl_sync(F, m, 0, kSetupLanes), b2 = __shfl_sync(F, c, 0, kSetupLanes);
+  const double b3 = __shfl_sync(F, v, 0, kSetupLanes);
+  const double mmm = __shfl_sync(F, m, 1, kSetupLanes) - b1, mvm = __shfl_sync(F, v, 1, kSetupLanes) - b3;
+  const double mcc = __shfl_sync(F, c, 2, kSetupLanes) - b2, mvc = __shfl_sync(F, v, 2, kSetupLanes) - b3;
+  const double mvv = __shfl_sync(F, v, 3, kSetupLanes) - b3;
+  double m0 = b1 / (1.0 - mmm);
+  double c0 = b2 / (1.0 - mcc);
+  double v0 = ((b3 + mvm * m0) + mvc * c0) / (1.0 - mvv);
+  if (!(m0 > 0.0)) m0 = 0.0;
+  if (!(v0 > 0.0)) v0 = 0.0;
+  if (!(c0 == c0)) c0 = 0.0;
+  if (r == 0) {
+    W.R.g0 = g0;
+    W.R.u0 = m0;
+    W.R.s0 = 0.0;
+    W.R.c0 = c0;
+    W.R.v0 = v0;
+  }
+}
+
+// initial_means (model.cuh), splicing models: the four passes on lanes 0..3
+__device__ void initial_means_lanes(const DevCfg& cfg, SetupShared& W, int r) {
+  double x0 = r == 1 ? 1.0 : 0.0, x1 = r == 2 ? 1.0 : 0.0, x2 = r == 3 ? 1.0 : 0.0;
+  if (r < 4) mean_cycle(cfg, W.R, x0, x1, x2);
+  const unsigned F = 0xffffffffu;
+  double b[3], col[3][3];
+  b[0] = __shfl_sync(F, x0, 0, kSetupLanes);
+  b[1] = __shfl_sync(F, x1, 0, kSetupLanes);
+  b[2] = __shfl_sync(F, x2, 0, kSetupLanes);
+  for (int i = 0; i < 3; ++i) {
+    col[i][0] = __shfl_sync(F, x0, i + 1, kSetupLanes);
+    col[i][1] = __shfl_sync(F, x1, i + 1, kSetupLanes);
+    col[i][2] = __shfl_sync(F, x2, i + 1, kSetupLanes);
+  }
+  if (r == 0) solve_initial_means(cfg, b, col, W.R);
+}
+
+__global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
+  __shared__ SetupShared sh[kSetupParticles];
+  const int r = threadIdx.x % kSetupLanes, slot = threadIdx.x / kSetupLanes;
+  const int64_t p = (int64_t)blockIdx.x * kSetupParticles + slot;
+  const bool here = p < A.n_particles;
+  const DevCfg& cfg = A.cfg;
+  const int S = cfg.n_steps;
+  SetupShared& W = sh[slot];
+  PRec& R = W.R;
+  const int model = !here ? 0 : A.models ? A.models[p] : A.model;
+  bool bad = !(model >= 1 && model <= 5);
+  // rates: lane k takes age step k; columns hcat(kon, koff, alpha, gamma, lambda, [beta], [scaling]),
+  // the model's varying rate expanded over the steps
+  if (!bad) {
+    const double* th = A.theta + p * A.ld_theta;
+    const int nk = model == 3 ? S : 1, na = model == 4 ? S : 1, ng = model == 5 ? S : 1;
+    const int ikoff = nk, ia = nk + 1, ig = ia + na, il = ig + ng;
+    int i = il + 1;
+    const double beta = cfg.splicing ? xexp10(th[i++]) : 0.0;
+    const double scal = cfg.scaling_column ? th[i++] : (model == 2 ? 0.0 : 1.0);
+    const double koff = xexp10(th[ikoff]), lam = xexp10(th[il]);
+    double kon = 0.0, alp = 0.0, gam = 0.0, amax = 0.0;
+    if (r < S) {
+      kon = xexp10(th[nk > 1 ? r : 0]);
+      alp = xexp10(th[ia + (na > 1 ? r : 0)]);
+      gam = xexp10(th[ig + (ng > 1 ? r : 0)]);
+      amax = alp * xpow(1.0 + (double)(r + 1) / (double)S, scal);
+      bad = !(kon < INFINITY) || !(alp < INFINITY) || !(gam < INFINITY);
+    }
+    bad = bad || !(koff < INFINITY) || lam != lam || scal != scal || scal < 0.0;
+    R.kon[r] = kon;
+    R.alp[r] = alp;
+    R.gam[r] = gam;
+    R.amax[r] = amax;
+    if (r == 0) {
+      R.koff = koff;
+      R.lam = lam;
+      R.beta = beta;
+      R.scal = scal;
+    }
+  }
+  const unsigned mine = ((1u << kSetupLanes) - 1u) << (slot * kSetupLanes);
+  bad = (__ballot_sync(0xffffffffu, bad) & mine) != 0u;
+  if (bad) {
+    // a harmless record: the trajectory sees no reactions
+    R.kon[r] = R.alp[r] = R.gam[r] = R.amax[r] = 0.0;
+    if (r == 0) {
+      R.koff = R.lam = R.beta = R.scal = R.g0 = R.u0 = R.s0 = R.c0 = R.v0 = 0.0;
+      R.cost = 1.0;
+      if (here) atomicOr(A.status, STF_NONFINITE);
+    }
+  } else if (r == 0) {
+    R.c0 = R.v0 = 0.0;
+  }
+  __syncwarp();
+  // (the lanes of a bad record run along, for the shuffles, and are not kept)
+  PRec keep = {};
+  if (bad && r == 0) keep = R;
+  if (cfg.splicing)
+    initial_means_lanes(cfg, W, r);
+  else
+    initial_moments_lanes(cfg, W, r);
+  // work estimate: switching + transcription + decay events over the horizon
+  double rate = 0.0, mine_k = 0.0;
+  if (r < S) {
+    const double pon = R.kon[r] / (R.kon[r] + R.koff);
+    mine_k = 2.0 * pon * R.koff + 2.0 * pon * R.amax[r];
+  }
+  for (int k = 0; k < S; ++k) rate = rate + __shfl_sync(0xffffffffu, mine_k, k, kSetupLanes);
+  if (r == 0) {
+    if (bad)
+      R = keep;
+    else
+      R.cost = (double)(cfg.ages[0] - cfg.t0) * rate / (double)S + 1.0;
+  }
+  __syncwarp();
+  if (!here) return;
+  const double* src = reinterpret_cast<const double*>(&R);
+  double* dst = reinterpret_cast<double*>(&A.rec[p]);
+  for (int i = r; i < (int)(sizeof(PRec) / sizeof(double)); i += kSetupLanes) dst[i] = src[i];
   // rates in log2 units (times log2 e), so the production kernel's waiting
   // time is -log2(U) / a0 without a conversion per event
   constexpr double kL2E = 1.4426950408889634;
-  PRecF F;
-  for (int k = 0; k < kMaxSteps; ++k) {
-    F.kon[k] = (float)(R.kon[k] * kL2E);
-    F.alp[k] = (float)(R.alp[k] * kL2E);
-    F.gam[k] = (float)(R.gam[k] * kL2E);
-    F.amax[k] = (float)(R.amax[k] * kL2E);
-  }
-  F.koff = (float)(R.koff * kL2E);
-  F.lam = (float)R.lam;
-  F.beta = (float)(R.beta * kL2E);
-  F.scal = (float)R.scal;
+  float kon = (float)(R.kon[r] * kL2E), alp = (float)(R.alp[r] * kL2E), gam = (float)(R.gam[r] * kL2E);
+  float amax = (float)(R.amax[r] * kL2E), koff = (float)(R.koff * kL2E), beta = (float)(R.beta * kL2E);
+  float lam = (float)R.lam, scal = (float)R.scal;
   if (A.fp32) {
     // rates beyond the FP32 range would stall the production kernel's clock
-    bool ok = F.koff < 1e30f && F.beta < 1e30f;
-    for (int k = 0; k < kMaxSteps; ++k) ok = ok && F.kon[k] < 1e30f && F.alp[k] < 1e30f && F.gam[k] < 1e30f;
-    if (!ok) {
-      atomicOr(A.status, STF_NONFINITE);
-      memset(&F, 0, sizeof(F));
+    const bool ok = koff < 1e30f && beta < 1e30f && kon < 1e30f && alp < 1e30f && gam < 1e30f;
+    if ((__ballot_sync(mine, !ok) & mine) != 0u) {
+      if (r == 0) atomicOr(A.status, STF_NONFINITE);
+      kon = alp = gam = amax = koff = lam = beta = scal = 0.0f;
     }
   }
-  A.recf[p] = F;
+  PRecF& F = A.recf[p];
+  F.kon[r] = kon;
+  F.alp[r] = alp;
+  F.gam[r] = gam;
+  F.amax[r] = amax;
+  if (r == 0) {
+    F.koff = koff;
+    F.lam = lam;
+    F.beta = beta;
+    F.scal = scal;
+  }
 }
 
 cudaError_t launch_setup(const SetupArgs& a, cudaStream_t s) {
   if (a.n_particles <= 0) return cudaSuccess;
-  int blocks = (int)((a.n_particles + 63) / 64);
-  setup_kernel<<<blocks, 64, 0, s>>>(a);
+  const int64_t blocks = (a.n_particles + kSetupParticles - 1) / kSetupParticles;
+  setup_kernel<<<(unsigned)blocks, 32, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -264,11 +452,17 @@ __device__ __forceinline__ __int128 shfl_xor_i128(__int128 v, int o) {
   return (__int128)(((unsigned __int128)(unsigned long long)hi << 64) | (unsigned __int128)lo);
 }
 
+// 1,024 threads per particle up to one particle per SM
+constexpr int kStatsWideParticles = 152;
+
 // NARROW: 64-bit sums of the squared counts (production mode: counts at most
 // 2^24, where FP32 increments stop, and at most 2^14 cells per group, so the
 // sums stay below 2^62); 128-bit otherwise.
-template <bool CAP32, bool NARROW>
-__global__ void __launch_bounds__(256) stats_kernel(StatsArgs A) {
+// THREADS: 256, or 1,024 where the launch has too few particles to fill the
+// GPU (the groups are then the parallelism: a particle alone with 55 groups
+// of 36 cells takes 90 us in 8 warps, 51 in 32).
+template <bool CAP32, bool NARROW, int THREADS>
+__global__ void __launch_bounds__(THREADS) stats_kernel(StatsArgs A) {
   __shared__ double mom[kMaxAges * kMaxConds * 5];
   __shared__ double wts[kMaxAges * kMaxConds];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -339,12 +533,14 @@ __global__ void __launch_bounds__(256) stats_kernel(StatsArgs A) {
 cudaError_t launch_stats(const StatsArgs& a, cudaStream_t s) {
   if (a.n_particles <= 0) return cudaSuccess;
   int blocks = (int)(a.n_particles < 1048576 ? a.n_particles : 1048576);
-  if (a.fp32 && a.max_group_cells <= 16384)
-    stats_kernel<true, true><<<blocks, 256, 0, s>>>(a);
+  if (a.fp32 && a.max_group_cells <= 16384 && blocks <= kStatsWideParticles)
+    stats_kernel<true, true, 1024><<<blocks, 1024, 0, s>>>(a);
+  else if (a.fp32 && a.max_group_cells <= 16384)
+    stats_kernel<true, true, 256><<<blocks, 256, 0, s>>>(a);
   else if (a.fp32)
-    stats_kernel<true, false><<<blocks, 256, 0, s>>>(a);
+    stats_kernel<true, false, 256><<<blocks, 256, 0, s>>>(a);
   else
-    stats_kernel<false, false><<<blocks, 256, 0, s>>>(a);
+    stats_kernel<false, false, 256><<<blocks, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -122,21 +122,14 @@ ABC_HD void mean_cycle(const DevCfg& cfg, const PRec& R, double& G, double& uu, 
   us = us * 0.5;
 }
 
-ABC_HD void initial_means(const DevCfg& cfg, PRec& R) {
-  double b0 = 0.0, b1 = 0.0, b2 = 0.0;
-  double c10 = 1.0, c11 = 0.0, c12 = 0.0;
-  double c20 = 0.0, c21 = 1.0, c22 = 0.0;
-  double c30 = 0.0, c31 = 0.0, c32 = 1.0;
-  mean_cycle(cfg, R, b0, b1, b2);
-  mean_cycle(cfg, R, c10, c11, c12);
-  mean_cycle(cfg, R, c20, c21, c22);
-  mean_cycle(cfg, R, c30, c31, c32);
-  double mGG = c10 - b0;
-  double muG = c11 - b1, muu = c21 - b1;
-  double msG = c12 - b2, msu = c22 - b2, mss = c32 - b2;
-  double g = b0 / (1.0 - mGG);
-  double u = (b1 + muG * g) / (1.0 - muu);
-  double s = cfg.splicing ? ((b2 + msG * g) + msu * u) / (1.0 - mss) : 0.0;
+// b: the cycle map of (0, 0, 0); c[i]: of the i-th unit vector
+ABC_HD void solve_initial_means(const DevCfg& cfg, const double b[3], const double c[3][3], PRec& R) {
+  double mGG = c[0][0] - b[0];
+  double muG = c[0][1] - b[1], muu = c[1][1] - b[1];
+  double msG = c[0][2] - b[2], msu = c[1][2] - b[2], mss = c[2][2] - b[2];
+  double g = b[0] / (1.0 - mGG);
+  double u = (b[1] + muG * g) / (1.0 - muu);
+  double s = cfg.splicing ? ((b[2] + msG * g) + msu * u) / (1.0 - mss) : 0.0;
   if (!(g > 0.0)) g = 0.0;
   if (g > 1.0) g = 1.0;
   if (!(u > 0.0)) u = 0.0;
@@ -158,70 +151,9 @@ ABC_HD void initial_means(const DevCfg& cfg, PRec& R) {
 //   V'   = alpha(t) E G + gamma E u + 2 alpha(t) C - 2 gamma V
 // Exponential sub-steps (16 per age step) with the sources averaged over the
 // sub-step.  E G is periodic by itself; with it fixed, the cycle map of
-// (E u, C, V) is affine with a lower-triangular matrix, solved directly.
+// (E u, C, V) is affine with a lower-triangular matrix, solved directly
+// (initial_moments_lanes in kernels_fp64.cu).
 // ---------------------------------------------------------------------------
-ABC_HD void moment_cycle(const DevCfg& cfg, const PRec& R, double* x) {
-  const int S = cfg.n_steps;
-  const double T = cfg.cycle;
-  const double h = (T / (double)S) / (double)kIcSub;
-  double g = x[0], m = x[1], c = x[2], v = x[3];
-  for (int k = 0; k < S; ++k) {
-    const double kG = R.kon[k] + R.koff;
-    const double Ginf = R.kon[k] / kG;
-    const double gam = R.gam[k];
-    double eG, phG, em, phm, ec, phc, ev, phv;
-    phi_pair(kG * h, eG, phG);
-    phi_pair(gam * h, em, phm);
-    phi_pair((kG + gam) * h, ec, phc);
-    phi_pair((2.0 * gam) * h, ev, phv);
-    for (int i = 0; i < kIcSub; ++i) {
-      const double ph = ((double)(k * kIcSub + i) + 0.5) * h;
-      const double a = R.alp[k] * xpow(1.0 + ph / T, R.scal);
-      const double Gavg = Ginf + (g - Ginf) * phG;
-      const double gn = Ginf + (g - Ginf) * eG;
-      const double mn = m * em + ((a * Gavg) * h) * phm;
-      const double cn = c * ec + ((a * (Gavg * (1.0 - Gavg))) * h) * phc;
-      const double src = (a * Gavg + gam * (0.5 * (m + mn))) + (2.0 * a) * (0.5 * (c + cn));
-      const double vn = v * ev + (src * h) * phv;
-      g = gn;
-      m = mn;
-      c = cn;
-      v = vn;
-    }
-  }
-  x[0] = g;
-  x[1] = m * 0.5;
-  x[2] = c * 0.5;
-  x[3] = v * 0.25 + m * 0.25;
-}
-
-ABC_HD void initial_moments(const DevCfg& cfg, PRec& R) {
-  double z[4] = {0.0, 0.0, 0.0, 0.0}, e[4] = {1.0, 0.0, 0.0, 0.0};
-  moment_cycle(cfg, R, z);
-  moment_cycle(cfg, R, e);
-  double g = z[0] / (1.0 - (e[0] - z[0]));
-  if (!(g > 0.0)) g = 0.0;
-  if (g > 1.0) g = 1.0;
-  double b[4] = {g, 0.0, 0.0, 0.0}, bm[4] = {g, 1.0, 0.0, 0.0};
-  double bc[4] = {g, 0.0, 1.0, 0.0}, bv[4] = {g, 0.0, 0.0, 1.0};
-  moment_cycle(cfg, R, b);
-  moment_cycle(cfg, R, bm);
-  moment_cycle(cfg, R, bc);
-  moment_cycle(cfg, R, bv);
-  const double mmm = bm[1] - b[1], mcc = bc[2] - b[2];
-  const double mvm = bm[3] - b[3], mvc = bc[3] - b[3], mvv = bv[3] - b[3];
-  double m = b[1] / (1.0 - mmm);
-  double c = b[2] / (1.0 - mcc);
-  double v = ((b[3] + mvm * m) + mvc * c) / (1.0 - mvv);
-  if (!(m > 0.0)) m = 0.0;
-  if (!(v > 0.0)) v = 0.0;
-  if (!(c == c)) c = 0.0;
-  R.g0 = g;
-  R.u0 = m;
-  R.s0 = 0.0;
-  R.c0 = c;
-  R.v0 = v;
-}
 
 // Unspliced count at the start of a trajectory, given the gene state G drawn
 // with probability g0: conditional mean E[u | G] = u0 + c0 / g0 (G = 1) or
@@ -249,9 +181,9 @@ ABC_HD int64_t initial_count(const PRec& R, int G, uint32_t wz, Rng& aux) {
   return poisson(aux, lam);
 }
 
-// theta -> record; returns 0 or a negative abc_status.
-// with_ic: also the SSA initial state and work estimate (not needed by the moment ODE)
-ABC_HD int parse_theta(const DevCfg& cfg, int model, const double* th, PRec& R, bool with_ic = true) {
+// theta -> rates of the record (the moment ODE's; the SSA's setup_kernel also
+// fills the initial state and work estimate); returns 0 or a negative abc_status.
+ABC_HD int parse_theta(const DevCfg& cfg, int model, const double* th, PRec& R) {
   const int S = cfg.n_steps;
   int i = 0;
   double lk[kMaxSteps], la[kMaxSteps], lg[kMaxSteps];
@@ -289,20 +221,6 @@ ABC_HD int parse_theta(const DevCfg& cfg, int model, const double* th, PRec& R, 
   for (int k = 0; k < S; ++k)
     if (!(R.kon[k] < INFINITY) || !(R.alp[k] < INFINITY) || !(R.gam[k] < INFINITY)) return -5;
   if (!(R.koff < INFINITY) || R.lam != R.lam || R.scal != R.scal || R.scal < 0.0) return -5;
-  if (!with_ic) return 0;
-  R.c0 = R.v0 = 0.0;
-  if (cfg.splicing)
-    initial_means(cfg, R);
-  else
-    initial_moments(cfg, R);
-  // work estimate: switching + transcription + decay events over the horizon
-  double horizon = (double)(cfg.ages[0] - cfg.t0);
-  double rate = 0.0;
-  for (int k = 0; k < S; ++k) {
-    double pon = R.kon[k] / (R.kon[k] + R.koff);
-    rate = rate + (2.0 * pon * R.koff + 2.0 * pon * R.amax[k]);
-  }
-  R.cost = horizon * rate / (double)S + 1.0;
   return 0;
 }
 

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kMomThreads) moment_kernel(MomArgs a) {
   for (int64_t p = blockIdx.x; p < a.P; p += gridDim.x) {
     if (threadIdx.x == 0) {
       DevCfg c1 = cfg;
-      s_bad = parse_theta(c1, a.model, a.theta + p * a.ld, R, false) ? 1 : 0;
+      s_bad = parse_theta(c1, a.model, a.theta + p * a.ld, R) ? 1 : 0;
     }
     __syncthreads();
     if (s_bad) {

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads) moment_kernel_f32(MomArgs a) {
   const LaneTri lt = lane_tri(lane);
   float* P1 = P0 + (size_t)nsub * NT;
   for (int64_t p = blockIdx.x; p < a.P; p += gridDim.x) {
-    if (threadIdx.x == 0) s_bad = parse_theta(cfg, a.model, a.theta + p * a.ld, R, false) ? 1 : 0;
+    if (threadIdx.x == 0) s_bad = parse_theta(cfg, a.model, a.theta + p * a.ld, R) ? 1 : 0;
     __syncthreads();
     if (s_bad) {
       for (int k = threadIdx.x; k < K; k += blockDim.x) a.stats[p * K + k] = NAN;

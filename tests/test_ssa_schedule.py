@@ -66,3 +66,32 @@ def test_lane_and_warp_halving_agree(built, tmp_path):
         assert np.array_equal(out[:, 0], out[:, 1]) and np.array_equal(out[:, 2], out[:, 3])
         n = np.arange(1200)
         assert (np.abs(out[:, 0] - n / 2) <= 4 * np.sqrt(n) + 1).all() and (out[:, 0] <= n).all()
+
+
+@pytest.mark.parametrize("n,n_steps,model,kw", [(1, 5, 1, {}), (3, 1, 4, {}), (4, 8, 3, {}), (5, 2, 5, {}),
+                                                (7, 5, 2, {"splicing": True}), (6, 8, 5, {"scaling_column": True})])
+def test_particle_records_match_oracle(built, orc, n, n_steps, model, kw):
+    """Rates, initial moments and statistics of particle groups that do not fill
+    a warp, for the smallest and largest numbers of age steps: the FP64 mode's
+    counts equal the oracle's, with an invalid parameter set between them."""
+    from abc_inference_transcription_gb300.host import Context
+    cfg = make_config("hour", precision=abi.FP64, **kw)
+    cfg.n_steps = n_steps
+    cells = synthetic_cells(n_per_pulse=10, n_per_chase=10, seed=2)
+    npar = abi.num_params(cfg, model)
+    rng = np.random.default_rng(n)
+    theta = rng.uniform(-1.0, 0.6, (n, npar))
+    if cfg.scaling_column:  # a negative size exponent is refused
+        theta[:, -1] = np.abs(theta[:, -1])
+    with Context(cfg, cells) as ctx:
+        got = ctx.simulate_cells(model, theta, seed=3)
+        ref = orc.simulate(cfg, cells, model, theta, seed=3)
+        for key in ("counts", "captured", "events", "hash"):
+            assert np.array_equal(got[key], ref[key]), key
+        assert np.array_equal(got["stats"], ref["stats"], equal_nan=True)
+        if n > 2:
+            bad = theta.copy()
+            bad[1, 0] = np.nan
+            with pytest.raises(abi.AbcError):
+                ctx.simulate(model, bad, seed=3)
+            assert np.array_equal(ctx.simulate(model, theta, seed=3), got["stats"], equal_nan=True)
