@@ -137,33 +137,61 @@ __global__ void __launch_bounds__(128, 1)
   const uint32_t lane_addr = tbase + ((uint32_t)(warp * 32) << 16);
   if (have) {
     const float* bias = g.bias ? g.bias + z * g.sBias : nullptr;
+    // A lane holds 32 neighbouring columns of its row, which it writes (and
+    // reads, EPI_DSILU) 16 bytes at a time: N and every row length are
+    // multiples of 16 values.  One value at a time, each warp store touched 32
+    // rows, and a hidden layer of 4 x 65,536 rows took 0.70 ms instead of
+    // 0.20.  The transposed copy is coalesced across the lanes.
 #pragma unroll 1
     for (int cc = 0; cc < BN / 32; ++cc) {
+      const int nb = n0 + cc * 32;
+      if (nb >= g.N) break;
       __syncwarp();
       uint32_t v[32];
       tmem_ld32(lane_addr + (uint32_t)(cc * 32), v);
       if (m >= g.M) continue;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int n = n0 + cc * 32 + j;
-        if (n >= g.N) continue;
-        const float a = __uint_as_float(v[j]);
-        if (EPI == EPI_HIDDEN) {
-          const float zz = a + (bias ? bias[n] : 0.0f);
-          if (g.outf) g.outf[z * g.sOutf + (int64_t)m * g.ldf + n] = zz;
-          const __nv_bfloat16 h = __float2bfloat16(zz * sigm(zz));
-          g.outh[z * g.sOuth + (int64_t)m * g.ldh + n] = h;
-          if (g.outhT) g.outhT[z * g.sOuthT + (int64_t)n * g.ldhT + m] = h;
-        } else if (EPI == EPI_LINEAR) {
-          g.outf[z * g.sOutf + (int64_t)m * g.ldf + n] = a + (bias ? bias[n] : 0.0f);
-        } else if (EPI == EPI_PARTIAL) {
-          g.outf[split * g.sSplit + z * g.sOutf + (int64_t)m * g.ldf + n] = a;
-        } else {
-          const float zp = g.zprev[z * g.sZ + (int64_t)m * g.ldz + n];
-          const float sg = sigm(zp);
-          const __nv_bfloat16 d = __float2bfloat16(a * (sg * (1.0f + zp * (1.0f - sg))));
-          g.outh[z * g.sOuth + (int64_t)m * g.ldh + n] = d;
-          if (g.outhT) g.outhT[z * g.sOuthT + (int64_t)n * g.ldhT + m] = d;
+      for (int q = 0; q < 4; ++q) {
+        const int n = nb + 8 * q;
+        if (n >= g.N) break;
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[8 * q + j]);
+        if (EPI == EPI_HIDDEN || EPI == EPI_LINEAR) {
+          if (bias) {
+            const float4 b0 = *(const float4*)(bias + n), b1 = *(const float4*)(bias + n + 4);
+            x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
+            x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
+          }
+        }
+        if (EPI == EPI_DSILU) {
+          const float* zp = g.zprev + z * g.sZ + (int64_t)m * g.ldz + n;
+          const float4 p0 = *(const float4*)zp, p1 = *(const float4*)(zp + 4);
+          const float zq[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float sg = sigm(zq[j]);
+            x[j] = x[j] * (sg * (1.0f + zq[j] * (1.0f - sg)));
+          }
+        }
+        if (EPI != EPI_DSILU && g.outf) {
+          float* o = g.outf + z * g.sOutf + (int64_t)m * g.ldf + n;
+          if (EPI == EPI_PARTIAL) o += split * g.sSplit;
+          *(float4*)o = make_float4(x[0], x[1], x[2], x[3]);
+          *(float4*)(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
+        }
+        if (EPI == EPI_HIDDEN || EPI == EPI_DSILU) {
+          __nv_bfloat16 h[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16(EPI == EPI_HIDDEN ? x[j] * sigm(x[j]) : x[j]);
+          uint4 pk;
+          memcpy(&pk, h, 16);
+          *(uint4*)(g.outh + z * g.sOuth + (int64_t)m * g.ldh + n) = pk;
+          if (g.outhT) {
+            __nv_bfloat16* oT = g.outhT + z * g.sOuthT + (int64_t)n * g.ldhT + m;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) oT[(int64_t)j * g.ldhT] = h[j];
+          }
         }
       }
     }
@@ -217,6 +245,10 @@ cudaError_t mlp_tc_gemm(int epi, const TcOperand& A, const TcOperand& B, const T
                         cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
   if ((A.ld * 2) % 16 || (B.ld * 2) % 16 || (A.member_stride * 2) % 16 || (B.member_stride * 2) % 16)
+    return cudaErrorInvalidValue;
+  // the epilogue's 16-byte accesses
+  if (g.N % 8 || g.ldf % 4 || g.ldh % 8 || g.ldz % 4 || g.sOutf % 4 || g.sSplit % 4 || g.sOuth % 8 || g.sZ % 4 ||
+      g.sBias % 4 || ((uintptr_t)g.outf | (uintptr_t)g.outh | (uintptr_t)g.zprev | (uintptr_t)g.bias) % 16)
     return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
   if (!make_map3(&ma, A.ptr, g.K, A.ld, A.rows, g.a_shared ? 1 : members, A.member_stride) ||
