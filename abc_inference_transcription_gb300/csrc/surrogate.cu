@@ -127,13 +127,27 @@ __global__ void norm_y_kernel(const double* st, int64_t N, int K, const double* 
   }
 }
 
-// per statistic: scale c = mean |y| over finite values (1 if none), then y <- asinh(y / c) in place
-__global__ void asinh_scale_kernel(double* st, int64_t N, int K, float* scale) {
+// per statistic: scale c = mean |y| over finite values (1 if none); the asinh
+// itself is asinh_fit_kernel's, over all values at once (in this kernel's one
+// block per statistic it took 0.9 ms for 40,000 x 53 values).  The columns lie
+// a row apart, so four values are loaded before they are added, in row order.
+__global__ void __launch_bounds__(256) abs_scale_kernel(const double* st, int64_t N, int K, double* scale,
+                                                        float* scale32) {
   __shared__ double red[256];
   __shared__ double cnt[256];
   const int c = blockIdx.x;
   double s = 0.0, n = 0.0;
-  for (int64_t i = threadIdx.x; i < N; i += blockDim.x) {
+  const int64_t step = blockDim.x;
+  int64_t i = threadIdx.x;
+  for (; i + 3 * step < N; i += 4 * step) {
+    double v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = st[(i + j * step) * K + c];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (isfinite(v[j])) { s += fabs(v[j]); n += 1.0; }
+  }
+  for (; i < N; i += step) {
     const double v = st[i * K + c];
     if (isfinite(v)) { s += fabs(v); n += 1.0; }
   }
@@ -144,14 +158,20 @@ __global__ void asinh_scale_kernel(double* st, int64_t N, int K, float* scale) {
     if (threadIdx.x < o) { red[threadIdx.x] += red[threadIdx.x + o]; cnt[threadIdx.x] += cnt[threadIdx.x + o]; }
     __syncthreads();
   }
-  double sc = cnt[0] > 0.0 ? red[0] / cnt[0] : 1.0;
-  if (!(sc > 1e-12)) sc = 1.0;
-  __syncthreads();
-  for (int64_t i = threadIdx.x; i < N; i += blockDim.x) {
-    const double v = st[i * K + c];
-    if (isfinite(v)) st[i * K + c] = asinh(v / sc);
+  if (threadIdx.x == 0) {
+    double sc = cnt[0] > 0.0 ? red[0] / cnt[0] : 1.0;
+    if (!(sc > 1e-12)) sc = 1.0;
+    scale[c] = sc;
+    scale32[c] = (float)sc;
   }
-  if (threadIdx.x == 0) scale[c] = (float)sc;
+}
+
+// y <- asinh(y / c) with the FP64 scales of the same data
+__global__ void asinh_fit_kernel(double* st, int64_t N, int K, const double* scale) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N * K; i += (int64_t)gridDim.x * blockDim.x) {
+    const double v = st[i];
+    if (isfinite(v)) st[i] = asinh(v / scale[i % K]);
+  }
 }
 
 __global__ void asinh_apply_kernel(double* st, int64_t N, int K, const float* scale) {
@@ -263,7 +283,7 @@ struct abc_surrogate {
   Buf<float> P, G, Am, Av, ymf, ysf, yscf;  // yscf: asinh scale per statistic (0: identity)
   Buf<__nv_bfloat16> Ph, PhT;   // BF16 weights as stored and transposed
   Buf<int> tcerr;                // tensor-core GEMM error word
-  Buf<double> xm, xs, ym, ys;
+  Buf<double> xm, xs, ym, ys, ysc;
   // training / batch scratch
   Buf<double> th64, st64;
   Buf<float> xn, yn, T, Z, Y;
@@ -382,7 +402,7 @@ int abc_surrogate_create(abc_surrogate** out, int in_dim, int n_stats, int ensem
 int abc_surrogate_destroy(abc_surrogate* s) {
   if (!s) return ABC_OK;
   cudaStreamSynchronize(s->stream);
-  s->yscf.release();
+  s->yscf.release(); s->ysc.release();
   s->P.release(); s->G.release(); s->Am.release(); s->Av.release(); s->Ph.release(); s->ymf.release();
   s->PhT.release(); s->tcerr.release(); s->X0T.release(); s->AhT.release(); s->dYT.release(); s->dZTa.release();
   s->dZTb.release();
@@ -420,7 +440,9 @@ static int load_training(abc_surrogate* s, const double* theta, const double* st
   SK(cudaMemcpyAsync(s->th64.p, theta, sizeof(double) * N * d.in_dim, cudaMemcpyHostToDevice, s->stream));
   SK(cudaMemcpyAsync(s->st64.p, stats, sizeof(double) * N * d.K, cudaMemcpyHostToDevice, s->stream));
   if (fit_norm) {
-    asinh_scale_kernel<<<d.K, 256, 0, s->stream>>>(s->st64.p, N, d.K, s->yscf.p);
+    SK(s->ysc.ensure((size_t)d.K));
+    abs_scale_kernel<<<d.K, 256, 0, s->stream>>>(s->st64.p, N, d.K, s->ysc.p, s->yscf.p);
+    asinh_fit_kernel<<<blocks(N * d.K), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->ysc.p);
     col_norm_kernel<<<d.in_dim, 256, 0, s->stream>>>(s->th64.p, N, d.in_dim, d.in_dim, s->xm.p, s->xs.p);
     col_norm_kernel<<<d.K, 256, 0, s->stream>>>(s->st64.p, N, d.K, d.K, s->ym.p, s->ys.p);
     SK(cudaGetLastError());
