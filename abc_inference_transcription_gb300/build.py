@@ -36,6 +36,7 @@ UNITS = {
     "noalloc.cu": [],
     "mlp.cu": [],
     "mlp_tc.cu": [],
+    "mlp_infer.cu": [],
     "surrogate.cu": [],
     "formats.cu": [],
 }

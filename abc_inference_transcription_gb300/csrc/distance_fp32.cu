@@ -333,32 +333,34 @@ cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int6
 //     v = sum_k (2 sig^4 + 4 sig^2 delta^2) / K^2 (delta = a (d - mu),
 //     sig = a sd), and L_pg = m - z sqrt(v).
 // keep[p] = 1 when L_pg <= X[g] for some gene (X = calibrated threshold).  A
-// draw is dropped only when it is confidently far from every gene.  Same
-// 128 x 128 tiling as dist_fast_kernel.
-template <int MODE>
+// draw is dropped only when it is confidently far from every gene.  Tiles of
+// 128 draws x 16 GJ genes, GJ genes per thread: 8, as dist_fast_kernel, or 1
+// for at most 32 genes, where the wide tile computes mostly padding (65,536
+// draws x 4 genes: 108 us wide, 41 narrow).
+template <int MODE, int GJ>
 __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restrict__ mu,
                                                           const float* __restrict__ var,
                                                           const float* __restrict__ sw,
                                                           const float* __restrict__ dw, int64_t P, int64_t G,
                                                           int K, const float* __restrict__ X, float z,
                                                           uint8_t* keep, float* err_out) {
+  constexpr int N2 = MODE ? 8 : 1, M2 = MODE ? GJ : 1, kGenes = 16 * GJ;
   __shared__ float sm[kDistKc][kDistTile];
   __shared__ float sv[kDistKc][kDistTile];
-  __shared__ float sa[kDistKc][kDistTile];
-  __shared__ float sd[kDistKc][kDistTile];
-  constexpr int N2 = MODE ? 8 : 1;
+  __shared__ float sa[kDistKc][kGenes];
+  __shared__ float sd[kDistKc][kGenes];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t g0 = (int64_t)blockIdx.x * kDistTile;
+  const int64_t g0 = (int64_t)blockIdx.x * kGenes;
   const int64_t p0 = (int64_t)blockIdx.y * kDistTile;
-  float acc[8][8], acc2[N2][N2];
+  float acc[8][GJ], acc2[N2][M2];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    for (int j = 0; j < GJ; ++j) acc[i][j] = 0.0f;
 #pragma unroll
   for (int i = 0; i < N2; ++i)
 #pragma unroll
-    for (int j = 0; j < N2; ++j) acc2[i][j] = 0.0f;
+    for (int j = 0; j < M2; ++j) acc2[i][j] = 0.0f;
   for (int k0 = 0; k0 < K; k0 += kDistKc) {
     for (int idx = threadIdx.x; idx < kDistKc * kDistTile; idx += 256) {
       const int r = idx / kDistKc, kk = idx - (idx / kDistKc) * kDistKc;
@@ -370,34 +372,36 @@ __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restric
         v = sqrtf(fmaxf(var[p * K + k], 0.0f));  // predictive std
         if (MODE == 0) v *= z;
       }
-      if (g < G && k < K) {
+      if (r < kGenes && g < G && k < K) {
         a = sw[g * K + k];
         d = dw[g * K + k];
       }
       sm[kk][r] = m;
       sv[kk][r] = v;
-      sa[kk][r] = a;
-      sd[kk][r] = d;
+      if (r < kGenes) {
+        sa[kk][r] = a;
+        sd[kk][r] = d;
+      }
     }
     __syncthreads();
     const int kc = (K - k0) < kDistKc ? (K - k0) : kDistKc;
 #pragma unroll 2
     for (int kk = 0; kk < kc; ++kk) {
-      float m[8], v[8], a[8], d[8];
+      float m[8], v[8], a[GJ], d[GJ];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         m[i] = sm[kk][ty + 16 * i];
         v[i] = sv[kk][ty + 16 * i];
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < GJ; ++j) {
         a[j] = sa[kk][tx + 16 * j];
         d[j] = sd[kk][tx + 16 * j];
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < GJ; ++j) {
           if (MODE == 0) {
             const float t = fmaxf(fabsf(fmaf(-a[j], m[i], d[j])) - a[j] * v[i], 0.0f);
             acc[i][j] = fmaf(t, t, acc[i][j]);
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restric
             const float sg = a[j] * v[i];
             const float s2 = sg * sg, d2 = dl * dl;
             acc[i][j] += d2 + s2;
-            acc2[i & (N2 - 1)][j & (N2 - 1)] = fmaf(s2, fmaf(4.0f, d2, 2.0f * s2), acc2[i & (N2 - 1)][j & (N2 - 1)]);
+            acc2[i & (N2 - 1)][j & (M2 - 1)] = fmaf(s2, fmaf(4.0f, d2, 2.0f * s2), acc2[i & (N2 - 1)][j & (M2 - 1)]);
           }
         }
     }
@@ -419,12 +423,12 @@ __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restric
     if (p >= P) continue;
     bool any = false;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < GJ; ++j) {
       const int64_t g = g0 + tx + 16 * j;
       if (g >= G) continue;
       // not clipped: far draws keep large predicted errors
       float e = acc[i][j] * invK;
-      if (MODE == 1) e -= z * sqrtf(acc2[i & (N2 - 1)][j & (N2 - 1)]) * invK;
+      if (MODE == 1) e -= z * sqrtf(acc2[i & (N2 - 1)][j & (M2 - 1)]) * invK;
       if (err_out) err_out[p * G + g] = e;
       any = any || (e <= X[g]);
     }
@@ -436,11 +440,16 @@ cudaError_t launch_dist_screen(const float* mu, const float* var, const float* s
                                int64_t G, int K, const float* X, float z, int mode, uint8_t* keep, float* err_out,
                                cudaStream_t s) {
   if (P <= 0 || G <= 0) return cudaSuccess;
-  dim3 grid((unsigned)((G + kDistTile - 1) / kDistTile), (unsigned)((P + kDistTile - 1) / kDistTile));
-  if (mode == 1)
-    dist_screen_kernel<1><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
+  const int genes = G <= 32 ? 16 : kDistTile;
+  dim3 grid((unsigned)((G + genes - 1) / genes), (unsigned)((P + kDistTile - 1) / kDistTile));
+  if (mode == 1 && genes == 16)
+    dist_screen_kernel<1, 1><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
+  else if (mode == 1)
+    dist_screen_kernel<1, 8><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
+  else if (genes == 16)
+    dist_screen_kernel<0, 1><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
   else
-    dist_screen_kernel<0><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
+    dist_screen_kernel<0, 8><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
   return cudaGetLastError();
 }
 

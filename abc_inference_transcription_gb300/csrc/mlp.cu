@@ -267,17 +267,30 @@ __global__ void mlp_adam_kernel(float* P, const float* G, float* m, float* v, __
 // Targets are learnt as z = (asinh(y / c) - m) / s (c = 0: z = (y - m) / s);
 // the predictive mean and variance map back through y = c sinh(m + s z)
 // (delta method for the variance).
-__global__ void mlp_combine_kernel(const float* Y, int N, int K, int out_pad, int members, int64_t sY,
-                                   const float* ymean, const float* ystd, const float* yscale, double* mean_out,
-                                   double* var_out, double* disagree, int aleatoric_only) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  float worst = 0.0f;
-  for (int k = 0; k < K; ++k) {
+// A block takes a few rows and its threads their (row, statistic) pairs, so the
+// outputs of the members are read coalesced and every lane of the FP64 pipe,
+// which bounds this (sinh and cosh), has work.  OUT = double: the caller's
+// mean and variance; float: the screen's, rounded once.  65,536 rows x 53
+// statistics with the asinh transform: 0.36 ms, 0.46 with a thread per row.
+constexpr int kCombinePairs = 2048;  // (row, statistic) pairs per block
+template <typename OUT>
+__global__ void __launch_bounds__(256) mlp_combine_kernel(const float* __restrict__ Y, int N, int K, int out_pad,
+                                                          int members, int64_t sY, int rows_per_block,
+                                                          const float* __restrict__ ymean,
+                                                          const float* __restrict__ ystd,
+                                                          const float* __restrict__ yscale, OUT* __restrict__ mean_out,
+                                                          OUT* __restrict__ var_out, double* __restrict__ disagree,
+                                                          int aleatoric_only) {
+  __shared__ float worst[kCombinePairs];
+  const int i0 = blockIdx.x * rows_per_block;
+  const int rows = min(rows_per_block, N - i0);
+  for (int q = threadIdx.x; q < rows * K; q += blockDim.x) {
+    const int i = q / K, k = q - i * K;
+    const float* y = Y + (int64_t)(i0 + i) * out_pad + k;
     float mu = 0.0f, mu2 = 0.0f, ale = 0.0f;
     for (int e = 0; e < members; ++e) {
-      const float a = Y[e * sY + (int64_t)i * out_pad + k];
-      const float lv = fminf(fmaxf(Y[e * sY + (int64_t)i * out_pad + K + k], kLvMin), kLvMax);
+      const float a = y[e * sY];
+      const float lv = fminf(fmaxf(y[e * sY + K], kLvMin), kLvMax);
       mu += a;
       mu2 += a * a;
       ale += __expf(lv);
@@ -287,20 +300,28 @@ __global__ void mlp_combine_kernel(const float* Y, int N, int K, int out_pad, in
     const float epi = fmaxf(mu2 * inv - mu * mu, 0.0f);
     ale *= inv;
     const float var = aleatoric_only ? ale : ale + epi;
-    worst = fmaxf(worst, sqrtf(epi / fmaxf(ale, 1e-12f)));
-    const double u = (double)mu * (double)ystd[k] + (double)ymean[k];
-    const double vu = (double)var * (double)ystd[k] * (double)ystd[k];
+    worst[q] = sqrtf(epi / fmaxf(ale, 1e-12f));
+    const double sd = (double)ystd[k];
+    const double u = (double)mu * sd + (double)ymean[k];
+    const double vu = (double)var * sd * sd;
     const double c = yscale ? (double)yscale[k] : 0.0;
+    const int64_t o = (int64_t)i0 * K + q;
     if (c > 0.0) {
       const double ch = c * cosh(u);
-      if (mean_out) mean_out[(int64_t)i * K + k] = c * sinh(u);
-      if (var_out) var_out[(int64_t)i * K + k] = ch * ch * vu;
+      if (mean_out) mean_out[o] = (OUT)(c * sinh(u));
+      if (var_out) var_out[o] = (OUT)(ch * ch * vu);
     } else {
-      if (mean_out) mean_out[(int64_t)i * K + k] = u;
-      if (var_out) var_out[(int64_t)i * K + k] = vu;
+      if (mean_out) mean_out[o] = (OUT)u;
+      if (var_out) var_out[o] = (OUT)vu;
     }
   }
-  if (disagree) disagree[i] = worst;
+  if (!disagree) return;
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+    float w = 0.0f;
+    for (int k = 0; k < K; ++k) w = fmaxf(w, worst[i * K + k]);
+    disagree[i0 + i] = w;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -499,12 +520,27 @@ cudaError_t mlp_adam(const MlpDims& d, int members, float* P, const float* G, fl
   return cudaGetLastError();
 }
 
+template <typename OUT>
+static cudaError_t combine(const MlpDims& d, int members, int N, const float* Y, const float* ymean,
+                           const float* ystd, const float* yscale, OUT* mean_out, OUT* var_out, double* disagree,
+                           int aleatoric_only, cudaStream_t s) {
+  const int rows = std::max(1, kCombinePairs / d.K);
+  mlp_combine_kernel<OUT><<<(N + rows - 1) / rows, 256, 0, s>>>(Y, N, d.K, d.out_pad, members, (int64_t)N * d.out_pad,
+                                                                rows, ymean, ystd, yscale, mean_out, var_out, disagree,
+                                                                aleatoric_only);
+  return cudaGetLastError();
+}
+
 cudaError_t mlp_combine(const MlpDims& d, int members, int N, const float* Y, const float* ymean, const float* ystd,
                         const float* yscale, double* mean_out, double* var_out, double* disagree, int aleatoric_only,
                         cudaStream_t s) {
-  mlp_combine_kernel<<<(N + 127) / 128, 128, 0, s>>>(Y, N, d.K, d.out_pad, members, (int64_t)N * d.out_pad, ymean,
-                                                     ystd, yscale, mean_out, var_out, disagree, aleatoric_only);
-  return cudaGetLastError();
+  return combine<double>(d, members, N, Y, ymean, ystd, yscale, mean_out, var_out, disagree, aleatoric_only, s);
+}
+
+cudaError_t mlp_combine32(const MlpDims& d, int members, int N, const float* Y, const float* ymean,
+                          const float* ystd, const float* yscale, float* mean_out, float* var_out, double* disagree,
+                          cudaStream_t s) {
+  return combine<float>(d, members, N, Y, ymean, ystd, yscale, mean_out, var_out, disagree, 0, s);
 }
 
 }  // namespace abc

@@ -23,34 +23,49 @@
 #include "kernels.h"
 #include "smem_attr.h"
 #include "mlp.cuh"
+#include "mlp_tc.cuh"
 #include "tcgen05.cuh"
 
 namespace abc {
+namespace tc {
+
+bool make_map3(CUtensorMap* map, const __nv_bfloat16* base, int64_t K, int64_t ld, int64_t rows, int64_t members,
+               int64_t member_stride) {
+  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  if (!encode) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
+            cudaSuccess ||
+        q != cudaDriverEntryPointSuccess || !fn)
+      return false;
+    encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
+  }
+  memset(map, 0, sizeof(*map));
+  const int64_t row_bytes = ld * 2;
+  int64_t mstride = member_stride * 2;
+  if (members <= 1) mstride = ((rows * row_bytes + 15) / 16) * 16;
+  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)(members < 1 ? 1 : members)};
+  cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)mstride};
+  cuuint32_t box[3] = {(cuuint32_t)kTcBK, 128, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace tc
+
 namespace {
 
 using namespace tc;
 
-constexpr int BM = 128, BN = 128, BK = 64;  // BK BF16 values = one 128-byte swizzled row
+constexpr int BM = 128, BN = 128, BK = kTcBK;
 constexpr int kStages = 3;
 constexpr uint32_t kTileBytes = BM * BK * 2;  // A and B tiles alike (BN = BM)
 constexpr uint32_t kStageBytes = 2 * kTileBytes;
 constexpr uint32_t kTmemCols = 128;
 constexpr int kSmem = 1024 + kStages * kStageBytes + 128;
-
-// D = F32, A = B = BF16, both K-major, M = 128, N = 128
-constexpr uint32_t kIdescBf16 =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(kIdescBf16), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
 
 template <int EPI>
 __global__ void __launch_bounds__(128, 1)
@@ -122,7 +137,7 @@ __global__ void __launch_bounds__(128, 1)
 #pragma unroll
       for (int kk = 0; kk < BK / 16; ++kk) {
         const uint64_t adv = (uint64_t)(kk * 32) >> 4;  // 16 BF16 = 32 bytes along K
-        mma_bf16(tbase, da + adv, db + adv, (c > c0 || kk > 0) ? 1u : 0u);
+        mma_bf16_128(tbase, da + adv, db + adv, (c > c0 || kk > 0) ? 1u : 0u);
       }
       mma_commit(&empty[st]);
     }
@@ -168,11 +183,10 @@ __global__ void __launch_bounds__(128, 1)
           const float* zp = g.zprev + z * g.sZ + (int64_t)m * g.ldz + n;
           const float4 p0 = *(const float4*)zp, p1 = *(const float4*)(zp + 4);
           const float zq[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+          float sg[8];
+          sigm8(zq, sg);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float sg = sigm(zq[j]);
-            x[j] = x[j] * (sg * (1.0f + zq[j] * (1.0f - sg)));
-          }
+          for (int j = 0; j < 8; ++j) x[j] = x[j] * (sg[j] * (1.0f + zq[j] * (1.0f - sg[j])));
         }
         if (EPI != EPI_DSILU && g.outf) {
           float* o = g.outf + z * g.sOutf + (int64_t)m * g.ldf + n;
@@ -181,9 +195,15 @@ __global__ void __launch_bounds__(128, 1)
           *(float4*)(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
         }
         if (EPI == EPI_HIDDEN || EPI == EPI_DSILU) {
+          if (EPI == EPI_HIDDEN) {
+            float sg[8];
+            sigm8(x, sg);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = x[j] * sg[j];
+          }
           __nv_bfloat16 h[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16(EPI == EPI_HIDDEN ? x[j] * sigm(x[j]) : x[j]);
+          for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16(x[j]);
           uint4 pk;
           memcpy(&pk, h, 16);
           *(uint4*)(g.outh + z * g.sOuth + (int64_t)m * g.ldh + n) = pk;
@@ -200,32 +220,6 @@ __global__ void __launch_bounds__(128, 1)
   __syncthreads();
   tc_fence_after();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(kTmemCols));
-}
-
-// 3D map over [members][rows][K] BF16 (K contiguous): box 64 x 128 x 1, 128-byte swizzle
-bool make_map3(CUtensorMap* map, const __nv_bfloat16* base, int64_t K, int64_t ld, int64_t rows, int64_t members,
-               int64_t member_stride) {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn)
-      return false;
-    encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-  }
-  memset(map, 0, sizeof(*map));
-  const int64_t row_bytes = ld * 2;
-  int64_t mstride = member_stride * 2;
-  if (members <= 1) mstride = ((rows * row_bytes + 15) / 16) * 16;
-  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)(members < 1 ? 1 : members)};
-  cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)mstride};
-  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)BM, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int EPI>

@@ -28,6 +28,9 @@ cudaError_t mlp_gather(const float* xn, const float* yn, int64_t N, const MlpDim
 cudaError_t mlp_forward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0, int64_t sX,
                         const __nv_bfloat16* WhT, const float* Pf, float* Z, __nv_bfloat16* Ah, __nv_bfloat16* AhT,
                         int ldT, float* Y, int* err, cudaStream_t s);
+bool mlp_infer_fits(const MlpDims& d);
+cudaError_t mlp_infer(const MlpDims& d, int members, int B, const __nv_bfloat16* X0, const __nv_bfloat16* WhT,
+                      const float* Pf, float* Y, int* err, int sms, cudaStream_t s);
 cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0T, const __nv_bfloat16* Wh,
                          const float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
                          __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZTa, __nv_bfloat16* dZTb, int ldT,
@@ -39,6 +42,9 @@ cudaError_t mlp_adam(const MlpDims& d, int members, float* P, const float* G, fl
 cudaError_t mlp_combine(const MlpDims& d, int members, int N, const float* Y, const float* ymean, const float* ystd,
                         const float* yscale, double* mean_out, double* var_out, double* disagree, int aleatoric_only,
                         cudaStream_t s);
+cudaError_t mlp_combine32(const MlpDims& d, int members, int N, const float* Y, const float* ymean,
+                          const float* ystd, const float* yscale, float* mean_out, float* var_out, double* disagree,
+                          cudaStream_t s);
 }  // namespace abc
 
 using namespace abc;
@@ -274,6 +280,7 @@ constexpr int kPredChunk = 65536;
 struct abc_surrogate {
   MlpDims d;
   int members = 4;
+  int sms = 0;
   uint64_t seed = 0;
   cudaStream_t stream = nullptr;
   std::string err;
@@ -373,7 +380,10 @@ int abc_surrogate_create(abc_surrogate** out, int in_dim, int n_stats, int ensem
   s->d = mlp_dims(in_dim, n_stats);
   s->members = ensemble;
   s->seed = seed;
-  if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete s;
     return ABC_ERR_CUDA;
   }
@@ -579,19 +589,29 @@ int abc_surrogate_set_norm(abc_surrogate* s, const double* xmean, const double* 
 
 // predictions for device theta rows [0, N): mean, total variance (aleatoric +
 // ensemble), disagreement = max_k sqrt(ensemble var / aleatoric var)
-static int predict_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_t n, double* d_mean, double* d_var,
-                         double* d_dis, int aleatoric_only = 0) {
+static int forward_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_t n) {
   const MlpDims& d = s->d;
   const int E = s->members;
   SK(s->X0.ensure((size_t)n * d.in_pad));
-  SK(s->Ah.ensure((size_t)E * 3 * n * d.H));
   SK(s->Y.ensure((size_t)E * n * d.out_pad));
   norm_x_kernel<<<blocks(n * d.in_pad), 256, 0, s->stream>>>(d_theta, n, d.in_dim, ld, s->xm.p, s->xs.p, d.in_pad,
                                                               nullptr, s->X0.p);
   SK(cudaGetLastError());
-  SK(mlp_forward(d, E, (int)n, s->X0.p, 0, s->PhT.p, s->P.p, nullptr, s->Ah.p, nullptr, 0, s->Y.p, s->tcerr.p,
-                 s->stream));
-  SK(mlp_combine(d, E, (int)n, s->Y.p, s->ymf.p, s->ysf.p, s->yscf.p, d_mean, d_var, d_dis, aleatoric_only,
+  if (mlp_infer_fits(d)) {
+    SK(mlp_infer(d, E, (int)n, s->X0.p, s->PhT.p, s->P.p, s->Y.p, s->tcerr.p, s->sms, s->stream));
+  } else {  // more than 128 statistics: layer by layer
+    SK(s->Ah.ensure((size_t)E * 3 * n * d.H));
+    SK(mlp_forward(d, E, (int)n, s->X0.p, 0, s->PhT.p, s->P.p, nullptr, s->Ah.p, nullptr, 0, s->Y.p, s->tcerr.p,
+                   s->stream));
+  }
+  return ABC_OK;
+}
+
+static int predict_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_t n, double* d_mean, double* d_var,
+                         double* d_dis) {
+  int st = forward_chunk(s, d_theta, ld, n);
+  if (st) return st;
+  SK(mlp_combine(s->d, s->members, (int)n, s->Y.p, s->ymf.p, s->ysf.p, s->yscf.p, d_mean, d_var, d_dis, 0,
                  s->stream));
   return ABC_OK;
 }
@@ -662,8 +682,6 @@ int abc_surrogate_screen_device(abc_surrogate* s, const double* d_theta, int ld_
   for (int64_t g = 0; g < G; ++g) hx[g] = (float)(thr[g] + margin);
   SK(cudaMemcpyAsync(s->X.p, hx.data(), sizeof(float) * G, cudaMemcpyHostToDevice, s->stream));
   SK(cudaMemsetAsync(d_keep, 0, (size_t)N, s->stream));
-  SK(s->pm.ensure((size_t)kPredChunk * K));
-  SK(s->pv.ensure((size_t)kPredChunk * K));
   SK(s->pd.ensure((size_t)kPredChunk));
   SK(s->pmf.ensure((size_t)kPredChunk * K));
   SK(s->pvf.ensure((size_t)kPredChunk * K));
@@ -671,10 +689,10 @@ int abc_surrogate_screen_device(abc_surrogate* s, const double* d_theta, int ld_
   if (err_out) SK(eo.ensure((size_t)N * G));
   for (int64_t p0 = 0; p0 < N; p0 += kPredChunk) {
     const int64_t n = std::min<int64_t>(kPredChunk, N - p0);
-    int st = predict_chunk(s, d_theta + p0 * ld_theta, ld_theta, n, s->pm.p, s->pv.p, s->pd.p, 0);
+    int st = forward_chunk(s, d_theta + p0 * ld_theta, ld_theta, n);
     if (st) return st;
-    d2f_kernel<<<blocks(n * K), 256, 0, s->stream>>>(s->pm.p, s->pmf.p, n * K);
-    d2f_kernel<<<blocks(n * K), 256, 0, s->stream>>>(s->pv.p, s->pvf.p, n * K);
+    SK(mlp_combine32(s->d, s->members, (int)n, s->Y.p, s->ymf.p, s->ysf.p, s->yscf.p, s->pmf.p, s->pvf.p, s->pd.p,
+                     s->stream));
     SK(launch_dist_screen(s->pmf.p, s->pvf.p, s->sw.p, s->dw.p, n, G, K, s->X.p, (float)z, s->screen_mode, d_keep + p0,
                           err_out ? eo.p + p0 * G : nullptr, s->stream));
     disagree_keep_kernel<<<blocks(n), 256, 0, s->stream>>>(s->pd.p, n, disagree_max, d_keep + p0);
