@@ -40,6 +40,12 @@ struct DBuf {
   }
 };
 
+// Workspace of the calls that need device memory only while they run: one
+// buffer of the context, carved into 256-byte aligned pieces (an allocation and
+// release per call and array cost 0.3 to 3 ms).  A buffer above kKeepWork is
+// given back when the call ends, so a large call does not hold its memory.
+constexpr size_t kKeepWork = size_t(512) << 20;
+
 // counts buffer budget per simulate chunk: 10^6 particles x 2,000 cells run as
 // one persistent launch (16 GB of the GB300's HBM), so the heaviest
 // trajectories of the whole batch start first
@@ -121,6 +127,7 @@ struct abc_ctx {
   DistInputs sel_in;             // inputs of the last selection (device buffers; stats as given)
   DBuf<int32_t> d_asp, d_asg;    // accepted pairs for abc_accept_errors
   DBuf<double> d_aerr;
+  DBuf<uint8_t> d_work;  // see kKeepWork
   DBuf<float4> d_ffg;
   DBuf<int32_t> d_pos;
   DBuf<uint8_t> d_flag;
@@ -136,6 +143,31 @@ static int fail(abc_ctx* c, int status, const std::string& msg) {
 static int cuda_fail(abc_ctx* c, cudaError_t e, const char* where) {
   return fail(c, e == cudaErrorMemoryAllocation ? ABC_ERR_NOMEM : ABC_ERR_CUDA,
               std::string(where) + ": " + cudaGetErrorString(e));
+}
+
+// Layout of a call's workspace: add() each piece, allocate() once, then at().
+struct Work {
+  size_t total = 0;
+  uint8_t* base = nullptr;
+  size_t add(size_t bytes) {
+    const size_t off = total;
+    total += (bytes + 255) & ~size_t(255);
+    return off;
+  }
+  cudaError_t allocate(abc_ctx* c) {
+    const cudaError_t e = c->d_work.ensure(total);
+    base = c->d_work.p;
+    return e;
+  }
+  template <typename T>
+  T* at(size_t off) const {
+    return reinterpret_cast<T*>(base + off);
+  }
+};
+
+// at the end of the call, after its stream has been waited for
+static void trim_work(abc_ctx* c) {
+  if (c->d_work.cap > kKeepWork) c->d_work.release();
 }
 
 #define CK(call)                                   \
@@ -247,6 +279,7 @@ int abc_destroy(abc_ctx* c) {
   c->d_segcount.release(); c->d_hist.release(); c->d_tcerr.release(); c->d_seg.release(); c->d_cand2.release();
   c->d_alen.release(); c->d_aoff.release(); c->d_out_idx.release(); c->d_gcursor.release();
   c->d_ncand.release(); c->d_fail.release(); c->d_thr.release();
+  c->d_asp.release(); c->d_asg.release(); c->d_aerr.release(); c->d_work.release();
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   for (cudaEvent_t e : c->sel_ev)
     if (e) cudaEventDestroy(e);
@@ -891,13 +924,15 @@ int abc_errors(abc_ctx* c, const double* data, const double* se, int64_t G, int 
   DistInputs in;
   int st = load_dist_inputs(c, data, se, G, K, n_fam, fam, stats, P, in);
   if (st) return st;
-  DBuf<double> out;
-  CK(out.ensure((size_t)P * G));
-  cudaError_t e = launch_dist_full(in, out.p, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(err_out, out.p, sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  out.release();
-  if (e != cudaSuccess) return cuda_fail(c, e, "abc_errors");
+  Work w;
+  const size_t o_out = w.add(sizeof(double) * (size_t)P * G);
+  CK(w.allocate(c));
+  CK(c->d_sw.ensure((size_t)G * K));
+  CK(c->d_dw.ensure((size_t)G * K));
+  CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, w.at<double>(o_out), c->stream));
+  CK(cudaMemcpyAsync(err_out, w.at<double>(o_out), sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  trim_work(c);
   return ABC_OK;
 }
 
@@ -1376,26 +1411,24 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   const bool f32 = cf.precision == ABC_FP32;
   const int grid = (int)std::min<int64_t>(P, (int64_t)c->sms * (f32 ? 16 : 8));
   const size_t scr_doubles = f32 ? (moment_f32_scratch_per_cta(a.nsub) + 7) / 8 : (size_t)2 * a.nsub * 100;
-  DBuf<double> d_theta, d_bm, d_ad, d_stats, d_mom, d_scr;
-  DBuf<int> d_it;
-  CK(d_theta.ensure((size_t)P * npar));
-  CK(d_bm.ensure((size_t)2 * A * 3));
-  CK(d_ad.ensure((size_t)A * J));
-  CK(d_stats.ensure((size_t)P * K));
-  CK(d_scr.ensure((size_t)grid * scr_doubles));
-  if (moments_out) CK(d_mom.ensure((size_t)P * J * A * 5));
-  if (iters_out) CK(d_it.ensure((size_t)P));
-  CK(cudaMemcpyAsync(d_theta.p, theta, sizeof(double) * P * npar, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(d_bm.p, beta_mom, sizeof(double) * 2 * A * 3, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(d_ad.p, age_dist, sizeof(double) * A * J, cudaMemcpyHostToDevice, c->stream));
+  Work w;
+  const size_t o_theta = w.add(sizeof(double) * (size_t)P * npar), o_bm = w.add(sizeof(double) * 2 * A * 3);
+  const size_t o_ad = w.add(sizeof(double) * (size_t)A * J), o_stats = w.add(sizeof(double) * (size_t)P * K);
+  const size_t o_scr = w.add(sizeof(double) * (size_t)grid * scr_doubles);
+  const size_t o_mom = w.add(moments_out ? sizeof(double) * (size_t)P * J * A * 5 : 0);
+  const size_t o_it = w.add(iters_out ? sizeof(int) * (size_t)P : 0);
+  CK(w.allocate(c));
+  CK(cudaMemcpyAsync(w.at<double>(o_theta), theta, sizeof(double) * P * npar, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(w.at<double>(o_bm), beta_mom, sizeof(double) * 2 * A * 3, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(w.at<double>(o_ad), age_dist, sizeof(double) * A * J, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemsetAsync(c->d_status.p, 0, sizeof(int), c->stream));
-  a.theta = d_theta.p;
-  a.beta_mom = d_bm.p;
-  a.age_dist = d_ad.p;
-  a.stats = d_stats.p;
-  a.moments = moments_out ? d_mom.p : nullptr;
-  a.iters = iters_out ? d_it.p : nullptr;
-  a.scratch = d_scr.p;
+  a.theta = w.at<double>(o_theta);
+  a.beta_mom = w.at<double>(o_bm);
+  a.age_dist = w.at<double>(o_ad);
+  a.stats = w.at<double>(o_stats);
+  a.moments = moments_out ? w.at<double>(o_mom) : nullptr;
+  a.iters = iters_out ? w.at<int>(o_it) : nullptr;
+  a.scratch = w.at<double>(o_scr);
   a.status = c->d_status.p;
   if (c->prof && !c->sel_ev[0]) {
     CK(cudaEventCreate(&c->sel_ev[0]));
@@ -1404,10 +1437,10 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   if (c->prof) CK(cudaEventRecord(c->sel_ev[0], c->stream));
   CK(f32 ? launch_moment_f32(a, grid, c->stream) : launch_moment(a, grid, c->stream));
   if (c->prof) CK(cudaEventRecord(c->sel_ev[1], c->stream));
-  CK(cudaMemcpyAsync(stats_out, d_stats.p, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(stats_out, a.stats, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
   if (moments_out)
-    CK(cudaMemcpyAsync(moments_out, d_mom.p, sizeof(double) * P * J * A * 5, cudaMemcpyDeviceToHost, c->stream));
-  if (iters_out) CK(cudaMemcpyAsync(iters_out, d_it.p, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(moments_out, a.moments, sizeof(double) * P * J * A * 5, cudaMemcpyDeviceToHost, c->stream));
+  if (iters_out) CK(cudaMemcpyAsync(iters_out, a.iters, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
   int hst = 0;
   CK(cudaMemcpyAsync(&hst, c->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1417,6 +1450,7 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
     c->sel_fast_ms = ms;
     c->sel_fast_passes = 1;
   }
+  trim_work(c);
   if (hst) return fail(c, ABC_ERR_NONFINITE, "abc_moment_simulate: non-finite rates for some particles (NaN rows)");
   return ABC_OK;
 }
@@ -1430,23 +1464,22 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   if (c->C > data_stats_max_cells(c->cfg.n_ages, c->cfg.n_conds))
     return fail(c, ABC_ERR_INVALID, "abc_data_stats: too many cells for the per-gene shared-memory table");
   const int64_t C = c->C;
-  for (int64_t i = 0; i < G * C; ++i)
-    if (u[i] < 0 || l[i] < 0 || u[i] > (1 << 20) || l[i] > (1 << 20))
-      return fail(c, ABC_ERR_INVALID, "abc_data_stats: counts must lie in [0, 2^20]");
   if (G == 0) return ABC_OK;
   const int K = 4 * c->cfg.n_ages + 3 * c->cfg.n_conds;
-  DBuf<int32_t> du, dl;
-  DBuf<double> dout, dse;
-  CK(du.ensure((size_t)G * C));
-  CK(dl.ensure((size_t)G * C));
-  CK(dout.ensure((size_t)G * (n_boot + 1) * K));
-  if (se_out) CK(dse.ensure((size_t)G * K));
-  CK(cudaMemcpyAsync(du.p, u, sizeof(int32_t) * G * C, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(dl.p, l, sizeof(int32_t) * G * C, cudaMemcpyHostToDevice, c->stream));
+  Work w;
+  const size_t o_u = w.add(sizeof(int32_t) * (size_t)G * C), o_l = w.add(sizeof(int32_t) * (size_t)G * C);
+  const size_t o_out = w.add(sizeof(double) * (size_t)G * (n_boot + 1) * K);
+  const size_t o_se = w.add(se_out ? sizeof(double) * (size_t)G * K : 0);
+  const size_t o_sums = w.add(data_stats_scratch(c->dcfg, G, n_boot, C));
+  CK(w.allocate(c));
+  double* dout = w.at<double>(o_out);
+  double* dse = se_out ? w.at<double>(o_se) : nullptr;
+  CK(cudaMemcpyAsync(w.at<int32_t>(o_u), u, sizeof(int32_t) * G * C, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(w.at<int32_t>(o_l), l, sizeof(int32_t) * G * C, cudaMemcpyHostToDevice, c->stream));
   DataStatsArgs a;
   a.cfg = c->dcfg;
-  a.u = du.p;
-  a.l = dl.p;
+  a.u = w.at<int32_t>(o_u);
+  a.l = w.at<int32_t>(o_l);
   a.G = G;
   a.C = C;
   a.cell_cond = c->d_cond.p;
@@ -1456,18 +1489,29 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   a.age_dist = c->d_age_dist.p;
   a.n_boot = n_boot;
   a.seed = seed;
-  a.out = dout.p;
+  a.out = dout;
+  a.sums = w.at<unsigned long long>(o_sums);
+  a.invalid = c->d_status.p;
   if (c->prof && !c->sel_ev[0]) {
     CK(cudaEventCreate(&c->sel_ev[0]));
     CK(cudaEventCreate(&c->sel_ev[1]));
   }
   if (c->prof) CK(cudaEventRecord(c->sel_ev[0], c->stream));
-  CK(launch_data_stats(a, se_out ? dse.p : nullptr, c->stream));
+  CK(launch_data_stats(a, dse, c->stream));
   if (c->prof) CK(cudaEventRecord(c->sel_ev[1], c->stream));
+  // the counts are checked where they are read (a pass over them on the host
+  // took a millisecond per 10^7): nothing is returned for invalid ones
+  int invalid = 0;
+  CK(cudaMemcpyAsync(&invalid, c->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (invalid) {
+    trim_work(c);
+    return fail(c, ABC_ERR_INVALID, "abc_data_stats: counts must lie in [0, 2^20]");
+  }
   // the estimate is resample 0 of each gene
-  CK(cudaMemcpy2DAsync(stats_out, sizeof(double) * K, dout.p, sizeof(double) * K * (n_boot + 1), sizeof(double) * K,
+  CK(cudaMemcpy2DAsync(stats_out, sizeof(double) * K, dout, sizeof(double) * K * (n_boot + 1), sizeof(double) * K,
                        (size_t)G, cudaMemcpyDeviceToHost, c->stream));
-  if (se_out) CK(cudaMemcpyAsync(se_out, dse.p, sizeof(double) * G * K, cudaMemcpyDeviceToHost, c->stream));
+  if (se_out) CK(cudaMemcpyAsync(se_out, dse, sizeof(double) * G * K, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (c->prof) {
     float ms = 0.0f;
@@ -1475,6 +1519,7 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
     c->sel_fast_ms = ms;
     c->sel_fast_passes = 1;
   }
+  trim_work(c);
   return ABC_OK;
 }
 
@@ -1487,26 +1532,20 @@ int abc_model_probs(abc_ctx* c, const int64_t* counts, int64_t G, int M, int n_b
   for (int64_t i = 0; i < G * M; ++i)
     if (counts[i] < 0) return fail(c, ABC_ERR_INVALID, "abc_model_probs: negative count");
   if (G == 0) return ABC_OK;
-  DBuf<int64_t> d_counts;
-  DBuf<double> d_out, d_boot;
-  cudaError_t e = d_counts.ensure((size_t)G * M);
-  if (e == cudaSuccess) e = d_out.ensure((size_t)3 * G * M);
-  if (e == cudaSuccess) e = d_boot.ensure((size_t)G * M * n_boot);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_counts.p, counts, sizeof(int64_t) * G * M, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess)
-    e = launch_model_probs(d_counts.p, G, M, n_boot, alpha, seed, d_out.p, d_out.p + G * M, d_out.p + 2 * G * M,
-                           d_boot.p, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(prob, d_out.p, sizeof(double) * G * M, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(lb, d_out.p + G * M, sizeof(double) * G * M, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ub, d_out.p + 2 * G * M, sizeof(double) * G * M, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  d_counts.release();
-  d_out.release();
-  d_boot.release();
-  if (e != cudaSuccess) return cuda_fail(c, e, "abc_model_probs");
+  const size_t n = (size_t)G * M;
+  Work w;
+  const size_t o_counts = w.add(sizeof(int64_t) * n), o_out = w.add(sizeof(double) * 3 * n);
+  const size_t o_boot = w.add(sizeof(double) * n * n_boot);
+  CK(w.allocate(c));
+  double* out = w.at<double>(o_out);
+  CK(cudaMemcpyAsync(w.at<int64_t>(o_counts), counts, sizeof(int64_t) * n, cudaMemcpyHostToDevice, c->stream));
+  CK(launch_model_probs(w.at<int64_t>(o_counts), G, M, n_boot, alpha, seed, out, out + n, out + 2 * n,
+                        w.at<double>(o_boot), c->stream));
+  CK(cudaMemcpyAsync(prob, out, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(lb, out + n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(ub, out + 2 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  trim_work(c);
   return ABC_OK;
 }
 
@@ -1517,35 +1556,27 @@ int abc_posterior_summary(abc_ctx* c, const double* theta, int64_t ld, int npar,
   if (!theta || !map || !mean || !lb || !ub || npar < 1 || ld < npar || !(q > 0.0 && q < 1.0))
     return fail(c, ABC_ERR_INVALID, "abc_posterior_summary: bad arguments");
   const int64_t G = c->sel_G, P = c->sel_P, total = c->sel_total;
-  DBuf<double> d_theta, d_scr, d_out;
-  DBuf<int64_t> d_n;
+  const size_t gn = (size_t)G * npar;
+  Work w;
+  const size_t o_theta = w.add(theta_on_device ? 0 : sizeof(double) * (size_t)P * ld);
+  const size_t o_scr = w.add(sizeof(double) * ((size_t)total * npar + 4 * gn)), o_out = w.add(sizeof(double) * 4 * gn);
+  const size_t o_n = w.add(sizeof(int64_t) * (size_t)G);
+  CK(w.allocate(c));
   const double* th = theta;
-  cudaError_t e = cudaSuccess;
   if (!theta_on_device) {
-    e = d_theta.ensure((size_t)P * ld);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(d_theta.p, theta, sizeof(double) * P * ld, cudaMemcpyHostToDevice, c->stream);
-    th = d_theta.p;
+    CK(cudaMemcpyAsync(w.at<double>(o_theta), theta, sizeof(double) * P * ld, cudaMemcpyHostToDevice, c->stream));
+    th = w.at<double>(o_theta);
   }
-  if (e == cudaSuccess) e = d_scr.ensure((size_t)total * npar + (size_t)4 * G * npar);
-  if (e == cudaSuccess) e = d_out.ensure((size_t)4 * G * npar);
-  if (e == cudaSuccess) e = d_n.ensure((size_t)G);
-  if (e == cudaSuccess)
-    e = launch_posterior_summary(c->d_aoff.p, c->d_out_idx.p, G, total, th, ld, npar, q, d_scr.p, d_out.p,
-                                 d_out.p + G * npar, d_out.p + 2 * G * npar, d_out.p + 3 * G * npar, d_n.p,
-                                 c->stream);
+  double* out = w.at<double>(o_out);
+  CK(launch_posterior_summary(c->d_aoff.p, c->d_out_idx.p, G, total, th, ld, npar, q, w.at<double>(o_scr), out, out + gn,
+                              out + 2 * gn, out + 3 * gn, w.at<int64_t>(o_n), c->stream));
   double* outs[4] = {map, mean, lb, ub};
-  for (int i = 0; i < 4 && e == cudaSuccess; ++i)
-    e = cudaMemcpyAsync(outs[i], d_out.p + (size_t)i * G * npar, sizeof(double) * G * npar, cudaMemcpyDeviceToHost,
-                        c->stream);
-  if (e == cudaSuccess && n_particles)
-    e = cudaMemcpyAsync(n_particles, d_n.p, sizeof(int64_t) * G, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  d_theta.release();
-  d_scr.release();
-  d_out.release();
-  d_n.release();
-  if (e != cudaSuccess) return cuda_fail(c, e, "abc_posterior_summary");
+  for (int i = 0; i < 4; ++i)
+    CK(cudaMemcpyAsync(outs[i], out + i * gn, sizeof(double) * gn, cudaMemcpyDeviceToHost, c->stream));
+  if (n_particles)
+    CK(cudaMemcpyAsync(n_particles, w.at<int64_t>(o_n), sizeof(int64_t) * G, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  trim_work(c);
   return ABC_OK;
 }
 

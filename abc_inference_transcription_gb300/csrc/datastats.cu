@@ -4,8 +4,8 @@
 // statistics: [pulse mean (A), pulse FF (A), chase mean (A), chase FF (A),
 // ratio (J), mean_corr (J), corr_mean (J)].
 //
-// Two phases: one CTA per (gene, resample) forms the integer sums, then one
-// thread per (gene, resample, statistic group) computes the statistics from
+// Two phases: one CTA per (gene, group of resamples) forms the integer sums,
+// then one thread per (gene, resample, statistic group) computes the statistics from
 // them.  Resample 0 is the estimate itself, 1..n_boot are bootstrap resamples
 // of the cells with replacement, drawn separately for
 // the pulse cells, the chase cells and all cells (ratios and correlations), as
@@ -29,18 +29,20 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// position in [0, n) of draw i of stream (seed, family, resample, gene):
-// floor(x n / 2^52) of a 52-bit uniform integer x, in exact integer arithmetic
-__device__ __forceinline__ int64_t draw_pos(uint64_t seed, int fam, int b, int64_t g, int64_t i, int64_t n) {
+// positions in [0, n) of draws 2 j and 2 j + 1 of stream (seed, family, resample,
+// gene): floor(x n / 2^52) of 52-bit uniform integers x, in exact integer
+// arithmetic; both come from one Philox block
+__device__ __forceinline__ void draw_pair(uint64_t seed, int fam, int b, int64_t g, int64_t j, int64_t n, int64_t& p0,
+                                          int64_t& p1) {
   U4 c;
-  c.x = (uint32_t)(i >> 1);
-  c.y = ((uint32_t)((uint64_t)i >> 33) & 0x3fffffffu) | (ST_AUX << 30);
+  c.x = (uint32_t)j;
+  c.y = ((uint32_t)((uint64_t)j >> 32) & 0x3fffffffu) | (ST_AUX << 30);
   c.z = (uint32_t)b | ((uint32_t)(fam + 1) << 24);
   c.w = (uint32_t)g;
   const U4 o = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-  const uint32_t hi = (i & 1) ? o.z : o.x, lo = (i & 1) ? o.w : o.y;
-  const uint64_t x = ((uint64_t)hi << 20) | (uint64_t)(lo >> 12);
-  return (int64_t)__umul64hi(x << 12, (uint64_t)n);
+  const uint64_t x0 = ((uint64_t)o.x << 20) | (uint64_t)(o.y >> 12), x1 = ((uint64_t)o.z << 20) | (uint64_t)(o.w >> 12);
+  p0 = (int64_t)__umul64hi(x0 << 12, (uint64_t)n);
+  p1 = (int64_t)__umul64hi(x1 << 12, (uint64_t)n);
 }
 
 // exact sample variance / covariance from integer sums: (n sxy - sx sy) / (n (n - 1))
@@ -55,98 +57,152 @@ __device__ __forceinline__ double sample_cov(unsigned long long n, unsigned long
 __device__ __forceinline__ double sample_cov_r(unsigned long long n, unsigned long long sx, unsigned long long sy,
                                                unsigned long long sxy, double d2, double r2) {
   const __int128 num = (__int128)n * (__int128)sxy - (__int128)sx * (__int128)sy;
-  return div_rn(i128_to_double(num), d2, r2);
-}
-
-// Exact 64-bit sums from 32-bit shared-memory atomics (the 64-bit form is far
-// slower): the low word takes the addend's low 32 bits, its carry out is read
-// from the returned old value, and the high word is touched only for a carry
-// or a non-zero high part (rare for counts).
-__device__ __forceinline__ void add64(unsigned* lo, unsigned* hi, unsigned long long v) {
-  const unsigned vl = (unsigned)v, vh = (unsigned)(v >> 32);
-  const unsigned old = atomicAdd(lo, vl);
-  const unsigned carry = old + vl < old ? 1u : 0u;
-  if (carry | vh) atomicAdd(hi, vh + carry);
+  const double x = i128_to_double(num);
+  return x == 0.0 && d2 > 0.0 ? x : div_rn(x, d2, r2);  // d2 = 0 (one cell): 0 / 0 is NaN
 }
 
 // Phase 1, one CTA per (gene, resample group): the integer sums of the
 // resamples b = blockIdx.y, blockIdx.y + gridDim.y, ...  The gene's cells are
-// first copied into shared memory in the group-sorted order, (u, l) and the
-// (condition, age) group of each, so that the draws (random cells) read
-// shared memory instead of scattered global lines.  Each warp accumulates
-// into its own copy of the sums (low and high words), so atomics contend only
-// within a warp; after each resample the copies are added and the nsum totals
-// written to S_out (integer sums: the order does not matter).
-constexpr int kWarps = kThreads / 32;
+// first copied into shared memory in the group-sorted order.  A resample
+// only counts how often each cell is drawn (one 16-bit counter per cell, two to a
+// word, one shared-memory atomic per draw); then a few lanes per (condition,
+// age) group add count x (1, u, l, u^2, l^2, u l) over its cells, which are
+// contiguous, in registers, and join with shuffles.  Six sums per draw through
+// shared-memory atomics took 3.15 ms for 2,000 genes x 2,000 cells x 100
+// resamples, this takes SUMS_MS: the draws' Philox blocks (two draws each) are
+// what is left.  Integer sums: the order does not matter.  The pulse and the
+// chase draws share the counters of one pass unless both use the same cells.
 constexpr size_t data_stats_smem_limit() { return 227 * 1024; }
+constexpr int kMaxCount = 1 << 20;  // abc_data_stats' limit of a count
 
-__global__ void __launch_bounds__(kThreads) data_sums_kernel(DataStatsArgs a, int64_t g0,
-                                                             unsigned long long* S_out) {
-  extern __shared__ unsigned long long sums[];
+struct Sums6 {
+  unsigned long long v[6];
+};
+
+// lanes per group: the largest power of two with groups x lanes <= kThreads, at most 32
+__device__ __forceinline__ int group_lanes(int groups) {
+  int L = 32;
+  while (L > 1 && L * groups > kThreads) L >>= 1;
+  return L;
+}
+
+// threads 0 .. groups * L - 1: the sums of cells [i0, i1) with counter offsets, joined over L lanes
+template <bool PAIR>
+__device__ __forceinline__ Sums6 group_sums(const int2* T, const unsigned short* mult, int64_t i0, int64_t i1, int sub,
+                                            int L, bool one) {
+  Sums6 s = {{0, 0, 0, 0, 0, 0}};
+  for (int64_t i = i0 + sub; i < i1; i += L) {
+    const unsigned long long m = one ? 1u : mult[i];
+    const int2 t = T[i];
+    const unsigned long long u = (unsigned)t.x, l = (unsigned)t.y;
+    if (PAIR) {
+      s.v[0] += m;
+      s.v[1] += m * u;
+      s.v[2] += m * l;
+      s.v[3] += m * (u * u);
+      s.v[4] += m * (l * l);
+      s.v[5] += m * (u * l);
+    } else {
+      const unsigned long long x = u + l;
+      s.v[0] += m;
+      s.v[1] += m * x;
+      s.v[2] += m * (x * x);
+    }
+  }
+  for (int o = L >> 1; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < (PAIR ? 6 : 3); ++q) s.v[q] += __shfl_xor_sync(0xffffffffu, s.v[q], o);
+  return s;
+}
+
+__device__ __forceinline__ void count_draws(const DataStatsArgs& a, unsigned* words, int fam, int b, int64_t g,
+                                            int64_t base, int64_t n) {
+  for (int64_t j = threadIdx.x; 2 * j < n; j += blockDim.x) {
+    int64_t p0, p1;
+    draw_pair(a.seed, fam, b, g, j, n, p0, p1);
+    p0 += base;
+    p1 += base;
+    // counters reach at most the number of draws, below 2^16 (data_stats_max_cells)
+    atomicAdd(&words[p0 >> 1], 1u << ((p0 & 1) * 16));
+    if (2 * j + 1 < n) atomicAdd(&words[p1 >> 1], 1u << ((p1 & 1) * 16));
+  }
+}
+
+__global__ void __launch_bounds__(kThreads) data_sums_kernel(DataStatsArgs a, int64_t g0, unsigned long long* S_out) {
+  extern __shared__ int2 T[];                                       // (u, l) per sorted cell
   const int A = a.cfg.n_ages, J = a.cfg.n_conds;
   const int nsum = 6 * A + 6 * J * A;
   const int64_t C = a.C;
-  unsigned* words = reinterpret_cast<unsigned*>(sums);               // per warp: lo[nsum], hi[nsum]
-  int2* T = reinterpret_cast<int2*>(sums + kWarps * nsum);           // (u, l) per sorted cell
-  unsigned short* grp = reinterpret_cast<unsigned short*>(T + C);   // condition * A + age
-  unsigned* lo = words + (threadIdx.x >> 5) * 2 * nsum;
-  unsigned* hi = lo + nsum;
-  const int ocs = 6 * A;                                              // offset of the all-cells sums
+  unsigned* words = reinterpret_cast<unsigned*>(T + C);             // times each cell was drawn, 16 bits each
+  const unsigned short* mult = reinterpret_cast<const unsigned short*>(words);
+  const int n_words = (int)((C + 1) / 2);
   const int64_t g = g0 + blockIdx.x;
   const int32_t* u = a.u + g * C;
   const int32_t* l = a.l + g * C;
+  bool bad = false;
   for (int64_t i = threadIdx.x; i < C; i += blockDim.x) {
     const int64_t id = a.cell_id[i];
     T[i] = make_int2(u[id], l[id]);
-    grp[i] = (unsigned short)(a.cell_cond[i] * A + a.cell_age[i]);
+    bad = bad || (unsigned)T[i].x > (unsigned)kMaxCount || (unsigned)T[i].y > (unsigned)kMaxCount;
   }
+  if (bad) *a.invalid = 1;
+  const int cp = a.cfg.pulse_stat, cc = a.cfg.chase_stat;
+  const int L2 = group_lanes(J * A), L1 = group_lanes(2 * A);
   for (int b = blockIdx.y; b <= a.n_boot; b += gridDim.y) {
-    for (int i = threadIdx.x; i < 2 * kWarps * nsum; i += blockDim.x) words[i] = 0u;
-    __syncthreads();
-    // pulse and chase cells (contiguous in the group-sorted cell order):
-    // per age (n, sx, sxx) at 3 A f + 3 ag
-    for (int f = 0; f < 2; ++f) {
-      const int cond = f == 0 ? a.cfg.pulse_stat : a.cfg.chase_stat;
-      const int64_t base = a.gstart[cond * A], n = a.gstart[(cond + 1) * A] - base;
-      for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const int64_t cell = base + (b == 0 ? i : draw_pos(a.seed, f, b, g, i, n));
-        const int2 t = T[cell];
-        const unsigned long long x = (unsigned long long)t.x + (unsigned long long)t.y;
-        const int o = 3 * A * f + 3 * ((int)grp[cell] - cond * A);
-        atomicAdd(&lo[o], 1u);
-        add64(&lo[o + 1], &hi[o + 1], x);
-        add64(&lo[o + 2], &hi[o + 2], x * x);
-      }
+    unsigned long long* out = S_out + ((int64_t)blockIdx.x * (a.n_boot + 1) + b) * nsum;
+    // pulse and chase cells: per age (n, sx, sxx) at 3 A f + 3 ag
+    for (int f0 = 0; f0 < 2; f0 += (cp == cc ? 1 : 2)) {
+      const int f1 = cp == cc ? f0 + 1 : 2;
+      __syncthreads();
+      for (int i = threadIdx.x; i < n_words; i += blockDim.x) words[i] = 0u;
+      __syncthreads();
+      if (b > 0)
+        for (int f = f0; f < f1; ++f) {
+          const int cond = f == 0 ? cp : cc;
+          const int64_t base = a.gstart[cond * A];
+          count_draws(a, words, f, b, g, base, a.gstart[(cond + 1) * A] - base);
+        }
+      __syncthreads();
+      const int grp = threadIdx.x / L1, f = grp / A, ag = grp - f * A;
+      const bool mine = grp < 2 * A && f >= f0 && f < f1;
+      const int gi = mine ? (f == 0 ? cp : cc) * A + ag : 0;
+      const Sums6 s = group_sums<false>(T, mult, mine ? a.gstart[gi] : 0, mine ? a.gstart[gi + 1] : 0,
+                                        threadIdx.x % L1, L1, b == 0);
+      if (mine && threadIdx.x % L1 == 0)
+        for (int q = 0; q < 3; ++q) out[3 * grp + q] = s.v[q];
     }
     // all cells: per (condition, age) (n, su, sl, suu, sll, sul)
-    for (int64_t i = threadIdx.x; i < C; i += blockDim.x) {
-      const int64_t cell = b == 0 ? i : draw_pos(a.seed, 2, b, g, i, C);
-      const int2 t = T[cell];
-      const unsigned long long uu = (unsigned long long)t.x, ll = (unsigned long long)t.y;
-      const int o = ocs + 6 * (int)grp[cell];
-      atomicAdd(&lo[o], 1u);
-      add64(&lo[o + 1], &hi[o + 1], uu);
-      add64(&lo[o + 2], &hi[o + 2], ll);
-      add64(&lo[o + 3], &hi[o + 3], uu * uu);
-      add64(&lo[o + 4], &hi[o + 4], ll * ll);
-      add64(&lo[o + 5], &hi[o + 5], uu * ll);
-    }
     __syncthreads();
-    unsigned long long* out = S_out + ((int64_t)blockIdx.x * (a.n_boot + 1) + b) * nsum;
-    for (int i = threadIdx.x; i < nsum; i += blockDim.x) {
-      unsigned long long t = 0ull;
-      for (int w = 0; w < kWarps; ++w)
-        t += ((unsigned long long)words[w * 2 * nsum + nsum + i] << 32) | words[w * 2 * nsum + i];
-      out[i] = t;
-    }
+    for (int i = threadIdx.x; i < n_words; i += blockDim.x) words[i] = 0u;
     __syncthreads();
+    if (b > 0) count_draws(a, words, 2, b, g, 0, C);
+    __syncthreads();
+    const int grp = threadIdx.x / L2;
+    const bool mine = grp < J * A;
+    const Sums6 s = group_sums<true>(T, mult, mine ? a.gstart[grp] : 0, mine ? a.gstart[grp + 1] : 0,
+                                     threadIdx.x % L2, L2, b == 0);
+    if (mine && threadIdx.x % L2 == 0)
+      for (int q = 0; q < 6; ++q) out[6 * A + 6 * grp + q] = s.v[q];
   }
 }
+
+// RN(1 / n) and RN(1 / (n (n - 1))) of the sample sizes 1..C, for phase 2: a
+// reciprocal each, instead of two divisions per group of every resample on the FP64 pipe
+__global__ void data_recip_kernel(int64_t C, double2* recip) {
+  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < 1 || n > C) return;
+  const double nd = (double)n;
+  recip[n] = make_double2(1.0 / nd, 1.0 / (nd * (double)(n - 1)));
+}
+
+// a / b for b > 0 given y = RN(1 / b): div_rn, and 0 without its slow path
+__device__ __forceinline__ double div_pos(double a, double b, double y) { return a == 0.0 ? a : div_rn(a, b, y); }
 
 // Phase 2, one thread per (gene, resample, item): items 0..2A-1 are the mean
 // and Fano factor of one (family, age) cell, items 2A..2A+J-1 the ratio,
 // mean_corr and corr_mean of one condition.
-__global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const unsigned long long* S_in) {
+__global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const unsigned long long* S_in,
+                                  const double2* __restrict__ recip) {
   const int A = a.cfg.n_ages, J = a.cfg.n_conds, K = 4 * A + 3 * J;
   const int nsum = 6 * A + 6 * J * A;
   const int items = 2 * A + J;
@@ -187,18 +243,21 @@ __global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const
       if (S[0] == 0) {
         m1[ag] = m2[ag] = v1[ag] = v2[ag] = c12[ag] = 0.0;
       } else {
-        // two reciprocals per group instead of five divisions
-        const double nd = (double)S[0], rn = 1.0 / nd;
-        m1[ag] = div_rn((double)S[1], nd, rn);
-        m2[ag] = div_rn((double)S[2], nd, rn);
-        const double d2 = nd * (double)(S[0] - 1), r2 = 1.0 / d2;
+        const double2 r = recip[S[0]];
+        const double nd = (double)S[0], rn = r.x;
+        m1[ag] = div_pos((double)S[1], nd, rn);
+        m2[ag] = div_pos((double)S[2], nd, rn);
+        const double d2 = nd * (double)(S[0] - 1), r2 = r.y;
         v1[ag] = sample_cov_r(S[0], S[1], S[1], S[3], d2, r2);
         v2[ag] = sample_cov_r(S[0], S[2], S[2], S[4], d2, r2);
         c12[ag] = sample_cov_r(S[0], S[1], S[2], S[5], d2, r2);
       }
     }
     // ratio of means (get_cond_specific_ratios)
-    const double mu = (double)suj / (double)nj, ml = (double)slj / (double)nj;
+    // nj = 0 (no cell of the condition drawn) keeps its 0 / 0
+    const double njd = (double)nj, rj = nj > 0 ? recip[nj].x : INFINITY;
+    const double mu = nj > 0 ? div_pos((double)suj, njd, rj) : (double)suj / njd;
+    const double ml = nj > 0 ? div_pos((double)slj, njd, rj) : (double)slj / njd;
     st[4 * A + j] = (mu + ml > 0.0) ? ml / (mu + ml) : 0.0;
     // age weights: the given distribution for the estimate; for a bootstrap
     // resample the resampled cells' age fractions within the condition
@@ -207,8 +266,7 @@ __global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const
       if (b == 0) {
         w[ag] = a.age_dist[ag * J + j];
       } else {
-        const double x = (double)Sg[6 * (j * A + ag)] / (double)nj;
-        w[ag] = x == x ? x : 0.0;
+        w[ag] = nj > 0 ? div_pos((double)Sg[6 * (j * A + ag)], njd, rj) : 0.0;
       }
     }
     // get_cond_specific_correlations
@@ -243,29 +301,44 @@ __global__ void data_se_kernel(const double* boot, int64_t G, int K, int n_boot,
 
 }  // namespace
 
+// (the limit of the earlier layout, which kept per-warp sums beside the 10 bytes
+// per cell: calls are accepted and refused as before)
 int64_t data_stats_max_cells(int n_ages, int n_conds) {
   const int64_t nsum = 6 * n_ages + 6 * n_conds * n_ages;
-  return ((int64_t)data_stats_smem_limit() - (int64_t)sizeof(unsigned long long) * nsum * kWarps) /
+  return ((int64_t)data_stats_smem_limit() - (int64_t)sizeof(unsigned long long) * nsum * (kThreads / 32)) /
          (int64_t)(sizeof(int2) + sizeof(unsigned short));
+}
+
+// the sums of at most ~256 MB of (gene, resample) pairs at a time
+static int64_t genes_at_a_time(const DevCfg& cfg, int64_t G, int n_boot, int64_t* per_gene) {
+  const int64_t nsum = 6 * cfg.n_ages + 6 * cfg.n_conds * cfg.n_ages;
+  *per_gene = (int64_t)(n_boot + 1) * nsum * (int64_t)sizeof(unsigned long long);
+  return std::max<int64_t>(1, std::min<int64_t>(G, ((int64_t)256 << 20) / *per_gene));
+}
+
+size_t data_stats_scratch(const DevCfg& cfg, int64_t G, int n_boot, int64_t C) {
+  int64_t per_gene = 0;
+  const int64_t chunk = genes_at_a_time(cfg, G, n_boot, &per_gene);
+  return (size_t)(chunk * per_gene) + sizeof(double2) * (size_t)(C + 1);
 }
 
 cudaError_t launch_data_stats(const DataStatsArgs& a, double* se, cudaStream_t s) {
   if (a.G <= 0) return cudaSuccess;
   const int A = a.cfg.n_ages, J = a.cfg.n_conds, K = 4 * A + 3 * J;
-  const int64_t nsum = 6 * A + 6 * J * A;
-  const size_t smem = sizeof(unsigned long long) * nsum * kWarps + (size_t)a.C * (sizeof(int2) + sizeof(unsigned short));
+  const size_t smem = (size_t)a.C * sizeof(int2) + sizeof(unsigned) * (size_t)((a.C + 1) / 2);
   if (smem > data_stats_smem_limit()) return cudaErrorInvalidValue;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(data_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  // the sums of at most ~256 MB of (gene, resample) pairs at a time
-  const int64_t per_gene = (int64_t)(a.n_boot + 1) * nsum * (int64_t)sizeof(unsigned long long);
-  const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(a.G, ((int64_t)256 << 20) / per_gene));
-  unsigned long long* S = nullptr;
-  cudaError_t e = cudaMallocAsync(&S, (size_t)(chunk * per_gene), s);
+  int64_t per_gene = 0;
+  const int64_t chunk = genes_at_a_time(a.cfg, a.G, a.n_boot, &per_gene);
+  unsigned long long* S = a.sums;
+  double2* recip = reinterpret_cast<double2*>(reinterpret_cast<char*>(S) + chunk * per_gene);
+  cudaError_t e = cudaMemsetAsync(a.invalid, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
-  for (int64_t g0 = 0; g0 < a.G && e == cudaSuccess; g0 += chunk) {
+  data_recip_kernel<<<(unsigned)(a.C / 256 + 1), 256, 0, s>>>(a.C, recip);
+  for (int64_t g0 = 0; g0 < a.G; g0 += chunk) {
     const int64_t ng = std::min<int64_t>(chunk, a.G - g0);
     // enough CTAs to fill the GPU several times over, resamples split among them
     const int64_t want = (int64_t)4 * 152 * 5;
@@ -273,12 +346,10 @@ cudaError_t launch_data_stats(const DataStatsArgs& a, double* se, cudaStream_t s
     data_sums_kernel<<<dim3((unsigned)ng, (unsigned)groups), kThreads, smem, s>>>(a, g0, S);
     const int64_t items = ng * (a.n_boot + 1) * (2 * A + J);
     const int64_t blocks = std::min<int64_t>((items + 127) / 128, 65536);
-    data_stats_kernel<<<(unsigned)blocks, 128, 0, s>>>(a, g0, ng, S);
+    data_stats_kernel<<<(unsigned)blocks, 128, 0, s>>>(a, g0, ng, S, recip);
     e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  const cudaError_t ef = cudaFreeAsync(S, s);
-  if (e != cudaSuccess) return e;
-  if (ef != cudaSuccess) return ef;
   if (a.n_boot < 2 || !se) return cudaSuccess;
   const int64_t n = a.G * K;
   data_se_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a.out, a.G, K, a.n_boot, se);

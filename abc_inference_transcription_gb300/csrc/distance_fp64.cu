@@ -411,19 +411,103 @@ __global__ void run_sort_kernel(const int32_t* sg, const int64_t* goff, const ui
   }
 }
 
-__global__ void dist_full_kernel(DistInputs in, double* err) {
-  const int64_t n = in.P * in.G;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / in.G, g = i - (i / in.G) * in.G;
-    err[i] = err_exact(in, p, g);
+// Full error matrix.  Errors are clipped at 10, and of a matrix over prior
+// draws most are: a block first evaluates its kFullTile x kFullTile pairs in
+// FP32 (two FMAs per term, as dist_fast_kernel) and writes 10 where that is
+// certain; only the other pairs are computed in FP64, whose narrow pipe took
+// the whole 0.97 ms for 3,001 x 500 pairs of 53 statistics (FULL_MS with 0.4 % below
+// the clip; all of them below it cost FULL_WORST).
+// Certain: K e32 > K sure.  With finite operands |e32 - e| <= B(e) =
+// 1.5 u (64 sqrt(e) + (K + 8) e) (distance.cuh), so e <= 10 implies e32 <= 10 + B(10), and
+// sure is 10 + 2 B(10).  An operand that is not finite in FP32 becomes
+// NaN, which no comparison holds for, so its pairs are computed in FP64.
+constexpr int kFullTile = 64, kFullKc = 16;
+__device__ __forceinline__ float finite_or_nan(float x) { return fabsf(x) < INFINITY ? x : __int_as_float(0x7fc00000); }
+
+__global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const float* __restrict__ sw,
+                                                        const float* __restrict__ dw, float sure, double* err) {
+  __shared__ float ss[kFullKc][kFullTile + 1], sa[kFullKc][kFullTile + 1], sd[kFullKc][kFullTile + 1];
+  __shared__ unsigned short todo[kFullTile * kFullTile];
+  __shared__ int n_todo;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31;
+  const int64_t g0 = (int64_t)blockIdx.x * kFullTile;
+  if (threadIdx.x == 0) n_todo = 0;
+  for (int64_t p0 = (int64_t)blockIdx.y * kFullTile; p0 < in.P; p0 += (int64_t)gridDim.y * kFullTile) {
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    for (int k0 = 0; k0 < in.K; k0 += kFullKc) {
+      __syncthreads();
+      for (int q = threadIdx.x; q < kFullKc * kFullTile; q += 256) {
+        const int r = q / kFullKc, kk = q - r * kFullKc, k = k0 + kk;
+        const int64_t p = p0 + r, g = g0 + r;
+        float s = 0.0f, a = 0.0f, d = 0.0f;
+        if (k < in.K) {
+          if (p < in.P) s = finite_or_nan(rn32_bits(in.stats[p * in.K + k]));
+          if (g < in.G) {
+            a = finite_or_nan(sw[g * in.K + k]);
+            d = finite_or_nan(dw[g * in.K + k]);
+          }
+        }
+        ss[kk][r] = s;
+        sa[kk][r] = a;
+        sd[kk][r] = d;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int kk = 0; kk < kFullKc; ++kk) {
+        float s[4], a[4], d[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          s[i] = ss[kk][ty + 16 * i];
+          a[i] = sa[kk][tx + 16 * i];
+          d[i] = sd[kk][tx + 16 * i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float t = fmaf(-a[j], s[i], d[j]);
+            acc[i][j] = fmaf(t, t, acc[i][j]);
+          }
+      }
+    }
+    const float limit = sure * (float)in.K;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int r = ty + 16 * i, c = tx + 16 * j;
+        const bool real = p0 + r < in.P && g0 + c < in.G;
+        const bool clip = acc[i][j] > limit;
+        if (real && clip) err[(p0 + r) * in.G + g0 + c] = 10.0;
+        const unsigned m = __ballot_sync(0xffffffffu, real && !clip);
+        int base = 0;
+        if (lane == 0 && m) base = atomicAdd(&n_todo, __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (real && !clip) todo[base + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(r * kFullTile + c);
+      }
+    __syncthreads();
+    const int n = n_todo;
+    for (int q = threadIdx.x; q < n; q += 256) {
+      const int64_t p = p0 + todo[q] / kFullTile, g = g0 + todo[q] % kFullTile;
+      err[p * in.G + g] = err_exact(in, p, g);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) n_todo = 0;
   }
 }
 
-cudaError_t launch_dist_full(const DistInputs& in, double* err, cudaStream_t s) {
-  const int64_t n = in.P * in.G;
-  if (n <= 0) return cudaSuccess;
-  int blocks = (int)((n + 255) / 256 < 65536 ? (n + 255) / 256 : 65536);
-  dist_full_kernel<<<blocks, 256, 0, s>>>(in, err);
+cudaError_t launch_dist_full(const DistInputs& in, float* sw, float* dw, double* err, cudaStream_t s) {
+  if (in.P <= 0 || in.G <= 0) return cudaSuccess;
+  cudaError_t e = launch_dist_prep(in, sw, dw, nullptr, 0, 1, s);
+  if (e) return e;
+  const float sure = 10.0f + 2.0f * dist_bound_f(10.0f, in.K);
+  const int64_t py = (in.P + kFullTile - 1) / kFullTile;
+  dim3 grid((unsigned)((in.G + kFullTile - 1) / kFullTile), (unsigned)(py < 65535 ? py : 65535));
+  dist_full_kernel<<<grid, 256, 0, s>>>(in, sw, dw, sure, err);
   return cudaGetLastError();
 }
 

@@ -172,8 +172,8 @@ cudaError_t launch_scan(const int64_t* cnt, int64_t G, int64_t* off, cudaStream_
 // in.rden.  sp, sg: n scratch entries each.
 cudaError_t launch_accepted_errors(const DistInputs& in, const int64_t* aoff, const int64_t* idx, int64_t G,
                                    int64_t p_base, int64_t n, int32_t* sp, int32_t* sg, double* err, cudaStream_t s);
-// full FP64 error matrix [P][G]
-cudaError_t launch_dist_full(const DistInputs& in, double* err, cudaStream_t s);
+// full FP64 error matrix [P][G]; sw, dw: G x K scratch values each
+cudaError_t launch_dist_full(const DistInputs& in, float* sw, float* dw, double* err, cudaStream_t s);
 
 // moment ODE (moment.cu)
 struct MomArgs {
@@ -212,7 +212,12 @@ struct DataStatsArgs {
   int n_boot;
   uint64_t seed;
   double* out;                // [G][n_boot + 1][K]
+  unsigned long long* sums;   // data_stats_scratch bytes
+  int* invalid;               // set when a count lies outside [0, 2^20]
 };
+// bytes of the group sums of the (gene, resample) pairs processed at a time,
+// and of the reciprocals of the sample sizes
+size_t data_stats_scratch(const DevCfg& cfg, int64_t G, int n_boot, int64_t C);
 cudaError_t launch_data_stats(const DataStatsArgs& a, double* se, cudaStream_t s);
 // cells that fit the per-gene shared-memory table of launch_data_stats
 int64_t data_stats_max_cells(int n_ages, int n_conds);
