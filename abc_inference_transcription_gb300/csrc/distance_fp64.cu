@@ -84,10 +84,13 @@ __device__ __forceinline__ double err_exact(const DistInputs& in, int64_t p, int
     const double rK = 1.0 / nK;
     for (int f = 0; f < in.n_fam; ++f) {
       double part = 0.0;
-      for (int q = 0; q < in.fam[f]; ++q, ++k) {
-        const double diff = d[k] - s[k];
-        part = part + div_rn(diff * diff, dn[k], ry[k]);
+      // unrolled for the loads of the next terms beside the chain of additions
+#pragma unroll 4
+      for (int q = 0; q < in.fam[f]; ++q) {
+        const double diff = __ldg(d + k + q) - __ldg(s + k + q);
+        part = part + div_rn(diff * diff, __ldg(dn + k + q), __ldg(ry + k + q));
       }
+      k += in.fam[f];
       tot = tot + div_rn(part, nK, rK);
     }
   } else {
@@ -412,30 +415,31 @@ __global__ void run_sort_kernel(const int32_t* sg, const int64_t* goff, const ui
 }
 
 // Full error matrix.  Errors are clipped at 10, and of a matrix over prior
-// draws most are: a block first evaluates its kFullTile x kFullTile pairs in
+// draws most are: a block first evaluates its kFullRows x kFullTile pairs in
 // FP32 (two FMAs per term, as dist_fast_kernel) and writes 10 where that is
 // certain; only the other pairs are computed in FP64, whose narrow pipe took
-// the whole 0.97 ms for 3,001 x 500 pairs of 53 statistics (FULL_MS with 0.4 % below
-// the clip; all of them below it cost FULL_WORST).
+// the whole 0.97 ms for 3,001 x 500 pairs of 53 statistics (0.08 with 0.4 %
+// of them below the clip; with all of them below it, as before).  32 particles
+// per block, so that such an input still fills the GPU evenly.
 // Certain: K e32 > K sure.  With finite operands |e32 - e| <= B(e) =
 // 1.5 u (64 sqrt(e) + (K + 8) e) (distance.cuh), so e <= 10 implies e32 <= 10 + B(10), and
 // sure is 10 + 2 B(10).  An operand that is not finite in FP32 becomes
 // NaN, which no comparison holds for, so its pairs are computed in FP64.
-constexpr int kFullTile = 64, kFullKc = 16;
+constexpr int kFullTile = 64, kFullRows = 32, kFullKc = 16;  // genes, particles, statistics
 __device__ __forceinline__ float finite_or_nan(float x) { return fabsf(x) < INFINITY ? x : __int_as_float(0x7fc00000); }
 
 __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const float* __restrict__ sw,
                                                         const float* __restrict__ dw, float sure, double* err) {
-  __shared__ float ss[kFullKc][kFullTile + 1], sa[kFullKc][kFullTile + 1], sd[kFullKc][kFullTile + 1];
-  __shared__ unsigned short todo[kFullTile * kFullTile];
+  __shared__ float ss[kFullKc][kFullRows + 1], sa[kFullKc][kFullTile + 1], sd[kFullKc][kFullTile + 1];
+  __shared__ unsigned short todo[kFullRows * kFullTile];
   __shared__ int n_todo;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31;
   const int64_t g0 = (int64_t)blockIdx.x * kFullTile;
   if (threadIdx.x == 0) n_todo = 0;
-  for (int64_t p0 = (int64_t)blockIdx.y * kFullTile; p0 < in.P; p0 += (int64_t)gridDim.y * kFullTile) {
-    float acc[4][4];
+  for (int64_t p0 = (int64_t)blockIdx.y * kFullRows; p0 < in.P; p0 += (int64_t)gridDim.y * kFullRows) {
+    float acc[2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
     for (int k0 = 0; k0 < in.K; k0 += kFullKc) {
@@ -445,28 +449,29 @@ __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const flo
         const int64_t p = p0 + r, g = g0 + r;
         float s = 0.0f, a = 0.0f, d = 0.0f;
         if (k < in.K) {
-          if (p < in.P) s = finite_or_nan(rn32_bits(in.stats[p * in.K + k]));
+          if (r < kFullRows && p < in.P) s = finite_or_nan(rn32_bits(in.stats[p * in.K + k]));
           if (g < in.G) {
             a = finite_or_nan(sw[g * in.K + k]);
             d = finite_or_nan(dw[g * in.K + k]);
           }
         }
-        ss[kk][r] = s;
+        if (r < kFullRows) ss[kk][r] = s;
         sa[kk][r] = a;
         sd[kk][r] = d;
       }
       __syncthreads();
 #pragma unroll 4
       for (int kk = 0; kk < kFullKc; ++kk) {
-        float s[4], a[4], d[4];
+        float s[2], a[4], d[4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) s[i] = ss[kk][ty + 16 * i];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          s[i] = ss[kk][ty + 16 * i];
           a[i] = sa[kk][tx + 16 * i];
           d[i] = sd[kk][tx + 16 * i];
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float t = fmaf(-a[j], s[i], d[j]);
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const flo
     }
     const float limit = sure * (float)in.K;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int r = ty + 16 * i, c = tx + 16 * j;
@@ -505,7 +510,7 @@ cudaError_t launch_dist_full(const DistInputs& in, float* sw, float* dw, double*
   cudaError_t e = launch_dist_prep(in, sw, dw, nullptr, 0, 1, s);
   if (e) return e;
   const float sure = 10.0f + 2.0f * dist_bound_f(10.0f, in.K);
-  const int64_t py = (in.P + kFullTile - 1) / kFullTile;
+  const int64_t py = (in.P + kFullRows - 1) / kFullRows;
   dim3 grid((unsigned)((in.G + kFullTile - 1) / kFullTile), (unsigned)(py < 65535 ? py : 65535));
   dist_full_kernel<<<grid, 256, 0, s>>>(in, sw, dw, sure, err);
   return cudaGetLastError();
