@@ -29,11 +29,17 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// floor(x n / 2^64) for n < 2^32, from two 32-bit products
+__device__ __forceinline__ uint32_t scaled(uint64_t x, uint32_t n) {
+  const uint64_t hi = (x >> 32) * n, lo = (x & 0xffffffffu) * (uint64_t)n;
+  return (uint32_t)((hi + (lo >> 32)) >> 32);
+}
+
 // positions in [0, n) of draws 2 j and 2 j + 1 of stream (seed, family, resample,
 // gene): floor(x n / 2^52) of 52-bit uniform integers x, in exact integer
 // arithmetic; both come from one Philox block
-__device__ __forceinline__ void draw_pair(uint64_t seed, int fam, int b, int64_t g, int64_t j, int64_t n, int64_t& p0,
-                                          int64_t& p1) {
+__device__ __forceinline__ void draw_pair(uint64_t seed, int fam, int b, int64_t g, int64_t j, int64_t n, uint32_t& p0,
+                                          uint32_t& p1) {
   U4 c;
   c.x = (uint32_t)j;
   c.y = ((uint32_t)((uint64_t)j >> 32) & 0x3fffffffu) | (ST_AUX << 30);
@@ -41,19 +47,13 @@ __device__ __forceinline__ void draw_pair(uint64_t seed, int fam, int b, int64_t
   c.w = (uint32_t)g;
   const U4 o = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
   const uint64_t x0 = ((uint64_t)o.x << 20) | (uint64_t)(o.y >> 12), x1 = ((uint64_t)o.z << 20) | (uint64_t)(o.w >> 12);
-  p0 = (int64_t)__umul64hi(x0 << 12, (uint64_t)n);
-  p1 = (int64_t)__umul64hi(x1 << 12, (uint64_t)n);
+  p0 = scaled(x0 << 12, (uint32_t)n);
+  p1 = scaled(x1 << 12, (uint32_t)n);
 }
 
-// exact sample variance / covariance from integer sums: (n sxy - sx sy) / (n (n - 1))
-__device__ __forceinline__ double sample_cov(unsigned long long n, unsigned long long sx, unsigned long long sy,
-                                             unsigned long long sxy) {
-  const __int128 num = (__int128)n * (__int128)sxy - (__int128)sx * (__int128)sy;
-  return i128_to_double(num) / ((double)n * (double)(n - 1));
-}
-
-// the same with the denominator d2 = n (n - 1) and r2 = RN(1 / d2) given: the
-// quotient through div_rn (correctly rounded, equal to the IEEE division)
+// exact sample variance / covariance from integer sums, (n sxy - sx sy) /
+// (n (n - 1)), with the denominator d2 and r2 = RN(1 / d2) given: the quotient
+// through div_rn (correctly rounded, equal to the IEEE division)
 __device__ __forceinline__ double sample_cov_r(unsigned long long n, unsigned long long sx, unsigned long long sy,
                                                unsigned long long sxy, double d2, double r2) {
   const __int128 num = (__int128)n * (__int128)sxy - (__int128)sx * (__int128)sy;
@@ -69,15 +69,11 @@ __device__ __forceinline__ double sample_cov_r(unsigned long long n, unsigned lo
 // age) group add count x (1, u, l, u^2, l^2, u l) over its cells, which are
 // contiguous, in registers, and join with shuffles.  Six sums per draw through
 // shared-memory atomics took 3.15 ms for 2,000 genes x 2,000 cells x 100
-// resamples, this takes SUMS_MS: the draws' Philox blocks (two draws each) are
+// resamples, this takes 2.1: the draws' Philox blocks (two draws each) are
 // what is left.  Integer sums: the order does not matter.  The pulse and the
 // chase draws share the counters of one pass unless both use the same cells.
 constexpr size_t data_stats_smem_limit() { return 227 * 1024; }
 constexpr int kMaxCount = 1 << 20;  // abc_data_stats' limit of a count
-
-struct Sums6 {
-  unsigned long long v[6];
-};
 
 // lanes per group: the largest power of two with groups x lanes <= kThreads, at most 32
 __device__ __forceinline__ int group_lanes(int groups) {
@@ -86,42 +82,54 @@ __device__ __forceinline__ int group_lanes(int groups) {
   return L;
 }
 
-// threads 0 .. groups * L - 1: the sums of cells [i0, i1) with counter offsets, joined over L lanes
-template <bool PAIR>
-__device__ __forceinline__ Sums6 group_sums(const int2* T, const unsigned short* mult, int64_t i0, int64_t i1, int sub,
-                                            int L, bool one) {
-  Sums6 s = {{0, 0, 0, 0, 0, 0}};
-  for (int64_t i = i0 + sub; i < i1; i += L) {
-    const unsigned long long m = one ? 1u : mult[i];
+// threads 0 .. groups * L - 1: the sums of cells [i0, i1), joined over L lanes.
+// U: 32-bit where no sum of the gene can reach 2^32 (counts up to 732 with
+// 2,000 cells), 64-bit otherwise.
+template <bool PAIR, typename U>
+__device__ __forceinline__ void group_sums(const int2* T, const unsigned short* mult, int i0, int i1, int sub, int L,
+                                           bool one, bool store, unsigned long long* out) {
+  U v[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = i0 + sub; i < i1; i += L) {
+    const U m = one ? 1u : mult[i];
     const int2 t = T[i];
-    const unsigned long long u = (unsigned)t.x, l = (unsigned)t.y;
+    const U u = (unsigned)t.x, l = (unsigned)t.y;
+    v[0] += m;
     if (PAIR) {
-      s.v[0] += m;
-      s.v[1] += m * u;
-      s.v[2] += m * l;
-      s.v[3] += m * (u * u);
-      s.v[4] += m * (l * l);
-      s.v[5] += m * (u * l);
+      const U mu = m * u, ml = m * l;
+      v[1] += mu;
+      v[2] += ml;
+      v[3] += mu * u;
+      v[4] += ml * l;
+      v[5] += mu * l;
     } else {
-      const unsigned long long x = u + l;
-      s.v[0] += m;
-      s.v[1] += m * x;
-      s.v[2] += m * (x * x);
+      const U x = u + l, mx = m * x;
+      v[1] += mx;
+      v[2] += mx * x;
     }
   }
   for (int o = L >> 1; o > 0; o >>= 1)
 #pragma unroll
-    for (int q = 0; q < (PAIR ? 6 : 3); ++q) s.v[q] += __shfl_xor_sync(0xffffffffu, s.v[q], o);
-  return s;
+    for (int q = 0; q < (PAIR ? 6 : 3); ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  if (store)
+    for (int q = 0; q < (PAIR ? 6 : 3); ++q) out[q] = v[q];
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void group_sums_any(bool narrow, const int2* T, const unsigned short* mult, int i0, int i1,
+                                               int sub, int L, bool one, bool store, unsigned long long* out) {
+  if (narrow)
+    group_sums<PAIR, unsigned>(T, mult, i0, i1, sub, L, one, store, out);
+  else
+    group_sums<PAIR, unsigned long long>(T, mult, i0, i1, sub, L, one, store, out);
 }
 
 __device__ __forceinline__ void count_draws(const DataStatsArgs& a, unsigned* words, int fam, int b, int64_t g,
                                             int64_t base, int64_t n) {
   for (int64_t j = threadIdx.x; 2 * j < n; j += blockDim.x) {
-    int64_t p0, p1;
+    uint32_t p0, p1;
     draw_pair(a.seed, fam, b, g, j, n, p0, p1);
-    p0 += base;
-    p1 += base;
+    p0 += (uint32_t)base;
+    p1 += (uint32_t)base;
     // counters reach at most the number of draws, below 2^16 (data_stats_max_cells)
     atomicAdd(&words[p0 >> 1], 1u << ((p0 & 1) * 16));
     if (2 * j + 1 < n) atomicAdd(&words[p1 >> 1], 1u << ((p1 & 1) * 16));
@@ -140,12 +148,17 @@ __global__ void __launch_bounds__(kThreads) data_sums_kernel(DataStatsArgs a, in
   const int32_t* u = a.u + g * C;
   const int32_t* l = a.l + g * C;
   bool bad = false;
+  unsigned most = 0;
   for (int64_t i = threadIdx.x; i < C; i += blockDim.x) {
     const int64_t id = a.cell_id[i];
     T[i] = make_int2(u[id], l[id]);
-    bad = bad || (unsigned)T[i].x > (unsigned)kMaxCount || (unsigned)T[i].y > (unsigned)kMaxCount;
+    const unsigned x = max((unsigned)T[i].x, (unsigned)T[i].y);
+    bad = bad || x > (unsigned)kMaxCount;
+    most = max(most, min(x, 1u << 20));
   }
   if (bad) *a.invalid = 1;
+  // the largest sum: C draws of a cell with (u + l)^2 <= 4 most^2
+  const bool narrow = __syncthreads_and(4ull * (unsigned long long)C * most * most < (1ull << 32)) != 0;
   const int cp = a.cfg.pulse_stat, cc = a.cfg.chase_stat;
   const int L2 = group_lanes(J * A), L1 = group_lanes(2 * A);
   for (int b = blockIdx.y; b <= a.n_boot; b += gridDim.y) {
@@ -166,10 +179,8 @@ __global__ void __launch_bounds__(kThreads) data_sums_kernel(DataStatsArgs a, in
       const int grp = threadIdx.x / L1, f = grp / A, ag = grp - f * A;
       const bool mine = grp < 2 * A && f >= f0 && f < f1;
       const int gi = mine ? (f == 0 ? cp : cc) * A + ag : 0;
-      const Sums6 s = group_sums<false>(T, mult, mine ? a.gstart[gi] : 0, mine ? a.gstart[gi + 1] : 0,
-                                        threadIdx.x % L1, L1, b == 0);
-      if (mine && threadIdx.x % L1 == 0)
-        for (int q = 0; q < 3; ++q) out[3 * grp + q] = s.v[q];
+      group_sums_any<false>(narrow, T, mult, mine ? a.gstart[gi] : 0, mine ? a.gstart[gi + 1] : 0, threadIdx.x % L1, L1,
+                            b == 0, mine && threadIdx.x % L1 == 0, out + 3 * grp);
     }
     // all cells: per (condition, age) (n, su, sl, suu, sll, sul)
     __syncthreads();
@@ -179,10 +190,8 @@ __global__ void __launch_bounds__(kThreads) data_sums_kernel(DataStatsArgs a, in
     __syncthreads();
     const int grp = threadIdx.x / L2;
     const bool mine = grp < J * A;
-    const Sums6 s = group_sums<true>(T, mult, mine ? a.gstart[grp] : 0, mine ? a.gstart[grp + 1] : 0,
-                                     threadIdx.x % L2, L2, b == 0);
-    if (mine && threadIdx.x % L2 == 0)
-      for (int q = 0; q < 6; ++q) out[6 * A + 6 * grp + q] = s.v[q];
+    group_sums_any<true>(narrow, T, mult, mine ? a.gstart[grp] : 0, mine ? a.gstart[grp + 1] : 0, threadIdx.x % L2, L2,
+                         b == 0, mine && threadIdx.x % L2 == 0, out + 6 * A + 6 * grp);
   }
 }
 
@@ -198,24 +207,29 @@ __global__ void data_recip_kernel(int64_t C, double2* recip) {
 // a / b for b > 0 given y = RN(1 / b): div_rn, and 0 without its slow path
 __device__ __forceinline__ double div_pos(double a, double b, double y) { return a == 0.0 ? a : div_rn(a, b, y); }
 
-// Phase 2, one thread per (gene, resample, item): items 0..2A-1 are the mean
-// and Fano factor of one (family, age) cell, items 2A..2A+J-1 the ratio,
-// mean_corr and corr_mean of one condition.
+// Phase 2, one thread per (gene, resample, item), bound by the FP64 pipe.  First
+// come the items of the conditions (ratio, mean_corr and corr_mean of condition
+// it), then those of the (family, age) cells (mean and Fano factor): with both
+// kinds in a warp each lane waited for the other's branch (3.2 ms against
+// 1.7 for 2,000 genes x 101 resamples).
 __global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const unsigned long long* S_in,
                                   const double2* __restrict__ recip) {
   const int A = a.cfg.n_ages, J = a.cfg.n_conds, K = 4 * A + 3 * J;
   const int nsum = 6 * A + 6 * J * A;
-  const int items = 2 * A + J;
-  const int64_t total = ng * (a.n_boot + 1) * items;
+  const int64_t sets = ng * (a.n_boot + 1);
+  const int64_t total = sets * (2 * A + J);
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t gb = t / items;  // (gene - g0) * (n_boot + 1) + resample
-    const int it = (int)(t - gb * items);
+    const bool cell = t >= sets * J;
+    const int64_t q = cell ? t - sets * J : t;
+    const int per = cell ? 2 * A : J;
+    const int64_t gb = q / per;  // (gene - g0) * (n_boot + 1) + resample
+    const int it = (int)(q - gb * per);
     const int b = (int)(gb % (a.n_boot + 1));
     const unsigned long long* Sp = S_in + gb * nsum;
     const unsigned long long* Sc = Sp + 3 * A;
     const unsigned long long* Sg = Sc + 3 * A;
     double* st = a.out + (g0 * (int64_t)(a.n_boot + 1) + gb) * K;
-    if (it < 2 * A) {
+    if (cell) {
       // mean and Fano factor of u + l per age cluster (get_mean_ccp_data, get_ff_ccp_data)
       const int f = it / A, ag = it - (it / A) * A;
       const unsigned long long* S = f == 0 ? Sp : Sc;
@@ -223,8 +237,10 @@ __global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const
       const unsigned long long n = S[3 * ag];
       double m = 0.0, ff = 0.0;
       if (n > 0) {
-        m = (double)S[3 * ag + 1] / (double)n;
-        const double v = sample_cov(n, S[3 * ag + 1], S[3 * ag + 1], S[3 * ag + 2]);
+        const double2 r = recip[n];
+        const double nd = (double)n;
+        m = div_pos((double)S[3 * ag + 1], nd, r.x);
+        const double v = sample_cov_r(n, S[3 * ag + 1], S[3 * ag + 1], S[3 * ag + 2], nd * (double)(n - 1), r.y);
         const double eps = (m == 0.0) ? 0.0001 : 0.0;
         ff = v / (m + eps);
       }
@@ -232,7 +248,7 @@ __global__ void data_stats_kernel(DataStatsArgs a, int64_t g0, int64_t ng, const
       st[off + A + ag] = ff;
       continue;
     }
-    const int j = it - 2 * A;
+    const int j = it;
     double m1[kMaxAges], m2[kMaxAges], v1[kMaxAges], v2[kMaxAges], c12[kMaxAges], w[kMaxAges];
     unsigned long long nj = 0, suj = 0, slj = 0;
     for (int ag = 0; ag < A; ++ag) {
@@ -309,11 +325,12 @@ int64_t data_stats_max_cells(int n_ages, int n_conds) {
          (int64_t)(sizeof(int2) + sizeof(unsigned short));
 }
 
-// the sums of at most ~256 MB of (gene, resample) pairs at a time
+// the sums of at most ~64 MB of (gene, resample) pairs at a time: they stay in
+// L2 between the phases
 static int64_t genes_at_a_time(const DevCfg& cfg, int64_t G, int n_boot, int64_t* per_gene) {
   const int64_t nsum = 6 * cfg.n_ages + 6 * cfg.n_conds * cfg.n_ages;
   *per_gene = (int64_t)(n_boot + 1) * nsum * (int64_t)sizeof(unsigned long long);
-  return std::max<int64_t>(1, std::min<int64_t>(G, ((int64_t)256 << 20) / *per_gene));
+  return std::max<int64_t>(1, std::min<int64_t>(G, ((int64_t)64 << 20) / *per_gene));
 }
 
 size_t data_stats_scratch(const DevCfg& cfg, int64_t G, int n_boot, int64_t C) {

@@ -101,3 +101,43 @@ def test_data_stats_gpu_bit_exact(built, orc):
     assert np.array_equal(st, want_st, equal_nan=True)
     assert np.array_equal(se, want_se, equal_nan=True)
     assert np.array_equal(st0, want_st, equal_nan=True) and se0 is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("per_pulse,n_ages,most,same,n_boot", [(10, 5, 3, False, 2), (11, 1, 700, False, 3),
+                                                               (200, 5, 40000, False, 2), (33, 8, 1 << 20, True, 4),
+                                                               (10, 2, 50, True, 0)])
+def test_data_stats_gpu_layouts_and_count_ranges(built, orc, per_pulse, n_ages, most, same, n_boot):
+    """Odd and even cell counts, one to eight age groups, 32- and 64-bit sums, the
+    pulse and chase statistics of one condition; counts outside the range are refused."""
+    from abc_inference_transcription_gb300 import abi
+    from abc_inference_transcription_gb300.host import Context
+    cfg = make_config("hour")
+    cfg.n_ages = n_ages
+    for a in range(n_ages):
+        cfg.ages[a] = (2 * a + 1) / (2 * n_ages) * cfg.cycle
+    if same:
+        cfg.chase_stat_cond = cfg.pulse_stat_cond
+    cells = synthetic_cells(n_per_pulse=max(per_pulse, 2 * n_ages), n_per_chase=max(per_pulse - 1, 2 * n_ages),
+                            n_ages=n_ages, seed=per_pulse)
+    rng = np.random.default_rng(most)
+    G, C = 7, cells.cond.shape[0]
+    u = rng.integers(0, most + 1, (G, C)).astype(np.int32)
+    l = (rng.integers(0, most + 1, (G, C)) * (rng.random((G, C)) < 0.3)).astype(np.int32)
+    u[0] = 0
+    l[1] = 0
+    u[2], l[2] = most, most
+    with Context(cfg, cells) as ctx:
+        got = ctx.data_stats(u, l, n_boot=n_boot, seed=11)
+        want = orc.data_stats(cfg, cells, u, l, n_boot=n_boot, seed=11)
+        assert np.array_equal(got[0], want[0], equal_nan=True)
+        assert (got[1] is None) == (want[1] is None)
+        if got[1] is not None:
+            assert np.array_equal(got[1], want[1], equal_nan=True)
+        for value in (-1, (1 << 20) + 1):
+            bad = u.copy()
+            bad[-1, -1] = value
+            with pytest.raises(abi.AbcError):
+                ctx.data_stats(bad, l, n_boot=n_boot)
+            with pytest.raises(abi.AbcError):
+                ctx.data_stats(u, bad, n_boot=n_boot)
