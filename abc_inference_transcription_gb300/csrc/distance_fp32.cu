@@ -1,33 +1,43 @@
 // distance_fp32.cu — FP32 particle x gene distance with a fused epilogue
 // (candidate emission or subsample export) and the per-gene threshold pass.
 // The P x G error matrix is never written in full.
+#include <atomic>
+
 #include "distance.cuh"
 #include "kernels.h"
+#include "smem_attr.h"
 
 namespace abc {
 
 // 256 threads = 16 x 16; thread (tx, ty) owns particles ty + 16 i and genes
 // tx + 16 j (i, j < 8) of a 128 x 128 tile.  Statistics stream through shared
 // memory kDistKc at a time, stored k-major so one row serves all threads.
+//
+// GJ genes per thread: 8, or 1 (a tile of 16 genes) for few genes, where the
+// wide tile computes mostly padding (32,768 rows x 4 genes of 53 statistics: 35 us wide, 14
+// narrow).  The rows are padded by one word: without it the 16 statistics of a
+// row go to one bank.
+template <int GJ>
 __global__ void __launch_bounds__(256) dist_fast_kernel(const float* __restrict__ s32,
                                                         const float* __restrict__ sw,
                                                         const float* __restrict__ dw, int64_t P, int64_t G,
                                                         int K, const float* __restrict__ X, Cand* cand,
                                                         float* cand_e, unsigned long long* n_cand, int64_t cap,
                                                         float* esub, int64_t stride, int64_t n_sub) {
-  __shared__ float ss[kDistKc][kDistTile];
-  __shared__ float sa[kDistKc][kDistTile];
-  __shared__ float sd[kDistKc][kDistTile];
+  constexpr int kGenes = 16 * GJ;
+  __shared__ float ss[kDistKc][kDistTile + 1];
+  __shared__ float sa[kDistKc][kGenes + 1];
+  __shared__ float sd[kDistKc][kGenes + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t g0 = (int64_t)blockIdx.x * kDistTile;
+  const int64_t g0 = (int64_t)blockIdx.x * kGenes;
   const int64_t r0 = (int64_t)blockIdx.y * kDistTile;  // row = particle (emit) or subsample row
   const bool sample = esub != nullptr;
   const int64_t nrows = sample ? n_sub : P;
-  float acc[8][8];
+  float acc[8][GJ];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    for (int j = 0; j < GJ; ++j) acc[i][j] = 0.0f;
 
   for (int k0 = 0; k0 < K; k0 += kDistKc) {
     // cooperative loads: 128 rows x kDistKc values for each of the three tiles
@@ -41,6 +51,7 @@ __global__ void __launch_bounds__(256) dist_fast_kernel(const float* __restrict_
         sv = s32[p * K + k];
       }
       ss[kk][r] = sv;
+      if (r >= kGenes) continue;
       const int64_t g = g0 + r;
       float av = 0.0f, dv = 0.0f;
       if (g < G && k < K) {
@@ -54,18 +65,18 @@ __global__ void __launch_bounds__(256) dist_fast_kernel(const float* __restrict_
     const int kc = (K - k0) < kDistKc ? (K - k0) : kDistKc;
 #pragma unroll 4
     for (int kk = 0; kk < kc; ++kk) {
-      float s[8], a[8], d[8];
+      float s[8], a[GJ], d[GJ];
 #pragma unroll
       for (int i = 0; i < 8; ++i) s[i] = ss[kk][ty + 16 * i];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < GJ; ++j) {
         a[j] = sa[kk][tx + 16 * j];
         d[j] = sd[kk][tx + 16 * j];
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < GJ; ++j) {
           float t = fmaf(-a[j], s[i], d[j]);
           acc[i][j] = fmaf(t, t, acc[i][j]);
         }
@@ -78,7 +89,7 @@ __global__ void __launch_bounds__(256) dist_fast_kernel(const float* __restrict_
     const int64_t row = r0 + ty + 16 * i;
     if (row >= nrows) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < GJ; ++j) {
       const int64_t g = g0 + tx + 16 * j;
       if (g >= G) continue;
       float e = fminf(acc[i][j] * invK, 10.0f);
@@ -104,75 +115,128 @@ cudaError_t launch_dist_fast(const float* s32, const float* sw, const float* dw,
                              float* esub, int64_t stride, int64_t n_sub, cudaStream_t s) {
   const int64_t rows = esub ? n_sub : P;
   if (rows <= 0 || G <= 0) return cudaSuccess;
-  dim3 grid((unsigned)((G + kDistTile - 1) / kDistTile), (unsigned)((rows + kDistTile - 1) / kDistTile));
-  dist_fast_kernel<<<grid, 256, 0, s>>>(s32, sw, dw, P, G, K, X, cand, cand_e, n_cand, cap, esub, stride, n_sub);
+  const int genes = G <= 32 ? 16 : kDistTile;
+  dim3 grid((unsigned)((G + genes - 1) / genes), (unsigned)((rows + kDistTile - 1) / kDistTile));
+  if (genes == 16)
+    dist_fast_kernel<1><<<grid, 256, 0, s>>>(s32, sw, dw, P, G, K, X, cand, cand_e, n_cand, cap, esub, stride, n_sub);
+  else
+    dist_fast_kernel<8><<<grid, 256, 0, s>>>(s32, sw, dw, P, G, K, X, cand, cand_e, n_cand, cap, esub, stride, n_sub);
   return cudaGetLastError();
 }
 
 // Cumulative histogram search shared by the threshold and refinement kernels:
 // the first bin at which the running count of hist[0..kHistBins) reaches k
-// (-1 if it never does).  One CTA of 256 threads; csum is 256 words of shared memory.
+// (-1 if it never does).  Called by every thread of a CTA of at least 256;
+// csum is 256 words of shared memory.  The first warp scans the 256 partial
+// counts by shuffles and one lane walks the 128 bins that hold the answer.
 __device__ int hist_find(const unsigned int* hist, int64_t k, unsigned int* csum) {
-  const int per = kHistBins / 256;
-  unsigned int local = 0;
-  for (int b = 0; b < per; ++b) local += hist[threadIdx.x * per + b];
-  csum[threadIdx.x] = local;
+  constexpr int per = kHistBins / 256;
+  if (threadIdx.x < 256) {
+    unsigned int local = 0;
+#pragma unroll
+    for (int b = 0; b < per; ++b) local += hist[threadIdx.x * per + b];
+    csum[threadIdx.x] = local;
+  }
   __syncthreads();
   int found = -1;
-  if (threadIdx.x == 0) {
-    unsigned long long run = 0;
-    for (int t = 0; t < 256 && found < 0; ++t) {
-      if (run + csum[t] >= (unsigned long long)k) {
-        for (int b = 0; b < per; ++b) {
-          run += hist[t * per + b];
-          if (run >= (unsigned long long)k) {
-            found = t * per + b;
-            break;
-          }
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    unsigned long long own = 0;
+    for (int b = 0; b < 8; ++b) own += csum[lane * 8 + b];
+    unsigned long long run = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += v;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, run >= (unsigned long long)k);
+    if (m && lane == __ffs(m) - 1) {
+      run -= own;
+      for (int c = lane * 8; found < 0; ++c) {
+        if (run + csum[c] < (unsigned long long)k) {
+          run += csum[c];
+          continue;
         }
-      } else {
-        run += csum[t];
+        for (int b = 0; found < 0; ++b) {
+          run += hist[c * per + b];
+          if (run >= (unsigned long long)k) found = c * per + b;
+        }
       }
     }
+    if (m) found = __shfl_sync(0xffffffffu, found, __ffs(m) - 1);
   }
-  return found;  // meaningful in thread 0
+  return found;  // meaningful in the first warp
 }
 
-// One CTA per gene: histogram of the subsample errors on a sqrt scale, then
-// the bin where the running count reaches k_sub gives X[g] (its upper edge
-// widened by twice the error bound b0_g + b1 e of the candidate pass).
-__global__ void __launch_bounds__(256) dist_threshold_kernel(const float* __restrict__ esub, int64_t n_sub,
-                                                             int64_t G, int64_t k_sub, const float* b0, float b1,
-                                                             float* X) {
-  __shared__ unsigned int hist[kHistBins];
+// Histogram of the subsample errors of GB neighbouring genes per CTA on a sqrt
+// scale, then per gene the bin where the running count reaches k_sub gives X[g]
+// (its upper edge widened by twice the error bound b0_g + b1 e of the candidate
+// pass).  The errors lie row by row, so eight genes at a time read whole 32-byte
+// sectors; the last bin, where almost all of them fall (the clip), is counted in
+// registers instead of by atomics on one word.  32,768 rows: 2,000 genes 0.32
+// ms with a CTA of 256 threads per gene, 0.093 now; 4 genes 80 us, 10 now.
+__global__ void __launch_bounds__(1024) dist_threshold_kernel(const float* __restrict__ esub, int64_t n_sub,
+                                                              int64_t G, int64_t k_sub, int log_gb, const float* b0,
+                                                              float b1, float* X) {
+  extern __shared__ unsigned int hist[];  // GB x kHistBins
   __shared__ unsigned int csum[256];
-  const int64_t g = blockIdx.x;
-  for (int b = threadIdx.x; b < kHistBins; b += blockDim.x) hist[b] = 0u;
+  const int GB = 1 << log_gb;
+  const int64_t g0 = (int64_t)blockIdx.x * GB;
+  for (int b = threadIdx.x; b < GB * kHistBins; b += blockDim.x) hist[b] = 0u;
   __syncthreads();
-  for (int64_t r = threadIdx.x; r < n_sub; r += blockDim.x) {
-    float e = esub[r * G + g];
-    if (e == e) atomicAdd(&hist[hist_bin(e)], 1u);
+  const int j = threadIdx.x & (GB - 1);
+  unsigned int last = 0;
+  if (g0 + j < G) {
+    unsigned int* h = hist + j * kHistBins;
+    const int64_t step = blockDim.x >> log_gb;
+    constexpr int kAhead = 16;  // loads in flight per thread
+    for (int64_t r0 = threadIdx.x >> log_gb; r0 < n_sub; r0 += kAhead * step) {
+      float e[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int64_t r = r0 + u * step;
+        e[u] = r < n_sub ? __ldg(esub + r * G + g0 + j) : __int_as_float(0x7fc00000);
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        if (e[u] >= 10.0f)  // the clip: the last bin
+          ++last;
+        else if (e[u] == e[u])
+          atomicAdd(&h[hist_bin(e[u])], 1u);
+      }
+    }
+    if (last) atomicAdd(&h[kHistBins - 1], last);
   }
   __syncthreads();
-  const int found = hist_find(hist, k_sub, csum);
-  if (threadIdx.x == 0) {
-    float x;
-    if (found < 0 || k_sub <= 0) {
-      x = INFINITY;
-    } else {
-      const float bg = b0[g];
-      const float up = hist_upper(found);
-      const float xp = up + 1.01f * (bg + b1 * up);
-      x = xp + 1.01f * (bg + b1 * xp);
+  for (int q = 0; q < GB && g0 + q < G; ++q) {
+    const int found = hist_find(hist + q * kHistBins, k_sub, csum);
+    if (threadIdx.x == 0) {
+      float x;
+      if (found < 0 || k_sub <= 0) {
+        x = INFINITY;
+      } else {
+        const float bg = b0[g0 + q];
+        const float up = hist_upper(found);
+        const float xp = up + 1.01f * (bg + b1 * up);
+        x = xp + 1.01f * (bg + b1 * xp);
+      }
+      X[g0 + q] = x;
     }
-    X[g] = x;
+    __syncthreads();  // csum is rewritten
   }
 }
 
 cudaError_t launch_dist_threshold(const float* esub, int64_t n_sub, int64_t G, int64_t k_sub, const float* b0,
                                   float b1, float* X, cudaStream_t s) {
   if (G <= 0) return cudaSuccess;
-  dist_threshold_kernel<<<(unsigned)G, 256, 0, s>>>(esub, n_sub, G, k_sub, b0, b1, X);
+  // as many genes per CTA as leave every multiprocessor one, at most 8 (128 KB of histograms)
+  int lg = 0;
+  while (lg < 3 && (G >> (lg + 1)) >= 152) ++lg;
+  const size_t smem = ((size_t)sizeof(unsigned int) * kHistBins) << lg;
+  static std::atomic<uint64_t> attr{0};  // devices where the limit is set, shared by all contexts
+  cudaError_t e = set_smem_once(attr, dist_threshold_kernel, (int)(sizeof(unsigned int) * kHistBins * 8));
+  if (e != cudaSuccess) return e;
+  dist_threshold_kernel<<<(unsigned)((G + (1 << lg) - 1) >> lg), 1024, smem, s>>>(esub, n_sub, G, k_sub, lg, b0, b1,
+                                                                                 X);
   return cudaGetLastError();
 }
 
@@ -223,6 +287,24 @@ __global__ void cand_hist_kernel(const Cand* cand, const float* e, int64_t n, un
     const float x = e[i];
     if (x == x) atomicAdd(&hist[(int64_t)cand[i].g * kHistBins + hist_bin(fmaxf(x, 0.0f))], 1u);
   }
+}
+
+// The same with the histograms of all genes in shared memory, for few genes:
+// with 4 of them the candidates' global atomics met on a few thousand words (300,000
+// candidates: 66 us, 14 here).
+constexpr int kSmemHistGenes = 12;  // 192 KB
+__global__ void __launch_bounds__(1024) cand_hist_smem_kernel(const Cand* cand, const float* e, int64_t n, int G,
+                                                              unsigned int* hist) {
+  extern __shared__ unsigned int sh[];  // G x kHistBins
+  for (int b = threadIdx.x; b < G * kHistBins; b += blockDim.x) sh[b] = 0u;
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float x = e[i];
+    if (x == x) atomicAdd(&sh[cand[i].g * kHistBins + hist_bin(fmaxf(x, 0.0f))], 1u);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < G * kHistBins; b += blockDim.x)
+    if (sh[b]) atomicAdd(&hist[b], sh[b]);
 }
 
 // Per gene: when at least k candidates have an FP32 error <= a (the upper edge
@@ -316,7 +398,15 @@ cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int6
   if (e != cudaSuccess) return e;
   if (G <= 0) return cudaSuccess;
   const int blocks = (int)((n + 255) / 256 < 16384 ? (n + 255) / 256 : 16384);
-  if (n > 0) cand_hist_kernel<<<blocks, 256, 0, s>>>(cand, cand_e, n, hist);
+  if (n > 0 && G <= kSmemHistGenes) {
+    static std::atomic<uint64_t> attr{0};
+    e = set_smem_once(attr, cand_hist_smem_kernel, (int)(sizeof(unsigned int) * kHistBins * kSmemHistGenes));
+    if (e != cudaSuccess) return e;
+    const int hb = (int)((n + 8191) / 8192 < 152 ? (n + 8191) / 8192 : 152);
+    cand_hist_smem_kernel<<<hb, 1024, sizeof(unsigned int) * kHistBins * (size_t)G, s>>>(cand, cand_e, n, (int)G, hist);
+  } else if (n > 0) {
+    cand_hist_kernel<<<blocks, 256, 0, s>>>(cand, cand_e, n, hist);
+  }
   refine_kernel<<<(unsigned)G, 256, 0, s>>>(hist, G, k, X, b0, b1, Xt);
   if (n > 0) cand_filter_kernel<<<blocks, 256, 0, s>>>(cand, cand_e, n, Xt, out, count);
   return cudaGetLastError();
@@ -345,10 +435,10 @@ __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restric
                                                           int K, const float* __restrict__ X, float z,
                                                           uint8_t* keep, float* err_out) {
   constexpr int N2 = MODE ? 8 : 1, M2 = MODE ? GJ : 1, kGenes = 16 * GJ;
-  __shared__ float sm[kDistKc][kDistTile];
-  __shared__ float sv[kDistKc][kDistTile];
-  __shared__ float sa[kDistKc][kGenes];
-  __shared__ float sd[kDistKc][kGenes];
+  __shared__ float sm[kDistKc][kDistTile + 1];
+  __shared__ float sv[kDistKc][kDistTile + 1];
+  __shared__ float sa[kDistKc][kGenes + 1];
+  __shared__ float sd[kDistKc][kGenes + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int64_t g0 = (int64_t)blockIdx.x * kGenes;
   const int64_t p0 = (int64_t)blockIdx.y * kDistTile;

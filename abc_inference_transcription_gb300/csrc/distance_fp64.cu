@@ -122,18 +122,22 @@ constexpr int kRecheckWarps = 8;
 constexpr int kRecheckCols = 24;
 constexpr int kRecheckLd = kRecheckCols + 1;
 
-__global__ void __launch_bounds__(kRecheckWarps * 32) recheck_grouped_kernel(DistInputs in, const int32_t* sp,
-                                                                             const int32_t* sg, int64_t n,
-                                                                             double* se64) {
-  __shared__ double rs_smem[kRecheckWarps * 32 * kRecheckLd];
+// WARPS: kRecheckWarps, or 1 while the chunks do not fill the GPU: a term's six
+// FP64 operations hold a scheduler's pipe whatever the number of pairs, so
+// the warps of a few chunks go to different ones (800 pairs of 53 statistics: 39 us in
+// blocks of 8 warps, 30 apart).
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) recheck_grouped_kernel(DistInputs in, const int32_t* sp,
+                                                                     const int32_t* sg, int64_t n, double* se64) {
+  __shared__ double rs_smem[WARPS * 32 * kRecheckLd];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int K = in.K;
   double* S = rs_smem + warp * 32 * kRecheckLd;
   const double nK = (double)K;
   const double rK = 1.0 / nK;
   const int64_t n_chunks = (n + 31) >> 5;
-  const int64_t wstride = (int64_t)gridDim.x * kRecheckWarps;
-  for (int64_t ch = (int64_t)blockIdx.x * kRecheckWarps + warp; ch < n_chunks; ch += wstride) {
+  const int64_t wstride = (int64_t)gridDim.x * WARPS;
+  for (int64_t ch = (int64_t)blockIdx.x * WARPS + warp; ch < n_chunks; ch += wstride) {
     const int64_t i = ch * 32 + lane;
     const bool mine = i < n;
     const int32_t p = mine ? sp[i] : 0;
@@ -177,10 +181,14 @@ __global__ void __launch_bounds__(kRecheckWarps * 32) recheck_grouped_kernel(Dis
       __syncwarp();
       if (mine) {
         const double* s = S + lane * kRecheckLd - c0;
-        for (int k = c0; k < c0 + cw; ++k) {
-          const double diff = __ldg(d + k) - s[k];
-          part = part + div_rn(diff * diff, __ldg(dn + k), __ldg(ry + k));
-          while (k + 1 == fend) {  // close this family and any empty ones after it
+        for (int k = c0; k < c0 + cw;) {
+          const int ke = fend > k && fend < c0 + cw ? fend : c0 + cw;  // the open family's terms of this chunk
+#pragma unroll 4
+          for (; k < ke; ++k) {
+            const double diff = __ldg(d + k) - s[k];
+            part = part + div_rn(diff * diff, __ldg(dn + k), __ldg(ry + k));
+          }
+          while (k == fend) {  // close this family and any empty ones after it
             tot = tot + div_rn(part, nK, rK);
             part = 0.0;
             ++f;
@@ -566,23 +574,29 @@ __global__ void __launch_bounds__(256) scatter_smem_kernel(const Cand* cand, int
 }
 
 __global__ void __launch_bounds__(1024) scan_kernel(const int64_t* cnt, int64_t G, int64_t* off) {
-  __shared__ int64_t part[1024];
+  __shared__ int64_t wsum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t per = (G + 1023) / 1024;
   const int64_t b = threadIdx.x * per;
-  int64_t s = 0;
-  for (int64_t i = b; i < b + per && i < G; ++i) s += cnt[i];
-  part[threadIdx.x] = s;
+  int64_t own = 0;
+  for (int64_t i = b; i < b + per && i < G; ++i) own += cnt[i];
+  int64_t run = own;  // inclusive scan over the warp, then over the warps
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t v = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += v;
+  }
+  if (lane == 31) wsum[warp] = run;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t run = 0;
-    for (int t = 0; t < 1024; ++t) {
-      int64_t v = part[t];
-      part[t] = run;
-      run += v;
+  if (warp == 0) {
+    int64_t w = wsum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t v = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += v;
     }
+    wsum[lane] = w;
   }
   __syncthreads();
-  int64_t run = part[threadIdx.x];
+  run += (warp ? wsum[warp - 1] : 0) - own;
   for (int64_t i = b; i < b + per && i < G; ++i) {
     off[i] = run;
     run += cnt[i];
@@ -742,12 +756,21 @@ static int grouped_blocks(int64_t n) {
   return (int)(want < 65536 ? want : 65536);
 }
 
+static void launch_recheck_grouped(const DistInputs& in, const int32_t* sp, const int32_t* sg, int64_t n, double* se64,
+                                   cudaStream_t s) {
+  const int64_t chunks = (n + 31) / 32;
+  if (chunks <= 4 * 152)  // at most a warp per scheduler
+    recheck_grouped_kernel<1><<<(unsigned)chunks, 32, 0, s>>>(in, sp, sg, n, se64);
+  else
+    recheck_grouped_kernel<kRecheckWarps><<<grouped_blocks(n), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, se64);
+}
+
 cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, const Cand* cand, int64_t n, int64_t* gcount,
                                            int64_t* goff, unsigned long long* gcursor, int32_t* sp, int32_t* sg,
                                            double* se64, cudaStream_t s) {
   cudaError_t err = launch_dist_group(cand, n, in.G, gcount, goff, gcursor, sp, sg, s);
   if (err || n <= 0) return err;
-  recheck_grouped_kernel<<<grouped_blocks(n), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, se64);
+  launch_recheck_grouped(in, sp, sg, n, se64, s);
   err = cudaGetLastError();
   if (err) return err;
   return launch_segsort(goff, in.G, sp, se64, nullptr, s);
@@ -868,7 +891,7 @@ cudaError_t launch_accepted_errors(const DistInputs& in, const int64_t* aoff, co
                                    int64_t p_base, int64_t n, int32_t* sp, int32_t* sg, double* err, cudaStream_t s) {
   if (G <= 0 || n <= 0) return cudaSuccess;
   accepted_pairs_kernel<<<(unsigned)G, 256, 0, s>>>(aoff, idx, G, p_base, sp, sg);
-  recheck_grouped_kernel<<<grouped_blocks(n), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, err);
+  launch_recheck_grouped(in, sp, sg, n, err, s);
   return cudaGetLastError();
 }
 
