@@ -1409,12 +1409,12 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   a.nsub = S * per_step;
   a.n_pulse_conds = n_pulse_conds;
   const bool f32 = cf.precision == ABC_FP32;
-  const int grid = (int)std::min<int64_t>(P, (int64_t)c->sms * (f32 ? 16 : 8));
-  const size_t scr_doubles = f32 ? (moment_f32_scratch_per_cta(a.nsub) + 7) / 8 : (size_t)2 * a.nsub * 100;
+  const int grid = (int)std::min<int64_t>(P, (int64_t)c->sms * 8);  // FP64 mode
+  const size_t scratch = f32 ? moment_f32_scratch(P, a.nsub, J * A) : sizeof(double) * (size_t)grid * 2 * a.nsub * 100;
   Work w;
   const size_t o_theta = w.add(sizeof(double) * (size_t)P * npar), o_bm = w.add(sizeof(double) * 2 * A * 3);
   const size_t o_ad = w.add(sizeof(double) * (size_t)A * J), o_stats = w.add(sizeof(double) * (size_t)P * K);
-  const size_t o_scr = w.add(sizeof(double) * (size_t)grid * scr_doubles);
+  const size_t o_scr = w.add(scratch);
   const size_t o_mom = w.add(moments_out ? sizeof(double) * (size_t)P * J * A * 5 : 0);
   const size_t o_it = w.add(iters_out ? sizeof(int) * (size_t)P : 0);
   CK(w.allocate(c));
@@ -1435,7 +1435,7 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
     CK(cudaEventCreate(&c->sel_ev[1]));
   }
   if (c->prof) CK(cudaEventRecord(c->sel_ev[0], c->stream));
-  CK(f32 ? launch_moment_f32(a, grid, c->stream) : launch_moment(a, grid, c->stream));
+  CK(f32 ? launch_moment_f32(a, c->stream) : launch_moment(a, grid, c->stream));
   if (c->prof) CK(cudaEventRecord(c->sel_ev[1], c->stream));
   CK(cudaMemcpyAsync(stats_out, a.stats, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
   if (moments_out)

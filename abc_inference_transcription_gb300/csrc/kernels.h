@@ -190,13 +190,13 @@ struct MomArgs {
   double* stats;           // [P][K]
   double* moments;         // [P][J][A][5] or null
   int* iters;              // [P] transient cycles or null
-  double* scratch;         // [grid][2][nsub][100]
+  double* scratch;         // FP64 mode: [grid][2][nsub][100]
   int* status;
 };
 cudaError_t launch_moment(const MomArgs& a, int grid, cudaStream_t s);
-// FP32 production mode (moment_fp32.cu); scratch: moment_f32_scratch_per_cta(nsub) bytes per CTA
-size_t moment_f32_scratch_per_cta(int nsub);
-cudaError_t launch_moment_f32(const MomArgs& a, int grid, cudaStream_t s);
+// FP32 production mode (moment_fp32.cu); scratch: moment_f32_scratch() bytes, pairs = conditions x ages
+size_t moment_f32_scratch(int64_t P, int nsub, int pairs);
+cudaError_t launch_moment_f32(const MomArgs& a, cudaStream_t s);
 
 // data-side statistics and bootstrap standard errors (datastats.cu)
 struct DataStatsArgs {

@@ -4,18 +4,36 @@
 //   [1, E G, Var G, E u, E l, Cov(G,u), Cov(G,l), Var u, Cov(u,l), Var l]
 // in which the moment matrix of scripts/model.jl:74-86 is lower triangular:
 // every moment depends only on itself and on moments listed before it.
-// Products of lower-triangular matrices stay lower triangular, so an
-// exponential product costs 220 FMA instead of 1000 and a substep 55 instead
-// of 100.  Taylor order 8 after scaling to a column-sum norm <= 1/2
-// (truncation < 6e-9, below FP32's 6e-8 resolution).  Substep and labelling indices are integers (the
-// grid is aligned with every breakpoint), so the per-substep work has no FP64
-// operation; rates, times and the statistics stay in FP64.  The transient
-// phase applies the one-cycle propagator (the ordered product of the cycle's
-// unlabelled substep propagators) once per cycle.  The default substep is
-// cycle / 80 (every pulse, chase and age of the reference grid is a multiple
-// of it): against the reference's recovered statistics it is as close as
-// cycle / 400, and within 3e-3 of it.
+// Products of such matrices keep not only the triangle but the pattern of
+// 38 entries that the matrix's dependencies allow (row_mask); the other 17 are
+// exact zeros and are neither stored nor multiplied.  Taylor order 8 after scaling
+// to a column-sum norm <= 1/2 (truncation < 6e-9, below FP32's 6e-8
+// resolution).  Substep and labelling indices are integers (the grid is aligned
+// with every breakpoint), so the per-substep work has no FP64 operation; rates,
+// times and the statistics stay in FP64.  The transient phase applies the
+// one-cycle propagator (the ordered product of the cycle's unlabelled substep
+// propagators) once per cycle.  The default substep is cycle / 80 (every pulse,
+// chase and age of the reference grid is a multiple of it): against the
+// reference's recovered statistics it is as close as cycle / 400, and within
+// 3e-3 of it.
+//
+// Kernels per chunk of particles:
+//   rates   a thread per particle;
+//   exp     a propagator per thread, its 38 entries in registers.  (A lane per
+//           entry of one product at a time, operands in shared memory, took
+//           some 60 times as many instructions.)
+//   cycle   the one-cycle propagators, a column of a quarter per thread;
+//   walk    a thread per particle: the transient, then the unlabelled stretch
+//           that the particle's trajectories share, walked once;
+//   paths   the labelled and chased rest of the trajectories, a lane per
+//           (condition, age);
+//   stats   capture and statistics.
+// 10,000 particles: 0.56 ms; 14.4 with one CTA per particle doing all of it,
+// trajectories from their first substep on.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -25,125 +43,225 @@ namespace abc {
 namespace {
 
 constexpr int NA = 10;
-constexpr int NT = NA * (NA + 1) / 2;  // 55 lower-triangular entries, row-major packed
-constexpr int kThreads = 128;
-constexpr int kWarps = kThreads / 32;
 constexpr int kTaylor = 8;
+constexpr int kNnz = 38, kQuads = 10;  // stored entries of a propagator; 16-byte pieces, the last one half padding
+constexpr int kExpThreads = 128;
+constexpr int kQuarters = 4;  // parts of the cycle multiplied separately
+constexpr int kCycleParticles = 8;
+constexpr int kPathParticles = 8;  // a warp of the path kernel: these x kPathGroup pairs, two per lane
+constexpr int kPathGroup = 2 * 32 / kPathParticles;
+constexpr int kMaxPairs = kMaxConds * kMaxAges;
+constexpr int kWalkStages = 8, kPathStages = 4;  // substeps whose propagators are on their way
 
-// packed index of (r, c), c <= r
-__host__ __device__ constexpr int tri(int r, int c) { return r * (r + 1) / 2 + c; }
-
-// the moment matrix times h in the permuted order (rows: 0 const, 1 EG, 2 VarG,
-// 3 Eu, 4 El, 5 CovGu, 6 CovGl, 7 Varu, 8 Covul, 9 Varl); rates already times h
-__device__ void build_tri(float* A, int lane, float kon, float koff, float al, float gam, float lam) {
-  for (int i = lane; i < NT; i += 32) A[i] = 0.0f;
-  __syncwarp();
-  if (lane == 0) {
-    const float ks = kon + koff, a1 = al * (1.0f - lam), a2 = al * lam;
-    A[tri(1, 0)] = kon;
-    A[tri(1, 1)] = -ks;
-    A[tri(2, 0)] = kon;
-    A[tri(2, 1)] = koff - kon;
-    A[tri(2, 2)] = -2.0f * ks;
-    A[tri(3, 1)] = a1;
-    A[tri(3, 3)] = -gam;
-    A[tri(4, 1)] = a2;
-    A[tri(4, 4)] = -gam;
-    A[tri(5, 2)] = a1;
-    A[tri(5, 5)] = -(ks + gam);
-    A[tri(6, 2)] = a2;
-    A[tri(6, 6)] = -(ks + gam);
-    A[tri(7, 1)] = a1;
-    A[tri(7, 3)] = gam;
-    A[tri(7, 5)] = 2.0f * a1;
-    A[tri(7, 7)] = -2.0f * gam;
-    A[tri(8, 5)] = a2;
-    A[tri(8, 6)] = a1;
-    A[tri(8, 8)] = -2.0f * gam;
-    A[tri(9, 1)] = a2;
-    A[tri(9, 4)] = gam;
-    A[tri(9, 6)] = 2.0f * a2;
-    A[tri(9, 9)] = -2.0f * gam;
-  }
-  __syncwarp();
-}
-
-// Output entries of a lane in a packed triangular product: o = lane and
-// o = lane + 32 (when < 55), with their (row, column), kept in registers (a
-// table in constant memory would serialise the lanes' distinct addresses).
-struct LaneTri {
-  int r0, c0, r1, c1;
-  bool has1;
+// (condition, age) pairs by the start of their labelling: labelled from substep
+// lo to hi, observed at end
+struct MomPlan {
+  int n;
+  int pair[kMaxPairs], lo[kMaxPairs], hi[kMaxPairs], end[kMaxPairs];
 };
 
-__device__ __forceinline__ void rc_of(int o, int& r, int& c) {
-  r = 0;
-  while ((r + 1) * (r + 2) / 2 <= o) ++r;
-  c = o - r * (r + 1) / 2;
+// Scratch of a chunk of n particles.  The particle is the fastest index of the
+// propagators: threads of neighbouring particles read and write whole lines.
+enum { kRateOn = 0, kRateAlp = kMaxSteps, kRateGam = 2 * kMaxSteps, kRateOff = 3 * kMaxSteps, kRateLam, kRateScal,
+       kRateBad, kRates };
+struct MomScratch {
+  float4* props;  // [labelled][substep][kQuads][n]
+  float4* phi;    // [kQuads][n]
+  float* start;   // [pairs, in plan order][n][NA]
+  float* mom;     // [n][pairs][5]
+  float* rates;   // [kRates][n]
+  int64_t n;
+};
+
+// columns of the stored entries of row r, as bits
+__device__ __forceinline__ constexpr unsigned row_mask(int r) {
+  return r == 0   ? 0x001u
+         : r == 1 ? 0x003u
+         : r == 2 ? 0x007u
+         : r == 3 ? 0x00bu
+         : r == 4 ? 0x013u
+         : r == 5 ? 0x027u
+         : r == 6 ? 0x047u
+         : r == 7 ? 0x0afu
+         : r == 8 ? 0x167u
+                  : 0x257u;
+}
+__device__ __forceinline__ bool stored(int r, int c) { return (row_mask(r) >> c) & 1u; }
+
+// position of the entry (r, c) among the stored ones (row by row)
+__device__ __forceinline__ int pos_of(int r, int c) {
+  constexpr int first[NA] = {0, 1, 3, 6, 9, 12, 16, 20, 26, 32};
+  return first[r] + __popc(row_mask(r) & ((1u << c) - 1u));
 }
 
-__device__ __forceinline__ LaneTri lane_tri(int lane) {
-  LaneTri t;
-  rc_of(lane, t.r0, t.c0);
-  t.has1 = lane + 32 < NT;
-  t.r1 = t.c1 = 0;
-  if (t.has1) rc_of(lane + 32, t.r1, t.c1);
-  return t;
+struct Prop {
+  float v[4 * kQuads];
+};
+
+__device__ __forceinline__ void set_quad(Prop& P, int i, float4 q) {
+  P.v[4 * i] = q.x;
+  P.v[4 * i + 1] = q.y;
+  P.v[4 * i + 2] = q.z;
+  P.v[4 * i + 3] = q.w;
 }
 
-__device__ __forceinline__ float tri_dot(const float* X, const float* Y, int r, int c) {
-  float s = 0.0f;
-  for (int k = c; k <= r; ++k) s = fmaf(X[tri(r, k)], Y[tri(k, c)], s);
-  return s;
+// src: the first piece, stride apart
+__device__ __forceinline__ void load_prop(const float4* src, int64_t stride, Prop& P) {
+#pragma unroll
+  for (int i = 0; i < kQuads; ++i) set_quad(P, i, src[i * stride]);
 }
 
-// Z = X Y, lower triangular, packed
-__device__ __forceinline__ void tri_mul(const float* X, const float* Y, float* Z, const LaneTri& t, int lane) {
-  const float z0 = tri_dot(X, Y, t.r0, t.c0);
-  const float z1 = t.has1 ? tri_dot(X, Y, t.r1, t.c1) : 0.0f;
-  Z[lane] = z0;
-  if (t.has1) Z[lane + 32] = z1;
-  __syncwarp();
-}
-
-__device__ void expm_tri(float* A, float* E, float* T, const LaneTri& t, int lane) {
-  float norm = 0.0f;
-  for (int c = 0; c < NA; ++c) {
-    float s = 0.0f;
-    for (int r = c; r < NA; ++r) s += fabsf(A[tri(r, c)]);
-    norm = fmaxf(norm, s);
+// y <- P y, each row from its first entry on
+__device__ __forceinline__ void apply(const Prop& P, float (&y)[NA]) {
+  float z[NA];
+  int i = 0;
+#pragma unroll
+  for (int r = 0; r < NA; ++r) {
+    float acc = 0.0f;
+#pragma unroll
+    for (int c = 0; c < NA; ++c)
+      if (stored(r, c)) acc = fmaf(P.v[i++], y[c], acc);
+    z[r] = acc;
   }
+#pragma unroll
+  for (int r = 0; r < NA; ++r) y[r] = z[r];
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
+// rates of one particle, times the substep
+__global__ void moment_rates_kernel(MomArgs a, int64_t p0, MomScratch ws) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n = ws.n;
+  if (i >= n) return;
+  PRec R;
+  const bool bad = parse_theta(a.cfg, a.model, a.theta + (p0 + i) * a.ld, R);
+  const double h = a.h;
+  float* out = ws.rates + i;
+  for (int k = 0; k < a.cfg.n_steps; ++k) {
+    out[(kRateOn + k) * n] = bad ? 0.0f : (float)(R.kon[k] * h);
+    out[(kRateAlp + k) * n] = bad ? 0.0f : (float)(R.alp[k] * h);
+    out[(kRateGam + k) * n] = bad ? 0.0f : (float)(R.gam[k] * h);
+  }
+  out[kRateOff * n] = bad ? 0.0f : (float)(R.koff * h);
+  out[kRateLam * n] = bad ? 0.0f : (float)R.lam;
+  out[kRateScal * n] = bad ? 0.0f : (float)R.scal;
+  out[kRateBad * n] = bad ? 1.0f : 0.0f;
+}
+
+// The propagator of one substep of one particle per thread (blockIdx.y: the substep,
+// the labelled ones second).  The generator in the permuted order (rows: 0 const,
+// 1 EG, 2 VarG, 3 Eu, 4 El, 5 CovGu, 6 CovGl, 7 Varu, 8 Covul, 9 Varl; rates
+// already times h):
+//   (1,0) kon (1,1) -ks | (2,0) kon (2,1) koff - kon (2,2) -2 ks | (3,1) a1 (3,3) -g |
+//   (4,1) a2 (4,4) -g | (5,2) a1 (5,5) -(ks + g) | (6,2) a2 (6,6) -(ks + g) |
+//   (7,1) a1 (7,3) g (7,5) 2 a1 (7,7) -2 g | (8,5) a2 (8,6) a1 (8,8) -2 g |
+//   (9,1) a2 (9,4) g (9,6) 2 a2 (9,9) -2 g,   ks = kon + koff, a1 = al (1 - lam), a2 = al lam
+__global__ void __launch_bounds__(kExpThreads) moment_exp_kernel(MomArgs a, MomScratch ws) {
+  const int64_t i = (int64_t)blockIdx.x * kExpThreads + threadIdx.x, n = ws.n;
+  if (i >= n) return;
+  const int lab = (int)blockIdx.y / a.nsub, idx = (int)blockIdx.y - lab * a.nsub, k = idx / a.per_step;
+  const float* m = ws.rates + i;
+  const float hf = (float)a.h, invT = (float)(1.0 / a.cfg.cycle);
+  const float ph = ((float)idx + 0.5f) * hf;
+  // alpha(t) = alpha_k size^s, size = 1 + phase / T (model.jl:25-27)
+  const float al = m[(kRateAlp + k) * n] * exp2f(m[kRateScal * n] * __log2f(fmaf(ph, invT, 1.0f)));
+  const float lam = lab ? m[kRateLam * n] : 0.0f;
+  const float kon = m[(kRateOn + k) * n], koff = m[kRateOff * n], g = m[(kRateGam + k) * n];
+  const float ks = kon + koff, a1 = al * (1.0f - lam), a2 = al * lam;
+  const float kd = koff - kon, ks2 = -2.0f * ks, kg = -(ks + g), a1d = 2.0f * a1, a2d = 2.0f * a2, g2 = -2.0f * g;
+  // column-sum norm
+  float norm = (0.0f + fabsf(kon)) + fabsf(kon);
+  norm = fmaxf(norm, ((((fabsf(ks) + fabsf(kd)) + fabsf(a1)) + fabsf(a2)) + fabsf(a1)) + fabsf(a2));
+  norm = fmaxf(norm, (fabsf(ks2) + fabsf(a1)) + fabsf(a2));
+  norm = fmaxf(norm, fabsf(g) + fabsf(g));
+  norm = fmaxf(norm, (fabsf(kg) + fabsf(a1d)) + fabsf(a2));
+  norm = fmaxf(norm, (fabsf(kg) + fabsf(a1)) + fabsf(a2d));
+  norm = fmaxf(norm, fabsf(g2));
   int sq = 0;
-  while (norm > 0.5f) {
+  while (norm > 0.5f && sq < 256) {  // (a norm beyond FP32's range ends here too)
     norm *= 0.5f;
     sq++;
   }
-  const float scale = ldexpf(1.0f, -sq);
-  const float d0 = t.r0 == t.c0 ? 1.0f : 0.0f, d1 = t.r1 == t.c1 ? 1.0f : 0.0f;
-  A[lane] *= scale;
-  E[lane] = d0;
-  if (t.has1) {
-    A[lane + 32] *= scale;
-    E[lane + 32] = d1;
+  const float sc = ldexpf(1.0f, -sq);
+  float A[NA][NA];  // only the entries named below are ever read
+  A[1][0] = A[2][0] = kon * sc;
+  A[1][1] = -ks * sc;
+  A[2][1] = kd * sc;
+  A[2][2] = ks2 * sc;
+  A[3][1] = A[5][2] = A[7][1] = A[8][6] = a1 * sc;
+  A[4][1] = A[6][2] = A[8][5] = A[9][1] = a2 * sc;
+  A[3][3] = A[4][4] = -g * sc;
+  A[5][5] = A[6][6] = kg * sc;
+  A[7][3] = A[9][4] = g * sc;
+  A[7][5] = a1d * sc;
+  A[9][6] = a2d * sc;
+  A[7][7] = A[8][8] = A[9][9] = g2 * sc;
+  constexpr unsigned kGen[NA] = {0x000u, 0x003u, 0x007u, 0x00au, 0x012u, 0x024u, 0x044u, 0x0aau, 0x160u, 0x252u};
+  // E <- I + A E / q, q = 8 .. 1.  Row r of A E needs rows up to r of E only, so
+  // descending rows overwrite in place.
+  Prop E;
+#pragma unroll
+  for (int r = 0; r < NA; ++r)
+#pragma unroll
+    for (int c = 0; c < NA; ++c)
+      if (stored(r, c)) E.v[pos_of(r, c)] = r == c ? 1.0f : 0.0f;
+#pragma unroll 1
+  for (int q = kTaylor; q >= 1; --q) {
+    const float inv = 1.0f / (float)q;
+#pragma unroll
+    for (int r = NA - 1; r >= 1; --r) {
+      float t[NA];
+#pragma unroll
+      for (int c = 0; c < NA; ++c) {
+        if (!stored(r, c)) continue;
+        float acc = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NA; ++j)
+          if (((kGen[r] >> j) & 1u) && stored(j, c)) acc = fmaf(A[r][j], E.v[pos_of(j, c)], acc);
+        t[c] = fmaf(acc, inv, r == c ? 1.0f : 0.0f);
+      }
+#pragma unroll
+      for (int c = 0; c < NA; ++c)
+        if (stored(r, c)) E.v[pos_of(r, c)] = t[c];
+    }
   }
-  __syncwarp();
-  for (int n = kTaylor; n >= 1; --n) {
-    tri_mul(A, E, T, t, lane);
-    const float inv = 1.0f / (float)n;
-    E[lane] = fmaf(T[lane], inv, d0);
-    if (t.has1) E[lane + 32] = fmaf(T[lane + 32], inv, d1);
-    __syncwarp();
-  }
+  // E <- E E, likewise
+#pragma unroll 1
   for (int s = 0; s < sq; ++s) {
-    tri_mul(E, E, T, t, lane);
-    E[lane] = T[lane];
-    if (t.has1) E[lane + 32] = T[lane + 32];
-    __syncwarp();
+#pragma unroll
+    for (int r = NA - 1; r >= 0; --r) {
+      float t[NA];
+#pragma unroll
+      for (int c = 0; c < NA; ++c) {
+        if (!stored(r, c)) continue;
+        float acc = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NA; ++j)
+          if (stored(r, j) && stored(j, c)) acc = fmaf(E.v[pos_of(r, j)], E.v[pos_of(j, c)], acc);
+        t[c] = acc;
+      }
+#pragma unroll
+      for (int c = 0; c < NA; ++c)
+        if (stored(r, c)) E.v[pos_of(r, c)] = t[c];
+    }
   }
+  E.v[kNnz] = E.v[kNnz + 1] = 0.0f;
+  float4* dst = ws.props + (int64_t)blockIdx.y * kQuads * n + i;
+#pragma unroll
+  for (int q = 0; q < kQuads; ++q)
+    dst[q * n] = make_float4(E.v[4 * q], E.v[4 * q + 1], E.v[4 * q + 2], E.v[4 * q + 3]);
 }
 
 // division map (model.jl:98-111) in the permuted order
-__device__ __forceinline__ void divide_p(float* v) {
+__device__ __forceinline__ void divide_p(float (&v)[NA]) {
   const float eu = v[3], el = v[4];
   v[5] *= 0.5f;
   v[6] *= 0.5f;
@@ -154,20 +272,6 @@ __device__ __forceinline__ void divide_p(float* v) {
   v[4] = 0.5f * el;
 }
 
-// y <- P y (P in shared or L1-resident global memory)
-__device__ __forceinline__ void step_tri_s(const float* P, float* y) {
-  float z[NA];
-#pragma unroll
-  for (int r = 0; r < NA; ++r) {
-    float acc = 0.0f;
-#pragma unroll
-    for (int c = 0; c <= r; ++c) acc = fmaf(P[tri(r, c)], y[c], acc);
-    z[r] = acc;
-  }
-#pragma unroll
-  for (int r = 0; r < NA; ++r) y[r] = z[r];
-}
-
 // original moment index of each permuted position
 __device__ __forceinline__ int orig_of(int r) {
   // 0 const, 1 EG(0), 2 VarG(3), 3 Eu(1), 4 El(2), 5 CovGu(4), 6 CovGl(5), 7 Varu(6), 8 Covul(7), 9 Varl(8)
@@ -175,175 +279,323 @@ __device__ __forceinline__ int orig_of(int r) {
   return map[r];
 }
 
-__global__ void __launch_bounds__(kThreads) moment_kernel_f32(MomArgs a) {
-  __shared__ float wsp[kWarps][3][NT];
-  __shared__ float ss[NA];
-  __shared__ double mom[kMaxConds * kMaxAges * 5];
-  __shared__ double ds[kMaxConds * kMaxAges * 5];
-  __shared__ PRec R;
-  __shared__ int s_bad;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const DevCfg& cfg = a.cfg;
-  const int J = cfg.n_conds, A = cfg.n_ages;
-  const int K = 4 * A + 3 * J;
-  const int nsub = a.nsub;
-  const double h = a.h, T = cfg.cycle;
-  float* P0 = reinterpret_cast<float*>(a.scratch) + (size_t)blockIdx.x * 2 * nsub * NT;
-  const LaneTri lt = lane_tri(lane);
-  float* P1 = P0 + (size_t)nsub * NT;
-  for (int64_t p = blockIdx.x; p < a.P; p += gridDim.x) {
-    if (threadIdx.x == 0) s_bad = parse_theta(cfg, a.model, a.theta + p * a.ld, R) ? 1 : 0;
-    __syncthreads();
-    if (s_bad) {
-      for (int k = threadIdx.x; k < K; k += blockDim.x) a.stats[p * K + k] = NAN;
-      if (threadIdx.x == 0) atomicOr(a.status, 1);
-      __syncthreads();
-      continue;
-    }
-    // ---- propagators for every substep, without and with labelling
-    float* Aw = wsp[warp][0];
-    float* Ew = wsp[warp][1];
-    float* Tw = wsp[warp][2];
-    const float hf = (float)h, invT = (float)(1.0 / T), scal = (float)R.scal, lamf = (float)R.lam;
-    const float koffh = (float)(R.koff * h);
-    for (int task = warp; task < 2 * nsub; task += kWarps) {
-      const int lab = task / nsub, idx = task - lab * nsub;
-      const int k = idx / a.per_step;
-      const float ph = ((float)idx + 0.5f) * hf;
-      // alpha(t) = alpha_k size^s, size = 1 + phase / T (model.jl:25-27)
-      const float al = (float)(R.alp[k] * h) * exp2f(scal * __log2f(fmaf(ph, invT, 1.0f)));
-      build_tri(Aw, lane, (float)(R.kon[k] * h), koffh, al, (float)(R.gam[k] * h), lab ? lamf : 0.0f);
-      expm_tri(Aw, Ew, Tw, lt, lane);
-      float* dst = (lab ? P1 : P0) + (size_t)idx * NT;
-      for (int i = lane; i < NT; i += 32) dst[i] = Ew[i];
-      __syncwarp();
-    }
-    __syncthreads();
-    // ---- one-cycle propagator without labelling, Phi = P[nsub-1] ... P[0]:
-    // each warp multiplies a contiguous quarter in order, warp 0 joins them
-    {
-      const int q0 = warp * nsub / kWarps, q1 = (warp + 1) * nsub / kWarps;
-      float* Q = wsp[warp][1];
-      float* Pi = wsp[warp][0];
-      Q[lane] = lt.r0 == lt.c0 ? 1.0f : 0.0f;
-      if (lt.has1) Q[lane + 32] = lt.r1 == lt.c1 ? 1.0f : 0.0f;
-      __syncwarp();
-      for (int i = q0; i < q1; ++i) {
-        const float* src = P0 + (size_t)i * NT;
-        Pi[lane] = src[lane];
-        if (lt.has1) Pi[lane + 32] = src[lane + 32];
-        __syncwarp();
-        tri_mul(Pi, Q, Tw, lt, lane);
-        Q[lane] = Tw[lane];
-        if (lt.has1) Q[lane + 32] = Tw[lane + 32];
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {
-      float* Phi = wsp[0][1];
-      for (int w = 1; w < kWarps; ++w) {
-        tri_mul(wsp[w][1], Phi, wsp[0][2], lt, lane);
-        Phi[lane] = wsp[0][2][lane];
-        if (lt.has1) Phi[lane + 32] = wsp[0][2][lane + 32];
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    // ---- transient phase (model.jl:114-142): one cycle from iv, then cycles
-    // until the moments of E G, E u, Var G, Cov(G,u), Var u change by <= 1 %
-    if (threadIdx.x == 0) {
-      const float* Phi = wsp[0][1];
-      float y[NA], e1[NA];
-      y[0] = 1.0f;
-      for (int r = 1; r < NA; ++r) y[r] = (float)a.iv[orig_of(r)];
-      step_tri_s(Phi, y);
-      for (int r = 0; r < NA; ++r) e1[r] = y[r];
-      int it = 0;
-      bool conv = false;
-      while (!conv && it <= 100) {
-        it++;
-        divide_p(y);
-        step_tri_s(Phi, y);
-        const int chk[5] = {1, 3, 2, 5, 7};
-        int nz = 0, ok = 0;
-        for (int q = 0; q < 5; ++q) {
-          const int r = chk[q];
-          if (e1[r] > 0.0f) {
-            nz++;
-            if (fabsf((e1[r] - y[r]) / e1[r]) <= 0.01f) ok++;
-          }
-        }
-        conv = ok == nz;
-        for (int r = 0; r < NA; ++r) e1[r] = y[r];
-      }
-      divide_p(y);
-      for (int r = 0; r < NA; ++r) ss[r] = y[r];
-      if (a.iters) a.iters[p] = it;
-    }
-    __syncthreads();
-    // ---- trajectories (model.jl:146-199), one (condition, age) per thread:
-    // global substep s (midpoint t0 + (s + 1/2) h), divisions at multiples of
-    // nsub, labelling iff s_lo <= s < s_hi, the end at s_end = (age - t0) / h
-    const double t0 = cfg.t0;
-    for (int t = threadIdx.x; t < J * A; t += blockDim.x) {
-      const int j = t / A, ai = t - (t / A) * A;
-      const double age = cfg.ages[ai];
-      const double texp = (age - cfg.pulse[j]) - cfg.chase[j];
-      const double tle = texp + cfg.pulse[j];
-      const int s_lo = (int)lround((texp - t0) / h), s_hi = (int)lround((tle - t0) / h);
-      const int s_end = (int)lround((age - t0) / h);
-      float y[NA];
+// One-cycle propagators without labelling, Phi = P[nsub-1] ... P[0]: the
+// columns of each contiguous quarter P[q1-1] ... P[q0], applied from the identity,
+// then those of the quarters' product.  Threads: column of quarter x particle.
+__global__ void __launch_bounds__(kCycleParticles * kQuarters * NA, 3) moment_cycle_kernel(int nsub, MomScratch ws) {
+  __shared__ float sq[kQuarters][4 * kQuads][kCycleParticles];
+  const int pi = threadIdx.x % kCycleParticles, w = threadIdx.x / (kCycleParticles * NA);
+  const int c = threadIdx.x / kCycleParticles % NA;
+  const int64_t i = (int64_t)blockIdx.x * kCycleParticles + pi, n = ws.n;
+  float q[NA];
 #pragma unroll
-      for (int r = 0; r < NA; ++r) y[r] = ss[r];
-      int idx = 0;
-      for (int s = 0; s < s_end; ++s) {
-        if (idx == nsub) {
-          idx = 0;
-          divide_p(y);
-        }
-        step_tri_s(((s >= s_lo && s < s_hi) ? P1 : P0) + (size_t)idx * NT, y);
-        ++idx;
-      }
-      double* mo = mom + t * 5;
-      mo[0] = y[3];
-      mo[1] = y[4];
-      mo[2] = y[7];
-      mo[3] = y[8];
-      mo[4] = y[9];
+  for (int r = 0; r < NA; ++r) q[r] = r == c ? 1.0f : 0.0f;
+  if (i < n) {
+    const int q1 = (w + 1) * nsub / kQuarters;
+#pragma unroll 1
+    for (int s = w * nsub / kQuarters; s < q1; ++s) {
+      float4 b[kQuads];  // every load under way before the first use
+#pragma unroll
+      for (int e = 0; e < kQuads; ++e) b[e] = ws.props[((int64_t)s * kQuads + e) * n + i];
+      Prop P;
+#pragma unroll
+      for (int e = 0; e < kQuads; ++e) set_quad(P, e, b[e]);
+      apply(P, q);
     }
-    __syncthreads();
-    if (a.moments)
-      for (int i = threadIdx.x; i < J * A * 5; i += blockDim.x) a.moments[p * (J * A * 5) + i] = mom[i];
-    // capture transform (model.jl:221-239) per (condition, age), then the
-    // statistics per condition on the lanes of warp 0
-    for (int t = threadIdx.x; t < J * A; t += blockDim.x) {
-      const int j = t / A, ai = t - (t / A) * A;
-      const double* bm = a.beta_mom + ((j < a.n_pulse_conds ? 0 : 1) * A + ai) * 3;
-      const double mb = bm[0], m2 = bm[1], vb = bm[2];
-      const double* sm = mom + (j * A + ai) * 5;
-      double* d = ds + (j * A + ai) * 5;
-      d[0] = sm[0] * mb;
-      d[1] = sm[1] * mb;
-      d[2] = ((mb - m2) * sm[0] + vb * (sm[0] * sm[0] + sm[2])) + mb * mb * sm[2];
-      d[4] = ((mb - m2) * sm[1] + vb * (sm[1] * sm[1] + sm[4])) + mb * mb * sm[4];
-      d[3] = vb * (sm[0] * sm[1] + sm[3]) + mb * mb * sm[3];
-    }
-    __syncthreads();
-    if (threadIdx.x < 32)
-      for (int j = threadIdx.x; j < J; j += 32) stats_from_moments_cond(cfg, ds, a.age_dist, a.stats + p * K, j);
-    __syncthreads();
   }
+#pragma unroll
+  for (int r = 0; r < NA; ++r)
+    if (stored(r, c)) sq[w][pos_of(r, c)][pi] = q[r];
+  __syncthreads();
+  if (w == 0) {
+    for (int v = 1; v < kQuarters; ++v) {
+      Prop P;
+#pragma unroll
+      for (int e = 0; e < kNnz; ++e) P.v[e] = sq[v][e][pi];
+      apply(P, q);
+    }
+#pragma unroll
+    for (int r = 0; r < NA; ++r)
+      if (stored(r, c)) sq[0][pos_of(r, c)][pi] = q[r];  // read by this column's thread alone until here
+    if (c < 4 * kQuads - kNnz) sq[0][kNnz + c][pi] = 0.0f;
+  }
+  __syncthreads();
+  if (w == 0 && i < n)
+    ws.phi[c * n + i] = make_float4(sq[0][4 * c][pi], sq[0][4 * c + 1][pi], sq[0][4 * c + 2][pi], sq[0][4 * c + 3][pi]);
+}
+
+// Transient phase (model.jl:114-142): one cycle from iv, then cycles until the
+// moments of E G, E u, Var G, Cov(G,u), Var u change by <= 1 %; then the
+// unlabelled substeps: global substep s (midpoint t0 + (s + 1/2) h), divisions
+// at multiples of nsub, the state kept where a pair's labelling starts.  A serial chain
+// of some 300 substeps per particle, few warps: each thread copies its
+// propagators kWalkStages substeps ahead into shared memory.
+__global__ void __launch_bounds__(32) moment_walk_kernel(MomArgs a, int64_t p0, MomScratch ws,
+                                                         const __grid_constant__ MomPlan plan) {
+  __shared__ float4 ring[kWalkStages][kQuads][32];
+  const int64_t i = (int64_t)blockIdx.x * 32 + threadIdx.x, n = ws.n;
+  const bool live = i < n && ws.rates[kRateBad * n + (i < n ? i : 0)] == 0.0f;
+  const unsigned lanes = __ballot_sync(0xffffffffu, live);
+  if (!live) return;
+  const int nsub = a.nsub, steps = plan.lo[plan.n - 1];
+  auto fetch = [&](int s, int sub) {  // sub = s mod nsub
+    if (s < steps)
+#pragma unroll
+      for (int q = 0; q < kQuads; ++q)
+        cp_async16(&ring[s % kWalkStages][q][threadIdx.x], ws.props + ((int64_t)sub * kQuads + q) * n + i);
+    cp_async_commit();
+  };
+  int ahead = 0;
+  for (int s = 0; s < kWalkStages - 1; ++s) {
+    fetch(s, ahead);
+    if (++ahead == nsub) ahead = 0;
+  }
+  Prop P;
+  load_prop(ws.phi + i, n, P);
+  float y[NA], e1[NA];
+  y[0] = 1.0f;
+#pragma unroll
+  for (int r = 1; r < NA; ++r) y[r] = (float)a.iv[orig_of(r)];
+  apply(P, y);
+#pragma unroll
+  for (int r = 0; r < NA; ++r) e1[r] = y[r];
+  int it = 0;
+  bool conv = false;
+  while (!conv && it <= 100) {
+    it++;
+    divide_p(y);
+    apply(P, y);
+    const int chk[5] = {1, 3, 2, 5, 7};
+    int nz = 0, ok = 0;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const int r = chk[q];
+      if (e1[r] > 0.0f) {
+        nz++;
+        if (fabsf((e1[r] - y[r]) / e1[r]) <= 0.01f) ok++;
+      }
+    }
+    conv = ok == nz;
+#pragma unroll
+    for (int r = 0; r < NA; ++r) e1[r] = y[r];
+  }
+  divide_p(y);
+  if (a.iters) a.iters[p0 + i] = it;
+  int q = 0, idx = 0;
+  for (int s = 0;; ++s) {
+    for (; q < plan.n && plan.lo[q] <= s; ++q) {
+      float* start = ws.start + ((int64_t)q * n + i) * NA;
+#pragma unroll
+      for (int r = 0; r < NA; r += 2) *reinterpret_cast<float2*>(start + r) = make_float2(y[r], y[r + 1]);
+    }
+    if (q == plan.n) break;
+    __syncwarp(lanes);  // the slot read last is free
+    fetch(s + kWalkStages - 1, ahead);
+    if (++ahead == nsub) ahead = 0;
+    if (idx == nsub) {
+      idx = 0;
+      divide_p(y);
+    }
+    ++idx;
+    cp_async_wait<kWalkStages - 1>();  // substep s is there: a thread reads only what it copied
+    load_prop(&ring[s % kWalkStages][0][threadIdx.x], 32, P);
+    apply(P, y);
+  }
+}
+
+// Trajectories (model.jl:146-199) from the start of their labelling.  A warp
+// holds kPathGroup neighbouring pairs (blockIdx.y) of kPathParticles particles:
+// the pairs walk the substeps together, each joining at its lo and leaving at
+// its end, so a particle's lanes read the same propagators, which the warp copies
+// kPathStages substeps ahead into shared memory.  What bounds it is reading them
+// from there (40 cycles of the multiprocessor's load path a substep, FMAs 38), so
+// a lane walks two neighbouring pairs on one read (10,000 particles: 226 us with one pair
+// per lane and 4 particles per warp, 153 now).  Groups of 8 neighbours by lo
+// take 131 steps for 32 of the reference's hourly pairs, groups of 32 take 232.
+__global__ void __launch_bounds__(32) moment_path_kernel(MomArgs a, MomScratch ws,
+                                                         const __grid_constant__ MomPlan plan) {
+  __shared__ float4 ring[kPathStages][2][kQuads][kPathParticles];
+  const int JA = plan.n, nsub = a.nsub, lane = threadIdx.x;
+  const int64_t n = ws.n;
+  const int pi = lane % kPathParticles, slot = (int)blockIdx.y * kPathGroup + lane / kPathParticles * 2;
+  const int64_t i = (int64_t)blockIdx.x * kPathParticles + pi;
+  const bool good = i < n && ws.rates[kRateBad * n + (i < n ? i : 0)] == 0.0f;
+  bool live[2];
+  int lo[2], hi[2], end[2];
+  unsigned first = 0x7fffffffu, last = 0, un = 0x7fffffffu, la = 0;
+  float y[2][NA];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    live[e] = good && slot + e < JA;
+    lo[e] = live[e] ? max(plan.lo[slot + e], 0) : 0x7fffffff;
+    end[e] = live[e] ? max(plan.end[slot + e], 0) : 0;
+    hi[e] = live[e] ? min(max(plan.hi[slot + e], 0), end[e]) : 0;
+    if (live[e]) {
+      first = min(first, (unsigned)lo[e]);
+      last = max(last, (unsigned)end[e]);
+      un = min(un, (unsigned)hi[e]);
+      la = max(la, (unsigned)hi[e]);
+    }
+#pragma unroll
+    for (int r = 0; r < NA; ++r) y[e][r] = live[e] ? ws.start[((int64_t)(slot + e) * n + i) * NA + r] : 0.0f;
+  }
+  // substeps s0 .. s1 of the warp; the unlabelled propagators serve from un on, the labelled ones up to la
+  const int s0 = (int)__reduce_min_sync(0xffffffffu, first), s1 = (int)__reduce_max_sync(0xffffffffu, last);
+  un = __reduce_min_sync(0xffffffffu, un);
+  la = __reduce_max_sync(0xffffffffu, la);
+  const int64_t src0 = lane / kPathParticles * n + min(i, n - 1);
+  auto fetch = [&](int s, int sub) {
+#pragma unroll
+    for (int lab = 0; lab < 2; ++lab) {
+      if (s >= s1 || (lab ? s >= (int)la : s < (int)un)) continue;
+      const float4* src = ws.props + (int64_t)(lab * nsub + sub) * kQuads * n + src0;
+      float4* dst = &ring[s % kPathStages][lab][0][0] + lane;
+#pragma unroll
+      for (int q = 0; q < kQuads * kPathParticles; q += 32)
+        if (q + lane < kQuads * kPathParticles) cp_async16(dst + q, src + q / kPathParticles * n);
+    }
+    cp_async_commit();
+  };
+  int idx = s0 % nsub, ahead = idx;
+  for (int t = 0; t < kPathStages - 1; ++t) {
+    fetch(s0 + t, ahead);
+    if (++ahead == nsub) ahead = 0;
+  }
+  for (int s = s0; s < s1; ++s) {
+    cp_async_wait<kPathStages - 2>();
+    __syncwarp();  // every lane's pieces of substep s are there, and the slot read last is free
+    fetch(s + kPathStages - 1, ahead);
+    if (++ahead == nsub) ahead = 0;
+    const bool on0 = s >= lo[0] && s < end[0], on1 = s >= lo[1] && s < end[1];
+    const bool lab0 = s < hi[0], lab1 = s < hi[1];
+    if (on0 || on1) {
+      const float4(*src)[kQuads][kPathParticles] = ring[s % kPathStages];
+      Prop P;
+      load_prop(&src[(on0 ? lab0 : lab1) ? 1 : 0][0][pi], kPathParticles, P);
+      if (on0) {
+        if (idx == 0 && s > 0) divide_p(y[0]);
+        apply(P, y[0]);
+      }
+      if (on1) {
+        if (on0 && lab0 != lab1) load_prop(&src[lab1 ? 1 : 0][0][pi], kPathParticles, P);
+        if (idx == 0 && s > 0) divide_p(y[1]);
+        apply(P, y[1]);
+      }
+    }
+    if (++idx == nsub) idx = 0;
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    if (!live[e]) continue;
+    float* mo = ws.mom + ((int64_t)i * JA + plan.pair[slot + e]) * 5;
+    mo[0] = y[e][3];
+    mo[1] = y[e][4];
+    mo[2] = y[e][7];
+    mo[3] = y[e][8];
+    mo[4] = y[e][9];
+  }
+}
+
+constexpr int kStatParticles = 8;
+inline size_t stat_smem(int pairs) { return (size_t)kStatParticles * pairs * 5 * sizeof(double); }
+
+// capture transform (model.jl:221-239) per (condition, age), then the
+// statistics per condition
+__global__ void __launch_bounds__(128) moment_stats_kernel(MomArgs a, int64_t p0, MomScratch ws) {
+  extern __shared__ double ds[];  // [particle][JA][5]
+  const DevCfg& cfg = a.cfg;
+  const int J = cfg.n_conds, A = cfg.n_ages, JA = J * A, K = 4 * A + 3 * J;
+  const int64_t i0 = (int64_t)blockIdx.x * kStatParticles, n = ws.n;
+  const int np = (int)min((int64_t)kStatParticles, n - i0);
+  const float* bad = ws.rates + kRateBad * n + i0;
+  for (int q = threadIdx.x; q < np * JA; q += blockDim.x) {
+    const int i = q / JA, t = q - i * JA;
+    if (bad[i] != 0.0f) continue;
+    const int j = t / A, ai = t - (t / A) * A;
+    const double* bm = a.beta_mom + ((j < a.n_pulse_conds ? 0 : 1) * A + ai) * 3;
+    const double mb = bm[0], m2 = bm[1], vb = bm[2];
+    double sm[5];
+#pragma unroll
+    for (int e = 0; e < 5; ++e) sm[e] = ws.mom[(i0 * JA + q) * 5 + e];
+    double* d = ds + (size_t)q * 5;
+    d[0] = sm[0] * mb;
+    d[1] = sm[1] * mb;
+    d[2] = ((mb - m2) * sm[0] + vb * (sm[0] * sm[0] + sm[2])) + mb * mb * sm[2];
+    d[4] = ((mb - m2) * sm[1] + vb * (sm[1] * sm[1] + sm[4])) + mb * mb * sm[4];
+    d[3] = vb * (sm[0] * sm[1] + sm[3]) + mb * mb * sm[3];
+    if (a.moments)
+#pragma unroll
+      for (int e = 0; e < 5; ++e) a.moments[((p0 + i0) * JA + q) * 5 + e] = sm[e];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < np * J; q += blockDim.x) {
+    const int i = q / J, j = q - i * J;
+    if (bad[i] == 0.0f)
+      stats_from_moments_cond(cfg, ds + (size_t)i * JA * 5, a.age_dist, a.stats + (p0 + i0 + i) * K, j);
+  }
+  for (int q = threadIdx.x; q < np * K; q += blockDim.x) {
+    const int i = q / K;
+    if (bad[i] == 0.0f) continue;
+    a.stats[(p0 + i0) * K + q] = NAN;
+    if (q == i * K) atomicOr(a.status, 1);
+  }
+}
+
+// particles per chunk: propagators of at most ~256 MB
+int64_t moment_chunk(int64_t P, int nsub) {
+  const int64_t bytes = (int64_t)2 * nsub * kQuads * (int64_t)sizeof(float4);
+  return std::max<int64_t>(1, std::min<int64_t>(P, ((int64_t)256 << 20) / bytes));
 }
 
 }  // namespace
 
-size_t moment_f32_scratch_per_cta(int nsub) { return (size_t)2 * nsub * NT * sizeof(float); }
+size_t moment_f32_scratch(int64_t P, int nsub, int pairs) {
+  const size_t n = (size_t)moment_chunk(P, nsub);
+  return n * ((2 * (size_t)nsub + 1) * kQuads * sizeof(float4) + ((size_t)pairs * (NA + 5) + kRates) * sizeof(float));
+}
 
-cudaError_t launch_moment_f32(const MomArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_moment_f32(const MomArgs& a, cudaStream_t s) {
   if (a.P <= 0) return cudaSuccess;
-  moment_kernel_f32<<<grid, kThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  const DevCfg& cfg = a.cfg;
+  const int A = cfg.n_ages, pairs = cfg.n_conds * A;
+  MomPlan plan;
+  plan.n = pairs;
+  int lo[kMaxPairs];
+  for (int t = 0; t < pairs; ++t) {
+    const double age = cfg.ages[t % A], texp = (age - cfg.pulse[t / A]) - cfg.chase[t / A];
+    lo[t] = (int)std::min(std::lround((texp - cfg.t0) / a.h), std::lround((age - cfg.t0) / a.h));
+    plan.pair[t] = t;
+  }
+  std::sort(plan.pair, plan.pair + pairs, [&](int x, int y) { return lo[x] != lo[y] ? lo[x] < lo[y] : x < y; });
+  for (int q = 0; q < pairs; ++q) {
+    const int t = plan.pair[q];
+    const double age = cfg.ages[t % A], texp = (age - cfg.pulse[t / A]) - cfg.chase[t / A];
+    plan.lo[q] = lo[t];
+    plan.hi[q] = (int)std::lround((texp + cfg.pulse[t / A] - cfg.t0) / a.h);
+    plan.end[q] = (int)std::lround((age - cfg.t0) / a.h);
+  }
+  const int64_t chunk = moment_chunk(a.P, a.nsub);
+  for (int64_t p0 = 0; p0 < a.P; p0 += chunk) {
+    const int64_t n = std::min<int64_t>(chunk, a.P - p0);
+    MomScratch ws;
+    ws.n = n;
+    ws.props = reinterpret_cast<float4*>(a.scratch);
+    ws.phi = ws.props + (size_t)n * 2 * a.nsub * kQuads;
+    ws.start = reinterpret_cast<float*>(ws.phi + (size_t)n * kQuads);
+    ws.mom = ws.start + (size_t)n * pairs * NA;
+    ws.rates = ws.mom + (size_t)n * pairs * 5;
+    moment_rates_kernel<<<(unsigned)((n + 31) / 32), 32, 0, s>>>(a, p0, ws);
+    moment_exp_kernel<<<dim3((unsigned)((n + kExpThreads - 1) / kExpThreads), 2 * a.nsub), kExpThreads, 0, s>>>(a, ws);
+    moment_cycle_kernel<<<(unsigned)((n + kCycleParticles - 1) / kCycleParticles), kCycleParticles * kQuarters * NA, 0,
+                          s>>>(a.nsub, ws);
+    moment_walk_kernel<<<(unsigned)((n + 31) / 32), 32, 0, s>>>(a, p0, ws, plan);
+    moment_path_kernel<<<dim3((unsigned)((n + kPathParticles - 1) / kPathParticles),
+                              (pairs + kPathGroup - 1) / kPathGroup), 32, 0, s>>>(a, ws, plan);
+    moment_stats_kernel<<<(unsigned)((n + kStatParticles - 1) / kStatParticles), 128, stat_smem(pairs), s>>>(a, p0, ws);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace abc
