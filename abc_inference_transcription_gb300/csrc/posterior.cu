@@ -5,10 +5,7 @@
 // FP64, built with -fmad=false: results are bit-identical to the C oracle.
 #include <cuda_runtime.h>
 
-#include <atomic>
-
 #include "common.cuh"
-#include "smem_attr.h"
 #include "kernels.h"
 
 namespace abc {
@@ -45,7 +42,7 @@ __global__ void post_gather_kernel(const int64_t* aoff, const int64_t* idx, cons
   }
 }
 
-constexpr int kPostSmem = 8192;   // columns up to this size are staged in shared memory
+constexpr int kPostSmem = 2048;   // columns up to this size are staged in shared memory (8 blocks of 18 KB per SM)
 constexpr int kSelThreads = 256;
 constexpr int kSelSmall = 64;     // candidate sets this small are ranked by counting
 
@@ -63,19 +60,20 @@ struct SelShared {
   unsigned hist[256];
   uint64_t cand[kSelSmall];
   uint64_t result;
-  int bin, cnt, ncand;
+  unsigned long long next;
+  int bin, cnt, ncand, upto;
   long long rr;
 };
 
-// The rank-th smallest (0-based) of the n keys K: radix select over 8-bit
-// digits from the top, narrowing to the digit bucket that holds the rank;
+// The rank-th smallest (0-based) of the n keys K (below 2^(top + 8)): radix
+// select over 8-bit digits from the top, narrowing to the digit bucket that holds the rank;
 // once the bucket has at most kSelSmall keys they are collected and the rank
 // is found by counting.  Every thread of the block calls it.
-__device__ uint64_t block_select(const uint64_t* K, int64_t n, int64_t rank, SelShared& sh) {
+__device__ uint64_t block_select(const uint64_t* K, int64_t n, int64_t rank, int top, SelShared& sh) {
   uint64_t prefix = 0, mask = 0;
   long long rr = rank;
   const int lane = threadIdx.x & 31;
-  for (int shift = 56; shift >= 0; shift -= 8) {
+  for (int shift = top; shift >= 0; shift -= 8) {
     for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.hist[i] = 0u;
     __syncthreads();
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -142,10 +140,44 @@ __device__ uint64_t block_select(const uint64_t* K, int64_t n, int64_t rank, Sel
   return prefix;
 }
 
+// The keys of rank and rank + 1 (rank alone, twice, if n = 1): the second is the first
+// again where it is repeated beyond that rank, else the smallest key above it, which one
+// more pass finds; a second select takes three.
+__device__ void block_select2(const uint64_t* K, int64_t n, int64_t rank, int top, SelShared& sh, uint64_t& a,
+                              uint64_t& b) {
+  a = block_select(K, n, rank, top, sh);
+  if (threadIdx.x == 0) {
+    sh.upto = 0;
+    sh.next = ~0ull;
+  }
+  __syncthreads();
+  int upto = 0;
+  uint64_t next = ~0ull;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const uint64_t k = K[i];
+    if (k <= a) ++upto;
+    else if (k < next) next = k;
+  }
+  for (int o = 16; o; o >>= 1) {
+    const uint64_t other = __shfl_xor_sync(0xffffffffu, next, o);
+    next = other < next ? other : next;
+  }
+  upto = __reduce_add_sync(0xffffffffu, upto);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&sh.upto, upto);
+    atomicMin(&sh.next, (unsigned long long)next);
+  }
+  __syncthreads();
+  b = sh.upto > rank + 1 || n == 1 ? a : sh.next;
+  __syncthreads();
+}
+
 // Per (parameter, gene) column of the gathered values, the order statistics
 // the two quantiles read: q4 = {v[j_lo - 1], v[j_lo], v[j_hi - 1], v[j_hi]} of
 // the sorted column (quantile_pos with p = 1 - q and p = q).  Columns longer
-// than kPostSmem are keyed in place in the scratch.
+// than kPostSmem are keyed in place in the scratch.  Bound by the barriers of the
+// passes: two selects and two extra passes instead of four selects, and eight blocks per
+// multiprocessor instead of three (487 genes x 6 parameters, 343 values each: 101 us, 55 now).
 __global__ void __launch_bounds__(kSelThreads) post_select_kernel(const int64_t* aoff, int64_t total, int64_t G,
                                                                   double* scratch, double q, double* q4) {
   extern __shared__ uint64_t sel_keys[];
@@ -173,11 +205,42 @@ __global__ void __launch_bounds__(kSelThreads) post_select_kernel(const int64_t*
   double gl, gh;
   quantile_pos(n, 1.0 - q, jl, gl);
   quantile_pos(n, q, jh, gh);
-  const int64_t ranks[4] = {jl - 1, jl, jh - 1, jh};
-  for (int r = 0; r < 4; ++r) {
-    const uint64_t k = block_select(K, n, ranks[r], sh);
-    if (threadIdx.x == 0) out[r] = dkey_inv(k);
+  for (int r = 0; r < 2; ++r) {
+    uint64_t a, b;
+    block_select2(K, n, (r ? jh : jl) - 1, 56, sh, a, b);
+    if (threadIdx.x == 0) {
+      out[2 * r] = dkey_inv(a);
+      out[2 * r + 1] = dkey_inv(b);
+    }
   }
+}
+
+// Means of the gathered columns, a thread per (parameter, gene).  The sum runs in the order of
+// the list (FP64, as the oracle's), so a column is one chain of additions; loads go
+// kMeanAhead values ahead of it (343 values per column: 40 us, where gathering through
+// the indices inside the chain took 100).
+constexpr int kMeanAhead = 8;
+__global__ void __launch_bounds__(32) post_mean_kernel(const int64_t* aoff, int64_t total, int64_t G, int npar,
+                                                       const double* scratch, double* mean) {
+  const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
+  if (t >= G * npar) return;
+  const int64_t c = t / G, g = t - c * G;
+  const int64_t o = aoff[g], n = aoff[g + 1] - o;
+  if (n == 0) return;
+  const double* v = scratch + c * total + o;
+  double s = 0.0, cur[kMeanAhead], nxt[kMeanAhead];
+#pragma unroll
+  for (int u = 0; u < kMeanAhead; ++u) cur[u] = u < n ? v[u] : 0.0;
+  for (int64_t i = 0; i < n; i += kMeanAhead) {
+#pragma unroll
+    for (int u = 0; u < kMeanAhead; ++u) nxt[u] = i + kMeanAhead + u < n ? v[i + kMeanAhead + u] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kMeanAhead; ++u)
+      if (i + u < n) s = s + cur[u];
+#pragma unroll
+    for (int u = 0; u < kMeanAhead; ++u) cur[u] = nxt[u];
+  }
+  mean[g * npar + c] = s / (double)n;
 }
 
 // One block per gene.  counts[g][m] = accepted particles of model group m.
@@ -186,8 +249,11 @@ __global__ void __launch_bounds__(kSelThreads) post_select_kernel(const int64_t*
 // bootstrap resamples of the sum(l) model labels (a multinomial draw, made
 // as conditional binomials from the (bootstrap, gene) Philox stream; the
 // block's threads take the resamples), with quantiles 1 - alpha and alpha of
-// the resampled proportions from the order statistics they read
-// (block_select on order-preserving keys; keys: G x M x n_boot scratch).
+// the resampled proportions from the order statistics they read.  The keys
+// (G x M x n_boot scratch) are the resampled counts: x / L rises with x, so only
+// the four that are read are divided, and the select starts at the highest digit of L.
+// Bound by the binomials' FP64 (487 genes, 2 groups, 100 resamples: 188 us with keys
+// of the divided proportions and four selects, 175 now).
 __global__ void __launch_bounds__(kSelThreads) model_probs_kernel(const int64_t* counts, int64_t G, int M,
                                                                   int n_boot, double alpha, uint64_t seed,
                                                                   double* prob, double* lb, double* ub,
@@ -237,7 +303,7 @@ __global__ void __launch_bounds__(kSelThreads) model_probs_kernel(const int64_t*
       else x = binomial(r, nrem, (double)l[m] / (double)lrem);
       nrem -= x;
       lrem -= l[m];
-      kv[(int64_t)m * n_boot + b] = dkey((double)x / (double)L);
+      kv[(int64_t)m * n_boot + b] = (uint64_t)x;
     }
   }
   __syncthreads();
@@ -245,14 +311,14 @@ __global__ void __launch_bounds__(kSelThreads) model_probs_kernel(const int64_t*
   double gl, gh;
   quantile_pos(n_boot, 1.0 - alpha, jl, gl);
   quantile_pos(n_boot, alpha, jh, gh);
-  const int64_t ranks[4] = {n_boot == 1 ? 0 : jl - 1, n_boot == 1 ? 0 : jl, n_boot == 1 ? 0 : jh - 1,
-                            n_boot == 1 ? 0 : jh};
+  const int top = (63 - __clzll(L)) / 8 * 8;
   for (int m = 0; m < M; ++m) {
-    double q[4];
-    for (int r = 0; r < 4; ++r) q[r] = dkey_inv(block_select(kv + (int64_t)m * n_boot, n_boot, ranks[r], sh));
+    uint64_t x[4];
+    block_select2(kv + (int64_t)m * n_boot, n_boot, n_boot == 1 ? 0 : jl - 1, top, sh, x[0], x[1]);
+    block_select2(kv + (int64_t)m * n_boot, n_boot, n_boot == 1 ? 0 : jh - 1, top, sh, x[2], x[3]);
     if (threadIdx.x == 0) {
-      LB[m] = quantile_mix(q[0], q[1], gl);
-      UB[m] = quantile_mix(q[2], q[3], gh);
+      LB[m] = quantile_mix((double)x[0] / (double)L, (double)x[1] / (double)L, gl);
+      UB[m] = quantile_mix((double)x[2] / (double)L, (double)x[3] / (double)L, gh);
     }
   }
 }
@@ -282,9 +348,6 @@ __global__ void post_summary_kernel(const int64_t* aoff, const int64_t* idx, con
     return;
   }
   map[t] = theta[(idx[o] - 1) * ld + c];
-  double s = 0.0;
-  for (int64_t i = 0; i < n; ++i) s = s + theta[(idx[o + i] - 1) * ld + c];
-  mean[t] = s / (double)n;
   const double* v4 = q4 + ((int64_t)c * G + g) * 4;
   int64_t j;
   double gl, gh;
@@ -304,9 +367,7 @@ cudaError_t launch_posterior_summary(const int64_t* aoff, const int64_t* idx, in
   if (total > 0) {
     post_gather_kernel<<<(unsigned)G, 256, 0, s>>>(aoff, idx, theta, ld, npar, total, scratch);
     constexpr int smem = kPostSmem * (int)sizeof(uint64_t);
-    static std::atomic<uint64_t> attr{0};  // devices where the limit is set, shared by all contexts
-    cudaError_t e = set_smem_once(attr, post_select_kernel, smem);
-    if (e != cudaSuccess) return e;
+    post_mean_kernel<<<(unsigned)((G * npar + 31) / 32), 32, 0, s>>>(aoff, total, G, npar, scratch, mean);
     post_select_kernel<<<(unsigned)(G * npar), kSelThreads, smem, s>>>(aoff, total, G, scratch, q, q4);
   }
   const int64_t n = G * npar;
