@@ -5,8 +5,8 @@
 //   (blockIdx.y = m tile + split * m tiles) for the weight gradients.
 // Warp 0 issues TMA loads (3D maps: reduction, rows, member; 64-wide BF16 boxes
 // with the 128-byte swizzle) into a 3-stage ring; one lane of warp 1 issues
-// tcgen05.mma.kind::f16 (M = N = 128, K = 16); all four warps then read their
-// 32 accumulator rows with tcgen05.ld and apply the fused epilogue (bias +
+// tcgen05.mma.kind::f16 (M = N = 128, K = 16); all eight warps then read their 32
+// accumulator rows x 64 columns with tcgen05.ld and apply the fused epilogue (bias +
 // SiLU, bias, one partial sum per reduction split, or the SiLU derivative), writing the
 // row-major result and, where the backward pass needs it, the transposed
 // BF16 copy.  Waits are bounded (about one second); a wait that runs out sets
@@ -66,9 +66,76 @@ constexpr uint32_t kTileBytes = BM * BK * 2;  // A and B tiles alike (BN = BM)
 constexpr uint32_t kStageBytes = 2 * kTileBytes;
 constexpr uint32_t kTmemCols = 128;
 constexpr int kSmem = 1024 + kStages * kStageBytes + 128;
+constexpr int kThreads = 256;
+constexpr int kChunk = 32;  // rows and columns of an epilogue chunk
+// row strides of a staged chunk, in words: 16-byte pieces of eight neighbouring lanes fall
+// on distinct banks, by rows and by columns
+constexpr int kRowF = kChunk + 4, kRowH = kChunk / 2 + 4;
+static_assert(kThreads / 32 * kChunk * kRowF * 4 <= kStages * kStageBytes, "the stages hold the warps' chunks");
+
+// What bounds the epilogue is the load/store path: a lane holds a row of the chunk, and a
+// 16-byte access per lane touches 32 rows.  Through shared memory the warp's
+// accesses take whole rows instead, 4 (FP32) or 8 (BF16) of them at a time.
+// rows, cols: what of the chunk is inside the matrix.
+__device__ __forceinline__ void store_rows_f32(float* sm, const float (&x)[kChunk], float* base, int64_t ld, int rows,
+                                               int cols, int lane) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *(float4*)(sm + lane * kRowF + 4 * q) = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+  __syncwarp();
+  const int r = lane / 8, c = lane % 8 * 4;
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+    if (4 * t + r < rows && c < cols) *(float4*)(base + (4 * t + r) * ld + c) = *(const float4*)(sm + (4 * t + r) * kRowF + c);
+  __syncwarp();
+}
+
+__device__ __forceinline__ void load_rows_f32(float* sm, float (&x)[kChunk], const float* base, int64_t ld, int rows,
+                                              int cols, int lane) {
+  const int r = lane / 8, c = lane % 8 * 4;
+  float4 v[8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+    v[t] = 4 * t + r < rows && c < cols ? *(const float4*)(base + (4 * t + r) * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int t = 0; t < 8; ++t) *(float4*)(sm + (4 * t + r) * kRowF + c) = v[t];
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 w = *(const float4*)(sm + lane * kRowF + 4 * q);
+    x[4 * q] = w.x; x[4 * q + 1] = w.y; x[4 * q + 2] = w.z; x[4 * q + 3] = w.w;
+  }
+  __syncwarp();
+}
+
+// also the transposed copy, whose accesses are whole columns as the lanes stand
+__device__ __forceinline__ void store_rows_bf16(float* sm, const float (&x)[kChunk], __nv_bfloat16* base, int64_t ld,
+                                                __nv_bfloat16* baseT, int64_t ldT, int rows, int cols, int lane) {
+  uint32_t* sw = reinterpret_cast<uint32_t*>(sm);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    __nv_bfloat16 h[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16(x[8 * q + j]);
+    uint4 pk;
+    memcpy(&pk, h, 16);
+    *(uint4*)(sw + lane * kRowH + 4 * q) = pk;
+    if (baseT && 8 * q < cols && lane < rows) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) baseT[(int64_t)(8 * q + j) * ldT + lane] = h[j];
+    }
+  }
+  __syncwarp();
+  const int r = lane / 4, c = lane % 4 * 8;
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (8 * t + r < rows && c < cols)
+      *(uint4*)(base + (8 * t + r) * ld + c) = *(const uint4*)(sw + (8 * t + r) * kRowH + c / 2);
+  __syncwarp();
+}
 
 template <int EPI>
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(kThreads, 2)
     mlp_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcGemm g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
@@ -143,77 +210,75 @@ __global__ void __launch_bounds__(128, 1)
     }
     mma_commit(done);  // arrives once every MMA above has completed
   }
-  // ---- epilogue: warp w holds accumulator rows 32 w .. 32 w + 31
+  // ---- epilogue: warp w holds accumulator rows 32 (w % 4) .. + 31, columns
+  // 64 (w / 4) .. + 63, in chunks staged where the operand tiles were: every
+  // copy has landed and every MMA has read its tiles once `done` has come.  N and
+  // every row length are multiples of 16 values.  4,096 rows x 256 x 4 members: a hidden
+  // layer 20 us with four warps and a row per lane, 14 now; its derivative 17.5, 13.6; a
+  // weight gradient 10.3, 8.7.
   bool have = work && mbar_wait(done, 0);
   have = __all_sync(0xffffffffu, have);
   if (work && !have && lane == 0) atomicOr(g.err, 4);
   tc_fence_after();
-  const int m = m0 + warp * 32 + lane;
-  const uint32_t lane_addr = tbase + ((uint32_t)(warp * 32) << 16);
-  if (have) {
-    const float* bias = g.bias ? g.bias + z * g.sBias : nullptr;
-    // A lane holds 32 neighbouring columns of its row, which it writes (and
-    // reads, EPI_DSILU) 16 bytes at a time: N and every row length are
-    // multiples of 16 values.  One value at a time, each warp store touched 32
-    // rows, and a hidden layer of 4 x 65,536 rows took 0.70 ms instead of
-    // 0.20.  The transposed copy is coalesced across the lanes.
+  const int m_w = m0 + warp % 4 * 32;
+  const uint32_t lane_addr = tbase + ((uint32_t)(warp % 4 * 32) << 16);
+  float* sm = reinterpret_cast<float*>(smem) + warp * kChunk * kRowF;
+  if (have && m_w < g.M) {
+    const int rows = min(kChunk, g.M - m_w);
 #pragma unroll 1
-    for (int cc = 0; cc < BN / 32; ++cc) {
-      const int nb = n0 + cc * 32;
+    for (int cc = warp / 4 * 2; cc < warp / 4 * 2 + 2; ++cc) {
+      const int nb = n0 + cc * kChunk;
       if (nb >= g.N) break;
-      __syncwarp();
-      uint32_t v[32];
-      tmem_ld32(lane_addr + (uint32_t)(cc * 32), v);
-      if (m >= g.M) continue;
+      const int cols = min(kChunk, g.N - nb);
+      float x[kChunk];
+      {
+        uint32_t v[32];
+        tmem_ld32(lane_addr + (uint32_t)(cc * kChunk), v);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int n = nb + 8 * q;
-        if (n >= g.N) break;
-        float x[8];
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
+      }
+      if ((EPI == EPI_HIDDEN || EPI == EPI_LINEAR) && g.bias) {
+        const float* bias = g.bias + z * g.sBias + nb;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[8 * q + j]);
-        if (EPI == EPI_HIDDEN || EPI == EPI_LINEAR) {
-          if (bias) {
-            const float4 b0 = *(const float4*)(bias + n), b1 = *(const float4*)(bias + n + 4);
-            x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
-            x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
-          }
-        }
-        if (EPI == EPI_DSILU) {
-          const float* zp = g.zprev + z * g.sZ + (int64_t)m * g.ldz + n;
-          const float4 p0 = *(const float4*)zp, p1 = *(const float4*)(zp + 4);
-          const float zq[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-          float sg[8];
-          sigm8(zq, sg);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) x[j] = x[j] * (sg[j] * (1.0f + zq[j] * (1.0f - sg[j])));
-        }
-        if (EPI != EPI_DSILU && g.outf) {
-          float* o = g.outf + z * g.sOutf + (int64_t)m * g.ldf + n;
-          if (EPI == EPI_PARTIAL) o += split * g.sSplit;
-          *(float4*)o = make_float4(x[0], x[1], x[2], x[3]);
-          *(float4*)(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
-        }
-        if (EPI == EPI_HIDDEN || EPI == EPI_DSILU) {
-          if (EPI == EPI_HIDDEN) {
-            float sg[8];
-            sigm8(x, sg);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = x[j] * sg[j];
-          }
-          __nv_bfloat16 h[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16(x[j]);
-          uint4 pk;
-          memcpy(&pk, h, 16);
-          *(uint4*)(g.outh + z * g.sOuth + (int64_t)m * g.ldh + n) = pk;
-          if (g.outhT) {
-            __nv_bfloat16* oT = g.outhT + z * g.sOuthT + (int64_t)n * g.ldhT + m;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) oT[(int64_t)j * g.ldhT] = h[j];
-          }
+        for (int q = 0; q < 8; ++q) {
+          if (4 * q >= cols) break;
+          const float4 b = *(const float4*)(bias + 4 * q);
+          x[4 * q] += b.x; x[4 * q + 1] += b.y; x[4 * q + 2] += b.z; x[4 * q + 3] += b.w;
         }
       }
+      if (EPI == EPI_DSILU) {
+        float zp[kChunk];
+        load_rows_f32(sm, zp, g.zprev + z * g.sZ + (int64_t)m_w * g.ldz + nb, g.ldz, rows, cols, lane);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float zq[8], sg[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) zq[j] = zp[8 * q + j];
+          sigm8(zq, sg);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[8 * q + j] = x[8 * q + j] * (sg[j] * (1.0f + zq[j] * (1.0f - sg[j])));
+        }
+      }
+      if (EPI != EPI_DSILU && g.outf) {
+        float* o = g.outf + z * g.sOutf + (int64_t)m_w * g.ldf + nb;
+        if (EPI == EPI_PARTIAL) o += split * g.sSplit;
+        store_rows_f32(sm, x, o, g.ldf, rows, cols, lane);
+      }
+      if (EPI == EPI_HIDDEN) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float xq[8], sg[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) xq[j] = x[8 * q + j];
+          sigm8(xq, sg);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[8 * q + j] = xq[j] * sg[j];
+        }
+      }
+      if (EPI == EPI_HIDDEN || EPI == EPI_DSILU)
+        store_rows_bf16(sm, x, g.outh + z * g.sOuth + (int64_t)m_w * g.ldh + nb, g.ldh,
+                        g.outhT ? g.outhT + z * g.sOuthT + (int64_t)nb * g.ldhT + m_w : nullptr, g.ldhT, rows, cols,
+                        lane);
     }
   }
   tc_fence_before();
@@ -229,7 +294,7 @@ cudaError_t launch_epi(const CUtensorMap& ma, const CUtensorMap& mb, const TcGem
   if (e != cudaSuccess) return e;
   const int n_mt = (g.M + BM - 1) / BM;
   dim3 grid((unsigned)((g.N + BN - 1) / BN), (unsigned)(n_mt * g.k_split), (unsigned)members);
-  mlp_tc_kernel<EPI><<<grid, 128, kSmem, s>>>(ma, mb, g);
+  mlp_tc_kernel<EPI><<<grid, kThreads, kSmem, s>>>(ma, mb, g);
   return cudaGetLastError();
 }
 
