@@ -119,148 +119,249 @@ __global__ void __launch_bounds__(256) mlp_gather_kernel(const float* xn, const 
 // Gaussian negative log-likelihood on standardised targets; dY = dL/dY / count.
 constexpr float kLvMin = -9.0f, kLvMax = 9.0f;
 
+// A launch has two kinds of blocks.  The first sum the loss over the pairs in the
+// order of nb blocks' grid-stride loops (a training run is reproducible bit for
+// bit), kLossBlocks of them at a time: one each, the launch was four waves of blocks
+// waiting for their loads (21 us for 4 x 4,096 rows of 53 statistics, 17 now).  The
+// others take kLossRows rows of the gradient each, whose transposed copy goes
+// through shared memory.
+constexpr int kLossRows = 32, kLossBlocks = 4;
 __global__ void __launch_bounds__(256) mlp_loss_kernel(const float* Y, const float* T, int B, int K, int out_pad,
                                                        float inv_count, __nv_bfloat16* dY, __nv_bfloat16* dYT, int ldT,
-                                                       float* loss_part, int64_t sY, int64_t sT) {
-  const int e = blockIdx.y;
-  float local = 0.0f;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < B * out_pad; idx += gridDim.x * blockDim.x) {
-    const int i = idx / out_pad, c = idx - (idx / out_pad) * out_pad;
-    float grad = 0.0f;
-    if (c < K) {
-      const float t = T[e * sT + (int64_t)i * K + c];
-      if (t == t) {
-        const float mu = Y[e * sY + (int64_t)i * out_pad + c];
-        const float lv_raw = Y[e * sY + (int64_t)i * out_pad + K + c];
-        const float lv = fminf(fmaxf(lv_raw, kLvMin), kLvMax);
-        const float r = t - mu;
-        const float ei = __expf(-lv);
-        local += 0.5f * (lv + r * r * ei);
-        grad = -r * ei * inv_count;
-      }
-    } else if (c < 2 * K) {
-      const float t = T[e * sT + (int64_t)i * K + (c - K)];
-      if (t == t) {
-        const float mu = Y[e * sY + (int64_t)i * out_pad + (c - K)];
-        const float lv_raw = Y[e * sY + (int64_t)i * out_pad + c];
-        const bool inside = lv_raw > kLvMin && lv_raw < kLvMax;
-        const float lv = fminf(fmaxf(lv_raw, kLvMin), kLvMax);
-        const float r = t - mu;
-        grad = inside ? 0.5f * (1.0f - r * r * __expf(-lv)) * inv_count : 0.0f;
-      }
-    }
-    const __nv_bfloat16 gb = __float2bfloat16(grad);
-    dY[e * sY + idx] = gb;
-    dYT[(int64_t)e * out_pad * ldT + (int64_t)c * ldT + i] = gb;
-  }
-  // block sum in a fixed order: warps by shuffles, then warp 0 over the warp sums
-  __shared__ float wsum[8];
-  for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = local;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w];
-    loss_part[e * gridDim.x + blockIdx.x] = t * inv_count;
-  }
-}
-
-// loss[e] += sum of the member's block partials, in block order (the epoch
-// loss accumulates over the batches in stream order).  The chain of additions
-// reads shared memory: from global memory 1,024 partials took 25 us.
-__global__ void __launch_bounds__(1024) mlp_loss_sum_kernel(const float* loss_part, int n_blocks, float* loss) {
-  __shared__ float part[1024];
-  const int e = blockIdx.x;
-  float t = 0.0f;
-  for (int b0 = 0; b0 < n_blocks; b0 += 1024) {
-    const int nb = min(1024, n_blocks - b0);
-    if ((int)threadIdx.x < nb) part[threadIdx.x] = loss_part[e * n_blocks + b0 + threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll 16
-      for (int b = 0; b < nb; ++b) t += part[b];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) loss[e] += t;
-}
-
-// out[z][i] = sum over the used reduction splits of part[split][z][i], in split
-// order, for the weights of every layer (the biases between them are column
-// sums); four parameters per thread, every block size a multiple of 16
-__global__ void __launch_bounds__(256) mlp_split_sum_kernel(const float* part, int used, int64_t sSplit, MlpDims d,
-                                                            float* out) {
-  const int z = blockIdx.y;
-  for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < d.n_params;
-       i += 4 * (int64_t)gridDim.x * blockDim.x) {
-    if ((i >= d.off_b1 && i < d.off_w2) || (i >= d.off_b2 && i < d.off_w3) || (i >= d.off_b3 && i < d.off_w4) ||
-        i >= d.off_b4)
-      continue;
-    const float* p = part + z * d.n_params + i;
-    float4 acc = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-    for (int sp = 0; sp < used; ++sp) {
-      const float4 v = *(const float4*)(p + sp * sSplit);
-      acc.x += v.x;
-      acc.y += v.y;
-      acc.z += v.z;
-      acc.w += v.w;
-    }
-    *(float4*)(out + z * d.n_params + i) = acc;
-  }
-}
-
-// db[n] = sum_i dZ[i][n] for every member, in row order (a training run is
-// reproducible bit for bit, and independent of the launch), from the transposed
-// copy [n][ldT].  The additions are one chain per column, so a warp takes a
-// column: its lanes load 256 rows at once (coalesced, the next 256 in flight) and
-// pass them through shared memory to the chain.  4,096 rows: 15 us, against
-// 39 with a lane per column and 266 down dZ's columns.
-constexpr int kColWarps = 4;
-__global__ void __launch_bounds__(32 * kColWarps) mlp_colsum_kernel(const __nv_bfloat16* dZT, int B, int N, int ldT,
-                                                                    int64_t sZT, float* db, int64_t sDb) {
-  __shared__ uint4 stage[kColWarps][32];
-  const int e = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = blockIdx.x * kColWarps + warp;
-  if (n >= N) return;
-  const __nv_bfloat16* row = dZT + e * sZT + (int64_t)n * ldT;
-  const uint4* src = reinterpret_cast<const uint4*>(row);
-  const int groups = B / 256;
-  float s = 0.0f;
-  uint4 nxt = {0u, 0u, 0u, 0u};
-  if (groups) nxt = src[lane];
-  for (int gq = 0; gq < groups; ++gq) {
-    stage[warp][lane] = nxt;
-    __syncwarp();
-    if (gq + 1 < groups) nxt = src[(gq + 1) * 32 + lane];
-#pragma unroll 8
-    for (int j = 0; j < 32; ++j) {
-      const uint4 p = stage[warp][j];
-      const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+                                                       float* loss_part, int nb, int64_t sY, int64_t sT) {
+  extern __shared__ __nv_bfloat16 tile[];  // [kLossRows][out_pad + 2]
+  __shared__ float wsum[kLossBlocks][8];
+  const int e = blockIdx.y, sum_blocks = (nb + kLossBlocks - 1) / kLossBlocks;
+  if ((int)blockIdx.x < sum_blocks) {
+    float local[kLossBlocks] = {};
+    const int v0 = blockIdx.x * kLossBlocks, n = B * out_pad;
+    for (int base = v0 * 256 + threadIdx.x; base < n; base += nb * 256) {
+      float t[kLossBlocks], mu[kLossBlocks], lv_raw[kLossBlocks];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {  // two BF16 values, the first in the low half
-        s += __uint_as_float(w[q] << 16);
-        s += __uint_as_float(w[q] & 0xffff0000u);
+      for (int u = 0; u < kLossBlocks; ++u) {
+        const int idx = base + u * 256;
+        const int i = idx / out_pad, c = idx - (idx / out_pad) * out_pad;
+        t[u] = __int_as_float(0x7fc00000);
+        mu[u] = lv_raw[u] = 0.0f;
+        if (v0 + u < nb && idx < n && c < K) {
+          const float* y = Y + e * sY + idx;
+          t[u] = T[e * sT + (int64_t)i * K + c];
+          mu[u] = y[0];
+          lv_raw[u] = y[K];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kLossBlocks; ++u) {
+        if (t[u] == t[u]) {
+          const float lv = fminf(fmaxf(lv_raw[u], kLvMin), kLvMax);
+          const float r = t[u] - mu[u];
+          const float ei = __expf(-lv);
+          local[u] += 0.5f * (lv + r * r * ei);
+        }
       }
     }
-    __syncwarp();
+    // block sums in a fixed order: warps by shuffles, then one thread over the warp sums
+#pragma unroll
+    for (int u = 0; u < kLossBlocks; ++u) {
+      for (int o = 16; o > 0; o >>= 1) local[u] += __shfl_xor_sync(0xffffffffu, local[u], o);
+      if ((threadIdx.x & 31) == 0) wsum[u][threadIdx.x >> 5] = local[u];
+    }
+    __syncthreads();
+    if (threadIdx.x < kLossBlocks && v0 + (int)threadIdx.x < nb) {
+      float t = 0.0f;
+      for (int w = 0; w < 8; ++w) t += wsum[threadIdx.x][w];
+      loss_part[e * nb + v0 + threadIdx.x] = t * inv_count;
+    }
+    return;
   }
-  for (int i = groups * 256; i < B; ++i) s += __bfloat162float(row[i]);
-  if (lane == 0) db[e * sDb + n] = s;
+  const int i0 = ((int)blockIdx.x - sum_blocks) * kLossRows, rows = min(kLossRows, B - i0), ld = out_pad + 2;
+#pragma unroll 4
+  for (int q = threadIdx.x; q < rows * K; q += blockDim.x) {
+    const int i = q / K, k = q - i * K;
+    const float* y = Y + e * sY + (int64_t)(i0 + i) * out_pad;
+    const float t = T[e * sT + (int64_t)i0 * K + q], mu = y[k], lv_raw = y[K + k];
+    float gm = 0.0f, gv = 0.0f;
+    if (t == t) {
+      const bool inside = lv_raw > kLvMin && lv_raw < kLvMax;
+      const float lv = fminf(fmaxf(lv_raw, kLvMin), kLvMax);
+      const float r = t - mu;
+      const float ei = __expf(-lv);
+      gm = -r * ei * inv_count;
+      gv = inside ? 0.5f * (1.0f - r * r * ei) * inv_count : 0.0f;
+    }
+    tile[i * ld + k] = __float2bfloat16(gm);
+    tile[i * ld + K + k] = __float2bfloat16(gv);
+  }
+  const int pad = out_pad - 2 * K;
+  for (int q = threadIdx.x; q < rows * pad; q += blockDim.x)
+    tile[q / pad * ld + 2 * K + q % pad] = __float2bfloat16(0.0f);
+  __syncthreads();
+  for (int q = threadIdx.x; q < rows * out_pad; q += blockDim.x) {
+    const int i = q / out_pad, c = q - i * out_pad;
+    dY[e * sY + (int64_t)i0 * out_pad + q] = tile[i * ld + c];
+  }
+  for (int q = threadIdx.x; q < out_pad * kLossRows; q += blockDim.x) {
+    const int c = q / kLossRows, i = q - c * kLossRows;
+    if (i < rows) dYT[(int64_t)e * out_pad * ldT + (int64_t)c * ldT + i0 + i] = tile[i * ld + c];
+  }
 }
 
-__global__ void mlp_adam_kernel(float* P, const float* G, float* m, float* v, __nv_bfloat16* Ph, int64_t n, float lr,
-                                float b1, float b2, float eps, float c1, float c2) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+// The reductions that end a backward pass, in one launch of three kinds of
+// blocks (blockIdx.x), so that the two serial ones run beside the third:
+//   columns  db[n] = sum_i dZ[i][n] for the output layer and the hidden ones, in
+//            row order (a training run is reproducible bit for bit, and
+//            independent of the launch), from the transposed copies [n][ldT].
+//            The additions are one chain per column.  A warp takes kColsPerWarp
+//            columns: it loads 256 rows of each at once (coalesced, the next 256 in
+//            flight) and passes them through shared memory to the chains, four
+//            lanes on one.  (A column per warp: the issue slots bound it, 40 us.
+//            32 columns: the loads, whose latency 110 warps do not hide);
+//   loss     loss[e] += sum of the member's block partials, in block order (the
+//            epoch loss accumulates over the batches in stream order);
+//   weights  sum over the reduction splits, in split order, of the weights of every
+//            layer (the biases between them are the column sums); four parameters per
+//            thread, every block size a multiple of 16.
+// 4,096 rows, 4 members: 61 + 6 + 11 us in six launches, 23 in one.
+constexpr int kRedThreads = 128, kColWarps = kRedThreads / 32, kColsPerWarp = 8;
+struct MlpReduce {
+  MlpDims d;
+  int B, ldT, col_blocks, n_loss, used;
+  const __nv_bfloat16* dYT;  // [members][out_pad][ldT]
+  const __nv_bfloat16* dZT;  // [layer][members][H][ldT]
+  int64_t sLayer;            // between the layers of dZT
+  const float* loss_part;    // [members][n_loss]
+  float* loss;
+  const float* part;  // [split][members][n_params]
+  int64_t sSplit;
+  float* out;  // [members][n_params]
+};
+__global__ void __launch_bounds__(kRedThreads) mlp_reduce_kernel(const MlpReduce a) {
+  __shared__ uint4 stage[kColWarps][kColsPerWarp][33];
+  __shared__ float lpart[1024];
+  const MlpDims& d = a.d;
+  const int e = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < a.col_blocks) {
+    const int n0 = (blockIdx.x * kColWarps + warp) * kColsPerWarp, total = d.out_pad + 3 * d.H;
+    if (n0 >= total) return;
+    // column n0 + j (every layer's columns are a multiple of kColsPerWarp: one layer per warp)
+    const __nv_bfloat16* rows;
+    int64_t off;
+    if (n0 < d.out_pad) {
+      rows = a.dYT + ((int64_t)e * d.out_pad + n0) * a.ldT;
+      off = d.off_b4 + n0;
+    } else {
+      const int layer = (n0 - d.out_pad) / d.H, n = n0 - d.out_pad - layer * d.H;
+      rows = a.dZT + layer * a.sLayer + ((int64_t)e * d.H + n) * a.ldT;
+      off = (layer == 0 ? d.off_b1 : layer == 1 ? d.off_b2 : d.off_b3) + n;
+    }
+    const int groups = a.B / 256, mine = lane / (32 / kColsPerWarp);
+    float s = 0.0f;
+    uint4 nxt[kColsPerWarp];
+    auto load = [&](int gq) {
+#pragma unroll
+      for (int j = 0; j < kColsPerWarp; ++j)
+        nxt[j] = reinterpret_cast<const uint4*>(rows + (int64_t)j * a.ldT)[gq * 32 + lane];
+    };
+    if (groups) load(0);
+    for (int gq = 0; gq < groups; ++gq) {
+#pragma unroll
+      for (int j = 0; j < kColsPerWarp; ++j) stage[warp][j][lane] = nxt[j];
+      __syncwarp();
+      if (gq + 1 < groups) load(gq + 1);
+#pragma unroll 8
+      for (int j = 0; j < 32; ++j) {
+        const uint4 p = stage[warp][mine][j];
+        const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // two BF16 values, the first in the low half
+          s += __uint_as_float(w[q] << 16);
+          s += __uint_as_float(w[q] & 0xffff0000u);
+        }
+      }
+      __syncwarp();
+    }
+    for (int i = groups * 256; i < a.B; ++i) s += __bfloat162float(rows[(int64_t)mine * a.ldT + i]);
+    if (lane % (32 / kColsPerWarp) == 0) a.out[e * d.n_params + off + mine] = s;
+    return;
+  }
+  if ((int)blockIdx.x == a.col_blocks) {
+    float t = 0.0f;
+    for (int b0 = 0; b0 < a.n_loss; b0 += 1024) {
+      const int nb = min(1024, a.n_loss - b0);
+      for (int b = threadIdx.x; b < nb; b += blockDim.x) lpart[b] = a.loss_part[e * a.n_loss + b0 + b];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+#pragma unroll 16
+        for (int b = 0; b < nb; ++b) t += lpart[b];
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) a.loss[e] += t;
+    return;
+  }
+  const int64_t i = 4 * ((int64_t)(blockIdx.x - a.col_blocks - 1) * kRedThreads + threadIdx.x);
+  if (i >= d.off_b4 || (i >= d.off_b1 && i < d.off_w2) || (i >= d.off_b2 && i < d.off_w3) ||
+      (i >= d.off_b3 && i < d.off_w4))
+    return;
+  const float* p = a.part + e * d.n_params + i;
+  float4 acc = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
+  for (int sp = 0; sp < a.used; ++sp) {
+    const float4 v = *(const float4*)(p + sp * a.sSplit);
+    acc.x += v.x;
+    acc.y += v.y;
+    acc.z += v.z;
+    acc.w += v.w;
+  }
+  *(float4*)(a.out + e * d.n_params + i) = acc;
+}
+
+// Adam, and the BF16 copies of the new weights as stored and transposed: a
+// block takes a 32 x 32 tile of a weight matrix, which it turns through shared
+// memory, or the biases (the last block).  4 members: 7 + 9 us in two launches, the second
+// writing every value to its own line, 9 in one.
+struct MlpAdam {
+  float lr, b1, b2, eps, c1, c2;
+};
+inline int mlp_tiles(int64_t rows, int64_t cols) { return (int)((rows + 31) / 32 * ((cols + 31) / 32)); }
+__global__ void __launch_bounds__(256) mlp_adam_kernel(MlpDims d, float* P, const float* G, float* m, float* v,
+                                                       __nv_bfloat16* Ph, __nv_bfloat16* PhT, MlpAdam o) {
+  __shared__ __nv_bfloat16 tile[32][34];
+  const int64_t base = blockIdx.y * d.n_params;
+  auto update = [&](int64_t i) {
     const float g = G[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * g;
-    const float vi = b2 * v[i] + (1.0f - b2) * g * g;
+    const float mi = o.b1 * m[i] + (1.0f - o.b1) * g;
+    const float vi = o.b2 * v[i] + (1.0f - o.b2) * g * g;
     m[i] = mi;
     v[i] = vi;
-    const float p = P[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    const float p = P[i] - o.lr * (mi * o.c1) / (sqrtf(vi * o.c2) + o.eps);
     P[i] = p;
-    Ph[i] = __float2bfloat16(p);
+    const __nv_bfloat16 h = __float2bfloat16(p);
+    Ph[i] = h;
+    return h;
+  };
+  const int64_t offs[4] = {d.off_w1, d.off_w2, d.off_w3, d.off_w4};
+  const int nr[4] = {d.in_pad, d.H, d.H, d.H}, nc[4] = {d.H, d.H, d.H, d.out_pad};
+  int b = blockIdx.x;
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const int R = nr[l], C = nc[l], tc = (C + 31) / 32, n = (R + 31) / 32 * tc;
+    if (b >= n) {
+      b -= n;
+      continue;
+    }
+    const int r0 = b / tc * 32, c0 = b % tc * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    for (int r = y; r < 32; r += 8)
+      if (r0 + r < R && c0 + x < C) tile[r][x] = update(base + offs[l] + (int64_t)(r0 + r) * C + c0 + x);
+    __syncthreads();
+    for (int c = y; c < 32; c += 8)
+      if (r0 + x < R && c0 + c < C) PhT[base + offs[l] + (int64_t)(c0 + c) * R + r0 + x] = tile[x][c];
+    return;
   }
+  const int64_t boff[4] = {d.off_b1, d.off_b2, d.off_b3, d.off_b4};
+#pragma unroll
+  for (int l = 0; l < 4; ++l)
+    for (int q = threadIdx.x; q < nc[l]; q += blockDim.x) PhT[base + boff[l] + q] = update(base + boff[l] + q);
 }
 
 // ensemble combination in standardised units -> caller units
@@ -418,8 +519,8 @@ cudaError_t mlp_forward(const MlpDims& d, int members, int B, const __nv_bfloat1
 // silu'(Z_l) with its transposed copy.
 cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0T, const __nv_bfloat16* Wh,
                          const float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
-                         __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZTa, __nv_bfloat16* dZTb, int ldT,
-                         float* Gf, float* Gpart, int* err, cudaStream_t s) {
+                         __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZT, int ldT, float* Gf, float* Gpart,
+                         float* loss, const float* loss_part, int* err, cudaStream_t s) {
   const int H = d.H;
   const int64_t sZ = 3 * (int64_t)B * H, sL = (int64_t)B * H, sLT = (int64_t)H * ldT, sP = d.n_params;
   const int splits = mlp_wgrad_splits(B);
@@ -439,25 +540,21 @@ cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat
     g.err = err;
     return mlp_tc_gemm(EPI_PARTIAL, A, Bg, g, members, s);
   };
-  // layer 4: dW4 = A3^T dY (M = H, N = out_pad), db4 = colsum(dY)
+  // layer 4: dW4 = A3^T dY (M = H, N = out_pad)
   {
     TcOperand A{AhT + 2 * sLT, ldT, H, 3 * sLT};
     TcOperand Bg{dYT, ldT, d.out_pad, (int64_t)d.out_pad * ldT};
     if ((e = wgrad(A, Bg, H, d.out_pad, d.off_w4))) return e;
-    mlp_colsum_kernel<<<dim3((d.out_pad + kColWarps - 1) / kColWarps, members), 32 * kColWarps, 0, s>>>(
-        dYT, B, d.out_pad, ldT, (int64_t)d.out_pad * ldT, Gf + d.off_b4, sP);
   }
   const __nv_bfloat16* grad_in = dY;
   int64_t s_gin = (int64_t)B * d.out_pad;
   int ld_gin = d.out_pad;
   const int64_t w_next[3] = {d.off_w2, d.off_w3, d.off_w4};
-  const int64_t b_off[3] = {d.off_b1, d.off_b2, d.off_b3};
   const int64_t w_off[3] = {d.off_w1, d.off_w2, d.off_w3};
   __nv_bfloat16* bufs[2] = {dZa, dZb};
-  __nv_bfloat16* bufsT[2] = {dZTa, dZTb};
   for (int layer = 2; layer >= 0; --layer) {
     __nv_bfloat16* dZ = bufs[layer & 1];
-    __nv_bfloat16* dZT = bufsT[layer & 1];
+    __nv_bfloat16* dZTl = dZT + layer * members * sLT;
     {
       // dZ_l = (grad_in W_{l+1}^T) silu'(Z_l): W_{l+1} stored [H][out] is the K-major [N = H][K = out] operand
       const int Kn = layer == 2 ? d.out_pad : H;
@@ -474,38 +571,52 @@ cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat
       g.outh = dZ;
       g.sOuth = sL;
       g.ldh = H;
-      g.outhT = dZT;
+      g.outhT = dZTl;
       g.sOuthT = sLT;
       g.ldhT = ldT;
       g.err = err;
       if ((e = mlp_tc_gemm(EPI_DSILU, A, Bw, g, members, s))) return e;
     }
     {
-      // dW_l = A_{l-1}^T dZ_l (M = in_l, N = H), db_l = colsum(dZ_l)
+      // dW_l = A_{l-1}^T dZ_l (M = in_l, N = H)
       const int Min = layer == 0 ? d.in_pad : H;
       TcOperand A = layer == 0 ? TcOperand{X0T, ldT, d.in_pad, (int64_t)d.in_pad * ldT}
                                : TcOperand{AhT + (layer - 1) * sLT, ldT, H, 3 * sLT};
-      TcOperand Bg{dZT, ldT, H, sLT};
+      TcOperand Bg{dZTl, ldT, H, sLT};
       if ((e = wgrad(A, Bg, Min, H, w_off[layer]))) return e;
-      mlp_colsum_kernel<<<dim3((H + kColWarps - 1) / kColWarps, members), 32 * kColWarps, 0, s>>>(dZT, B, H, ldT, sLT,
-                                                                                             Gf + b_off[layer], sP);
     }
     grad_in = dZ;
     s_gin = sL;
     ld_gin = H;
   }
-  mlp_split_sum_kernel<<<dim3((unsigned)((d.n_params / 4 + 255) / 256), members), 256, 0, s>>>(
-      Gpart, used, sP * members, d, Gf);
+  MlpReduce r{};
+  r.d = d;
+  r.B = B;
+  r.ldT = ldT;
+  r.col_blocks = (d.out_pad + 3 * H + kColWarps * kColsPerWarp - 1) / (kColWarps * kColsPerWarp);
+  r.n_loss = mlp_loss_blocks(B, d.out_pad);
+  r.used = used;
+  r.dYT = dYT;
+  r.dZT = dZT;
+  r.sLayer = members * sLT;
+  r.loss_part = loss_part;
+  r.loss = loss;
+  r.part = Gpart;
+  r.sSplit = sP * members;
+  r.out = Gf;
+  const int wblocks = (int)((d.n_params / 4 + kRedThreads - 1) / kRedThreads);
+  mlp_reduce_kernel<<<dim3(r.col_blocks + 1 + wblocks, members), kRedThreads, 0, s>>>(r);
   return cudaGetLastError();
 }
 
 cudaError_t mlp_loss(const MlpDims& d, int members, int B, int valid_rows, const float* Y, const float* T,
-                     __nv_bfloat16* dY, __nv_bfloat16* dYT, int ldT, float* loss, float* loss_part, cudaStream_t s) {
+                     __nv_bfloat16* dY, __nv_bfloat16* dYT, int ldT, float* loss_part, cudaStream_t s) {
   const float inv = 1.0f / (float)(std::max(1, valid_rows) * d.K);
   const int nb = mlp_loss_blocks(B, d.out_pad);
-  mlp_loss_kernel<<<dim3(nb, members), 256, 0, s>>>(Y, T, B, d.K, d.out_pad, inv, dY, dYT, ldT, loss_part,
-                                                    (int64_t)B * d.out_pad, (int64_t)B * d.K);
-  mlp_loss_sum_kernel<<<members, 1024, 0, s>>>(loss_part, nb, loss);
+  const int tiles = (B + kLossRows - 1) / kLossRows;
+  const size_t smem = (size_t)kLossRows * (d.out_pad + 2) * sizeof(__nv_bfloat16);
+  mlp_loss_kernel<<<dim3((nb + kLossBlocks - 1) / kLossBlocks + tiles, members), 256, smem, s>>>(Y, T, B, d.K, d.out_pad, inv, dY, dYT, ldT, loss_part, nb,
+                                                              (int64_t)B * d.out_pad, (int64_t)B * d.K);
   return cudaGetLastError();
 }
 
@@ -514,9 +625,8 @@ cudaError_t mlp_adam(const MlpDims& d, int members, float* P, const float* G, fl
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.0f / (1.0f - powf(b1, (float)step));
   const float c2 = 1.0f / (1.0f - powf(b2, (float)step));
-  const int64_t n = d.n_params * members;
-  mlp_adam_kernel<<<blocks_for(n, 256), 256, 0, s>>>(P, G, m, v, Ph, n, lr, b1, b2, eps, c1, c2);
-  mlp_weights_t_kernel<<<blocks_for(n, 256), 256, 0, s>>>(P, d, members, PhT);
+  const int tiles = mlp_tiles(d.in_pad, d.H) + 2 * mlp_tiles(d.H, d.H) + mlp_tiles(d.H, d.out_pad);
+  mlp_adam_kernel<<<dim3(tiles + 1, members), 256, 0, s>>>(d, P, G, m, v, Ph, PhT, MlpAdam{lr, b1, b2, eps, c1, c2});
   return cudaGetLastError();
 }
 

@@ -33,10 +33,10 @@ cudaError_t mlp_infer(const MlpDims& d, int members, int B, const __nv_bfloat16*
                       const float* Pf, float* Y, int* err, int sms, cudaStream_t s);
 cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0T, const __nv_bfloat16* Wh,
                          const float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
-                         __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZTa, __nv_bfloat16* dZTb, int ldT,
-                         float* Gf, float* Gpart, int* err, cudaStream_t s);
+                         __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZT, int ldT, float* Gf, float* Gpart,
+                         float* loss, const float* loss_part, int* err, cudaStream_t s);
 cudaError_t mlp_loss(const MlpDims& d, int members, int B, int valid_rows, const float* Y, const float* T,
-                     __nv_bfloat16* dY, __nv_bfloat16* dYT, int ldT, float* loss, float* loss_part, cudaStream_t s);
+                     __nv_bfloat16* dY, __nv_bfloat16* dYT, int ldT, float* loss_part, cudaStream_t s);
 cudaError_t mlp_adam(const MlpDims& d, int members, float* P, const float* G, float* m, float* v,
                      __nv_bfloat16* Ph, __nv_bfloat16* PhT, float lr, int step, cudaStream_t s);
 cudaError_t mlp_combine(const MlpDims& d, int members, int N, const float* Y, const float* ymean, const float* ystd,
@@ -295,7 +295,7 @@ struct abc_surrogate {
   Buf<double> th64, st64;
   Buf<float> xn, yn, T, Z, Y;
   Buf<__nv_bfloat16> X0, Ah, dY, dZa, dZb;
-  Buf<__nv_bfloat16> X0T, AhT, dYT, dZTa, dZTb;  // [features][ldT] copies for the weight gradients
+  Buf<__nv_bfloat16> X0T, AhT, dYT, dZT;  // [features][ldT] copies for the weight gradients
   int ldT = 0;
   Buf<float> loss, loss_part;  // per-member loss; per-block partial sums of the loss kernel
   Buf<float> Gpart;            // weight-gradient partial sums, one slice per reduction split
@@ -336,8 +336,7 @@ static int ensure_batch(abc_surrogate* s, int B) {
   SK(s->X0T.ensure(E * d.in_pad * lt));
   SK(s->AhT.ensure(E * 3 * d.H * lt));
   SK(s->dYT.ensure(E * d.out_pad * lt));
-  SK(s->dZTa.ensure(E * d.H * lt));
-  SK(s->dZTb.ensure(E * d.H * lt));
+  SK(s->dZT.ensure(E * 3 * d.H * lt));
   SK(s->loss.ensure(E));
   SK(s->loss_part.ensure(E * (size_t)mlp_loss_blocks(B, d.out_pad)));
   SK(s->Gpart.ensure((size_t)mlp_wgrad_splits(B) * E * (size_t)d.n_params));
@@ -363,9 +362,9 @@ static int train_step(abc_surrogate* s, int B, int64_t base, int valid, int64_t 
   SK(mlp_gather(s->xn.p, s->yn.p, N, d, B, base, s->perm.p, E, s->X0.p, s->X0T.p, s->ldT, s->T.p, s->stream));
   SK(mlp_forward(d, E, B, s->X0.p, (int64_t)B * d.in_pad, s->PhT.p, s->P.p, s->Z.p, s->Ah.p, s->AhT.p, s->ldT,
                  s->Y.p, s->tcerr.p, s->stream));
-  SK(mlp_loss(d, E, B, valid, s->Y.p, s->T.p, s->dY.p, s->dYT.p, s->ldT, s->loss.p, s->loss_part.p, s->stream));
-  SK(mlp_backward(d, E, B, s->X0T.p, s->Ph.p, s->Z.p, s->AhT.p, s->dY.p, s->dYT.p, s->dZa.p, s->dZb.p, s->dZTa.p,
-                  s->dZTb.p, s->ldT, s->G.p, s->Gpart.p, s->tcerr.p, s->stream));
+  SK(mlp_loss(d, E, B, valid, s->Y.p, s->T.p, s->dY.p, s->dYT.p, s->ldT, s->loss_part.p, s->stream));
+  SK(mlp_backward(d, E, B, s->X0T.p, s->Ph.p, s->Z.p, s->AhT.p, s->dY.p, s->dYT.p, s->dZa.p, s->dZb.p, s->dZT.p,
+                  s->ldT, s->G.p, s->Gpart.p, s->loss.p, s->loss_part.p, s->tcerr.p, s->stream));
   return ABC_OK;
 }
 
@@ -414,8 +413,7 @@ int abc_surrogate_destroy(abc_surrogate* s) {
   cudaStreamSynchronize(s->stream);
   s->yscf.release(); s->ysc.release();
   s->P.release(); s->G.release(); s->Am.release(); s->Av.release(); s->Ph.release(); s->ymf.release();
-  s->PhT.release(); s->tcerr.release(); s->X0T.release(); s->AhT.release(); s->dYT.release(); s->dZTa.release();
-  s->dZTb.release();
+  s->PhT.release(); s->tcerr.release(); s->X0T.release(); s->AhT.release(); s->dYT.release(); s->dZT.release();
   s->ysf.release(); s->xm.release(); s->xs.release(); s->ym.release(); s->ys.release(); s->th64.release();
   s->st64.release(); s->xn.release(); s->yn.release(); s->T.release(); s->Z.release(); s->Y.release();
   s->X0.release(); s->Ah.release(); s->dY.release(); s->dZa.release(); s->dZb.release(); s->loss.release();

@@ -90,3 +90,33 @@ def test_screen_gene_tiles_agree(built, mode, genes, rows):
         assert np.array_equal(low, np.concatenate([p[0] for p in parts], axis=1))
         assert np.array_equal(kept, np.logical_or.reduce([p[1] for p in parts])) and n == kept.sum()
         assert np.array_equal(kept, (low.astype(np.float32) <= np.float32(0.5)).any(axis=1))
+
+
+@pytest.mark.parametrize("rows,K", [(1, 53), (31, 8), (33, 53), (255, 53), (256, 8), (257, 53), (1100, 53)])
+def test_gradients_at_batch_edges(built, rows, K):
+    """Batches around the 32 rows of a gradient tile, the 256 rows of a column
+    sum's stage and the loss's block partials, outputs with (53) and without (8)
+    padding, against the FP64 network that rounds to BF16 where the GPU does.
+    Gradients within 2e-2 of their norm, as for the batch of 96."""
+    from abc_inference_transcription_gb300 import surrogate as S
+    from oracle import mlp_ref
+
+    rng = np.random.default_rng(rows)
+    theta, stats = rng.uniform(-3, 3, (rows, 5)), rng.normal(2.0, 1.5, (rows, K))
+    if rows > 1:
+        stats[0, 2] = np.nan
+    with S.Surrogate(5, K, ensemble=2, seed=11) as sg:
+        p = sg.params()
+        p = p + rng.normal(0, 0.02, p.shape).astype(np.float32)
+        sg.set_params(p)
+        norm = np.zeros(5), np.full(5, 1.7), np.full(K, 2.0), np.full(K, 1.5)
+        sg.set_norm(*norm)
+        loss, grads = sg.gradients(theta, stats)
+        d = mlp_ref.dims(5, K)
+        for e in range(2):
+            rl, rg = mlp_ref.loss_and_grads(p[e], d, theta, stats, *norm)
+            assert abs(loss[e] - rl) <= 2e-4 * abs(rl) + 1e-6
+            for name in ("w1", "b1", "w2", "b2", "w3", "b3", "w4", "b4"):
+                a, b = d[name]
+                got, want = grads[e, a:b].astype(np.float64), rg[a:b]
+                assert np.linalg.norm(got - want) < 2e-2 * max(np.linalg.norm(want), 1e-12), (e, name)
