@@ -141,3 +141,21 @@ def test_data_stats_gpu_layouts_and_count_ranges(built, orc, per_pulse, n_ages, 
                 ctx.data_stats(bad, l, n_boot=n_boot)
             with pytest.raises(abi.AbcError):
                 ctx.data_stats(u, bad, n_boot=n_boot)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("per_pulse", [1620, 1770, 1775])
+def test_data_stats_gpu_many_cells(built, orc, per_pulse):
+    """Cells whose (u, l) fit in shared memory beside the counters (17,820), and
+    just below the limit, where they are read through the order (19,470, 19,525)."""
+    from abc_inference_transcription_gb300.host import Context
+    cfg = make_config("hour")
+    cells = synthetic_cells(n_per_pulse=per_pulse, n_per_chase=per_pulse, seed=per_pulse)
+    C = cells.cond.shape[0]
+    rng = np.random.default_rng(per_pulse)
+    u = rng.integers(0, 60, (2, C)).astype(np.int32)
+    l = rng.integers(0, 9, (2, C)).astype(np.int32)
+    with Context(cfg, cells) as ctx:
+        got = ctx.data_stats(u, l, n_boot=2, seed=5)
+    for a, b in zip(got, orc.data_stats(cfg, cells, u, l, n_boot=2, seed=5)):
+        assert np.array_equal(a, b, equal_nan=True)
