@@ -537,6 +537,10 @@ cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat
   const int nk = (B + 63) / 64, per = (nk + splits - 1) / splits;
   const int used = (nk + per - 1) / per;  // splits that receive reduction chunks
   cudaError_t e;
+  // dW4 = A3^T dY (M = H, N = out_pad), dW_l = A_{l-1}^T dZ_l (M = in_l, N = H)
+  TcOperand wa[kWgradGemms], wb[kWgradGemms];
+  TcGemm wg[kWgradGemms];
+  int n_wg = 0;
   auto wgrad = [&](const TcOperand& A, const TcOperand& Bg, int M, int N, int64_t off) {
     TcGemm g{};
     g.M = M;
@@ -548,14 +552,12 @@ cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat
     g.sSplit = sP * members;
     g.ldf = N;
     g.err = err;
-    return mlp_tc_gemm(EPI_PARTIAL, A, Bg, g, members, s);
+    wa[n_wg] = A;
+    wb[n_wg] = Bg;
+    wg[n_wg++] = g;
   };
-  // layer 4: dW4 = A3^T dY (M = H, N = out_pad)
-  {
-    TcOperand A{AhT + 2 * sLT, ldT, H, 3 * sLT};
-    TcOperand Bg{dYT, ldT, d.out_pad, (int64_t)d.out_pad * ldT};
-    if ((e = wgrad(A, Bg, H, d.out_pad, d.off_w4))) return e;
-  }
+  wgrad(TcOperand{AhT + 2 * sLT, ldT, H, 3 * sLT}, TcOperand{dYT, ldT, d.out_pad, (int64_t)d.out_pad * ldT}, H,
+        d.out_pad, d.off_w4);
   const __nv_bfloat16* grad_in = dY;
   int64_t s_gin = (int64_t)B * d.out_pad;
   int ld_gin = d.out_pad;
@@ -587,18 +589,15 @@ cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat
       g.err = err;
       if ((e = mlp_tc_gemm(EPI_DSILU, A, Bw, g, members, s))) return e;
     }
-    {
-      // dW_l = A_{l-1}^T dZ_l (M = in_l, N = H)
-      const int Min = layer == 0 ? d.in_pad : H;
-      TcOperand A = layer == 0 ? TcOperand{X0T, ldT, d.in_pad, (int64_t)d.in_pad * ldT}
-                               : TcOperand{AhT + (layer - 1) * sLT, ldT, H, 3 * sLT};
-      TcOperand Bg{dZTl, ldT, H, sLT};
-      if ((e = wgrad(A, Bg, Min, H, w_off[layer]))) return e;
-    }
+    const int Min = layer == 0 ? d.in_pad : H;
+    wgrad(layer == 0 ? TcOperand{X0T, ldT, d.in_pad, (int64_t)d.in_pad * ldT}
+                     : TcOperand{AhT + (layer - 1) * sLT, ldT, H, 3 * sLT},
+          TcOperand{dZTl, ldT, H, sLT}, Min, H, w_off[layer]);
     grad_in = dZ;
     s_gin = sL;
     ld_gin = H;
   }
+  if ((e = mlp_tc_wgrads(wa, wb, wg, members, s))) return e;
   MlpReduce r{};
   r.d = d;
   r.B = B;

@@ -90,6 +90,9 @@ inline int mlp_loss_blocks(int B, int out_pad) {
   return n < 1024 ? n : 1024;
 }
 
+// the weight gradients (EPI_PARTIAL) of the four layers
+constexpr int kWgradGemms = 4;
+cudaError_t mlp_tc_wgrads(const TcOperand* A, const TcOperand* B, const TcGemm* g, int members, cudaStream_t s);
 cudaError_t mlp_tc_gemm(int epi, const TcOperand& A, const TcOperand& B, const TcGemm& g, int members,
                         cudaStream_t s);
 

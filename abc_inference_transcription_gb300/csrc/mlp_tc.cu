@@ -134,9 +134,10 @@ __device__ __forceinline__ void store_rows_bf16(float* sm, const float (&x)[kChu
   __syncwarp();
 }
 
+// one output tile: tile (mt + split * m tiles, nt) of member z
 template <int EPI>
-__global__ void __launch_bounds__(kThreads, 2)
-    mlp_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcGemm g) {
+__device__ __forceinline__ void gemm_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemm& g, int my, int nt,
+                                          int z) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (su32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full = (uint64_t*)(smem + kStages * kStageBytes);
@@ -144,10 +145,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint64_t* done = empty + kStages;
   uint32_t* tslot = (uint32_t*)(done + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int z = blockIdx.z;
   const int n_mt = (g.M + BM - 1) / BM;
-  const int mt = blockIdx.y % n_mt, split = blockIdx.y / n_mt;
-  const int m0 = mt * BM, n0 = blockIdx.x * BN;
+  const int mt = my % n_mt, split = my / n_mt;
+  const int m0 = mt * BM, n0 = nt * BN;
   const int nk = (g.K + BK - 1) / BK;
   const int per = (nk + g.k_split - 1) / g.k_split;
   const int c0 = split * per, c1 = min(nk, c0 + per);
@@ -214,8 +214,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   // 64 (w / 4) .. + 63, in chunks staged where the operand tiles were: every
   // copy has landed and every MMA has read its tiles once `done` has come.  N and
   // every row length are multiples of 16 values.  4,096 rows x 256 x 4 members: a hidden
-  // layer 20 us with four warps and a row per lane, 14 now; its derivative 17.5, 13.6; a
-  // weight gradient 10.3, 8.7.
+  // layer 20 us with four warps and a row per lane, 14 now; its derivative 17.5, 13.6.
   bool have = work && mbar_wait(done, 0);
   have = __all_sync(0xffffffffu, have);
   if (work && !have && lane == 0) atomicOr(g.err, 4);
@@ -288,6 +287,26 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 template <int EPI>
+__global__ void __launch_bounds__(kThreads, 2)
+    mlp_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcGemm g) {
+  gemm_tile<EPI>(tmA, tmB, g, blockIdx.y, blockIdx.x, blockIdx.z);
+}
+
+// The weight gradients of every layer in one launch: alone, none of them fills the
+// GPU (4,096 rows, 4 members: four launches 35 us, 21.5 in one).
+struct WgradSet {
+  CUtensorMap a[kWgradGemms], b[kWgradGemms];
+  TcGemm g[kWgradGemms];
+  int first[kWgradGemms + 1];  // first block of each, counting n tiles, then m tiles and splits
+};
+__global__ void __launch_bounds__(kThreads, 2) mlp_wgrad_kernel(const __grid_constant__ WgradSet w) {
+  int l = 0;
+  while (l + 1 < kWgradGemms && (int)blockIdx.x >= w.first[l + 1]) ++l;
+  const int i = blockIdx.x - w.first[l], n_nt = (w.g[l].N + BN - 1) / BN;
+  gemm_tile<EPI_PARTIAL>(w.a[l], w.b[l], w.g[l], i / n_nt, i % n_nt, blockIdx.y);
+}
+
+template <int EPI>
 cudaError_t launch_epi(const CUtensorMap& ma, const CUtensorMap& mb, const TcGemm& g, int members, cudaStream_t s) {
   static std::atomic<uint64_t> attr{0};  // devices where the limit is set, shared by all contexts
   cudaError_t e = set_smem_once(attr, mlp_tc_kernel<EPI>, kSmem);
@@ -300,23 +319,45 @@ cudaError_t launch_epi(const CUtensorMap& ma, const CUtensorMap& mb, const TcGem
 
 }  // namespace
 
-cudaError_t mlp_tc_gemm(int epi, const TcOperand& A, const TcOperand& B, const TcGemm& g, int members,
-                        cudaStream_t s) {
-  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
+static cudaError_t gemm_maps(const TcOperand& A, const TcOperand& B, const TcGemm& g, int members, CUtensorMap* ma,
+                             CUtensorMap* mb) {
   if ((A.ld * 2) % 16 || (B.ld * 2) % 16 || (A.member_stride * 2) % 16 || (B.member_stride * 2) % 16)
     return cudaErrorInvalidValue;
   // the epilogue's 16-byte accesses
   if (g.N % 8 || g.ldf % 4 || g.ldh % 8 || g.ldz % 4 || g.sOutf % 4 || g.sSplit % 4 || g.sOuth % 8 || g.sZ % 4 ||
       g.sBias % 4 || ((uintptr_t)g.outf | (uintptr_t)g.outh | (uintptr_t)g.zprev | (uintptr_t)g.bias) % 16)
     return cudaErrorInvalidValue;
-  CUtensorMap ma, mb;
-  if (!make_map3(&ma, A.ptr, g.K, A.ld, A.rows, g.a_shared ? 1 : members, A.member_stride) ||
-      !make_map3(&mb, B.ptr, g.K, B.ld, B.rows, members, B.member_stride))
+  if (!make_map3(ma, A.ptr, g.K, A.ld, A.rows, g.a_shared ? 1 : members, A.member_stride) ||
+      !make_map3(mb, B.ptr, g.K, B.ld, B.rows, members, B.member_stride))
     return cudaErrorInvalidValue;
+  return cudaSuccess;
+}
+
+cudaError_t mlp_tc_wgrads(const TcOperand* A, const TcOperand* B, const TcGemm* g, int members, cudaStream_t s) {
+  WgradSet w;
+  w.first[0] = 0;
+  for (int l = 0; l < kWgradGemms; ++l) {
+    cudaError_t e = gemm_maps(A[l], B[l], g[l], members, &w.a[l], &w.b[l]);
+    if (e != cudaSuccess) return e;
+    w.g[l] = g[l];
+    w.first[l + 1] = w.first[l] + (g[l].N + BN - 1) / BN * ((g[l].M + BM - 1) / BM) * g[l].k_split;
+  }
+  static std::atomic<uint64_t> attr{0};
+  cudaError_t e = set_smem_once(attr, mlp_wgrad_kernel, kSmem);
+  if (e != cudaSuccess) return e;
+  mlp_wgrad_kernel<<<dim3((unsigned)w.first[kWgradGemms], (unsigned)members), kThreads, kSmem, s>>>(w);
+  return cudaGetLastError();
+}
+
+cudaError_t mlp_tc_gemm(int epi, const TcOperand& A, const TcOperand& B, const TcGemm& g, int members,
+                        cudaStream_t s) {
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
+  CUtensorMap ma, mb;
+  cudaError_t e = gemm_maps(A, B, g, members, &ma, &mb);
+  if (e != cudaSuccess) return e;
   switch (epi) {
     case EPI_HIDDEN: return launch_epi<EPI_HIDDEN>(ma, mb, g, members, s);
     case EPI_LINEAR: return launch_epi<EPI_LINEAR>(ma, mb, g, members, s);
-    case EPI_PARTIAL: return launch_epi<EPI_PARTIAL>(ma, mb, g, members, s);
     default: return launch_epi<EPI_DSILU>(ma, mb, g, members, s);
   }
 }
