@@ -1409,8 +1409,7 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   a.nsub = S * per_step;
   a.n_pulse_conds = n_pulse_conds;
   const bool f32 = cf.precision == ABC_FP32;
-  const int grid = (int)std::min<int64_t>(P, (int64_t)c->sms * 8);  // FP64 mode
-  const size_t scratch = f32 ? moment_f32_scratch(P, a.nsub, J * A) : sizeof(double) * (size_t)grid * 2 * a.nsub * 100;
+  const size_t scratch = f32 ? moment_f32_scratch(P, a.nsub, J * A) : moment_f64_scratch(P, a.nsub, J * A);
   Work w;
   const size_t o_theta = w.add(sizeof(double) * (size_t)P * npar), o_bm = w.add(sizeof(double) * 2 * A * 3);
   const size_t o_ad = w.add(sizeof(double) * (size_t)A * J), o_stats = w.add(sizeof(double) * (size_t)P * K);
@@ -1435,7 +1434,7 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
     CK(cudaEventCreate(&c->sel_ev[1]));
   }
   if (c->prof) CK(cudaEventRecord(c->sel_ev[0], c->stream));
-  CK(f32 ? launch_moment_f32(a, c->stream) : launch_moment(a, grid, c->stream));
+  CK(f32 ? launch_moment_f32(a, c->stream) : launch_moment(a, c->stream));
   if (c->prof) CK(cudaEventRecord(c->sel_ev[1], c->stream));
   CK(cudaMemcpyAsync(stats_out, a.stats, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
   if (moments_out)

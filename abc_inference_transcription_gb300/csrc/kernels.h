@@ -190,11 +190,12 @@ struct MomArgs {
   double* stats;           // [P][K]
   double* moments;         // [P][J][A][5] or null
   int* iters;              // [P] transient cycles or null
-  double* scratch;         // FP64 mode: [grid][2][nsub][100]
+  void* scratch;           // moment_f64_scratch() or moment_f32_scratch() bytes
   int* status;
 };
-cudaError_t launch_moment(const MomArgs& a, int grid, cudaStream_t s);
-// FP32 production mode (moment_fp32.cu); scratch: moment_f32_scratch() bytes, pairs = conditions x ages
+// FP64 mode (moment.cu) and FP32 production mode (moment_fp32.cu); pairs = conditions x ages
+size_t moment_f64_scratch(int64_t P, int nsub, int pairs);
+cudaError_t launch_moment(const MomArgs& a, cudaStream_t s);
 size_t moment_f32_scratch(int64_t P, int nsub, int pairs);
 cudaError_t launch_moment_f32(const MomArgs& a, cudaStream_t s);
 

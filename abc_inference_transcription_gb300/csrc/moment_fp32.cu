@@ -33,16 +33,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cmath>
 
-#include "common.cuh"
-#include "kernels.h"
-#include "model.cuh"
+#include "moment.cuh"
 
 namespace abc {
 namespace {
 
-constexpr int NA = 10;
 constexpr int kTaylor = 8;
 constexpr int kNnz = 38, kQuads = 10;  // stored entries of a propagator; 16-byte pieces, the last one half padding
 constexpr int kExpThreads = 128;
@@ -50,15 +46,7 @@ constexpr int kQuarters = 4;  // parts of the cycle multiplied separately
 constexpr int kCycleParticles = 8;
 constexpr int kPathParticles = 8;  // a warp of the path kernel: these x kPathGroup pairs, two per lane
 constexpr int kPathGroup = 2 * 32 / kPathParticles;
-constexpr int kMaxPairs = kMaxConds * kMaxAges;
 constexpr int kWalkStages = 8, kPathStages = 4;  // substeps whose propagators are on their way
-
-// (condition, age) pairs by the start of their labelling: labelled from substep
-// lo to hi, observed at end
-struct MomPlan {
-  int n;
-  int pair[kMaxPairs], lo[kMaxPairs], hi[kMaxPairs], end[kMaxPairs];
-};
 
 // Scratch of a chunk of n particles.  The particle is the fastest index of the
 // propagators: threads of neighbouring particles read and write whole lines.
@@ -496,85 +484,18 @@ __global__ void __launch_bounds__(32) moment_path_kernel(MomArgs a, MomScratch w
   }
 }
 
-constexpr int kStatParticles = 8;
-inline size_t stat_smem(int pairs) { return (size_t)kStatParticles * pairs * 5 * sizeof(double); }
-
-// capture transform (model.jl:221-239) per (condition, age), then the
-// statistics per condition
-__global__ void __launch_bounds__(128) moment_stats_kernel(MomArgs a, int64_t p0, MomScratch ws) {
-  extern __shared__ double ds[];  // [particle][JA][5]
-  const DevCfg& cfg = a.cfg;
-  const int J = cfg.n_conds, A = cfg.n_ages, JA = J * A, K = 4 * A + 3 * J;
-  const int64_t i0 = (int64_t)blockIdx.x * kStatParticles, n = ws.n;
-  const int np = (int)min((int64_t)kStatParticles, n - i0);
-  const float* bad = ws.rates + kRateBad * n + i0;
-  for (int q = threadIdx.x; q < np * JA; q += blockDim.x) {
-    const int i = q / JA, t = q - i * JA;
-    if (bad[i] != 0.0f) continue;
-    const int j = t / A, ai = t - (t / A) * A;
-    const double* bm = a.beta_mom + ((j < a.n_pulse_conds ? 0 : 1) * A + ai) * 3;
-    const double mb = bm[0], m2 = bm[1], vb = bm[2];
-    double sm[5];
-#pragma unroll
-    for (int e = 0; e < 5; ++e) sm[e] = ws.mom[(i0 * JA + q) * 5 + e];
-    double* d = ds + (size_t)q * 5;
-    d[0] = sm[0] * mb;
-    d[1] = sm[1] * mb;
-    d[2] = ((mb - m2) * sm[0] + vb * (sm[0] * sm[0] + sm[2])) + mb * mb * sm[2];
-    d[4] = ((mb - m2) * sm[1] + vb * (sm[1] * sm[1] + sm[4])) + mb * mb * sm[4];
-    d[3] = vb * (sm[0] * sm[1] + sm[3]) + mb * mb * sm[3];
-    if (a.moments)
-#pragma unroll
-      for (int e = 0; e < 5; ++e) a.moments[((p0 + i0) * JA + q) * 5 + e] = sm[e];
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < np * J; q += blockDim.x) {
-    const int i = q / J, j = q - i * J;
-    if (bad[i] == 0.0f)
-      stats_from_moments_cond(cfg, ds + (size_t)i * JA * 5, a.age_dist, a.stats + (p0 + i0 + i) * K, j);
-  }
-  for (int q = threadIdx.x; q < np * K; q += blockDim.x) {
-    const int i = q / K;
-    if (bad[i] == 0.0f) continue;
-    a.stats[(p0 + i0) * K + q] = NAN;
-    if (q == i * K) atomicOr(a.status, 1);
-  }
-}
-
-// particles per chunk: propagators of at most ~256 MB
-int64_t moment_chunk(int64_t P, int nsub) {
-  const int64_t bytes = (int64_t)2 * nsub * kQuads * (int64_t)sizeof(float4);
-  return std::max<int64_t>(1, std::min<int64_t>(P, ((int64_t)256 << 20) / bytes));
-}
-
 }  // namespace
 
 size_t moment_f32_scratch(int64_t P, int nsub, int pairs) {
-  const size_t n = (size_t)moment_chunk(P, nsub);
+  const size_t n = (size_t)moment_chunk(P, nsub, kQuads * sizeof(float4));
   return n * ((2 * (size_t)nsub + 1) * kQuads * sizeof(float4) + ((size_t)pairs * (NA + 5) + kRates) * sizeof(float));
 }
 
 cudaError_t launch_moment_f32(const MomArgs& a, cudaStream_t s) {
   if (a.P <= 0) return cudaSuccess;
-  const DevCfg& cfg = a.cfg;
-  const int A = cfg.n_ages, pairs = cfg.n_conds * A;
-  MomPlan plan;
-  plan.n = pairs;
-  int lo[kMaxPairs];
-  for (int t = 0; t < pairs; ++t) {
-    const double age = cfg.ages[t % A], texp = (age - cfg.pulse[t / A]) - cfg.chase[t / A];
-    lo[t] = (int)std::min(std::lround((texp - cfg.t0) / a.h), std::lround((age - cfg.t0) / a.h));
-    plan.pair[t] = t;
-  }
-  std::sort(plan.pair, plan.pair + pairs, [&](int x, int y) { return lo[x] != lo[y] ? lo[x] < lo[y] : x < y; });
-  for (int q = 0; q < pairs; ++q) {
-    const int t = plan.pair[q];
-    const double age = cfg.ages[t % A], texp = (age - cfg.pulse[t / A]) - cfg.chase[t / A];
-    plan.lo[q] = lo[t];
-    plan.hi[q] = (int)std::lround((texp + cfg.pulse[t / A] - cfg.t0) / a.h);
-    plan.end[q] = (int)std::lround((age - cfg.t0) / a.h);
-  }
-  const int64_t chunk = moment_chunk(a.P, a.nsub);
+  const MomPlan plan = moment_plan(a);
+  const int pairs = plan.n;
+  const int64_t chunk = moment_chunk(a.P, a.nsub, kQuads * sizeof(float4));
   for (int64_t p0 = 0; p0 < a.P; p0 += chunk) {
     const int64_t n = std::min<int64_t>(chunk, a.P - p0);
     MomScratch ws;
@@ -591,7 +512,8 @@ cudaError_t launch_moment_f32(const MomArgs& a, cudaStream_t s) {
     moment_walk_kernel<<<(unsigned)((n + 31) / 32), 32, 0, s>>>(a, p0, ws, plan);
     moment_path_kernel<<<dim3((unsigned)((n + kPathParticles - 1) / kPathParticles),
                               (pairs + kPathGroup - 1) / kPathGroup), 32, 0, s>>>(a, ws, plan);
-    moment_stats_kernel<<<(unsigned)((n + kStatParticles - 1) / kStatParticles), 128, stat_smem(pairs), s>>>(a, p0, ws);
+    moment_stats_kernel<float><<<(unsigned)((n + kStatParticles - 1) / kStatParticles), 128, stat_smem(pairs), s>>>(
+        a, p0, n, ws.mom, ws.rates + kRateBad * n);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
