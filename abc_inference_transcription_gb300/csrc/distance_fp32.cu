@@ -424,17 +424,15 @@ cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int6
 //     sig = a sd), and L_pg = m - z sqrt(v).
 // keep[p] = 1 when L_pg <= X[g] for some gene (X = calibrated threshold).  A
 // draw is dropped only when it is confidently far from every gene.  Tiles of
-// 128 draws x 16 GJ genes, GJ genes per thread: 8, as dist_fast_kernel, or 1
-// for at most 32 genes, where the wide tile computes mostly padding (65,536
-// draws x 4 genes: 108 us wide, 41 narrow).
-template <int MODE, int GJ>
+// 128 draws x 128 genes, 8 x 8 per thread, as dist_fast_kernel.
+template <int MODE>
 __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restrict__ mu,
                                                           const float* __restrict__ var,
                                                           const float* __restrict__ sw,
                                                           const float* __restrict__ dw, int64_t P, int64_t G,
                                                           int K, const float* __restrict__ X, float z,
                                                           uint8_t* keep, float* err_out) {
-  constexpr int N2 = MODE ? 8 : 1, M2 = MODE ? GJ : 1, kGenes = 16 * GJ;
+  constexpr int GJ = 8, N2 = MODE ? 8 : 1, M2 = MODE ? GJ : 1, kGenes = 16 * GJ;
   __shared__ float sm[kDistKc][kDistTile + 1];
   __shared__ float sv[kDistKc][kDistTile + 1];
   __shared__ float sa[kDistKc][kGenes + 1];
@@ -526,20 +524,120 @@ __global__ void __launch_bounds__(256) dist_screen_kernel(const float* __restric
   }
 }
 
+// The same for up to GC genes: a thread takes a draw, with the errors to every
+// gene in registers, and reads the genes' terms of a statistic as broadcasts.
+// What bounds it is the shared-memory reads: 2 + GC / 2 words per statistic and
+// draw, where the tile of draws x genes reads 2 per gene, padding included (65,536 draws
+// x 53 statistics x 4 genes: 108 us in tiles of 128 genes, 32 in tiles of 16,
+// 15 here).
+constexpr int kScreenRows = 128, kScreenKc = 32;
+template <int MODE, int GC>
+__global__ void __launch_bounds__(kScreenRows) dist_screen_rows_kernel(const float* __restrict__ mu,
+                                                                       const float* __restrict__ var,
+                                                                       const float* __restrict__ sw,
+                                                                       const float* __restrict__ dw, int64_t P, int G,
+                                                                       int K, const float* __restrict__ X, float z,
+                                                                       uint8_t* keep, float* err_out) {
+  __shared__ float sm[kScreenRows][kScreenKc + 1], sv[kScreenRows][kScreenKc + 1];
+  __shared__ float4 sa[kScreenKc][GC / 4], sd[kScreenKc][GC / 4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t p0 = (int64_t)blockIdx.x * kScreenRows;
+  float acc[GC], acc2[MODE ? GC : 1];
+#pragma unroll
+  for (int j = 0; j < GC; ++j) acc[j] = 0.0f;
+#pragma unroll
+  for (int j = 0; j < (MODE ? GC : 1); ++j) acc2[j] = 0.0f;
+  for (int k0 = 0; k0 < K; k0 += kScreenKc) {
+    const int k = k0 + lane;
+    // a warp's 32 rows, eight at a time
+    for (int r0 = warp * 32; r0 < warp * 32 + 32; r0 += 8) {
+      float m[8], v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int64_t p = p0 + r0 + u;
+        const bool in = p < P && k < K;
+        m[u] = in ? mu[p * K + k] : 0.0f;
+        v[u] = in ? var[p * K + k] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float s = sqrtf(fmaxf(v[u], 0.0f));  // predictive std
+        sm[r0 + u][lane] = m[u];
+        sv[r0 + u][lane] = MODE == 0 ? s * z : s;
+      }
+    }
+    for (int q = threadIdx.x; q < kScreenKc * GC; q += kScreenRows) {
+      const int g = q / kScreenKc, kk = q - g * kScreenKc;
+      const bool in = g < G && k0 + kk < K;
+      reinterpret_cast<float*>(sa[kk])[g] = in ? sw[(int64_t)g * K + k0 + kk] : 0.0f;
+      reinterpret_cast<float*>(sd[kk])[g] = in ? dw[(int64_t)g * K + k0 + kk] : 0.0f;
+    }
+    __syncthreads();
+    const int kc = (K - k0) < kScreenKc ? (K - k0) : kScreenKc;
+#pragma unroll 2
+    for (int kk = 0; kk < kc; ++kk) {
+      const float m = sm[threadIdx.x][kk], v = sv[threadIdx.x][kk];
+#pragma unroll
+      for (int q = 0; q < GC / 4; ++q) {
+        const float4 a4 = sa[kk][q], d4 = sd[kk][q];
+        const float a[4] = {a4.x, a4.y, a4.z, a4.w}, d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = 4 * q + u;
+          if (MODE == 0) {
+            const float t = fmaxf(fabsf(fmaf(-a[u], m, d[u])) - a[u] * v, 0.0f);
+            acc[j] = fmaf(t, t, acc[j]);
+          } else {
+            const float dl = fmaf(-a[u], m, d[u]);
+            const float sg = a[u] * v;
+            const float s2 = sg * sg, d2 = dl * dl;
+            acc[j] += d2 + s2;
+            acc2[MODE ? j : 0] = fmaf(s2, fmaf(4.0f, d2, 2.0f * s2), acc2[MODE ? j : 0]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const int64_t p = p0 + threadIdx.x;
+  if (p >= P) return;
+  const float invK = 1.0f / (float)K;
+  bool any = false;
+#pragma unroll
+  for (int j = 0; j < GC; ++j) {
+    if (j >= G) break;
+    float e = acc[j] * invK;  // not clipped: far draws keep large predicted errors
+    if (MODE == 1) e -= z * sqrtf(acc2[MODE ? j : 0]) * invK;
+    if (err_out) err_out[p * G + j] = e;
+    any = any || (e <= X[j]);
+  }
+  if (any) keep[p] = 1;
+}
+
+template <int MODE>
+static void launch_screen(const float* mu, const float* var, const float* sw, const float* dw, int64_t P, int64_t G,
+                          int K, const float* X, float z, uint8_t* keep, float* err_out, cudaStream_t s) {
+  const unsigned rows = (unsigned)((P + kScreenRows - 1) / kScreenRows);
+  if (G <= 4)
+    dist_screen_rows_kernel<MODE, 4><<<rows, kScreenRows, 0, s>>>(mu, var, sw, dw, P, (int)G, K, X, z, keep, err_out);
+  else if (G <= 16)
+    dist_screen_rows_kernel<MODE, 16><<<rows, kScreenRows, 0, s>>>(mu, var, sw, dw, P, (int)G, K, X, z, keep, err_out);
+  else if (G <= 32)
+    dist_screen_rows_kernel<MODE, 32><<<rows, kScreenRows, 0, s>>>(mu, var, sw, dw, P, (int)G, K, X, z, keep, err_out);
+  else
+    dist_screen_kernel<MODE><<<dim3((unsigned)((G + kDistTile - 1) / kDistTile),
+                                    (unsigned)((P + kDistTile - 1) / kDistTile)), 256, 0, s>>>(mu, var, sw, dw, P, G, K,
+                                                                                              X, z, keep, err_out);
+}
+
 cudaError_t launch_dist_screen(const float* mu, const float* var, const float* sw, const float* dw, int64_t P,
                                int64_t G, int K, const float* X, float z, int mode, uint8_t* keep, float* err_out,
                                cudaStream_t s) {
   if (P <= 0 || G <= 0) return cudaSuccess;
-  const int genes = G <= 32 ? 16 : kDistTile;
-  dim3 grid((unsigned)((G + genes - 1) / genes), (unsigned)((P + kDistTile - 1) / kDistTile));
-  if (mode == 1 && genes == 16)
-    dist_screen_kernel<1, 1><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
-  else if (mode == 1)
-    dist_screen_kernel<1, 8><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
-  else if (genes == 16)
-    dist_screen_kernel<0, 1><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
+  if (mode == 1)
+    launch_screen<1>(mu, var, sw, dw, P, G, K, X, z, keep, err_out, s);
   else
-    dist_screen_kernel<0, 8><<<grid, 256, 0, s>>>(mu, var, sw, dw, P, G, K, X, z, keep, err_out);
+    launch_screen<0>(mu, var, sw, dw, P, G, K, X, z, keep, err_out, s);
   return cudaGetLastError();
 }
 

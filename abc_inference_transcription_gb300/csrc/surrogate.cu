@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/abcgpu.h"
+#include "distance.cuh"
 #include "kernels.h"
 #include "mlp.cuh"
 
@@ -71,19 +72,40 @@ struct Buf {
   }
 };
 
-// column mean / standard deviation over finite values (two passes)
-__global__ void col_norm_kernel(const double* X, int64_t N, int ld, int cols, double* mean, double* sd) {
+// f(x) for rows tid, tid + 256, ... of column c, in row order.  The columns lie a
+// row apart and a block takes one, so what bounds it is the latency of the loads:
+// kColAhead are under way at a time.
+constexpr int kColAhead = 16;
+template <typename F>
+__device__ __forceinline__ void each_row(const double* X, int64_t N, int ld, int c, F f) {
+  const int64_t step = blockDim.x;
+  int64_t i = threadIdx.x;
+  for (; i + (kColAhead - 1) * step < N; i += kColAhead * step) {
+    double v[kColAhead];
+#pragma unroll
+    for (int j = 0; j < kColAhead; ++j) v[j] = X[(i + j * step) * ld + c];
+#pragma unroll
+    for (int j = 0; j < kColAhead; ++j) f(v[j]);
+  }
+  for (; i < N; i += step) f(X[i * ld + c]);
+}
+__device__ __forceinline__ bool finite_bits(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
+
+// column mean / standard deviation over finite values (two passes; 40,000 rows x
+// 53 columns: 85 us one load at a time, 52 now)
+__global__ void __launch_bounds__(256, 2) col_norm_kernel(const double* X, int64_t N, int ld, int cols, double* mean,
+                                                       double* sd) {
   __shared__ double red[256];
   __shared__ double cnt[256];
   const int c = blockIdx.x;
   if (c >= cols) return;
-  double s = 0.0, n = 0.0;
-  for (int64_t i = threadIdx.x; i < N; i += blockDim.x) {
-    const double v = X[i * ld + c];
-    if (isfinite(v)) { s += v; n += 1.0; }
-  }
+  double s = 0.0;
+  int n = 0;
+  each_row(X, N, ld, c, [&](double v) {
+    if (finite_bits(v)) { s += v; ++n; }
+  });
   red[threadIdx.x] = s;
-  cnt[threadIdx.x] = n;
+  cnt[threadIdx.x] = (double)n;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if (threadIdx.x < o) { red[threadIdx.x] += red[threadIdx.x + o]; cnt[threadIdx.x] += cnt[threadIdx.x + o]; }
@@ -93,10 +115,9 @@ __global__ void col_norm_kernel(const double* X, int64_t N, int ld, int cols, do
   const double nn = cnt[0];
   __syncthreads();
   double q = 0.0;
-  for (int64_t i = threadIdx.x; i < N; i += blockDim.x) {
-    const double v = X[i * ld + c];
-    if (isfinite(v)) q += (v - mu) * (v - mu);
-  }
+  each_row(X, N, ld, c, [&](double v) {
+    if (finite_bits(v)) q += (v - mu) * (v - mu);
+  });
   red[threadIdx.x] = q;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
@@ -110,55 +131,70 @@ __global__ void col_norm_kernel(const double* X, int64_t N, int ld, int cols, do
   }
 }
 
+// Standardised values (v - mean) / sd, rounded to float.  The columns' means,
+// deviations and their correctly rounded reciprocals stand in shared memory, so
+// that a quotient is three FP64 operations (div_rn, equal to the division)
+// and the rounding to float none: the FP64 pipe bounds both kernels (65,536 x 14 inputs:
+// 18 us with divisions, 12 now; 40,000 x 53 targets: 45, 28).
+constexpr int kNormCols = 256;  // statistics, at most
+struct NormCols {
+  double mean[kNormCols], sd[kNormCols], rsd[kNormCols];
+  __device__ __forceinline__ void load(const double* m, const double* s, int cols) {
+    for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+      mean[c] = m[c];
+      sd[c] = s[c];
+      rsd[c] = 1.0 / s[c];
+    }
+    __syncthreads();
+  }
+  __device__ __forceinline__ float apply(double v, int c) const {
+    const double d = v - mean[c];
+    return rn32_bits((__double_as_longlong(d) << 1) == 0 ? d / sd[c] : div_rn(d, sd[c], rsd[c]));
+  }
+};
+
 // theta (FP64, row stride ld) -> standardised FP32 [N][in_pad] (zero padding)
-__global__ void norm_x_kernel(const double* th, int64_t N, int in_dim, int ld, const double* mean, const double* sd,
-                              int in_pad, float* xf, __nv_bfloat16* xh) {
+__global__ void __launch_bounds__(256) norm_x_kernel(const double* th, int64_t N, int in_dim, int ld,
+                                                     const double* mean, const double* sd, int in_pad, float* xf,
+                                                     __nv_bfloat16* xh) {
+  __shared__ NormCols cols;
+  cols.load(mean, sd, in_dim);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N * in_pad;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / in_pad;
     const int c = (int)(i - r * in_pad);
-    float v = 0.0f;
-    if (c < in_dim) v = (float)((th[r * ld + c] - mean[c]) / sd[c]);
+    const float v = c < in_dim ? cols.apply(th[r * ld + c], c) : 0.0f;
     if (xf) xf[i] = v;
     if (xh) xh[i] = __float2bfloat16(v);
   }
 }
 
 // statistics -> standardised FP32 targets, NaN where not finite
-__global__ void norm_y_kernel(const double* st, int64_t N, int K, const double* mean, const double* sd, float* yf) {
+__global__ void __launch_bounds__(256) norm_y_kernel(const double* st, int64_t N, int K, const double* mean,
+                                                     const double* sd, float* yf) {
+  __shared__ NormCols cols;
+  cols.load(mean, sd, K);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N * K; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % K);
     const double v = st[i];
-    yf[i] = isfinite(v) ? (float)((v - mean[c]) / sd[c]) : __int_as_float(0x7fc00000);
+    yf[i] = finite_bits(v) ? cols.apply(v, (int)(i % K)) : __int_as_float(0x7fc00000);
   }
 }
 
 // per statistic: scale c = mean |y| over finite values (1 if none); the asinh
 // itself is asinh_fit_kernel's, over all values at once (in this kernel's one
-// block per statistic it took 0.9 ms for 40,000 x 53 values).  The columns lie
-// a row apart, so four values are loaded before they are added, in row order.
-__global__ void __launch_bounds__(256) abs_scale_kernel(const double* st, int64_t N, int K, double* scale,
+// block per statistic it took 0.9 ms for 40,000 x 53 values).
+__global__ void __launch_bounds__(256, 2) abs_scale_kernel(const double* st, int64_t N, int K, double* scale,
                                                         float* scale32) {
   __shared__ double red[256];
   __shared__ double cnt[256];
   const int c = blockIdx.x;
-  double s = 0.0, n = 0.0;
-  const int64_t step = blockDim.x;
-  int64_t i = threadIdx.x;
-  for (; i + 3 * step < N; i += 4 * step) {
-    double v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = st[(i + j * step) * K + c];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (isfinite(v[j])) { s += fabs(v[j]); n += 1.0; }
-  }
-  for (; i < N; i += step) {
-    const double v = st[i * K + c];
-    if (isfinite(v)) { s += fabs(v); n += 1.0; }
-  }
+  double s = 0.0;
+  int n = 0;
+  each_row(st, N, K, c, [&](double v) {
+    if (finite_bits(v)) { s += fabs(v); ++n; }
+  });
   red[threadIdx.x] = s;
-  cnt[threadIdx.x] = n;
+  cnt[threadIdx.x] = (double)n;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if (threadIdx.x < o) { red[threadIdx.x] += red[threadIdx.x + o]; cnt[threadIdx.x] += cnt[threadIdx.x + o]; }
@@ -206,6 +242,8 @@ __global__ void count_keep_kernel(const uint8_t* keep, int64_t N, unsigned long 
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(n, c);
 }
 
+// of the kernels that keep the columns' terms per block
+int norm_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 152 * 8); }
 int blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 65536); }
 
 // Survivor compaction in ascending row order: per-1024-row counts, one scan,
@@ -226,15 +264,22 @@ __global__ void compact_count_kernel(const uint8_t* keep, int64_t N, unsigned in
   }
 }
 
-__global__ void compact_scan_kernel(unsigned int* counts, int64_t nb, unsigned long long* total) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned long long run = 0;
-  for (int64_t b = 0; b < nb; ++b) {
-    const unsigned int c = counts[b];
-    counts[b] = (unsigned int)run;
-    run += c;
+// exclusive prefix sums in place, a warp (one thread alone took 18 us for 489 counts)
+__global__ void __launch_bounds__(32) compact_scan_kernel(unsigned int* counts, int64_t nb,
+                                                          unsigned long long* total) {
+  unsigned int run = 0;
+  for (int64_t b0 = 0; b0 < nb; b0 += 32) {
+    const int64_t b = b0 + threadIdx.x;
+    const unsigned int c = b < nb ? counts[b] : 0u;
+    unsigned int incl = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)threadIdx.x >= o) incl += v;
+    }
+    if (b < nb) counts[b] = run + incl - c;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  *total = run;
+  if (threadIdx.x == 0) *total = run;
 }
 
 __global__ void compact_scatter_kernel(const uint8_t* keep, int64_t N, const unsigned int* start, const double* th,
@@ -460,9 +505,9 @@ static int load_training(abc_surrogate* s, const double* theta, const double* st
   } else {
     asinh_apply_kernel<<<blocks(N * d.K), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->yscf.p);
   }
-  norm_x_kernel<<<blocks(N * d.in_pad), 256, 0, s->stream>>>(s->th64.p, N, d.in_dim, d.in_dim, s->xm.p, s->xs.p,
+  norm_x_kernel<<<norm_blocks(N * d.in_pad), 256, 0, s->stream>>>(s->th64.p, N, d.in_dim, d.in_dim, s->xm.p, s->xs.p,
                                                               d.in_pad, s->xn.p, nullptr);
-  norm_y_kernel<<<blocks(N * d.K), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->ym.p, s->ys.p, s->yn.p);
+  norm_y_kernel<<<norm_blocks(N * d.K), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->ym.p, s->ys.p, s->yn.p);
   SK(cudaGetLastError());
   return ABC_OK;
 }
@@ -592,7 +637,7 @@ static int forward_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_
   const int E = s->members;
   SK(s->X0.ensure((size_t)n * d.in_pad));
   SK(s->Y.ensure((size_t)E * n * d.out_pad));
-  norm_x_kernel<<<blocks(n * d.in_pad), 256, 0, s->stream>>>(d_theta, n, d.in_dim, ld, s->xm.p, s->xs.p, d.in_pad,
+  norm_x_kernel<<<norm_blocks(n * d.in_pad), 256, 0, s->stream>>>(d_theta, n, d.in_dim, ld, s->xm.p, s->xs.p, d.in_pad,
                                                               nullptr, s->X0.p);
   SK(cudaGetLastError());
   if (mlp_infer_fits(d)) {
