@@ -235,13 +235,6 @@ ABC_HD double wsum(const double* w, const double* x, int A) {
   for (int a = 1; a < A; ++a) s = s + w[a] * x[a];
   return s;
 }
-ABC_HD double wcov(const double* x, const double* y, const double* w, int A) {
-  double mx = wsum(w, x, A), my = wsum(w, y, A);
-  double s = w[0] * ((x[0] - mx) * (y[0] - my));
-  for (int a = 1; a < A; ++a) s = s + w[a] * ((x[a] - mx) * (y[a] - my));
-  return s;
-}
-
 // the statistics of condition j (its ratio, mean_corr and corr_mean, and the
 // pulse or chase means and Fano factors when j is that condition); conditions
 // write disjoint entries, so they may run in any order or in parallel
@@ -258,13 +251,22 @@ ABC_HD void stats_from_moments_cond(const DevCfg& cfg, const double* m, const do
       cv[a] = g[3];
       vl[a] = g[4];
     }
-    double swu = wsum(w, mu, A), swl = wsum(w, ml, A);
+    const double swu = wsum(w, mu, A), swl = wsum(w, ml, A);
     st[4 * A + j] = swl / (swu + swl);
-    double tvu = wsum(w, vu, A) + wcov(mu, mu, w, A);
-    double tvl = wsum(w, vl, A) + wcov(ml, ml, w, A);
-    double stds = sqrt(fabs(tvu * tvl));
+    // wcov(mu, mu), wcov(ml, ml) and wcov(mu, ml): the means above and the deviations once
+    double suu = 0.0, sll = 0.0, sul = 0.0;
+    for (int a = 0; a < A; ++a) {
+      const double du = mu[a] - swu, dl = ml[a] - swl;
+      const double pu = w[a] * (du * du), pl = w[a] * (dl * dl), pc = w[a] * (du * dl);
+      suu = a ? suu + pu : pu;
+      sll = a ? sll + pl : pl;
+      sul = a ? sul + pc : pc;
+    }
+    const double tvu = wsum(w, vu, A) + suu;
+    const double tvl = wsum(w, vl, A) + sll;
+    const double stds = sqrt(fabs(tvu * tvl));
     st[4 * A + J + j] = wsum(w, cv, A) / stds;
-    st[4 * A + 2 * J + j] = wcov(mu, ml, w, A) / stds;
+    st[4 * A + 2 * J + j] = sul / stds;
     int off = (j == cfg.pulse_stat) ? 0 : (j == cfg.chase_stat) ? 2 * A : -1;
     if (off >= 0) {
       for (int a = 0; a < A; ++a) {
