@@ -107,8 +107,8 @@ struct abc_ctx {
   DBuf<float> d_tcA, d_tcB, d_cg32, d_b0, d_Y, d_Xt, d_seg_e;
   DBuf<uint8_t> d_rowbad;  // per particle of the candidate pass: a statistic is NaN
   DBuf<double> d_cg64;
-  DBuf<unsigned> d_tcflags, d_segcount, d_hist;
-  DBuf<int> d_tcerr;
+  DBuf<unsigned> d_tcstat, d_hist;  // d_tcstat: kTcFlags operand flags, the pass's error word, then per-CTA counts
+  void* h_pin = nullptr;            // pinned words for small results (kPinBytes)
   DBuf<Cand> d_seg, d_cand2;
   int64_t seg_cap = int64_t(1) << 16;
   DBuf<int32_t> d_sp, d_sg;
@@ -275,14 +275,15 @@ int abc_destroy(abc_ctx* c) {
   c->d_out_err.release(); c->d_sw.release(); c->d_dw.release(); c->d_s32.release(); c->d_X.release();
   c->d_esub.release(); c->d_cand.release(); c->d_sp.release(); c->d_gcount.release(); c->d_goff.release();
   c->d_cande.release(); c->d_den.release(); c->d_rden.release(); c->d_tcA.release(); c->d_tcB.release(); c->d_rowbad.release(); c->d_cg32.release(); c->d_b0.release();
-  c->d_Y.release(); c->d_Xt.release(); c->d_seg_e.release(); c->d_cg64.release(); c->d_tcflags.release();
-  c->d_segcount.release(); c->d_hist.release(); c->d_tcerr.release(); c->d_seg.release(); c->d_cand2.release();
+  c->d_Y.release(); c->d_Xt.release(); c->d_seg_e.release(); c->d_cg64.release(); c->d_tcstat.release();
+  c->d_hist.release(); c->d_seg.release(); c->d_cand2.release();
   c->d_alen.release(); c->d_aoff.release(); c->d_out_idx.release(); c->d_gcursor.release();
   c->d_ncand.release(); c->d_fail.release(); c->d_thr.release();
   c->d_asp.release(); c->d_asg.release(); c->d_aerr.release(); c->d_work.release();
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   for (cudaEvent_t e : c->sel_ev)
     if (e) cudaEventDestroy(e);
+  if (c->h_pin) cudaFreeHost(c->h_pin);
   cudaStreamDestroy(c->stream);
   delete c;
   return ABC_OK;
@@ -904,7 +905,9 @@ static int load_dist_inputs(abc_ctx* c, const double* data, const double* se, in
   in.se = c->d_se.p;
   CK(c->d_den.ensure((size_t)G * K));
   CK(c->d_rden.ensure((size_t)G * K));
-  CK(launch_dist_den(in, c->d_den.p, c->d_rden.p, c->stream));
+  CK(c->d_sw.ensure((size_t)G * K));
+  CK(c->d_dw.ensure((size_t)G * K));
+  CK(launch_dist_den(in, c->d_den.p, c->d_rden.p, c->d_sw.p, c->d_dw.p, c->stream));
   in.den = c->d_den.p;
   in.rden = c->d_rden.p;
   if (stats_on_device) {
@@ -927,8 +930,6 @@ int abc_errors(abc_ctx* c, const double* data, const double* se, int64_t G, int 
   Work w;
   const size_t o_out = w.add(sizeof(double) * (size_t)P * G);
   CK(w.allocate(c));
-  CK(c->d_sw.ensure((size_t)G * K));
-  CK(c->d_dw.ensure((size_t)G * K));
   CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, w.at<double>(o_out), c->stream));
   CK(cudaMemcpyAsync(err_out, w.at<double>(o_out), sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -986,20 +987,39 @@ static int candidate_pass_simt(abc_ctx* c, const DistInputs& in, int64_t* n) {
   return fail(c, ABC_ERR_CAPACITY, "candidate buffer overflow");
 }
 
+// Small results come back through pinned words of the context: a copy to pageable
+// memory makes the host wait for it, one after the other.
+constexpr size_t kPinBytes = 4096;
+constexpr int kTcFlags = 3;  // words of launch_tc_prep's flags
+static int pinned_words(abc_ctx* c) {
+  if (!c->h_pin) CK(cudaMallocHost(&c->h_pin, kPinBytes));
+  return ABC_OK;
+}
+
 // Tensor-core candidate pass: each CTA appends to its own segment; the
-// segments are concatenated into d_cand / d_cande.
-static int candidate_pass_tc(abc_ctx* c, const DistInputs& in, int nh, int64_t* n) {
+// segments are concatenated into d_cand / d_cande.  *redo: the operands left the
+// range of the pass (prepare_candidate_pass) and nothing was found; the FP32 pass
+// serves them.
+static int candidate_pass_tc(abc_ctx* c, const DistInputs& in, int nh, int64_t* n, bool* redo) {
   const int grid = tc_grid(in.P, in.G, c->sms);
   const TcLayout L = tc_layout(in.K, nh);
   CK(launch_tc_y(c->d_X.p, c->d_cg64.p, in.G, in.K, c->d_Y.p, c->stream));
-  CK(c->d_segcount.ensure((size_t)grid));
-  CK(c->d_tcerr.ensure(1));
-  std::vector<unsigned> cnt((size_t)grid);
+  int st = pinned_words(c);
+  if (st) return st;
+  unsigned* seg_count = c->d_tcstat.p + kTcFlags + 1;
+  std::vector<unsigned> big;
+  unsigned* stat = static_cast<unsigned*>(c->h_pin);
+  const size_t words = kTcFlags + 1 + (size_t)grid;
+  if (words * sizeof(unsigned) > kPinBytes) {
+    big.resize(words);
+    stat = big.data();
+  }
+  const unsigned* cnt = stat + kTcFlags + 1;
+  *redo = false;
   for (int attempt = 0; attempt < 2; ++attempt) {
     CK(c->d_seg.ensure((size_t)grid * (size_t)c->seg_cap));
     CK(c->d_seg_e.ensure((size_t)grid * (size_t)c->seg_cap));
-    CK(cudaMemsetAsync(c->d_segcount.p, 0, sizeof(unsigned) * grid, c->stream));
-    CK(cudaMemsetAsync(c->d_tcerr.p, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->d_tcstat.p + kTcFlags, 0, sizeof(unsigned) * (1 + (size_t)grid), c->stream));
     TcArgs a;
     a.P = in.P;
     a.G = in.G;
@@ -1014,20 +1034,26 @@ static int candidate_pass_tc(abc_ctx* c, const DistInputs& in, int nh, int64_t* 
     a.cand = c->d_seg.p;
     a.cand_e = c->d_seg_e.p;
     a.seg_cap = c->seg_cap;
-    a.seg_count = c->d_segcount.p;
-    a.err = c->d_tcerr.p;
-    int st = prof_begin(c);
+    a.seg_count = seg_count;
+    a.err = reinterpret_cast<int*>(c->d_tcstat.p + kTcFlags);
+    st = prof_begin(c);
     if (st) return st;
     CK(launch_dist_tc(nh, c->d_tcA.p, c->d_tcB.p, a, grid, c->stream));
     st = prof_end(c);
     if (st) return st;
-    int herr = 0;
-    CK(cudaMemcpyAsync(cnt.data(), c->d_segcount.p, sizeof(unsigned) * grid, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&herr, c->d_tcerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(stat, c->d_tcstat.p, sizeof(unsigned) * words, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (herr)
-      return fail(c, ABC_ERR_CUDA,
-                  "tensor-core distance pass: a bounded wait ran out (code " + std::to_string(herr) + ")");
+    if (stat[kTcFlags])
+      return fail(c, ABC_ERR_CUDA, "tensor-core distance pass: a bounded wait ran out (code " +
+                                       std::to_string((int)stat[kTcFlags]) + ")");
+    float maxw, maxs2;
+    memcpy(&maxw, &stat[1], 4);
+    memcpy(&maxs2, &stat[2], 4);
+    if (stat[0] || (double)maxw * (double)maxs2 * (4.0 * in.K) > 1e37) {
+      *redo = true;
+      *n = 0;
+      return ABC_OK;
+    }
     int64_t total = 0, mx = 0;
     for (int b = 0; b < grid; ++b) {
       total += cnt[b];
@@ -1039,7 +1065,7 @@ static int candidate_pass_tc(abc_ctx* c, const DistInputs& in, int nh, int64_t* 
     if (mx <= c->seg_cap) {
       CK(c->d_cand.ensure((size_t)std::max<int64_t>(total, 1)));
       CK(c->d_cande.ensure((size_t)std::max<int64_t>(total, 1)));
-      CK(launch_tc_gather(c->d_seg.p, c->d_seg_e.p, c->d_segcount.p, grid, c->seg_cap, c->d_cg32.p, in.K, c->d_cand.p,
+      CK(launch_tc_gather(c->d_seg.p, c->d_seg_e.p, seg_count, grid, c->seg_cap, c->d_cg32.p, in.K, c->d_cand.p,
                           c->d_cande.p, c->stream));
       *n = total;
       return ABC_OK;
@@ -1050,15 +1076,14 @@ static int candidate_pass_tc(abc_ctx* c, const DistInputs& in, int nh, int64_t* 
 }
 
 // Operands of the candidate pass and its error bound |e32 - e| <= b0[g] + b1 e.
-// Tensor cores (the requested mode) unless an operand is infinite or w s^2
-// could leave the FP32 range; then the FP32 CUDA-core pass.
-static int prepare_candidate_pass(abc_ctx* c, const DistInputs& in, int* dmode_out, float* b1_out) {
+// Tensor cores in mode `want`; whether an operand is infinite or w s^2 could
+// leave the FP32 range is told after the pass (candidate_pass_tc), and the caller
+// then starts again with want = 0, the FP32 CUDA-core pass.
+static int prepare_candidate_pass(abc_ctx* c, const DistInputs& in, int want, int* dmode_out, float* b1_out) {
   const int64_t G = in.G, P = in.P;
   const int K = in.K;
-  CK(c->d_sw.ensure((size_t)G * K));
-  CK(c->d_dw.ensure((size_t)G * K));
   CK(c->d_b0.ensure((size_t)G));
-  int dmode = c->dist_mode;
+  int dmode = want;
   float b1 = 0.0f;
   if (dmode == 3 && !tc_mode3_fits(K)) dmode = 2;  // gene rows too long to stay in shared memory
   if (dmode) {
@@ -1069,25 +1094,17 @@ static int prepare_candidate_pass(abc_ctx* c, const DistInputs& in, int* dmode_o
     CK(c->d_cg64.ensure((size_t)G));
     CK(c->d_cg32.ensure((size_t)G));
     CK(c->d_Y.ensure((size_t)G));
-    CK(c->d_tcflags.ensure(3));
-    CK(cudaMemsetAsync(c->d_tcflags.p, 0, sizeof(unsigned) * 3, c->stream));
+    CK(c->d_tcstat.ensure(kTcFlags + 1 + (size_t)tc_grid(P, G, c->sms)));
+    CK(cudaMemsetAsync(c->d_tcstat.p, 0, sizeof(unsigned) * kTcFlags, c->stream));
     const double beta = tc_beta(K, dmode);
     CK(launch_tc_prep(in, dmode, beta, c->d_tcA.p, c->d_tcB.p, c->d_rowbad.p, c->d_cg64.p, c->d_cg32.p, c->d_b0.p,
-                      c->d_tcflags.p, c->stream));
-    unsigned fl[3];
-    CK(cudaMemcpyAsync(fl, c->d_tcflags.p, sizeof(fl), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    float maxw, maxs2;
-    memcpy(&maxw, &fl[1], 4);
-    memcpy(&maxs2, &fl[2], 4);
-    if (fl[0] || (double)maxw * (double)maxs2 * (4.0 * K) > 1e37) dmode = 0;
-    else b1 = (float)(4.0 * beta);
-  }
-  // FP32 statistics of every particle for the CUDA-core pass; the tensor-core
-  // pass needs them only for the threshold subsample (converted there)
-  if (dmode == 0) CK(c->d_s32.ensure((size_t)P * K));
-  CK(launch_dist_prep(in, c->d_sw.p, c->d_dw.p, dmode == 0 ? c->d_s32.p : nullptr, P, 1, c->stream));
-  if (dmode == 0) {
+                      c->d_tcstat.p, c->stream));
+    b1 = (float)(4.0 * beta);
+  } else {
+    // FP32 statistics of every particle for the CUDA-core pass; the tensor-core
+    // pass needs them only for the threshold subsample (converted there)
+    CK(c->d_s32.ensure((size_t)P * K));
+    CK(launch_dist_rows32(in, c->d_s32.p, P, 1, c->stream));
     // 1.5 u (64 sqrt(e) + (K + 8) e) <= 48 u + 1.5 u (K + 40) e, u = 2^-24
     const double u = 5.9604644775390625e-08;
     b1 = (float)(1.5 * u * (K + 40));
@@ -1126,54 +1143,62 @@ static int select_impl(abc_ctx* c, const double* data, const double* se, int64_t
   CK(c->d_gcursor.ensure((size_t)G));
   CK(c->d_alen.ensure((size_t)G));
   CK(c->d_aoff.ensure((size_t)G + 1));
-  CK(c->d_fail.ensure((size_t)G));
-  c->sel_fast_ms = 0.0;
-  c->sel_fast_passes = 0;
-  int dmode = 0;
-  float b1 = 0.0f;
-  st = prepare_candidate_pass(c, in, &dmode, &b1);
+  CK(c->d_fail.ensure((size_t)G + 1));  // their number, then per gene
+  st = pinned_words(c);
   if (st) return st;
   const int64_t kq = mode == 1 ? (int64_t)std::ceil(eps_or_q * (double)P) : 0;
-  std::vector<float> hX((size_t)G);
-  if (mode == 0 || mode == 2) {
-    CK(launch_x_from_thr(mode == 2 ? c->d_thr.p : nullptr, eps_or_q, G, c->d_b0.p, b1, c->d_X.p, c->stream));
-  } else {
-    // thresholds from a strided subsample
-    const int64_t n_sub = std::min<int64_t>(P, 32768);
-    const int64_t stride = std::max<int64_t>(1, P / n_sub);
-    const int64_t k_sub = (int64_t)std::ceil(2.0 * eps_or_q * (double)n_sub) + 16;
-    if (k_sub >= n_sub) {
-      std::fill(hX.begin(), hX.end(), INFINITY);
-      CK(cudaMemcpyAsync(c->d_X.p, hX.data(), sizeof(float) * G, cudaMemcpyHostToDevice, c->stream));
-    } else {
-      CK(c->d_esub.ensure((size_t)n_sub * G));
-      int64_t sub_stride = stride;
-      if (dmode) {
-        // the subsample rows, compacted
-        CK(c->d_s32.ensure((size_t)n_sub * K));
-        CK(launch_dist_prep(in, c->d_sw.p, c->d_dw.p, c->d_s32.p, n_sub, stride, c->stream));
-        sub_stride = 1;
-      }
-      CK(launch_dist_fast(c->d_s32.p, c->d_sw.p, c->d_dw.p, P, G, K, nullptr, nullptr, nullptr, nullptr, 0,
-                          c->d_esub.p, sub_stride, n_sub, c->stream));
-      CK(launch_dist_threshold(c->d_esub.p, n_sub, G, k_sub, c->d_b0.p, b1, c->d_X.p, c->stream));
-      if (dmode) {
-        // about k_sub of every n_sub particles per gene pass X: size the per-CTA
-        // segments for that (with room for imbalance) so one pass suffices
-        const int grid = tc_grid(P, G, c->sms);
-        const double est = (double)G * (double)k_sub * ((double)P / (double)n_sub);
-        const int64_t want = (int64_t)(1.5 * est / grid) + 4096;
-        c->seg_cap = std::max(c->seg_cap, std::min<int64_t>(want, kCandLimit / grid + 1));
-      }
-      CK(cudaMemcpyAsync(hX.data(), c->d_X.p, sizeof(float) * G, cudaMemcpyDeviceToHost, c->stream));
-    }
-  }
+  int dmode = 0;
+  float b1 = 0.0f;
   int64_t ncand = 0;
+  bool redo = true;
+  for (int want = c->dist_mode; redo; want = 0) {
+    redo = false;
+    c->sel_fast_ms = 0.0;
+    c->sel_fast_passes = 0;
+    st = prepare_candidate_pass(c, in, want, &dmode, &b1);
+    if (st) return st;
+    if (mode == 0 || mode == 2) {
+      CK(launch_x_from_thr(mode == 2 ? c->d_thr.p : nullptr, eps_or_q, G, c->d_b0.p, b1, c->d_X.p, c->stream));
+    } else {
+      // thresholds from a strided subsample
+      const int64_t n_sub = std::min<int64_t>(P, 32768);
+      const int64_t stride = std::max<int64_t>(1, P / n_sub);
+      const int64_t k_sub = (int64_t)std::ceil(2.0 * eps_or_q * (double)n_sub) + 16;
+      if (k_sub >= n_sub) {
+        CK(launch_fill(c->d_X.p, G, INFINITY, c->stream));
+      } else {
+        CK(c->d_esub.ensure((size_t)n_sub * G));
+        int64_t sub_stride = stride;
+        if (dmode) {
+          // the subsample rows, compacted
+          CK(c->d_s32.ensure((size_t)n_sub * K));
+          CK(launch_dist_rows32(in, c->d_s32.p, n_sub, stride, c->stream));
+          sub_stride = 1;
+        }
+        CK(launch_dist_fast(c->d_s32.p, c->d_sw.p, c->d_dw.p, P, G, K, nullptr, nullptr, nullptr, nullptr, 0,
+                            c->d_esub.p, sub_stride, n_sub, c->stream));
+        CK(launch_dist_threshold(c->d_esub.p, n_sub, G, k_sub, c->d_b0.p, b1, c->d_X.p, c->stream));
+        if (dmode) {
+          // about k_sub of every n_sub particles per gene pass X: size the per-CTA
+          // segments for that (with room for imbalance) so one pass suffices
+          const int grid = tc_grid(P, G, c->sms);
+          const double est = (double)G * (double)k_sub * ((double)P / (double)n_sub);
+          const int64_t want_cap = (int64_t)(1.5 * est / grid) + 4096;
+          c->seg_cap = std::max(c->seg_cap, std::min<int64_t>(want_cap, kCandLimit / grid + 1));
+        }
+      }
+    }
+    st = dmode ? candidate_pass_tc(c, in, dmode, &ncand, &redo) : candidate_pass_simt(c, in, &ncand);
+    if (st) return st;
+  }
+  int64_t total = 0;
   c->sel_rechecked = 0;
   c->sel_cands_emitted = 0;
   for (int round = 0; round < 4; ++round) {
-    st = dmode ? candidate_pass_tc(c, in, dmode, &ncand) : candidate_pass_simt(c, in, &ncand);
-    if (st) return st;
+    if (round > 0) {
+      st = dmode ? candidate_pass_tc(c, in, dmode, &ncand, &redo) : candidate_pass_simt(c, in, &ncand);
+      if (st) return st;
+    }
     const Cand* rc = c->d_cand.p;
     const float* Xacc = c->d_X.p;
     int64_t nre = ncand;
@@ -1184,10 +1209,10 @@ static int select_impl(abc_ctx* c, const double* data, const double* se, int64_t
       CK(c->d_cand2.ensure((size_t)std::max<int64_t>(ncand, 1)));
       CK(launch_refine(c->d_cand.p, c->d_cande.p, ncand, G, kq, c->d_X.p, c->d_b0.p, b1, c->d_hist.p, c->d_Xt.p,
                        c->d_cand2.p, c->d_ncand.p, c->stream));
-      unsigned long long h = 0;
-      CK(cudaMemcpyAsync(&h, c->d_ncand.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+      unsigned long long* h = static_cast<unsigned long long*>(c->h_pin);
+      CK(cudaMemcpyAsync(h, c->d_ncand.p, sizeof(*h), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
-      nre = (int64_t)h;
+      nre = (int64_t)*h;
       rc = c->d_cand2.p;
       Xacc = c->d_Xt.p;
     }
@@ -1210,38 +1235,37 @@ static int select_impl(abc_ctx* c, const double* data, const double* se, int64_t
                                         c->d_cnt2.p,
                                         c->d_dirty.p, c->stream));
     }
-    CK(cudaMemsetAsync(c->d_fail.p, 0, sizeof(int) * G, c->stream));
+    CK(cudaMemsetAsync(c->d_fail.p, 0, sizeof(int) * (size_t)(G + 1), c->stream));
     CK(launch_dist_accept_len(c->d_goff.p, c->d_se64.p, G, mode == 2 ? 0 : mode, eps_or_q,
                               mode == 2 ? c->d_thr.p : nullptr, kq, Xacc, c->d_b0.p, b1, c->d_alen.p, c->d_fail.p,
-                              !c->sel_errors, c->stream));
-    c->sel_cands_emitted += ncand;
-    if (c->sel_errors) {
-      c->sel_rechecked += nre;
-    } else {
-      unsigned long long hc[2] = {0ull, 0ull};
-      CK(cudaMemcpyAsync(hc, c->d_cnt2.p, sizeof(hc), cudaMemcpyDeviceToHost, c->stream));
-      CK(cudaStreamSynchronize(c->stream));
-      c->sel_rechecked += (int64_t)(hc[0] + hc[1]);
-    }
-    if (mode != 1) break;
-    std::vector<int> hf((size_t)G);
-    CK(cudaMemcpyAsync(hf.data(), c->d_fail.p, sizeof(int) * G, cudaMemcpyDeviceToHost, c->stream));
+                              c->d_fail.p + 1, !c->sel_errors, c->stream));
+    CK(launch_scan(c->d_alen.p, G, c->d_aoff.p, c->stream));
+    struct Result {
+      unsigned long long rechecked[2];
+      int64_t total;
+      int n_fail;
+    }* r = static_cast<Result*>(c->h_pin);
+    r->rechecked[0] = r->rechecked[1] = 0;
+    if (!c->sel_errors)
+      CK(cudaMemcpyAsync(r->rechecked, c->d_cnt2.p, sizeof(r->rechecked), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&r->total, c->d_aoff.p + G, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&r->n_fail, c->d_fail.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    bool any = false;
-    for (int64_t g = 0; g < G; ++g) {
-      if (hf[g]) {
-        any = true;
-        hX[g] = (round >= 1 || !(hX[g] < INFINITY)) ? INFINITY : 4.0f * hX[g] + 0.1f;
-      }
-    }
-    if (!any) break;
+    c->sel_cands_emitted += ncand;
+    c->sel_rechecked += c->sel_errors ? nre : (int64_t)(r->rechecked[0] + r->rechecked[1]);
+    total = r->total;
+    if (mode != 1 || r->n_fail == 0) break;
     if (round == 3) return fail(c, ABC_ERR_CAPACITY, "top-q selection did not converge");
+    // the genes whose threshold was too narrow
+    std::vector<int> hf((size_t)G);
+    std::vector<float> hX((size_t)G);
+    CK(cudaMemcpyAsync(hf.data(), c->d_fail.p + 1, sizeof(int) * G, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(hX.data(), c->d_X.p, sizeof(float) * G, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    for (int64_t g = 0; g < G; ++g)
+      if (hf[g]) hX[g] = (round >= 1 || !(hX[g] < INFINITY)) ? INFINITY : 4.0f * hX[g] + 0.1f;
     CK(cudaMemcpyAsync(c->d_X.p, hX.data(), sizeof(float) * G, cudaMemcpyHostToDevice, c->stream));
   }
-  CK(launch_scan(c->d_alen.p, G, c->d_aoff.p, c->stream));
-  int64_t total = 0;
-  CK(cudaMemcpyAsync(&total, c->d_aoff.p + G, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   CK(c->d_out_idx.ensure((size_t)std::max<int64_t>(total, 1)));
   CK(c->d_out_err.ensure((size_t)std::max<int64_t>(total, 1)));
   CK(launch_dist_compact(c->d_goff.p, c->d_sp.p, c->d_se64.p, c->d_aoff.p, G, 0, c->d_out_idx.p, c->d_out_err.p,
@@ -1287,15 +1311,19 @@ int abc_errors_candidate(abc_ctx* c, const double* data, const double* se, int64
   if (st) return st;
   int dmode = 0;
   float b1 = 0.0f;
-  st = prepare_candidate_pass(c, in, &dmode, &b1);
-  if (st) return st;
   CK(c->d_X.ensure((size_t)G));
   CK(c->d_ncand.ensure(1));
   CK(launch_fill(c->d_X.p, G, INFINITY, c->stream));
   int64_t n = 0;
   c->cand_cap = std::max<int64_t>(c->cand_cap, P * G);
-  st = dmode ? candidate_pass_tc(c, in, dmode, &n) : candidate_pass_simt(c, in, &n);
-  if (st) return st;
+  bool redo = true;
+  for (int want = c->dist_mode; redo; want = 0) {
+    redo = false;
+    st = prepare_candidate_pass(c, in, want, &dmode, &b1);
+    if (st) return st;
+    st = dmode ? candidate_pass_tc(c, in, dmode, &n, &redo) : candidate_pass_simt(c, in, &n);
+    if (st) return st;
+  }
   DBuf<float> out;
   CK(out.ensure((size_t)P * G));
   CK(launch_fill(out.p, P * G, NAN, c->stream));

@@ -13,35 +13,31 @@
 
 namespace abc {
 
-// sw, dw for every (g, k); s32[r][k] = stats[r * stride][k] for r < s32_rows.
-__global__ void dist_prep_kernel(DistInputs in, float* sw, float* dw, float* s32, int64_t s32_rows,
-                                 int64_t stride) {
-  const int64_t n_gk = in.G * in.K;
-  const int64_t n_pk = s32 ? s32_rows * in.K : 0;
+// Terms of every (g, k): den = (se^2 + 0.01 d^2) + eps, rden = RN(1/den), and in
+// FP32 sw = sqrt(w), dw = sqrt(w) d with w = rden; den and rden may be null.
+__global__ void dist_den_kernel(DistInputs in, double* den, double* rden, float* sw, float* dw) {
+  const int64_t n = in.G * in.K;
   const double sig2 = 0.1 * 0.1;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_gk + n_pk;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if (i < n_gk) {
-      const double d = in.data[i], e = in.se[i];
-      const double eps = (e + d != 0.0) ? 0.0 : 0.0001;
-      const double w = 1.0 / ((e * e + sig2 * (d * d)) + eps);
-      const double a = sqrt(w);
-      sw[i] = (float)a;
-      dw[i] = (float)(a * d);
-    } else {
-      const int64_t j = i - n_gk;
-      const int64_t r = j / in.K, k = j - r * in.K;
-      s32[j] = (float)in.stats[(r * stride) * in.K + k];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double d = in.data[i], e = in.se[i];
+    const double eps = (e + d != 0.0) ? 0.0 : 0.0001;
+    const double b = (e * e + sig2 * (d * d)) + eps;
+    const double w = 1.0 / b;
+    if (den) {
+      den[i] = b;
+      rden[i] = w;
     }
+    const double a = sqrt(w);
+    sw[i] = (float)a;
+    dw[i] = (float)(a * d);
   }
 }
 
-cudaError_t launch_dist_prep(const DistInputs& in, float* sw, float* dw, float* s32, int64_t s32_rows,
-                             int64_t stride, cudaStream_t s) {
-  const int64_t n = in.G * in.K + (s32 ? s32_rows * in.K : 0);
+cudaError_t launch_dist_den(const DistInputs& in, double* den, double* rden, float* sw, float* dw, cudaStream_t s) {
+  const int64_t n = in.G * in.K;
   if (n <= 0) return cudaSuccess;
-  int blocks = (int)((n + 255) / 256 < 65536 ? (n + 255) / 256 : 65536);
-  dist_prep_kernel<<<blocks, 256, 0, s>>>(in, sw, dw, s32, s32_rows, stride);
+  int blocks = (int)((n + 63) / 64 < 4096 ? (n + 63) / 64 : 4096);
+  dist_den_kernel<<<blocks, 64, 0, s>>>(in, den, rden, sw, dw);
   return cudaGetLastError();
 }
 
@@ -51,20 +47,19 @@ __device__ __forceinline__ double den_term(double d, double e) {
   return (e * e + sig2 * (d * d)) + eps;
 }
 
-__global__ void dist_den_kernel(DistInputs in, double* den, double* rden) {
-  const int64_t n = in.G * in.K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double b = den_term(in.data[i], in.se[i]);
-    den[i] = b;
-    rden[i] = 1.0 / b;
+// s32[r][k] = stats[r * stride][k] rounded to float, r < rows; a warp per row
+__global__ void __launch_bounds__(256) dist_rows32_kernel(DistInputs in, float* s32, int64_t rows, int64_t stride) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8) {
+    const double* src = in.stats + r * stride * in.K;
+    for (int k = lane; k < in.K; k += 32) s32[r * in.K + k] = rn32_bits(src[k]);
   }
 }
 
-cudaError_t launch_dist_den(const DistInputs& in, double* den, double* rden, cudaStream_t s) {
-  const int64_t n = in.G * in.K;
-  if (n <= 0) return cudaSuccess;
-  int blocks = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
-  dist_den_kernel<<<blocks, 256, 0, s>>>(in, den, rden);
+cudaError_t launch_dist_rows32(const DistInputs& in, float* s32, int64_t rows, int64_t stride, cudaStream_t s) {
+  if (rows <= 0 || in.K <= 0) return cudaSuccess;
+  const int64_t blocks = (rows + 7) / 8;
+  dist_rows32_kernel<<<(unsigned)(blocks < 65536 ? blocks : 65536), 256, 0, s>>>(in, s32, rows, stride);
   return cudaGetLastError();
 }
 
@@ -513,10 +508,8 @@ __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const flo
   }
 }
 
-cudaError_t launch_dist_full(const DistInputs& in, float* sw, float* dw, double* err, cudaStream_t s) {
+cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, double* err, cudaStream_t s) {
   if (in.P <= 0 || in.G <= 0) return cudaSuccess;
-  cudaError_t e = launch_dist_prep(in, sw, dw, nullptr, 0, 1, s);
-  if (e) return e;
   const float sure = 10.0f + 2.0f * dist_bound_f(10.0f, in.K);
   const int64_t py = (in.P + kFullRows - 1) / kFullRows;
   dim3 grid((unsigned)((in.G + kFullTile - 1) / kFullTile), (unsigned)(py < 65535 ? py : 65535));
@@ -809,7 +802,7 @@ cudaError_t launch_dist_group_certify_sort(const DistInputs& in, const Cand* can
 // ---------------------------------------------------------------------------
 __global__ void accept_len_kernel(const int64_t* goff, const double* se64, int64_t G, int mode, double eps_all,
                                   const double* eps_g, int64_t k, const float* X, const float* b0, float b1,
-                                  int64_t* alen, int* fail, bool approx) {
+                                  int64_t* alen, int* n_fail, int* fail, bool approx) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G) return;
   const double eps = eps_g ? eps_g[g] : eps_all;
@@ -845,17 +838,20 @@ __global__ void accept_len_kernel(const int64_t* goff, const double* se64, int64
       // certified values: the k-th error may be above its stored value by its bound
       ok = (approx ? E[k - 1] + approx_bound(E[k - 1]) : E[k - 1]) <= L;
     }
-    if (!ok) fail[g] = 1;
+    if (!ok) {
+      fail[g] = 1;
+      atomicAdd(n_fail, 1);
+    }
   }
   alen[g] = len;
 }
 
 cudaError_t launch_dist_accept_len(const int64_t* goff, const double* se64, int64_t G, int mode, double eps,
                                    const double* eps_g, int64_t k, const float* X, const float* b0, float b1,
-                                   int64_t* alen, int* fail, bool approx, cudaStream_t s) {
+                                   int64_t* alen, int* n_fail, int* fail, bool approx, cudaStream_t s) {
   if (G <= 0) return cudaSuccess;
   accept_len_kernel<<<(unsigned)((G + 127) / 128), 128, 0, s>>>(goff, se64, G, mode, eps, eps_g, k, X, b0, b1,
-                                                                alen, fail, approx);
+                                                                alen, n_fail, fail, approx);
   return cudaGetLastError();
 }
 

@@ -112,10 +112,8 @@ cudaError_t launch_dist_tc(int mode, const void* A, const void* B, const TcArgs&
 cudaError_t launch_tc_gather(const Cand* seg, const float* seg_e, const unsigned* count, int n_seg, int64_t seg_cap,
                              const float* cg, int K, Cand* out, float* out_e, cudaStream_t s);
 
-// per (g,k): sw = sqrt(w), dw = sqrt(w) d in FP32, w = 1/((se^2 + 0.01 d^2) + eps)
-// and s32[r][k] = stats[r stride][k] in FP32 for r < s32_rows (s32 may be null)
-cudaError_t launch_dist_prep(const DistInputs& in, float* sw, float* dw, float* s32, int64_t s32_rows,
-                             int64_t stride, cudaStream_t s);
+// s32[r][k] = stats[r stride][k] in FP32, r < rows
+cudaError_t launch_dist_rows32(const DistInputs& in, float* s32, int64_t rows, int64_t stride, cudaStream_t s);
 // FP32 direct distance: emit (p, g) with min(10, err32) <= X[g] (mode emit), or
 // write err32 of the particles p = row*stride into esub[row][g] (mode sample).
 cudaError_t launch_dist_fast(const float* s32, const float* sw, const float* dw, int64_t P, int64_t G, int K,
@@ -139,8 +137,9 @@ cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int6
                           const float* b0, float b1, unsigned int* hist, float* Xt, Cand* out,
                           unsigned long long* count, cudaStream_t s);
 // den[g][k] = (se^2 + 0.01 d^2) + eps_gk, the denominators of the error terms,
-// evaluated as in the per-term FP64 expression (bit-identical), and rden = 1/den.
-cudaError_t launch_dist_den(const DistInputs& in, double* den, double* rden, cudaStream_t s);
+// evaluated as in the per-term FP64 expression (bit-identical), and rden = 1/den
+// (both may be null); sw = sqrt(w), dw = sqrt(w) d in FP32, w = 1/den.
+cudaError_t launch_dist_den(const DistInputs& in, double* den, double* rden, float* sw, float* dw, cudaStream_t s);
 // Group candidates by gene (goff: G + 1 offsets; sp, sg: particle and gene per
 // entry), evaluate their FP64 errors in the reference's operation order (se64;
 // needs in.den and in.rden) and sort each gene's list by (err, p).
@@ -162,7 +161,7 @@ cudaError_t launch_dist_group_certify_sort(const DistInputs& in, const Cand* can
 // X[g] could have excluded a member of the top k.
 cudaError_t launch_dist_accept_len(const int64_t* goff, const double* se64, int64_t G, int mode, double eps,
                                    const double* eps_g, int64_t k, const float* X, const float* b0, float b1,
-                                   int64_t* alen, int* fail, bool approx, cudaStream_t s);
+                                   int64_t* alen, int* n_fail, int* fail, bool approx, cudaStream_t s);
 // compact the accepted prefixes: idx (1-based particle index + p_base) and err.
 cudaError_t launch_dist_compact(const int64_t* goff, const int32_t* sp, const double* se64, const int64_t* aoff,
                                 int64_t G, int64_t p_base, int64_t* idx, double* err, cudaStream_t s);
@@ -173,7 +172,7 @@ cudaError_t launch_scan(const int64_t* cnt, int64_t G, int64_t* off, cudaStream_
 cudaError_t launch_accepted_errors(const DistInputs& in, const int64_t* aoff, const int64_t* idx, int64_t G,
                                    int64_t p_base, int64_t n, int32_t* sp, int32_t* sg, double* err, cudaStream_t s);
 // full FP64 error matrix [P][G]; sw, dw: G x K scratch values each
-cudaError_t launch_dist_full(const DistInputs& in, float* sw, float* dw, double* err, cudaStream_t s);
+cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, double* err, cudaStream_t s);
 
 // moment ODE (moment.cu)
 struct MomArgs {
