@@ -62,19 +62,22 @@ cudaError_t launch_prior(const PriorArgs& a, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// theta -> rates, thinning bounds and initial state, eight lanes per particle
+// theta -> rates, thinning bounds and initial state, LANES lanes per particle
 // (model.cuh has the formulas; every operation and its order are the
 // oracle's, so the record is bit-identical).  One thread per particle ran
 // six dependent passes over a cycle's 80 sub-steps, 0.69 ms for one particle
-// and for 10,000 alike; this takes 0.10 and 0.6 ms, bound by the FP64 pipe.  Here lane k holds age step k; the sub-steps' rates and
-// sources, which depend on E G alone, are computed side by side and only the
-// four recurrences stay serial, the passes from different start values on
-// different lanes.  8 lanes rather than 32: the serial parts then occupy
-// the narrow FP64 pipe once for four particles.
+// and for 10,000 alike.  Here lane k holds age step k, the sub-steps' rates and
+// sources are computed side by side, and only the recurrences stay serial, two
+// operations each, the passes from different start values on different lanes.
+// Bound by the FP64 pipe, which a warp's instruction holds whatever the
+// number of lanes with work: 8 lanes per particle, so that the serial parts
+// occupy it once for four particles, or 32 while the particles' warps do not fill the
+// GPU.  100 particles: 107 us with 8 lanes and sources inside the recurrences, 73 now; 10,000:
+// 455 us, 342 now.
 // ---------------------------------------------------------------------------
-constexpr int kSetupLanes = 8;
+constexpr int kSetupLanes = 8;  // 32 up to kSetupWide particles
+constexpr int64_t kSetupWide = 4 * 152;  // a warp per scheduler
 static_assert(kSetupLanes >= kMaxSteps, "lane k holds age step k");
-constexpr int kSetupParticles = 32 / kSetupLanes;  // per block (one warp)
 constexpr int kMaxSub = kMaxSteps * kIcSub;
 
 struct SetupShared {
@@ -83,9 +86,12 @@ struct SetupShared {
   double ec[kMaxSteps], phc[kMaxSteps], ev[kMaxSteps], phv[kMaxSteps];
   double g[kMaxSub];  // E G at the start of each sub-step, then 2 alpha
   double aG[kMaxSub], sm[kMaxSub], sc[kMaxSub];  // alpha E G, sources of E u and Cov(G, u)
+  double x[4][kMaxSub + 1];  // E u from 0 and from 1, Cov from 0 and from 1, at the sub-steps' ends
+  double w2[kMaxSub];        // sources of Var u (those of two starts overwrite sm and sc)
 };
 
 // initial_moments (model.cuh) by the particle's lanes; lane 0 writes the record
+template <int LANES>
 __device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) {
   const int S = cfg.n_steps, N = S * kIcSub;
   const double T = cfg.cycle;
@@ -105,7 +111,7 @@ __device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) 
     const double gi = W.ginf[k], eG = W.eG[k];
     for (int i = 0; i < kIcSub; ++i) g = gi + (g - gi) * eG;
   }
-  const double z0 = __shfl_sync(0xffffffffu, g, 0, kSetupLanes), e0 = __shfl_sync(0xffffffffu, g, 1, kSetupLanes);
+  const double z0 = __shfl_sync(0xffffffffu, g, 0, LANES), e0 = __shfl_sync(0xffffffffu, g, 1, LANES);
   double g0 = z0 / (1.0 - (e0 - z0));
   if (!(g0 > 0.0)) g0 = 0.0;
   if (g0 > 1.0) g0 = 1.0;
@@ -118,7 +124,7 @@ __device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) 
     }
   }
   __syncwarp();
-  for (int q = r; q < N; q += kSetupLanes) {
+  for (int q = r; q < N; q += LANES) {
     const int k = q / kIcSub;
     const double ph = ((double)q + 0.5) * h;
     const double a = W.R.alp[k] * xpow(1.0 + ph / T, W.R.scal);
@@ -130,29 +136,50 @@ __device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) 
     W.g[q] = 2.0 * a;
   }
   __syncwarp();
-  // the cycle map of (E u, Cov, Var u) from 0, (1, 0, 0), (0, 1, 0), (0, 0, 1) on lanes 0..3
-  double m = r == 1 ? 1.0 : 0.0, c = r == 2 ? 1.0 : 0.0, v = r == 3 ? 1.0 : 0.0;
-  for (int k = 0; k < S; ++k) {
-    const double gam = W.R.gam[k], em = W.em[k], ec = W.ec[k], ev = W.ev[k], phv = W.phv[k];
-    for (int i = 0; i < kIcSub; ++i) {
-      const int q = k * kIcSub + i;
-      const double mn = m * em + W.sm[q];
-      const double cn = c * ec + W.sc[q];
-      const double src = (W.aG[q] + gam * (0.5 * (m + mn))) + W.g[q] * (0.5 * (c + cn));
-      v = v * ev + (src * h) * phv;
-      m = mn;
-      c = cn;
+  // the cycle map of (E u, Cov, Var u) from 0, (1, 0, 0), (0, 1, 0), (0, 0, 1): E u and
+  // Cov depend on their own start alone (lanes 0..3 of x), the sources of Var u
+  // on both, for three pairs of starts, and Var u is a recurrence on them
+  const unsigned F = 0xffffffffu;
+  {
+    double y = (double)(r & 1);
+    const double* E = (r & 2) ? W.ec : W.em;
+    const double* s = (r & 2) ? W.sc : W.sm;
+    if (r < 4) W.x[r][0] = y;
+    for (int k = 0; k < S; ++k) {
+      const double ek = E[k];
+      for (int i = 0; i < kIcSub; ++i) {
+        const int q = k * kIcSub + i;
+        y = y * ek + s[q];
+        if (r < 4) W.x[r][q + 1] = y;
+      }
     }
   }
+  __syncwarp();
+  for (int item = r; item < 3 * N; item += LANES) {
+    const int start = item / N, q = item - start * N, k = q / kIcSub;
+    const double* m = W.x[start == 1 ? 1 : 0];
+    const double* c = W.x[start == 2 ? 3 : 2];
+    const double src = (W.aG[q] + W.R.gam[k] * (0.5 * (m[q] + m[q + 1]))) + W.g[q] * (0.5 * (c[q] + c[q + 1]));
+    (start == 0 ? W.sm : start == 1 ? W.sc : W.w2)[q] = (src * h) * W.phv[k];
+  }
+  __syncwarp();
+  double v = r == 3 ? 1.0 : 0.0;
+  {
+    const double* w = r == 1 ? W.sc : r == 2 ? W.w2 : W.sm;
+    for (int k = 0; k < S; ++k) {
+      const double ev = W.ev[k];
+      for (int i = 0; i < kIcSub; ++i) v = v * ev + w[k * kIcSub + i];
+    }
+  }
+  double m = W.x[r == 1 ? 1 : 0][N], c = W.x[r == 2 ? 3 : 2][N];
   v = v * 0.25 + m * 0.25;
   m = m * 0.5;
   c = c * 0.5;
-  const unsigned F = 0xffffffffu;
-  const double b1 = __shfl_sync(F, m, 0, kSetupLanes), b2 = __shfl_sync(F, c, 0, kSetupLanes);
-  const double b3 = __shfl_sync(F, v, 0, kSetupLanes);
-  const double mmm = __shfl_sync(F, m, 1, kSetupLanes) - b1, mvm = __shfl_sync(F, v, 1, kSetupLanes) - b3;
-  const double mcc = __shfl_sync(F, c, 2, kSetupLanes) - b2, mvc = __shfl_sync(F, v, 2, kSetupLanes) - b3;
-  const double mvv = __shfl_sync(F, v, 3, kSetupLanes) - b3;
+  const double b1 = __shfl_sync(F, m, 0, LANES), b2 = __shfl_sync(F, c, 0, LANES);
+  const double b3 = __shfl_sync(F, v, 0, LANES);
+  const double mmm = __shfl_sync(F, m, 1, LANES) - b1, mvm = __shfl_sync(F, v, 1, LANES) - b3;
+  const double mcc = __shfl_sync(F, c, 2, LANES) - b2, mvc = __shfl_sync(F, v, 2, LANES) - b3;
+  const double mvv = __shfl_sync(F, v, 3, LANES) - b3;
   double m0 = b1 / (1.0 - mmm);
   double c0 = b2 / (1.0 - mcc);
   double v0 = ((b3 + mvm * m0) + mvc * c0) / (1.0 - mvv);
@@ -169,25 +196,28 @@ __device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) 
 }
 
 // initial_means (model.cuh), splicing models: the four passes on lanes 0..3
+template <int LANES>
 __device__ void initial_means_lanes(const DevCfg& cfg, SetupShared& W, int r) {
   double x0 = r == 1 ? 1.0 : 0.0, x1 = r == 2 ? 1.0 : 0.0, x2 = r == 3 ? 1.0 : 0.0;
   if (r < 4) mean_cycle(cfg, W.R, x0, x1, x2);
   const unsigned F = 0xffffffffu;
   double b[3], col[3][3];
-  b[0] = __shfl_sync(F, x0, 0, kSetupLanes);
-  b[1] = __shfl_sync(F, x1, 0, kSetupLanes);
-  b[2] = __shfl_sync(F, x2, 0, kSetupLanes);
+  b[0] = __shfl_sync(F, x0, 0, LANES);
+  b[1] = __shfl_sync(F, x1, 0, LANES);
+  b[2] = __shfl_sync(F, x2, 0, LANES);
   for (int i = 0; i < 3; ++i) {
-    col[i][0] = __shfl_sync(F, x0, i + 1, kSetupLanes);
-    col[i][1] = __shfl_sync(F, x1, i + 1, kSetupLanes);
-    col[i][2] = __shfl_sync(F, x2, i + 1, kSetupLanes);
+    col[i][0] = __shfl_sync(F, x0, i + 1, LANES);
+    col[i][1] = __shfl_sync(F, x1, i + 1, LANES);
+    col[i][2] = __shfl_sync(F, x2, i + 1, LANES);
   }
   if (r == 0) solve_initial_means(cfg, b, col, W.R);
 }
 
+template <int LANES>
 __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
+  constexpr int kSetupParticles = 32 / LANES;  // per block (one warp)
   __shared__ SetupShared sh[kSetupParticles];
-  const int r = threadIdx.x % kSetupLanes, slot = threadIdx.x / kSetupLanes;
+  const int r = threadIdx.x % LANES, slot = threadIdx.x / LANES;
   const int64_t p = (int64_t)blockIdx.x * kSetupParticles + slot;
   const bool here = p < A.n_particles;
   const DevCfg& cfg = A.cfg;
@@ -215,10 +245,12 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
       bad = !(kon < INFINITY) || !(alp < INFINITY) || !(gam < INFINITY);
     }
     bad = bad || !(koff < INFINITY) || lam != lam || scal != scal || scal < 0.0;
-    R.kon[r] = kon;
-    R.alp[r] = alp;
-    R.gam[r] = gam;
-    R.amax[r] = amax;
+    if (r < kMaxSteps) {
+      R.kon[r] = kon;
+      R.alp[r] = alp;
+      R.gam[r] = gam;
+      R.amax[r] = amax;
+    }
     if (r == 0) {
       R.koff = koff;
       R.lam = lam;
@@ -226,11 +258,11 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
       R.scal = scal;
     }
   }
-  const unsigned mine = ((1u << kSetupLanes) - 1u) << (slot * kSetupLanes);
+  const unsigned mine = (0xffffffffu >> (32 - LANES)) << (slot * LANES);
   bad = (__ballot_sync(0xffffffffu, bad) & mine) != 0u;
   if (bad) {
     // a harmless record: the trajectory sees no reactions
-    R.kon[r] = R.alp[r] = R.gam[r] = R.amax[r] = 0.0;
+    if (r < kMaxSteps) R.kon[r] = R.alp[r] = R.gam[r] = R.amax[r] = 0.0;
     if (r == 0) {
       R.koff = R.lam = R.beta = R.scal = R.g0 = R.u0 = R.s0 = R.c0 = R.v0 = 0.0;
       R.cost = 1.0;
@@ -244,16 +276,16 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
   PRec keep = {};
   if (bad && r == 0) keep = R;
   if (cfg.splicing)
-    initial_means_lanes(cfg, W, r);
+    initial_means_lanes<LANES>(cfg, W, r);
   else
-    initial_moments_lanes(cfg, W, r);
+    initial_moments_lanes<LANES>(cfg, W, r);
   // work estimate: switching + transcription + decay events over the horizon
   double rate = 0.0, mine_k = 0.0;
   if (r < S) {
     const double pon = R.kon[r] / (R.kon[r] + R.koff);
     mine_k = 2.0 * pon * R.koff + 2.0 * pon * R.amax[r];
   }
-  for (int k = 0; k < S; ++k) rate = rate + __shfl_sync(0xffffffffu, mine_k, k, kSetupLanes);
+  for (int k = 0; k < S; ++k) rate = rate + __shfl_sync(0xffffffffu, mine_k, k, LANES);
   if (r == 0) {
     if (bad)
       R = keep;
@@ -264,12 +296,13 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
   if (!here) return;
   const double* src = reinterpret_cast<const double*>(&R);
   double* dst = reinterpret_cast<double*>(&A.rec[p]);
-  for (int i = r; i < (int)(sizeof(PRec) / sizeof(double)); i += kSetupLanes) dst[i] = src[i];
+  for (int i = r; i < (int)(sizeof(PRec) / sizeof(double)); i += LANES) dst[i] = src[i];
   // rates in log2 units (times log2 e), so the production kernel's waiting
   // time is -log2(U) / a0 without a conversion per event
   constexpr double kL2E = 1.4426950408889634;
-  float kon = (float)(R.kon[r] * kL2E), alp = (float)(R.alp[r] * kL2E), gam = (float)(R.gam[r] * kL2E);
-  float amax = (float)(R.amax[r] * kL2E), koff = (float)(R.koff * kL2E), beta = (float)(R.beta * kL2E);
+  const int rk = r < kMaxSteps ? r : kMaxSteps - 1;
+  float kon = (float)(R.kon[rk] * kL2E), alp = (float)(R.alp[rk] * kL2E), gam = (float)(R.gam[rk] * kL2E);
+  float amax = (float)(R.amax[rk] * kL2E), koff = (float)(R.koff * kL2E), beta = (float)(R.beta * kL2E);
   float lam = (float)R.lam, scal = (float)R.scal;
   if (A.fp32) {
     // rates beyond the FP32 range would stall the production kernel's clock
@@ -280,10 +313,12 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
     }
   }
   PRecF& F = A.recf[p];
-  F.kon[r] = kon;
-  F.alp[r] = alp;
-  F.gam[r] = gam;
-  F.amax[r] = amax;
+  if (r < kMaxSteps) {
+    F.kon[r] = kon;
+    F.alp[r] = alp;
+    F.gam[r] = gam;
+    F.amax[r] = amax;
+  }
   if (r == 0) {
     F.koff = koff;
     F.lam = lam;
@@ -294,8 +329,12 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
 
 cudaError_t launch_setup(const SetupArgs& a, cudaStream_t s) {
   if (a.n_particles <= 0) return cudaSuccess;
-  const int64_t blocks = (a.n_particles + kSetupParticles - 1) / kSetupParticles;
-  setup_kernel<<<(unsigned)blocks, 32, 0, s>>>(a);
+  if (a.n_particles <= kSetupWide) {
+    setup_kernel<32><<<(unsigned)a.n_particles, 32, 0, s>>>(a);
+  } else {
+    constexpr int per = 32 / kSetupLanes;
+    setup_kernel<kSetupLanes><<<(unsigned)((a.n_particles + per - 1) / per), 32, 0, s>>>(a);
+  }
   return cudaGetLastError();
 }
 
