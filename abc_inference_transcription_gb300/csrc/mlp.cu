@@ -472,7 +472,9 @@ cudaError_t mlp_gather(const float* xn, const float* yn, int64_t N, const MlpDim
 // for the weight gradients; null for inference), Y: [members][B][out_pad].
 cudaError_t mlp_forward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0, int64_t sX,
                         const __nv_bfloat16* WhT, const float* Pf, float* Z, __nv_bfloat16* Ah, __nv_bfloat16* AhT,
-                        int ldT, float* Y, int* err, cudaStream_t s) {
+                        int ldT, float* Y, int* err, int sms, cudaStream_t s) {
+  if (Z && AhT && sX && mlp_infer_fits(d))
+    return mlp_train_forward(d, members, B, X0, WhT, Pf, Z, AhT, ldT, Y, err, sms, s);
   const int H = d.H;
   const int64_t sZ = 3 * (int64_t)B * H, sL = (int64_t)B * H, sLT = (int64_t)H * ldT;
   const int64_t w_off[4] = {d.off_w1, d.off_w2, d.off_w3, d.off_w4};
@@ -528,9 +530,9 @@ cudaError_t mlp_forward(const MlpDims& d, int members, int B, const __nv_bfloat1
 // training run is reproducible bit for bit); dZ_l = (dZ_{l+1} W_{l+1}^T)
 // silu'(Z_l) with its transposed copy.
 cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0T, const __nv_bfloat16* Wh,
-                         const float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
+                         float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
                          __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZT, int ldT, float* Gf, float* Gpart,
-                         float* loss, const float* loss_part, int* err, cudaStream_t s) {
+                         float* loss, const float* loss_part, int* err, int sms, cudaStream_t s) {
   const int H = d.H;
   const int64_t sZ = 3 * (int64_t)B * H, sL = (int64_t)B * H, sLT = (int64_t)H * ldT, sP = d.n_params;
   const int splits = mlp_wgrad_splits(B);
@@ -564,10 +566,12 @@ cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat
   const int64_t w_next[3] = {d.off_w2, d.off_w3, d.off_w4};
   const int64_t w_off[3] = {d.off_w1, d.off_w2, d.off_w3};
   __nv_bfloat16* bufs[2] = {dZa, dZb};
+  const bool fused = mlp_infer_fits(d);
+  if (fused && (e = mlp_train_backward(d, members, B, dY, Wh, Z, dZT, ldT, err, sms, s))) return e;
   for (int layer = 2; layer >= 0; --layer) {
     __nv_bfloat16* dZ = bufs[layer & 1];
     __nv_bfloat16* dZTl = dZT + layer * members * sLT;
-    {
+    if (!fused) {
       // dZ_l = (grad_in W_{l+1}^T) silu'(Z_l): W_{l+1} stored [H][out] is the K-major [N = H][K = out] operand
       const int Kn = layer == 2 ? d.out_pad : H;
       TcOperand A{grad_in, ld_gin, B, s_gin};

@@ -96,4 +96,12 @@ cudaError_t mlp_tc_wgrads(const TcOperand* A, const TcOperand* B, const TcGemm* 
 cudaError_t mlp_tc_gemm(int epi, const TcOperand& A, const TcOperand& B, const TcGemm& g, int members,
                         cudaStream_t s);
 
+// all layers in one kernel (mlp_infer.cu); false: the outputs are too wide for it
+bool mlp_infer_fits(const MlpDims& d);
+cudaError_t mlp_train_forward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0, const __nv_bfloat16* WhT,
+                              const float* Pf, float* Z, __nv_bfloat16* AhT, int ldT, float* Y, int* err, int sms,
+                              cudaStream_t s);
+cudaError_t mlp_train_backward(const MlpDims& d, int members, int B, const __nv_bfloat16* dY, const __nv_bfloat16* Wh,
+                               float* Z, __nv_bfloat16* dZT, int ldT, int* err, int sms, cudaStream_t s);
+
 }  // namespace abc

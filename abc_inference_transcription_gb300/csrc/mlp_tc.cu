@@ -67,47 +67,7 @@ constexpr uint32_t kStageBytes = 2 * kTileBytes;
 constexpr uint32_t kTmemCols = 128;
 constexpr int kSmem = 1024 + kStages * kStageBytes + 128;
 constexpr int kThreads = 256;
-constexpr int kChunk = 32;  // rows and columns of an epilogue chunk
-// row strides of a staged chunk, in words: 16-byte pieces of eight neighbouring lanes fall
-// on distinct banks, by rows and by columns
-constexpr int kRowF = kChunk + 4, kRowH = kChunk / 2 + 4;
 static_assert(kThreads / 32 * kChunk * kRowF * 4 <= kStages * kStageBytes, "the stages hold the warps' chunks");
-
-// What bounds the epilogue is the load/store path: a lane holds a row of the chunk, and a
-// 16-byte access per lane touches 32 rows.  Through shared memory the warp's
-// accesses take whole rows instead, 4 (FP32) or 8 (BF16) of them at a time.
-// rows, cols: what of the chunk is inside the matrix.
-__device__ __forceinline__ void store_rows_f32(float* sm, const float (&x)[kChunk], float* base, int64_t ld, int rows,
-                                               int cols, int lane) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-    *(float4*)(sm + lane * kRowF + 4 * q) = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-  __syncwarp();
-  const int r = lane / 8, c = lane % 8 * 4;
-#pragma unroll
-  for (int t = 0; t < 8; ++t)
-    if (4 * t + r < rows && c < cols) *(float4*)(base + (4 * t + r) * ld + c) = *(const float4*)(sm + (4 * t + r) * kRowF + c);
-  __syncwarp();
-}
-
-__device__ __forceinline__ void load_rows_f32(float* sm, float (&x)[kChunk], const float* base, int64_t ld, int rows,
-                                              int cols, int lane) {
-  const int r = lane / 8, c = lane % 8 * 4;
-  float4 v[8];
-#pragma unroll
-  for (int t = 0; t < 8; ++t)
-    v[t] = 4 * t + r < rows && c < cols ? *(const float4*)(base + (4 * t + r) * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int t = 0; t < 8; ++t) *(float4*)(sm + (4 * t + r) * kRowF + c) = v[t];
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float4 w = *(const float4*)(sm + lane * kRowF + 4 * q);
-    x[4 * q] = w.x; x[4 * q + 1] = w.y; x[4 * q + 2] = w.z; x[4 * q + 3] = w.w;
-  }
-  __syncwarp();
-}
-
 // also the transposed copy, whose accesses are whole columns as the lanes stand
 __device__ __forceinline__ void store_rows_bf16(float* sm, const float (&x)[kChunk], __nv_bfloat16* base, int64_t ld,
                                                 __nv_bfloat16* baseT, int64_t ldT, int rows, int cols, int lane) {

@@ -28,14 +28,13 @@ cudaError_t mlp_gather(const float* xn, const float* yn, int64_t N, const MlpDim
                        cudaStream_t s);
 cudaError_t mlp_forward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0, int64_t sX,
                         const __nv_bfloat16* WhT, const float* Pf, float* Z, __nv_bfloat16* Ah, __nv_bfloat16* AhT,
-                        int ldT, float* Y, int* err, cudaStream_t s);
-bool mlp_infer_fits(const MlpDims& d);
+                        int ldT, float* Y, int* err, int sms, cudaStream_t s);
 cudaError_t mlp_infer(const MlpDims& d, int members, int B, const __nv_bfloat16* X0, const __nv_bfloat16* WhT,
                       const float* Pf, float* Y, int* err, int sms, cudaStream_t s);
 cudaError_t mlp_backward(const MlpDims& d, int members, int B, const __nv_bfloat16* X0T, const __nv_bfloat16* Wh,
-                         const float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
+                         float* Z, const __nv_bfloat16* AhT, const __nv_bfloat16* dY, const __nv_bfloat16* dYT,
                          __nv_bfloat16* dZa, __nv_bfloat16* dZb, __nv_bfloat16* dZT, int ldT, float* Gf, float* Gpart,
-                         float* loss, const float* loss_part, int* err, cudaStream_t s);
+                         float* loss, const float* loss_part, int* err, int sms, cudaStream_t s);
 cudaError_t mlp_loss(const MlpDims& d, int members, int B, int valid_rows, const float* Y, const float* T,
                      __nv_bfloat16* dY, __nv_bfloat16* dYT, int ldT, float* loss_part, cudaStream_t s);
 cudaError_t mlp_adam(const MlpDims& d, int members, float* P, const float* G, float* m, float* v,
@@ -406,10 +405,10 @@ static int train_step(abc_surrogate* s, int B, int64_t base, int valid, int64_t 
   const int E = s->members;
   SK(mlp_gather(s->xn.p, s->yn.p, N, d, B, base, s->perm.p, E, s->X0.p, s->X0T.p, s->ldT, s->T.p, s->stream));
   SK(mlp_forward(d, E, B, s->X0.p, (int64_t)B * d.in_pad, s->PhT.p, s->P.p, s->Z.p, s->Ah.p, s->AhT.p, s->ldT,
-                 s->Y.p, s->tcerr.p, s->stream));
+                 s->Y.p, s->tcerr.p, s->sms, s->stream));
   SK(mlp_loss(d, E, B, valid, s->Y.p, s->T.p, s->dY.p, s->dYT.p, s->ldT, s->loss_part.p, s->stream));
   SK(mlp_backward(d, E, B, s->X0T.p, s->Ph.p, s->Z.p, s->AhT.p, s->dY.p, s->dYT.p, s->dZa.p, s->dZb.p, s->dZT.p,
-                  s->ldT, s->G.p, s->Gpart.p, s->loss.p, s->loss_part.p, s->tcerr.p, s->stream));
+                  s->ldT, s->G.p, s->Gpart.p, s->loss.p, s->loss_part.p, s->tcerr.p, s->sms, s->stream));
   return ABC_OK;
 }
 
@@ -645,7 +644,7 @@ static int forward_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_
   } else {  // more than 128 statistics: layer by layer
     SK(s->Ah.ensure((size_t)E * 3 * n * d.H));
     SK(mlp_forward(d, E, (int)n, s->X0.p, 0, s->PhT.p, s->P.p, nullptr, s->Ah.p, nullptr, 0, s->Y.p, s->tcerr.p,
-                   s->stream));
+                   s->sms, s->stream));
   }
   return ABC_OK;
 }

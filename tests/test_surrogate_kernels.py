@@ -120,3 +120,30 @@ def test_gradients_at_batch_edges(built, rows, K):
                 a, b = d[name]
                 got, want = grads[e, a:b].astype(np.float64), rg[a:b]
                 assert np.linalg.norm(got - want) < 2e-2 * max(np.linalg.norm(want), 1e-12), (e, name)
+
+
+@pytest.mark.parametrize("rows,K", [(130, 140), (257, 120), (20000, 53)])
+def test_gradients_of_wide_outputs_and_many_tiles(built, rows, K):
+    """Outputs too wide for the fused training passes (280 columns: layer by layer), of
+    two output tiles (240), and batches of more row tiles than the GPU has SMs, against the FP64
+    network; bounds as above."""
+    from abc_inference_transcription_gb300 import surrogate as S
+    from oracle import mlp_ref
+
+    rng = np.random.default_rng(rows)
+    theta, stats = rng.uniform(-3, 3, (rows, 5)), rng.normal(2.0, 1.5, (rows, K))
+    with S.Surrogate(5, K, ensemble=2, seed=12) as sg:
+        p = sg.params()
+        p = p + rng.normal(0, 0.02, p.shape).astype(np.float32)
+        sg.set_params(p)
+        norm = np.zeros(5), np.full(5, 1.7), np.full(K, 2.0), np.full(K, 1.5)
+        sg.set_norm(*norm)
+        loss, grads = sg.gradients(theta, stats)
+        d = mlp_ref.dims(5, K)
+        for e in range(2):
+            rl, rg = mlp_ref.loss_and_grads(p[e], d, theta, stats, *norm)
+            assert abs(loss[e] - rl) <= 2e-4 * abs(rl) + 1e-6
+            for name in ("w1", "b1", "w2", "b2", "w3", "b3", "w4", "b4"):
+                a, b = d[name]
+                got, want = grads[e, a:b].astype(np.float64), rg[a:b]
+                assert np.linalg.norm(got - want) < 2e-2 * max(np.linalg.norm(want), 1e-12), (e, name)
