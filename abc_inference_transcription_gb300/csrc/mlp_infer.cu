@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(kInferThreads, KIND == kPredict ? 2 : 1)
   uint64_t* xfull = empty + kRing;
   uint64_t* acc_full = xfull + 1;
   uint64_t* act_ready = acc_full + 1;
-  uint64_t* drain = act_ready + 1;
+  uint64_t* act_free = act_ready + 1;  // once per tile, where acc_full completes once per layer
+  uint64_t* drain = act_free + 1;
   uint32_t* tslot = (uint32_t*)(drain + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t sbase = su32(smem);
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(kInferThreads, KIND == kPredict ? 2 : 1)
     mbar_init(xfull, 1);
     mbar_init(acc_full, 1);
     mbar_init(act_ready, 32 * kEpiWarps);
+    mbar_init(act_free, 1);
     mbar_init(drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(kInferThreads, KIND == kPredict ? 2 : 1)
         for (int l = 0; l < L && ok; ++l) {
           if (l == 0) {
             // the last layer of the previous tile has read the activations
-            if (ti > 0 && !mbar_wait(acc_full, (uint32_t)(L * ti - 1) & 1u)) {
+            if (ti > 0 && !mbar_wait(act_free, (uint32_t)(ti - 1) & 1u)) {
               ok = false;
               break;
             }
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(kInferThreads, KIND == kPredict ? 2 : 1)
               }
             }
           if (ok) mma_commit(acc_full);
+          if (ok && l == L - 1) mma_commit(act_free);
         }
       }
       if (!ok) atomicOr(g.err, 2);
