@@ -72,7 +72,7 @@ cudaError_t launch_prior(const PriorArgs& a, cudaStream_t s) {
 // Bound by the FP64 pipe, which a warp's instruction holds whatever the
 // number of lanes with work: 8 lanes per particle, so that the serial parts
 // occupy it once for four particles, or 32 while the particles' warps do not fill the
-// GPU.  100 particles: 107 us with 8 lanes and sources inside the recurrences, 73 now; 10,000:
+// GPU.  One particle: 107 us with 8 lanes and sources inside the recurrences, 73 now; 10,000:
 // 455 us, 342 now.
 // ---------------------------------------------------------------------------
 constexpr int kSetupLanes = 8;  // 32 up to kSetupWide particles
@@ -90,7 +90,7 @@ struct SetupShared {
   double w2[kMaxSub];        // sources of Var u (those of two starts overwrite sm and sc)
 };
 
-// initial_moments (model.cuh) by the particle's lanes; lane 0 writes the record
+// The periodic moments by the particle's lanes; lane 0 writes the record
 template <int LANES>
 __device__ void initial_moments_lanes(const DevCfg& cfg, SetupShared& W, int r) {
   const int S = cfg.n_steps, N = S * kIcSub;

@@ -279,10 +279,6 @@ ABC_HD void stats_from_moments_cond(const DevCfg& cfg, const double* m, const do
   }
 }
 
-ABC_HD void stats_from_moments(const DevCfg& cfg, const double* m, const double* age_dist, double* st) {
-  for (int j = 0; j < cfg.n_conds; ++j) stats_from_moments_cond(cfg, m, age_dist, st, j);
-}
-
 // int128 -> double with the oracle's rounding (exact below 2^62).
 ABC_HD double i128_to_double(__int128 x) {
   const __int128 lim = ((__int128)1) << 62;
