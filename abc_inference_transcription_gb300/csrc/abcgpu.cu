@@ -13,6 +13,7 @@
 
 #include "../../include/abcgpu.h"
 #include "distance.cuh"
+#include "host_pages.h"
 #include "kernels.h"
 
 using namespace abc;
@@ -122,6 +123,9 @@ struct abc_ctx {
   int64_t cand_cap = int64_t(1) << 22;
   int64_t sel_G = 0, sel_P = 0, sel_total = 0, sel_cands = 0, sel_rechecked = 0, sel_cands_emitted = 0;
   bool sel_ready = false;
+  int64_t* out_idx = nullptr;  // arrays of the next selection's result (abc_select_output)
+  double* out_err = nullptr;
+  size_t out_cap = 0;
   bool sel_errors = true;        // selections keep the FP64 error of every accepted pair
   bool sel_errors_exact = true;  // the last selection's stored errors are FP64
   DistInputs sel_in;             // inputs of the last selection (device buffers; stats as given)
@@ -687,6 +691,7 @@ int abc_simulate_batch(abc_ctx* c, const int32_t* models, const double* theta, i
   CK(cudaMemcpyAsync(c->d_theta.p, theta, sizeof(double) * P * ld_theta, cudaMemcpyHostToDevice, c->stream));
   st = enqueue_chain(c, 0, c->d_models.p, c->d_theta.p, ld_theta, P, seed, particle_offset, c->d_stats.p);
   if (st) return st;
+  make_present(stats_out, sizeof(double) * P * K);
   CK(cudaMemcpyAsync(stats_out, c->d_stats.p, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
   return finish_status(c);
 }
@@ -710,6 +715,7 @@ int abc_simulate(abc_ctx* c, int model, const double* theta, int64_t P, uint64_t
   CK(cudaMemcpyAsync(c->d_theta.p, theta, sizeof(double) * P * npar, cudaMemcpyHostToDevice, c->stream));
   st = enqueue_simulate(c, model, nullptr, c->d_theta.p, npar, P, seed, particle_offset, c->d_stats.p, false);
   if (st) return st;
+  make_present(stats_out, sizeof(double) * P * K);
   CK(cudaMemcpyAsync(stats_out, c->d_stats.p, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
   return finish_status(c);
 }
@@ -931,6 +937,7 @@ int abc_errors(abc_ctx* c, const double* data, const double* se, int64_t G, int 
   const size_t o_out = w.add(sizeof(double) * (size_t)P * G);
   CK(w.allocate(c));
   CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, w.at<double>(o_out), c->stream));
+  make_present(err_out, sizeof(double) * P * G);
   CK(cudaMemcpyAsync(err_out, w.at<double>(o_out), sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   trim_work(c);
@@ -959,6 +966,16 @@ static int prof_end(abc_ctx* c) {
   return ABC_OK;
 }
 
+// The arrays named by abc_select_output, made present behind the candidate pass:
+// the longest wait of a selection.
+static void present_outputs(abc_ctx* c) {
+  make_present(c->out_idx, sizeof(int64_t) * c->out_cap);
+  make_present(c->out_err, sizeof(double) * c->out_cap);
+  c->out_idx = nullptr;
+  c->out_err = nullptr;
+  c->out_cap = 0;
+}
+
 // FP32 candidate pass on the CUDA cores; candidates and their FP32 errors in
 // d_cand / d_cande, count in *n.
 static int candidate_pass_simt(abc_ctx* c, const DistInputs& in, int64_t* n) {
@@ -970,6 +987,7 @@ static int candidate_pass_simt(abc_ctx* c, const DistInputs& in, int64_t* n) {
     if (st) return st;
     CK(launch_dist_fast(c->d_s32.p, c->d_sw.p, c->d_dw.p, in.P, in.G, in.K, c->d_X.p, c->d_cand.p, c->d_cande.p,
                         c->d_ncand.p, c->cand_cap, nullptr, 0, 0, c->stream));
+    present_outputs(c);
     st = prof_end(c);
     if (st) return st;
     unsigned long long h = 0;
@@ -1039,6 +1057,7 @@ static int candidate_pass_tc(abc_ctx* c, const DistInputs& in, int nh, int64_t* 
     st = prof_begin(c);
     if (st) return st;
     CK(launch_dist_tc(nh, c->d_tcA.p, c->d_tcB.p, a, grid, c->stream));
+    present_outputs(c);
     st = prof_end(c);
     if (st) return st;
     CK(cudaMemcpyAsync(stat, c->d_tcstat.p, sizeof(unsigned) * words, cudaMemcpyDeviceToHost, c->stream));
@@ -1116,8 +1135,35 @@ static int prepare_candidate_pass(abc_ctx* c, const DistInputs& in, int want, in
   return ABC_OK;
 }
 
-// mode 0: err <= eps; mode 1: top ceil(q P) per gene; mode 2: err <= thr[g] per gene
+int abc_select_output(abc_ctx* c, int64_t* particle_idx, double* err, int64_t capacity) {
+  if (!c) return ABC_ERR_INVALID;
+  if (capacity < 0) return fail(c, ABC_ERR_INVALID, "abc_select_output: negative capacity");
+  c->out_idx = particle_idx;
+  c->out_err = err;
+  c->out_cap = (size_t)capacity;
+  return ABC_OK;
+}
+
+static int select_run(abc_ctx* c, const double* data, const double* se, int64_t G, int K, int n_fam,
+                      const int32_t* fam, const double* stats, bool stats_on_device, int64_t P, int mode,
+                      double eps_or_q, const double* thr, int64_t* n_accepted_total);
+
+// The named output arrays belong to one selection, whether it succeeds or not.
 static int select_impl(abc_ctx* c, const double* data, const double* se, int64_t G, int K, int n_fam,
+                       const int32_t* fam, const double* stats, bool stats_on_device, int64_t P, int mode,
+                       double eps_or_q, const double* thr, int64_t* n_accepted_total) {
+  const int st = select_run(c, data, se, G, K, n_fam, fam, stats, stats_on_device, P, mode, eps_or_q, thr,
+                            n_accepted_total);
+  if (c) {
+    c->out_idx = nullptr;
+    c->out_err = nullptr;
+    c->out_cap = 0;
+  }
+  return st;
+}
+
+// mode 0: err <= eps; mode 1: top ceil(q P) per gene; mode 2: err <= thr[g] per gene
+static int select_run(abc_ctx* c, const double* data, const double* se, int64_t G, int K, int n_fam,
                        const int32_t* fam, const double* stats, bool stats_on_device, int64_t P, int mode,
                        double eps_or_q, const double* thr, int64_t* n_accepted_total) {
   if (!c) return ABC_ERR_INVALID;
@@ -1464,6 +1510,8 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   if (c->prof) CK(cudaEventRecord(c->sel_ev[0], c->stream));
   CK(f32 ? launch_moment_f32(a, c->stream) : launch_moment(a, c->stream));
   if (c->prof) CK(cudaEventRecord(c->sel_ev[1], c->stream));
+  make_present(stats_out, sizeof(double) * P * K);
+  if (moments_out) make_present(moments_out, sizeof(double) * P * J * A * 5);
   CK(cudaMemcpyAsync(stats_out, a.stats, sizeof(double) * P * K, cudaMemcpyDeviceToHost, c->stream));
   if (moments_out)
     CK(cudaMemcpyAsync(moments_out, a.moments, sizeof(double) * P * J * A * 5, cudaMemcpyDeviceToHost, c->stream));
@@ -1526,6 +1574,8 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   if (c->prof) CK(cudaEventRecord(c->sel_ev[0], c->stream));
   CK(launch_data_stats(a, dse, c->stream));
   if (c->prof) CK(cudaEventRecord(c->sel_ev[1], c->stream));
+  make_present(stats_out, sizeof(double) * G * K);
+  if (se_out) make_present(se_out, sizeof(double) * G * K);
   // the counts are checked where they are read (a pass over them on the host
   // took a millisecond per 10^7): nothing is returned for invalid ones
   int invalid = 0;

@@ -15,6 +15,7 @@
 
 #include "../../include/abcgpu.h"
 #include "distance.cuh"
+#include "host_pages.h"
 #include "kernels.h"
 #include "mlp.cuh"
 
@@ -658,9 +659,8 @@ static int predict_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_
   return ABC_OK;
 }
 
-int abc_surrogate_predict_device(abc_surrogate* s, const double* d_theta, int ld_theta, int64_t N, double* d_mean,
-                                 double* d_var, double* d_disagree) {
-  if (!s) return ABC_ERR_INVALID;
+static int predict_launch(abc_surrogate* s, const double* d_theta, int ld_theta, int64_t N, double* d_mean,
+                          double* d_var, double* d_disagree) {
   if (!s->normed) return sfail(s, ABC_ERR_STATE, "surrogate not trained");
   if (!d_theta || N < 0 || ld_theta < s->d.in_dim) return sfail(s, ABC_ERR_INVALID, "bad arguments");
   for (int64_t p0 = 0; p0 < N; p0 += kPredChunk) {
@@ -669,6 +669,14 @@ int abc_surrogate_predict_device(abc_surrogate* s, const double* d_theta, int ld
                            d_var ? d_var + p0 * s->d.K : nullptr, d_disagree ? d_disagree + p0 : nullptr);
     if (st) return st;
   }
+  return ABC_OK;
+}
+
+int abc_surrogate_predict_device(abc_surrogate* s, const double* d_theta, int ld_theta, int64_t N, double* d_mean,
+                                 double* d_var, double* d_disagree) {
+  if (!s) return ABC_ERR_INVALID;
+  const int st = predict_launch(s, d_theta, ld_theta, N, d_mean, d_var, d_disagree);
+  if (st) return st;
   SK(cudaStreamSynchronize(s->stream));
   return check_tc(s);
 }
@@ -683,7 +691,13 @@ int abc_surrogate_predict(abc_surrogate* s, const double* theta, int64_t N, doub
   SK(s->pv.ensure((size_t)N * K));
   SK(s->pd.ensure((size_t)N));
   SK(cudaMemcpyAsync(s->th64.p, theta, sizeof(double) * N * s->d.in_dim, cudaMemcpyHostToDevice, s->stream));
-  int st = abc_surrogate_predict_device(s, s->th64.p, s->d.in_dim, N, s->pm.p, s->pv.p, s->pd.p);
+  int st = predict_launch(s, s->th64.p, s->d.in_dim, N, s->pm.p, s->pv.p, s->pd.p);
+  if (st) return st;
+  make_present(mean, sizeof(double) * N * K);
+  make_present(var, sizeof(double) * N * K);
+  make_present(disagree, sizeof(double) * N);
+  SK(cudaStreamSynchronize(s->stream));
+  st = check_tc(s);
   if (st) return st;
   if (mean) SK(cudaMemcpy(mean, s->pm.p, sizeof(double) * N * K, cudaMemcpyDeviceToHost));
   if (var) SK(cudaMemcpy(var, s->pv.p, sizeof(double) * N * K, cudaMemcpyDeviceToHost));

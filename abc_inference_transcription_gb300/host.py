@@ -15,6 +15,7 @@ library raises ImportError, a failing call raises AbcError).
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 
@@ -83,7 +84,7 @@ class Context:
 
     # -- prior ---------------------------------------------------------------
     def sample_prior(self, model: int, n: int, seed: int, prior: AbcPrior, offset: int = 0) -> np.ndarray:
-        th = np.zeros((n, self.num_params(model)))
+        th = np.empty((n, self.num_params(model)))
         self._check(self.lib.abc_sample_prior(self.h, model, n, seed, offset, C.byref(prior), ptr(th)))
         return th
 
@@ -97,7 +98,7 @@ class Context:
         th = np.ascontiguousarray(theta, np.float64)
         if th.ndim != 2 or th.shape[1] != self.num_params(model):
             raise ValueError(f"theta must be P x {self.num_params(model)}")
-        out = np.zeros((th.shape[0], self.K))
+        out = np.empty((th.shape[0], self.K))
         self._check(self.lib.abc_simulate(self.h, model, ptr(th), th.shape[0], seed, offset, ptr(out)))
         return out
 
@@ -110,7 +111,7 @@ class Context:
         """Mixed-model batch: theta rows padded to the largest npar."""
         m = np.ascontiguousarray(models, np.int32)
         th = np.ascontiguousarray(theta, np.float64)
-        out = np.zeros((th.shape[0], self.K))
+        out = np.empty((th.shape[0], self.K))
         self._check(self.lib.abc_simulate_batch(self.h, ptr(m, C.c_int32), ptr(th), th.shape[1], th.shape[0], seed,
                                                 offset, ptr(out)))
         return out
@@ -189,7 +190,7 @@ class Context:
         s = np.ascontiguousarray(stats, np.float64)
         G, K = d.shape
         nf, f = self._fam(families, K)
-        out = np.zeros((s.shape[0], G))
+        out = np.empty((s.shape[0], G))
         self._check(self.lib.abc_errors(self.h, ptr(d), ptr(e), G, K, nf, ptr(f, C.c_int32), ptr(s), s.shape[0],
                                         ptr(out)))
         return out
@@ -202,7 +203,7 @@ class Context:
         s = np.ascontiguousarray(stats, np.float64)
         G, K = d.shape
         nf, f = self._fam(families, K)
-        out = np.zeros((s.shape[0], G), np.float32)
+        out = np.empty((s.shape[0], G), np.float32)
         b0 = np.zeros(G)
         b1, used = C.c_double(), C.c_int()
         self._check(self.lib.abc_errors_candidate(self.h, ptr(d), ptr(e), G, K, nf, ptr(f, C.c_int32), ptr(s),
@@ -224,16 +225,39 @@ class Context:
         nf, f = self._fam(families, K)
         tot = C.c_int64()
         self._check(self.lib.abc_set_select_errors(self.h, int(errors)))
+        own = self._output(G, s.shape[0], mode, eps_or_q, errors)
         self._check(self.lib.abc_errors_select(self.h, ptr(d), ptr(e), G, K, nf, ptr(f, C.c_int32), ptr(s),
                                                s.shape[0], mode, float(eps_or_q), C.byref(tot)))
-        return self._fetch(G, tot.value, errors)
+        return self._fetch(G, tot.value, errors, own)
 
-    def _fetch(self, G: int, total: int, errors: bool = True):
+    # Results of a top-q selection allocated before it, from 2 MB (below, the
+    # allocator hands out memory whose pages are present) up to 2^28 pairs (a
+    # selection has no more candidates).
+    _OWN_MIN, _OWN_MAX = 1 << 18, 1 << 28
+
+    def _output(self, G: int, n: int, mode: int, q: float, errors: bool):
+        """(indices, errors) of a top-q selection, whose size is known beforehand,
+        named to the library so that it makes their pages present while the
+        device works; None where the size is not known."""
+        if mode != 1 or not 0.0 < q <= 1.0:
+            return None
+        total = G * math.ceil(q * n)
+        if not self._OWN_MIN <= total <= self._OWN_MAX:
+            return None
+        idx = np.empty(total, np.int64)
+        err = np.empty(total) if errors else None
+        self._check(self.lib.abc_select_output(self.h, ptr(idx, C.c_int64), ptr(err), total))
+        return idx, err
+
+    def _fetch(self, G: int, total: int, errors: bool = True, own=None):
         self._last_total = total
         self._sel_G = G
         off = np.zeros(G + 1, np.int64)
-        idx = np.empty(max(total, 1), np.int64)
-        err = np.empty(max(total, 1)) if errors else None
+        if own is not None and own[0].shape[0] == total:
+            idx, err = own
+        else:  # fewer than q of the particles have an error
+            idx = np.empty(max(total, 1), np.int64)
+            err = np.empty(max(total, 1)) if errors else None
         self._check(self.lib.abc_accept_fetch(self.h, ptr(off, C.c_int64), ptr(idx, C.c_int64), ptr(err)))
         return off, idx[:total], (err[:total] if errors else None)
 
@@ -262,16 +286,17 @@ class Context:
         nf, f = self._fam(families, K)
         tot = C.c_int64()
         self._check(self.lib.abc_set_select_errors(self.h, int(errors)))
+        own = self._output(G, n, mode, eps_or_q, errors)
         self._check(self.lib.abc_errors_select_device(self.h, ptr(d), ptr(e), G, K, nf, ptr(f, C.c_int32),
                                                       C.c_void_p(d_stats), n, mode, float(eps_or_q), ptr(t),
                                                       C.byref(tot)))
-        return self._fetch(G, tot.value, errors)
+        return self._fetch(G, tot.value, errors, own)
 
     def accept_errors(self) -> np.ndarray:
         """FP64 errors of the last selection's accepted pairs (computed for them
         alone when the selection returned indices only)."""
         total = int(getattr(self, "_last_total", 0))
-        out = np.zeros(total)
+        out = np.empty(total)
         if total:
             self._check(self.lib.abc_accept_errors(self.h, ptr(out)))
         return out
@@ -295,9 +320,9 @@ class Context:
         th = np.ascontiguousarray(theta, np.float64)
         P = th.shape[0]
         A, J = self.cfg.n_ages, self.cfg.n_conds
-        st = np.zeros((P, nstats(A, J)))
-        mo = np.zeros((P, J, A, 5)) if moments else None
-        it = np.zeros(P, np.int32)
+        st = np.empty((P, nstats(A, J)))
+        mo = np.empty((P, J, A, 5)) if moments else None
+        it = np.empty(P, np.int32)
         self._check(self.lib.abc_moment_simulate(self.h, model, ptr(th), P, ptr(np.ascontiguousarray(iv, np.float64)),
                                                  float(h_max), ptr(np.ascontiguousarray(beta_mom, np.float64)),
                                                  n_pulse_conds, ptr(np.ascontiguousarray(age_dist, np.float64)),
@@ -314,8 +339,8 @@ class Context:
         ll = np.ascontiguousarray(l, np.int32)
         G = uu.shape[0]
         K = nstats(self.cfg.n_ages, self.cfg.n_conds)
-        st = np.zeros((G, K))
-        se = np.zeros((G, K)) if n_boot >= 2 else None
+        st = np.empty((G, K))
+        se = np.empty((G, K)) if n_boot >= 2 else None
         self._check(self.lib.abc_data_stats(self.h, ptr(uu, C.c_int32), ptr(ll, C.c_int32), G, int(n_boot),
                                             C.c_uint64(seed), ptr(st), ptr(se)))
         return st, se

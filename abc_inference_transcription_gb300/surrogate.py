@@ -65,13 +65,13 @@ class Surrogate:
         th = np.ascontiguousarray(theta, np.float64)
         st = np.ascontiguousarray(stats, np.float64)
         loss = np.zeros(self.members)
-        g = np.zeros(self.members * self.n_params, np.float32)
+        g = np.empty(self.members * self.n_params, np.float32)
         self._check(self.lib.abc_surrogate_gradients(self.h, ptr(th), ptr(st), th.shape[0], ptr(loss),
                                                      ptr(g, C.c_float)))
         return loss, g.reshape(self.members, self.n_params)
 
     def params(self) -> np.ndarray:
-        p = np.zeros(self.members * self.n_params, np.float32)
+        p = np.empty(self.members * self.n_params, np.float32)
         self._check(self.lib.abc_surrogate_get_params(self.h, ptr(p, C.c_float)))
         return p.reshape(self.members, self.n_params)
 
@@ -93,7 +93,7 @@ class Surrogate:
     def predict(self, theta: np.ndarray):
         th = np.ascontiguousarray(theta, np.float64)
         n = th.shape[0]
-        mean, var, dis = np.zeros((n, self.K)), np.zeros((n, self.K)), np.zeros(n)
+        mean, var, dis = np.empty((n, self.K)), np.empty((n, self.K)), np.empty(n)
         self._check(self.lib.abc_surrogate_predict(self.h, ptr(th), n, ptr(mean), ptr(var), ptr(dis)))
         return mean, var, dis
 

@@ -257,6 +257,13 @@ int abc_set_select_errors(abc_ctx* ctx, int keep_errors);
  * lists needs.  The statistics of the selection must still be in place (a
  * d_stats pointer given to abc_errors_select_device). */
 int abc_accept_errors(abc_ctx* ctx, double* err);
+/* The arrays that the next selection's result will be fetched into, where their
+ * size is known before it (a top-q selection of G genes returns at most
+ * G ceil(q P) pairs): the selection makes their pages present while the device
+ * works, so that abc_accept_fetch copies at the rate of the link.  Optional; the
+ * contents are not touched, and the pointers are forgotten when that selection
+ * returns.  err may be NULL. */
+int abc_select_output(abc_ctx* ctx, int64_t* particle_idx, double* err, int64_t capacity);
 /* gene_offsets: G+1 entries; particle_idx: 1-based, n_accepted_total entries;
  * err: FP64 errors of the accepted pairs (may be NULL; must be NULL after a
  * selection with abc_set_select_errors(ctx, 0)). */
