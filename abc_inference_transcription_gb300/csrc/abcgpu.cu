@@ -1245,7 +1245,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
       st = dmode ? candidate_pass_tc(c, in, dmode, &ncand, &redo) : candidate_pass_simt(c, in, &ncand);
       if (st) return st;
     }
-    const Cand* rc = c->d_cand.p;
+    Cand* rc = c->d_cand.p;
     const float* Xacc = c->d_X.p;
     int64_t nre = ncand;
     if (mode == 1) {
@@ -1266,7 +1266,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
     CK(c->d_sp.ensure((size_t)std::max<int64_t>(nre, 1)));
     CK(c->d_sg.ensure((size_t)std::max<int64_t>(nre, 1)));
     if (c->sel_errors) {
-      CK(launch_dist_group_recheck_sort(in, rc, nre, c->d_gcount.p, c->d_goff.p, c->d_gcursor.p, c->d_sp.p,
+      CK(launch_dist_group_recheck_sort(in, rc, c->d_cande.p, nre, c->d_gcount.p, c->d_goff.p, c->d_gcursor.p, c->d_sp.p,
                                         c->d_sg.p, c->d_se64.p, c->stream));
     } else {
       // indices only: certified FP32 errors, FP64 where they cannot decide
@@ -1275,7 +1275,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
       CK(c->d_flag.ensure((size_t)std::max<int64_t>(nre, 1)));
       CK(c->d_cnt2.ensure(2));
       CK(c->d_dirty.ensure((size_t)G));
-      CK(launch_dist_group_certify_sort(in, rc, nre, mode, eps_or_q, mode == 2 ? c->d_thr.p : nullptr,
+      CK(launch_dist_group_certify_sort(in, rc, c->d_cande.p, nre, mode, eps_or_q, mode == 2 ? c->d_thr.p : nullptr,
                                         c->d_gcount.p, c->d_goff.p, c->d_gcursor.p, c->d_sp.p, c->d_sg.p,
                                         c->d_se64.p, c->d_ffg.p, c->d_pos.p, c->d_flag.p,
                                         c->d_cnt2.p,

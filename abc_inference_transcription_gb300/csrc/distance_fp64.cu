@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <atomic>
 
-#include "bitonic.cuh"
 #include "smem_attr.h"
 #include "distance.cuh"
 #include "kernels.h"
@@ -608,13 +607,20 @@ __global__ void scatter_kernel(const Cand* cand, int64_t n, const int64_t* goff,
   }
 }
 
-// Per-gene sort by (err, p), NaN last, ties by index.  Segments up to
-// kSortSmem entries run the register-resident bitonic network of bitonic.cuh
-// (EPT = n2 / 1024 entries per thread, n2 the padded power of two) on keys
+// Per-gene sort by (err, p), NaN last, ties by index, a block per gene, on keys
 // that are the bit patterns of the errors (monotone for the non-negative
-// errors; NaN canonicalised to one pattern) with the index as tie-break;
-// padding slots carry (all ones, INT32_MAX), above every real entry.  Longer
-// segments run the same network on (err, p) in global memory.
+// errors; NaN canonicalised to one pattern).
+// - up to kSortDirect entries: each thread counts the entries below its own;
+// - longer lists: entries go to 4,096 equal bins of the list's range of FP32
+//   errors (a monotone map), in shared memory, and each counts the entries
+//   below its own in its bin.  Up to kSortCap entries in one window, written in
+//   place; longer lists in windows of whole bins, each with a read of the list,
+//   by way of tmp_key and tmp_p (as many entries as the list);
+// - lists with more than kBinMax entries in a bin (mostly exact ties, as at the
+//   clip value), whose counting would cost more: a bitonic network, in shared
+//   memory up to kSortCap entries, in global memory above.
+// Bound by latency of shared memory and barriers; two blocks of 512 threads per
+// SM (112 KB each) overlap them.
 __device__ __forceinline__ bool key_less(double ea, int32_t pa, double eb, int32_t pb) {
   const bool na = ea != ea, nb = eb != eb;
   if (na != nb) return nb;
@@ -622,7 +628,6 @@ __device__ __forceinline__ bool key_less(double ea, int32_t pa, double eb, int32
   return ea < eb || (ea == eb && pa < pb);
 }
 
-constexpr int kSortSmem = 8192;  // segments up to this size sort in registers
 constexpr uint64_t kNanKey = 0x7ff8000000000000ull;
 
 __device__ __forceinline__ uint64_t err_key(double e) {
@@ -631,73 +636,209 @@ __device__ __forceinline__ uint64_t err_key(double e) {
   return (uint64_t)__double_as_longlong(e);
 }
 
-template <int EPT>
-__device__ void sort_segment_regs(int32_t* P, double* E, int m, int n2, uint64_t* sK, int32_t* sP) {
-  const int t = threadIdx.x;
-  const int nt = n2 / EPT > 32 ? n2 / EPT : 32;  // threads holding entries
-  const bool act = t < nt;
-  uint64_t key[EPT];
-  int32_t pp[EPT];
-#pragma unroll
-  for (int e = 0; e < EPT; ++e) {
-    const int i = t * EPT + e;
-    const bool real = act && i < m;
-    key[e] = real ? err_key(E[i]) : ~0ull;
-    pp[e] = real ? P[i] : 0x7fffffff;
-  }
-  bitonic_regs<EPT>(key, pp, n2, sK, sP);
-#pragma unroll
-  for (int e = 0; e < EPT; ++e) {
-    const int i = t * EPT + e;
-    if (act && i < m) {
-      E[i] = __longlong_as_double((long long)key[e]);
-      P[i] = pp[e];
+__device__ __forceinline__ bool sort_key_less(uint64_t ka, int32_t pa, uint64_t kb, int32_t pb) {
+  return ka < kb || (ka == kb && pa < pb);
+}
+__device__ __forceinline__ bool sort_key_less(double ea, int32_t pa, double eb, int32_t pb) {
+  return key_less(ea, pa, eb, pb);
+}
+
+constexpr int kSortThreads = 512, kSortCap = 8192, kSortBins = 4096, kSortDirect = 512, kBinMax = 512;
+constexpr int kSortSmem = kSortCap * (int)(sizeof(uint64_t) + sizeof(int32_t)) + kSortBins * (int)sizeof(int);
+
+// FP32 value of a key that is not NaN; rounding to nearest keeps the order
+__device__ __forceinline__ float key_value(uint64_t key) { return rn32_bits(__longlong_as_double((long long)key)); }
+
+// Non-decreasing in key: every step rounds monotonically.  A range of zero
+// width (scale 0 or infinite) sends all to one bin, found too full.
+__device__ __forceinline__ int sort_bin(uint64_t key, float lo, float scale) {
+  if (key >= kNanKey) return kSortBins - 1;
+  return (int)fminf((key_value(key) - lo) * scale, (float)(kSortBins - 1));
+}
+
+// All-ascending bitonic network (the first step of every merge of size k pairs
+// i with i ^ (k - 1), the others i with i ^ j) over n2, a power of two, entries
+// of K and P; those from n on are absent and above all others.
+template <typename Key>
+__device__ void bitonic(Key* K, int32_t* P, int64_t n, int64_t n2) {
+  for (int64_t k = 2; k <= n2; k <<= 1) {
+    for (int64_t j = k >> 1; j > 0; j >>= 1) {
+      const int64_t flip = j == (k >> 1) ? k - 1 : j;
+      for (int64_t i = threadIdx.x; i < n; i += kSortThreads) {
+        const int64_t q = i ^ flip;
+        if (q > i && q < n) {
+          const Key ka = K[i], kb = K[q];
+          const int32_t pa = P[i], pb = P[q];
+          if (sort_key_less(kb, pb, ka, pa)) {
+            K[i] = kb;
+            K[q] = ka;
+            P[i] = pb;
+            P[q] = pa;
+          }
+        }
+      }
+      __syncthreads();
     }
   }
 }
 
-__global__ void __launch_bounds__(1024, 1) segsort_kernel(const int64_t* goff, int32_t* sp, double* se64,
-                                                          const int* dirty) {
+__global__ void __launch_bounds__(kSortThreads, 2) segsort_kernel(const int64_t* goff, int32_t* sp, double* se64,
+                                                                  const int* dirty, uint64_t* tmp_key,
+                                                                  int32_t* tmp_p) {
   extern __shared__ uint64_t sort_smem[];
+  __shared__ unsigned int s_lo, s_hi;
+  __shared__ int s_warp[kSortThreads / 32], s_most;
   const int64_t g = blockIdx.x;
   if (dirty && !dirty[g]) return;
   const int64_t base = goff[g];
   const int64_t n = goff[g + 1] - base;
   if (n <= 1) return;
+  const int t = threadIdx.x, lane = t & 31;
   int32_t* P = sp + base;
   double* E = se64 + base;
-  int64_t n2 = 1;
-  while (n2 < n) n2 <<= 1;
-  if (n2 <= kSortSmem) {
-    uint64_t* sK = sort_smem;
-    int32_t* sP = reinterpret_cast<int32_t*>(sort_smem + kSortSmem);
-    const int m = (int)n, w = (int)n2;
-    if (w <= 1024) sort_segment_regs<1>(P, E, m, w, sK, sP);
-    else if (w == 2048) sort_segment_regs<2>(P, E, m, w, sK, sP);
-    else if (w == 4096) sort_segment_regs<4>(P, E, m, w, sK, sP);
-    else sort_segment_regs<8>(P, E, m, w, sK, sP);
+  uint64_t* sK = sort_smem;
+  int32_t* sP = reinterpret_cast<int32_t*>(sK + kSortCap);
+  int* bins = sP + kSortCap;
+  if (n <= kSortDirect) {
+    const int m = (int)n;
+    uint64_t key = 0;
+    int32_t p = 0;
+    if (t < m) {
+      sK[t] = key = err_key(E[t]);
+      sP[t] = p = P[t];
+    }
+    __syncthreads();
+    if (t < m) {
+      int r = 0;
+#pragma unroll 4
+      for (int j = 0; j < m; ++j) r += sort_key_less(sK[j], sP[j], key, p) ? 1 : 0;
+      E[r] = __longlong_as_double((long long)key);
+      P[r] = p;
+    }
     return;
   }
-  for (int64_t k = 2; k <= n2; k <<= 1) {
-    for (int64_t j = k >> 1; j > 0; j >>= 1) {
-      for (int64_t i = threadIdx.x; i < n2; i += blockDim.x) {
-        int64_t partner;
-        if (j == (k >> 1))
-          partner = i ^ (k - 1);  // flip step
-        else
-          partner = i ^ j;
-        if (partner > i && partner < n) {
-          double ea = E[i], eb = E[partner];
-          int32_t pa = P[i], pb = P[partner];
-          if (key_less(eb, pb, ea, pa)) {
-            E[i] = eb;
-            E[partner] = ea;
-            P[i] = pb;
-            P[partner] = pa;
-          }
-        }
+  // range of the errors, as FP32 (the patterns of non-negative floats are ordered)
+  if (t == 0) {
+    s_lo = 0xffffffffu;
+    s_hi = 0;
+    s_most = 0;
+  }
+  for (int b = t; b < kSortBins; b += kSortThreads) bins[b] = 0;
+  __syncthreads();
+  unsigned int lo_u = 0xffffffffu, hi_u = 0;
+#pragma unroll 4
+  for (int64_t i = t; i < n; i += kSortThreads) {
+    const uint64_t key = err_key(E[i]);
+    if (key < kNanKey) {
+      const unsigned int u = __float_as_uint(key_value(key));
+      lo_u = min(lo_u, u);
+      hi_u = max(hi_u, u);
+    }
+  }
+  lo_u = __reduce_min_sync(0xffffffffu, lo_u);
+  hi_u = __reduce_max_sync(0xffffffffu, hi_u);
+  if (lane == 0) {
+    atomicMin(&s_lo, lo_u);
+    atomicMax(&s_hi, hi_u);
+  }
+  __syncthreads();
+  const float lo = s_lo <= s_hi ? __uint_as_float(s_lo) : 0.0f, hi = __uint_as_float(s_hi);
+  const float scale = hi > lo ? (float)kSortBins / (hi - lo) : 0.0f;
+#pragma unroll 4
+  for (int64_t i = t; i < n; i += kSortThreads) atomicAdd(&bins[sort_bin(err_key(E[i]), lo, scale)], 1);
+  __syncthreads();
+  // exclusive prefix sums of the bins, eight of them per thread, and the fullest
+  constexpr int kPer = kSortBins / kSortThreads;
+  int cnt[kPer], sum = 0, most = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    cnt[q] = bins[t * kPer + q];
+    sum += cnt[q];
+    most = max(most, cnt[q]);
+  }
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 31) s_warp[t >> 5] = inc;
+  if (lane == 0) atomicMax(&s_most, most);
+  __syncthreads();
+  int at = inc - sum;
+  for (int w = 0; w < (t >> 5); ++w) at += s_warp[w];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    bins[t * kPer + q] = at;
+    at += cnt[q];
+  }
+  __syncthreads();
+  if (s_most > kBinMax) {
+    int64_t n2 = 1;
+    while (n2 < n) n2 <<= 1;
+    if (n > kSortCap) {
+      bitonic(E, P, n, n2);
+      return;
+    }
+    for (int i = t; i < (int)n; i += kSortThreads) {
+      sK[i] = err_key(E[i]);
+      sP[i] = P[i];
+    }
+    __syncthreads();
+    bitonic(sK, sP, n, n2);
+    for (int i = t; i < (int)n; i += kSortThreads) {
+      E[i] = __longlong_as_double((long long)sK[i]);
+      P[i] = sP[i];
+    }
+    return;
+  }
+  const bool whole = n <= kSortCap;
+  uint64_t* out_key = whole ? reinterpret_cast<uint64_t*>(E) : tmp_key + base;
+  int32_t* out_p = whole ? P : tmp_p + base;
+  for (int b0 = 0; b0 < kSortBins;) {
+    // the window: bins b0 to b1 - 1, positions first to first + m - 1 of the list
+    const int first = bins[b0];
+    int b1 = kSortBins, m = (int)n - first;
+    if (m > kSortCap) {
+      int below = b0, above = kSortBins;  // the last b1 with bins[b1] - first <= kSortCap
+      while (above - below > 1) {
+        const int mid = (below + above) >> 1;
+        if (bins[mid] - first <= kSortCap) below = mid; else above = mid;
       }
-      __syncthreads();
+      b1 = below;
+      m = bins[b1] - first;
+    }
+    __syncthreads();  // the bins are read; the window before is written
+#pragma unroll 4
+    for (int64_t i = t; i < n; i += kSortThreads) {
+      const uint64_t key = err_key(E[i]);
+      const int b = sort_bin(key, lo, scale);
+      if (b >= b0 && b < b1) {
+        const int slot = atomicAdd(&bins[b], 1) - first;
+        sK[slot] = key;
+        sP[slot] = P[i];
+      }
+    }
+    __syncthreads();
+    // bins[b] is now the end of bin b
+    for (int i = t; i < m; i += kSortThreads) {
+      const uint64_t key = sK[i];
+      const int32_t p = sP[i];
+      const int b = sort_bin(key, lo, scale);
+      const int s = b == b0 ? 0 : bins[b - 1] - first, e = bins[b] - first;
+      int r = first + s;
+      for (int j = s; j < e; ++j) r += sort_key_less(sK[j], sP[j], key, p) ? 1 : 0;
+      out_key[r] = key;
+      out_p[r] = p;
+    }
+    b0 = b1;
+  }
+  if (!whole) {
+    __syncthreads();
+    for (int64_t i = t; i < n; i += kSortThreads) {
+      E[i] = __longlong_as_double((long long)out_key[i]);
+      P[i] = out_p[i];
     }
   }
 }
@@ -733,13 +874,16 @@ cudaError_t launch_dist_group(const Cand* cand, int64_t n, int64_t G, int64_t* g
   return cudaGetLastError();
 }
 
+// tmp: the grouped candidates' own buffers, which nothing reads after the
+// grouping (Cand is two 32-bit words, room for a key per entry)
 static cudaError_t launch_segsort(const int64_t* goff, int64_t G, int32_t* sp, double* se64, const int* dirty,
-                                  cudaStream_t s) {
-  constexpr int smem = kSortSmem * (int)(sizeof(uint64_t) + sizeof(int32_t));
+                                  Cand* tmp, float* tmp_e, cudaStream_t s) {
+  static_assert(sizeof(Cand) == sizeof(uint64_t) && sizeof(float) == sizeof(int32_t), "scratch of the sort");
   static std::atomic<uint64_t> attr{0};  // devices where the limit is set, shared by all contexts
-  cudaError_t err = set_smem_once(attr, segsort_kernel, smem);
+  cudaError_t err = set_smem_once(attr, segsort_kernel, kSortSmem);
   if (err) return err;
-  segsort_kernel<<<(unsigned)G, 1024, smem, s>>>(goff, sp, se64, dirty);
+  segsort_kernel<<<(unsigned)G, kSortThreads, kSortSmem, s>>>(goff, sp, se64, dirty, reinterpret_cast<uint64_t*>(tmp),
+                                                              reinterpret_cast<int32_t*>(tmp_e));
   return cudaGetLastError();
 }
 
@@ -758,7 +902,7 @@ static void launch_recheck_grouped(const DistInputs& in, const int32_t* sp, cons
     recheck_grouped_kernel<kRecheckWarps><<<grouped_blocks(n), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, se64);
 }
 
-cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, const Cand* cand, int64_t n, int64_t* gcount,
+cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, Cand* cand, float* cand_e, int64_t n, int64_t* gcount,
                                            int64_t* goff, unsigned long long* gcursor, int32_t* sp, int32_t* sg,
                                            double* se64, cudaStream_t s) {
   cudaError_t err = launch_dist_group(cand, n, in.G, gcount, goff, gcursor, sp, sg, s);
@@ -766,10 +910,10 @@ cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, const Cand* can
   launch_recheck_grouped(in, sp, sg, n, se64, s);
   err = cudaGetLastError();
   if (err) return err;
-  return launch_segsort(goff, in.G, sp, se64, nullptr, s);
+  return launch_segsort(goff, in.G, sp, se64, nullptr, cand, cand_e, s);
 }
 
-cudaError_t launch_dist_group_certify_sort(const DistInputs& in, const Cand* cand, int64_t n, int mode, double eps,
+cudaError_t launch_dist_group_certify_sort(const DistInputs& in, Cand* cand, float* cand_e, int64_t n, int mode, double eps,
                                            const double* eps_g, int64_t* gcount, int64_t* goff,
                                            unsigned long long* gcursor, int32_t* sp, int32_t* sg, double* se64,
                                            float4* gt, int32_t* pos, uint8_t* flag,
@@ -786,7 +930,7 @@ cudaError_t launch_dist_group_certify_sort(const DistInputs& in, const Cand* can
                                                                          counts);
   const int list_blocks = 152 * 8;
   recheck_list_kernel<<<list_blocks, 128, 0, s>>>(in, sp, sg, pos, counts, se64);
-  err = launch_segsort(goff, in.G, sp, se64, nullptr, s);
+  err = launch_segsort(goff, in.G, sp, se64, nullptr, cand, cand_e, s);
   if (err) return err;
   err = cudaMemsetAsync(dirty, 0, sizeof(int) * (size_t)in.G, s);
   if (err) return err;
@@ -794,7 +938,7 @@ cudaError_t launch_dist_group_certify_sort(const DistInputs& in, const Cand* can
   ambiguous_kernel<<<blocks, 256, 0, s>>>(sg, goff, se64, n, mode, eps, eps_g, pos, counts + 1, flag);
   recheck_list_kernel<<<list_blocks, 128, 0, s>>>(in, sp, sg, pos, counts + 1, se64);
   run_sort_kernel<<<blocks, 256, 0, s>>>(sg, goff, flag, n, sp, se64, dirty);
-  return launch_segsort(goff, in.G, sp, se64, dirty, s);
+  return launch_segsort(goff, in.G, sp, se64, dirty, cand, cand_e, s);
 }
 
 // ---------------------------------------------------------------------------

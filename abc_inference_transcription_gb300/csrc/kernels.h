@@ -143,7 +143,7 @@ cudaError_t launch_dist_den(const DistInputs& in, double* den, double* rden, flo
 // Group candidates by gene (goff: G + 1 offsets; sp, sg: particle and gene per
 // entry), evaluate their FP64 errors in the reference's operation order (se64;
 // needs in.den and in.rden) and sort each gene's list by (err, p).
-cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, const Cand* cand, int64_t n, int64_t* gcount,
+cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, Cand* cand, float* cand_e, int64_t n, int64_t* gcount,
                                            int64_t* goff, unsigned long long* gcursor, int32_t* sp, int32_t* sg,
                                            double* se64, cudaStream_t s);
 // The same grouping and order with certified FP32 errors instead of FP64 ones
@@ -151,7 +151,7 @@ cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, const Cand* can
 // value or, where that cannot decide the order or the threshold (mode 0/2:
 // eps or eps_g), its FP64 error.  Scratch: gt (G x K float4), pos and flag
 // (n), counts (2: pairs computed in FP64 before / after the sort), dirty (G).
-cudaError_t launch_dist_group_certify_sort(const DistInputs& in, const Cand* cand, int64_t n, int mode, double eps,
+cudaError_t launch_dist_group_certify_sort(const DistInputs& in, Cand* cand, float* cand_e, int64_t n, int mode, double eps,
                                            const double* eps_g, int64_t* gcount, int64_t* goff,
                                            unsigned long long* gcursor, int32_t* sp, int32_t* sg, double* se64,
                                            float4* gt, int32_t* pos, uint8_t* flag,
