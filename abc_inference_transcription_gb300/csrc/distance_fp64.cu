@@ -611,16 +611,19 @@ __global__ void scatter_kernel(const Cand* cand, int64_t n, const int64_t* goff,
 // that are the bit patterns of the errors (monotone for the non-negative
 // errors; NaN canonicalised to one pattern).
 // - up to kSortDirect entries: each thread counts the entries below its own;
-// - longer lists: entries go to 4,096 equal bins of the list's range of FP32
-//   errors (a monotone map), in shared memory, and each counts the entries
-//   below its own in its bin.  Up to kSortCap entries in one window, written in
-//   place; longer lists in windows of whole bins, each with a read of the list,
-//   by way of tmp_key and tmp_p (as many entries as the list);
-// - lists with more than kBinMax entries in a bin (mostly exact ties, as at the
-//   clip value), whose counting would cost more: a bitonic network, in shared
-//   memory up to kSortCap entries, in global memory above.
+// - longer lists: entries go to 4,096 bins, a monotone map of (error, index):
+//   3,072 equal bins of the range of the errors below the clip value in FP32, then
+//   1,023 equal ranges of the particle index for errors at the clip value, where ties
+//   are the rule, then everything above.  Up to kSortCap entries in shared
+//   memory, longer lists by way of tmp_key and tmp_p (as many entries as the list).
+//   Windows of whole bins are then finished in shared memory: each entry
+//   counts those below it in its bin, or, where a bin holds more than kBinMax,
+//   the window goes through a bitonic network;
+// - a bin of more than kSortCap entries (ties elsewhere than at the clip value):
+//   a bitonic network over the list in global memory.
 // Bound by latency of shared memory and barriers; two blocks of 512 threads per
-// SM (112 KB each) overlap them.
+// SM (112 KB each) overlap them.  2,000 lists of 5,450 entries take 0.234 ms (a
+// bitonic network over 8,192 register entries: 1.69).
 __device__ __forceinline__ bool key_less(double ea, int32_t pa, double eb, int32_t pb) {
   const bool na = ea != ea, nb = eb != eb;
   if (na != nb) return nb;
@@ -644,17 +647,24 @@ __device__ __forceinline__ bool sort_key_less(double ea, int32_t pa, double eb, 
 }
 
 constexpr int kSortThreads = 512, kSortCap = 8192, kSortBins = 4096, kSortDirect = 512, kBinMax = 512;
+constexpr int kValueBins = 3072;
+constexpr uint64_t kClipKey = 0x4024000000000000ull;  // 10.0
 constexpr int kSortSmem = kSortCap * (int)(sizeof(uint64_t) + sizeof(int32_t)) + kSortBins * (int)sizeof(int);
 
 // FP32 value of a key that is not NaN; rounding to nearest keeps the order
 __device__ __forceinline__ float key_value(uint64_t key) { return rn32_bits(__longlong_as_double((long long)key)); }
 
-// Non-decreasing in key: every step rounds monotonically.  A range of zero
-// width (scale 0 or infinite) sends all to one bin, found too full.
-__device__ __forceinline__ int sort_bin(uint64_t key, float lo, float scale) {
-  if (key >= kNanKey) return kSortBins - 1;
-  return (int)fminf((key_value(key) - lo) * scale, (float)(kSortBins - 1));
-}
+// The map to bins.  Non-decreasing in (key, p): every step rounds monotonically.
+// A range of zero width (scale 0 or infinite) sends all of it to one bin.
+struct SortMap {
+  float lo, scale, p_scale;
+  int p_lo;
+  __device__ __forceinline__ int bin(uint64_t key, int32_t p) const {
+    if (key < kClipKey) return (int)fminf((key_value(key) - lo) * scale, (float)(kValueBins - 1));
+    if (key > kClipKey) return kSortBins - 1;
+    return kValueBins + (int)fminf((float)(p - p_lo) * p_scale, (float)(kSortBins - kValueBins - 2));
+  }
+};
 
 // All-ascending bitonic network (the first step of every merge of size k pairs
 // i with i ^ (k - 1), the others i with i ^ j) over n2, a power of two, entries
@@ -686,7 +696,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) segsort_kernel(const int64_t*
                                                                   const int* dirty, uint64_t* tmp_key,
                                                                   int32_t* tmp_p) {
   extern __shared__ uint64_t sort_smem[];
-  __shared__ unsigned int s_lo, s_hi;
+  __shared__ unsigned int s_lo, s_hi, s_plo, s_phi;
   __shared__ int s_warp[kSortThreads / 32], s_most;
   const int64_t g = blockIdx.x;
   if (dirty && !dirty[g]) return;
@@ -717,35 +727,48 @@ __global__ void __launch_bounds__(kSortThreads, 2) segsort_kernel(const int64_t*
     }
     return;
   }
-  // range of the errors, as FP32 (the patterns of non-negative floats are ordered)
+  // range of the errors below the clip value, as FP32 (the patterns of
+  // non-negative floats are ordered), and of the indices at it
   if (t == 0) {
-    s_lo = 0xffffffffu;
-    s_hi = 0;
+    s_lo = s_plo = 0xffffffffu;
+    s_hi = s_phi = 0;
     s_most = 0;
   }
   for (int b = t; b < kSortBins; b += kSortThreads) bins[b] = 0;
   __syncthreads();
-  unsigned int lo_u = 0xffffffffu, hi_u = 0;
+  unsigned int lo_u = 0xffffffffu, hi_u = 0, plo_u = 0xffffffffu, phi_u = 0;
 #pragma unroll 4
   for (int64_t i = t; i < n; i += kSortThreads) {
     const uint64_t key = err_key(E[i]);
-    if (key < kNanKey) {
+    const unsigned int p = (unsigned int)P[i];
+    if (key < kClipKey) {
       const unsigned int u = __float_as_uint(key_value(key));
       lo_u = min(lo_u, u);
       hi_u = max(hi_u, u);
+    } else if (key == kClipKey) {
+      plo_u = min(plo_u, p);
+      phi_u = max(phi_u, p);
     }
   }
   lo_u = __reduce_min_sync(0xffffffffu, lo_u);
   hi_u = __reduce_max_sync(0xffffffffu, hi_u);
+  plo_u = __reduce_min_sync(0xffffffffu, plo_u);
+  phi_u = __reduce_max_sync(0xffffffffu, phi_u);
   if (lane == 0) {
     atomicMin(&s_lo, lo_u);
     atomicMax(&s_hi, hi_u);
+    atomicMin(&s_plo, plo_u);
+    atomicMax(&s_phi, phi_u);
   }
   __syncthreads();
-  const float lo = s_lo <= s_hi ? __uint_as_float(s_lo) : 0.0f, hi = __uint_as_float(s_hi);
-  const float scale = hi > lo ? (float)kSortBins / (hi - lo) : 0.0f;
+  SortMap map;
+  const float hi = __uint_as_float(s_hi);
+  map.lo = s_lo <= s_hi ? __uint_as_float(s_lo) : 0.0f;
+  map.scale = hi > map.lo ? (float)kValueBins / (hi - map.lo) : 0.0f;
+  map.p_lo = s_plo <= s_phi ? (int)s_plo : 0;
+  map.p_scale = s_plo < s_phi ? (float)(kSortBins - kValueBins - 1) / (float)(s_phi - s_plo) : 0.0f;
 #pragma unroll 4
-  for (int64_t i = t; i < n; i += kSortThreads) atomicAdd(&bins[sort_bin(err_key(E[i]), lo, scale)], 1);
+  for (int64_t i = t; i < n; i += kSortThreads) atomicAdd(&bins[map.bin(err_key(E[i]), P[i])], 1);
   __syncthreads();
   // exclusive prefix sums of the bins, eight of them per thread, and the fullest
   constexpr int kPer = kSortBins / kSortThreads;
@@ -774,72 +797,70 @@ __global__ void __launch_bounds__(kSortThreads, 2) segsort_kernel(const int64_t*
     at += cnt[q];
   }
   __syncthreads();
-  if (s_most > kBinMax) {
+  if (s_most > kSortCap) {
     int64_t n2 = 1;
     while (n2 < n) n2 <<= 1;
-    if (n > kSortCap) {
-      bitonic(E, P, n, n2);
-      return;
-    }
-    for (int i = t; i < (int)n; i += kSortThreads) {
-      sK[i] = err_key(E[i]);
-      sP[i] = P[i];
-    }
-    __syncthreads();
-    bitonic(sK, sP, n, n2);
-    for (int i = t; i < (int)n; i += kSortThreads) {
-      E[i] = __longlong_as_double((long long)sK[i]);
-      P[i] = sP[i];
-    }
+    bitonic(E, P, n, n2);
     return;
   }
+  // entries by bin; afterwards bins[b] is the end of bin b
   const bool whole = n <= kSortCap;
-  uint64_t* out_key = whole ? reinterpret_cast<uint64_t*>(E) : tmp_key + base;
-  int32_t* out_p = whole ? P : tmp_p + base;
+  uint64_t* by_key = whole ? sK : tmp_key + base;
+  int32_t* by_p = whole ? sP : tmp_p + base;
+#pragma unroll 4
+  for (int64_t i = t; i < n; i += kSortThreads) {
+    const uint64_t key = err_key(E[i]);
+    const int32_t p = P[i];
+    const int slot = atomicAdd(&bins[map.bin(key, p)], 1);
+    by_key[slot] = key;
+    by_p[slot] = p;
+  }
+  __syncthreads();
   for (int b0 = 0; b0 < kSortBins;) {
     // the window: bins b0 to b1 - 1, positions first to first + m - 1 of the list
-    const int first = bins[b0];
-    int b1 = kSortBins, m = (int)n - first;
-    if (m > kSortCap) {
-      int below = b0, above = kSortBins;  // the last b1 with bins[b1] - first <= kSortCap
-      while (above - below > 1) {
-        const int mid = (below + above) >> 1;
-        if (bins[mid] - first <= kSortCap) below = mid; else above = mid;
+    const int first = b0 ? bins[b0 - 1] : 0;
+    int b1 = kSortBins;
+    if ((int)n - first > kSortCap) {
+      int above = kSortBins;  // the last b1 with bins[b1 - 1] - first <= kSortCap: at least one bin
+      b1 = b0 + 1;
+      while (above - b1 > 1) {
+        const int mid = (b1 + above) >> 1;
+        if (bins[mid - 1] - first <= kSortCap) b1 = mid; else above = mid;
       }
-      b1 = below;
-      m = bins[b1] - first;
     }
-    __syncthreads();  // the bins are read; the window before is written
+    const int m = bins[b1 - 1] - first;
+    bool crowded = false;
+    for (int b = b0 + t; b < b1; b += kSortThreads)
+      crowded = crowded || bins[b] - (b ? bins[b - 1] : 0) > kBinMax;
+    if (!whole) {
 #pragma unroll 4
-    for (int64_t i = t; i < n; i += kSortThreads) {
-      const uint64_t key = err_key(E[i]);
-      const int b = sort_bin(key, lo, scale);
-      if (b >= b0 && b < b1) {
-        const int slot = atomicAdd(&bins[b], 1) - first;
-        sK[slot] = key;
-        sP[slot] = P[i];
+      for (int i = t; i < m; i += kSortThreads) {
+        sK[i] = by_key[first + i];
+        sP[i] = by_p[first + i];
       }
     }
-    __syncthreads();
-    // bins[b] is now the end of bin b
-    for (int i = t; i < m; i += kSortThreads) {
-      const uint64_t key = sK[i];
-      const int32_t p = sP[i];
-      const int b = sort_bin(key, lo, scale);
-      const int s = b == b0 ? 0 : bins[b - 1] - first, e = bins[b] - first;
-      int r = first + s;
-      for (int j = s; j < e; ++j) r += sort_key_less(sK[j], sP[j], key, p) ? 1 : 0;
-      out_key[r] = key;
-      out_p[r] = p;
+    if (__syncthreads_or(crowded)) {
+      int n2 = 1;
+      while (n2 < m) n2 <<= 1;
+      bitonic(sK, sP, m, n2);
+      for (int i = t; i < m; i += kSortThreads) {
+        E[first + i] = __longlong_as_double((long long)sK[i]);
+        P[first + i] = sP[i];
+      }
+    } else {
+      for (int i = t; i < m; i += kSortThreads) {
+        const uint64_t key = sK[i];
+        const int32_t p = sP[i];
+        const int b = map.bin(key, p);
+        const int s = b ? bins[b - 1] - first : 0, e = bins[b] - first;
+        int r = first + s;
+        for (int j = s; j < e; ++j) r += sort_key_less(sK[j], sP[j], key, p) ? 1 : 0;
+        E[r] = __longlong_as_double((long long)key);
+        P[r] = p;
+      }
     }
     b0 = b1;
-  }
-  if (!whole) {
-    __syncthreads();
-    for (int64_t i = t; i < n; i += kSortThreads) {
-      E[i] = __longlong_as_double((long long)out_key[i]);
-      P[i] = out_p[i];
-    }
+    __syncthreads();  // before the next window's entries take their place
   }
 }
 

@@ -1,8 +1,8 @@
 """The per-gene sort at the list lengths where its path changes: counting over
 the whole list up to 512 entries, one window of bins up to 8,192, several
-windows above, and the bitonic networks for lists with crowded bins (one far
-entry, or exact ties).  eps = 10 accepts every particle, so that a list is as
-long as the particles are many."""
+windows above; the bitonic networks for crowded bins (one far entry, or exact
+ties); ties at the clip value, binned by index.  eps = 10 accepts every
+particle, so that a list is as long as the particles are many."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ from abc_inference_transcription_gb300.config import REF_FAMILIES, make_config
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", ["spread", "crowded", "ties"])
+@pytest.mark.parametrize("shape", ["spread", "crowded", "ties", "clipped", "all clipped"])
 @pytest.mark.parametrize("n", [1, 2, 33, 511, 512, 513, 4097, 8191, 8192, 8193, 16385, 40001])
 def test_lists_of_every_length(built, orc, n, shape):
     from abc_inference_transcription_gb300.host import Context
@@ -26,6 +26,8 @@ def test_lists_of_every_length(built, orc, n, shape):
         far = 1e-4 * far
         far[0] = 0.35
     stats = base * (1.0 + far * rng.uniform(-1.0, 1.0, (n, K)))
+    if shape in ("clipped", "all clipped"):
+        stats[rng.random(n) < (0.9 if shape == "clipped" else 1.1)] *= 3.0
     if shape == "ties":
         stats = stats[rng.integers(0, min(n, 7), n)]
     if n > 40:
