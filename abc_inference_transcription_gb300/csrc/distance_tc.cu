@@ -946,7 +946,8 @@ __global__ void tc_gather_kernel(const Cand* seg, const float* seg_e, const unsi
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const Cand cd = seg[(int64_t)b * seg_cap + i];
     out[off + i] = cd;
-    out_e[off + i] = fminf((seg_e[(int64_t)b * seg_cap + i] + cg[cd.g]) * invK, 10.0f);
+    const float e = (seg_e[(int64_t)b * seg_cap + i] + cg[cd.g]) * invK;
+    out_e[off + i] = e > 10.0f ? e : fminf(e, 10.0f);  // not clipped; NaN becomes 10
   }
 }
 

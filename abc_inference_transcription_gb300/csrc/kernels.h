@@ -125,17 +125,19 @@ cudaError_t launch_dist_fast(const float* s32, const float* sw, const float* dw,
 cudaError_t launch_dist_threshold(const float* esub, int64_t n_sub, int64_t G, int64_t k_sub, const float* b0,
                                   float b1, float* X, cudaStream_t s);
 cudaError_t launch_fill(float* x, int64_t n, float v, cudaStream_t s);
-// dense[p G + g] = e of candidate (p, g)
+// dense[p G + g] = e of candidate (p, g), clipped at 10
 cudaError_t launch_scatter_errors(const Cand* cand, const float* e, int64_t n, int64_t G, float* out, cudaStream_t s);
 // X[g] = e_g + 2 B_g(e_g) for e_g = thr[g] (or eps when thr is null); +inf for e_g >= 10, -1 for e_g < 0.
 cudaError_t launch_x_from_thr(const double* thr, double eps, int64_t G, const float* b0, float b1, float* X,
                               cudaStream_t s);
 // top-k refinement before the FP64 recheck: per-gene histogram of the
-// candidates' FP32 errors, a tighter Xt <= X from the bin completing k, and
-// the candidates with e <= Xt appended to out (count in *count).
-cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int64_t G, int64_t k, const float* X,
-                          const float* b0, float b1, unsigned int* hist, float* Xt, Cand* out,
-                          unsigned long long* count, cudaStream_t s);
+// candidates' FP32 errors (hist: G x (kHistBins + 1)), a tighter Xt <= X from the
+// bin completing k, and the candidates with e <= Xt appended to out (count in
+// *count).  Of those surely at the clip value only the ones below p_end[g] (of P
+// particles) are kept: enough for any k smallest, as ties are ordered by index.
+cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int64_t P, int64_t G, int64_t k,
+                          const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, int* p_end,
+                          Cand* out, unsigned long long* count, cudaStream_t s);
 // den[g][k] = (se^2 + 0.01 d^2) + eps_gk, the denominators of the error terms,
 // evaluated as in the per-term FP64 expression (bit-identical), and rden = 1/den
 // (both may be null); sw = sqrt(w), dw = sqrt(w) d in FP32, w = 1/den.
