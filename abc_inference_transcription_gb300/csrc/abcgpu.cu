@@ -136,7 +136,8 @@ struct abc_ctx {
   DBuf<int32_t> d_pos;
   DBuf<uint8_t> d_flag;
   DBuf<unsigned long long> d_cnt2;
-  DBuf<int> d_dirty, d_pend;
+  DBuf<int> d_dirty;
+  DBuf<float2> d_cut;
 };
 
 static int fail(abc_ctx* c, int status, const std::string& msg) {
@@ -275,7 +276,7 @@ int abc_destroy(abc_ctx* c) {
   c->d_events.release(); c->d_hash.release(); c->d_misc.release(); c->d_status.release();
   c->d_data.release(); c->d_se.release(); c->d_sel_stats.release(); c->d_se64.release(); c->d_sg.release();
   c->d_ffg.release(); c->d_pos.release(); c->d_flag.release(); c->d_cnt2.release();
-  c->d_dirty.release(); c->d_pend.release();
+  c->d_dirty.release(); c->d_cut.release();
   c->d_out_err.release(); c->d_sw.release(); c->d_dw.release(); c->d_s32.release(); c->d_X.release();
   c->d_esub.release(); c->d_cand.release(); c->d_sp.release(); c->d_gcount.release(); c->d_goff.release();
   c->d_cande.release(); c->d_den.release(); c->d_rden.release(); c->d_tcA.release(); c->d_tcB.release(); c->d_rowbad.release(); c->d_cg32.release(); c->d_b0.release();
@@ -1252,10 +1253,10 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
       // only candidates that can still be among the k smallest go to the FP64 recheck
       CK(c->d_hist.ensure((size_t)G * (kHistBins + 1)));
       CK(c->d_Xt.ensure((size_t)G));
-      CK(c->d_pend.ensure((size_t)G));
+      CK(c->d_cut.ensure((size_t)G));
       CK(c->d_cand2.ensure((size_t)std::max<int64_t>(ncand, 1)));
       CK(launch_refine(c->d_cand.p, c->d_cande.p, ncand, P, G, kq, c->d_X.p, c->d_b0.p, b1, c->d_hist.p, c->d_Xt.p,
-                       c->d_pend.p, c->d_cand2.p, c->d_ncand.p, c->stream));
+                       c->d_cut.p, c->d_cand2.p, c->d_ncand.p, c->stream));
       unsigned long long* h = static_cast<unsigned long long*>(c->h_pin);
       CK(cudaMemcpyAsync(h, c->d_ncand.p, sizeof(*h), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));

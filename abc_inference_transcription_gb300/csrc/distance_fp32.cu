@@ -284,22 +284,21 @@ cudaError_t launch_x_from_thr(const double* thr, double eps, int64_t G, const fl
 // A candidate whose error is certainly above the clip value 10, so that it is 10:
 // |e32 - err| <= b0 + b1 err (twice that covers the rounding here).  Only an
 // unclipped e32 can say so: the tensor-core pass's, not that of dist_fast_kernel.
-__device__ __forceinline__ bool surely_clipped(float e, float b0, float b1) {
-  return e > 10.0f && e < INFINITY && e > fmaf(2.0f, fmaf(10.0f, b1, b0), 10.0f);
-}
+__device__ __forceinline__ float sure_clip(float b0, float b1) { return fmaf(2.0f, fmaf(10.0f, b1, b0), 10.0f); }
+__device__ __forceinline__ bool surely_clipped(float e, float sure) { return e > sure && e < INFINITY; }
 
 // Histogram of the candidates' FP32 errors per gene (G x kCandBins counters:
 // kHistBins of errors, then the surely clipped ones).
 constexpr int kCandBins = kHistBins + 1;
-__device__ __forceinline__ int cand_bin(float e, const float* b0, int32_t g, float b1) {
-  return e > 10.0f && surely_clipped(e, b0[g], b1) ? kHistBins : hist_bin(fminf(fmaxf(e, 0.0f), 10.0f));
+__device__ __forceinline__ int cand_bin(float e, float sure) {
+  return surely_clipped(e, sure) ? kHistBins : hist_bin(fminf(fmaxf(e, 0.0f), 10.0f));
 }
 __global__ void cand_hist_kernel(const Cand* cand, const float* e, int64_t n, const float* b0, float b1,
                                  unsigned int* hist) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float x = e[i];
     const int32_t g = cand[i].g;
-    if (x == x) atomicAdd(&hist[(int64_t)g * kCandBins + cand_bin(x, b0, g, b1)], 1u);
+    if (x == x) atomicAdd(&hist[(int64_t)g * kCandBins + cand_bin(x, sure_clip(b0[g], b1))], 1u);
   }
 }
 
@@ -310,12 +309,14 @@ constexpr int kSmemHistGenes = 12;  // 192 KB
 __global__ void __launch_bounds__(1024) cand_hist_smem_kernel(const Cand* cand, const float* e, int64_t n, int G,
                                                               const float* b0, float b1, unsigned int* hist) {
   extern __shared__ unsigned int sh[];  // G x kCandBins
+  __shared__ float sure[kSmemHistGenes];
+  if (threadIdx.x < G) sure[threadIdx.x] = sure_clip(b0[threadIdx.x], b1);
   for (int b = threadIdx.x; b < G * kCandBins; b += blockDim.x) sh[b] = 0u;
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float x = e[i];
     const int32_t g = cand[i].g;
-    if (x == x) atomicAdd(&sh[g * kCandBins + cand_bin(x, b0, g, b1)], 1u);
+    if (x == x) atomicAdd(&sh[g * kCandBins + cand_bin(x, sure[g])], 1u);
   }
   __syncthreads();
   for (int b = threadIdx.x; b < G * kCandBins; b += blockDim.x)
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(1024) cand_hist_smem_kernel(const Cand* cand, 
 // pairs so instead of 8 x 10^6 (2.4 ms for the selection, 113 before).
 __global__ void __launch_bounds__(256) refine_kernel(const unsigned int* hist, int64_t P, int64_t G, int64_t k,
                                                      const float* X, const float* b0, float b1, float* Xt,
-                                                     int* p_end) {
+                                                     float2* cut) {
   __shared__ unsigned int csum[256];
   const int64_t g = blockIdx.x;
   const int found = hist_find(hist + g * kCandBins, k, csum);
@@ -360,26 +361,27 @@ __global__ void __launch_bounds__(256) refine_kernel(const unsigned int* hist, i
       const int64_t cand = c + hist[g * kCandBins + kHistBins];
       end = min(P, k + (P - cand) + c);
     }
-    p_end[g] = (int)min(end, (int64_t)INT32_MAX);
+    cut[g] = make_float2(sure_clip(b0[g], b1), __int_as_float((int)min(end, (int64_t)INT32_MAX)));
   }
 }
 
 // Keep candidates with e <= Xt[g] (e clipped at 10, as the error is) that are not
-// surely clipped or have an index below p_end[g].  A block takes 4 x 256 candidates per
+// surely clipped or have an index below p_end[g] (cut[g]: the bound of sure
+// clipping and p_end; looked at only where Xt lets clipped ones pass).  A block takes 4 x 256 candidates per
 // iteration and appends its kept ones with one global atomic (positions from
 // the warps' ballots), so the shared output counter sees one atomic per 1,024
 // candidates instead of one per warp.
 constexpr int kFilterItems = 4;
 __global__ void __launch_bounds__(256) cand_filter_kernel(const Cand* cand, const float* e, int64_t n, const float* Xt,
-                                                          const int* p_end, const float* b0, float b1, Cand* out,
-                                                          unsigned long long* count) {
+                                                          const float2* cut, Cand* out, unsigned long long* count) {
   __shared__ unsigned int wc[kFilterItems * 8];
   __shared__ unsigned long long base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t per = (int64_t)kFilterItems * blockDim.x;
   for (int64_t i0 = (int64_t)blockIdx.x * per; i0 < n; i0 += (int64_t)gridDim.x * per) {
-    bool keep[kFilterItems];
+    bool keep[kFilterItems], tie = false;
     Cand cd[kFilterItems];
+    float x[kFilterItems];
     unsigned m[kFilterItems];
 #pragma unroll
     for (int j = 0; j < kFilterItems; ++j) {
@@ -387,12 +389,22 @@ __global__ void __launch_bounds__(256) cand_filter_kernel(const Cand* cand, cons
       keep[j] = false;
       if (i < n) {
         cd[j] = cand[i];
-        const float x = e[i];
-        if (x > 10.0f)
-          keep[j] = Xt[cd[j].g] >= 10.0f && (cd[j].p < p_end[cd[j].g] || !surely_clipped(x, b0[cd[j].g], b1));
-        else
-          keep[j] = x <= Xt[cd[j].g];
+        x[j] = e[i];
+        keep[j] = (x[j] > 10.0f ? 10.0f : x[j]) <= Xt[cd[j].g];
+        tie = tie || (keep[j] && x[j] > 10.0f);
       }
+    }
+    if (tie) {
+#pragma unroll
+      for (int j = 0; j < kFilterItems; ++j) {
+        if (keep[j] && x[j] > 10.0f) {
+          const float2 c = cut[cd[j].g];
+          keep[j] = !surely_clipped(x[j], c.x) || cd[j].p < __float_as_int(c.y);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kFilterItems; ++j) {
       m[j] = __ballot_sync(0xffffffffu, keep[j]);
       if (lane == 0) wc[j * 8 + warp] = __popc(m[j]);
     }
@@ -427,7 +439,7 @@ cudaError_t launch_scatter_errors(const Cand* cand, const float* e, int64_t n, i
 }
 
 cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int64_t P, int64_t G, int64_t k,
-                          const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, int* p_end,
+                          const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, float2* cut,
                           Cand* out, unsigned long long* count, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(unsigned int) * (size_t)G * kCandBins, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, sizeof(unsigned long long), s);
@@ -444,8 +456,8 @@ cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int6
   } else if (n > 0) {
     cand_hist_kernel<<<blocks, 256, 0, s>>>(cand, cand_e, n, b0, b1, hist);
   }
-  refine_kernel<<<(unsigned)G, 256, 0, s>>>(hist, P, G, k, X, b0, b1, Xt, p_end);
-  if (n > 0) cand_filter_kernel<<<blocks, 256, 0, s>>>(cand, cand_e, n, Xt, p_end, b0, b1, out, count);
+  refine_kernel<<<(unsigned)G, 256, 0, s>>>(hist, P, G, k, X, b0, b1, Xt, cut);
+  if (n > 0) cand_filter_kernel<<<blocks, 256, 0, s>>>(cand, cand_e, n, Xt, cut, out, count);
   return cudaGetLastError();
 }
 

@@ -646,7 +646,7 @@ __device__ __forceinline__ bool sort_key_less(double ea, int32_t pa, double eb, 
   return key_less(ea, pa, eb, pb);
 }
 
-constexpr int kSortThreads = 512, kSortCap = 8192, kSortBins = 4096, kSortDirect = 512, kBinMax = 512;
+constexpr int kSortThreads = 512, kSortCap = 8192, kSortBins = 4096, kSortDirect = 256, kBinMax = 512;
 constexpr int kValueBins = 3072;
 constexpr uint64_t kClipKey = 0x4024000000000000ull;  // 10.0
 constexpr int kSortSmem = kSortCap * (int)(sizeof(uint64_t) + sizeof(int32_t)) + kSortBins * (int)sizeof(int);
@@ -973,8 +973,10 @@ __global__ void accept_len_kernel(const int64_t* goff, const double* se64, int64
   const double eps = eps_g ? eps_g[g] : eps_all;
   const double* E = se64 + goff[g];
   const int64_t n = goff[g + 1] - goff[g];
-  // number of finite (non-NaN) entries: NaN sorts last
+  // number of finite (non-NaN) entries: NaN sorts last, and most lists have none
+  // (a search of its own doubled the chain of dependent reads: 6.7 us for 4 genes)
   int64_t lo = 0, hi = n;
+  if (n > 0 && E[n - 1] == E[n - 1]) lo = n;
   while (lo < hi) {
     int64_t mid = (lo + hi) >> 1;
     if (E[mid] == E[mid]) lo = mid + 1; else hi = mid;

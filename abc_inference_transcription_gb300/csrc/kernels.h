@@ -133,10 +133,10 @@ cudaError_t launch_x_from_thr(const double* thr, double eps, int64_t G, const fl
 // top-k refinement before the FP64 recheck: per-gene histogram of the
 // candidates' FP32 errors (hist: G x (kHistBins + 1)), a tighter Xt <= X from the
 // bin completing k, and the candidates with e <= Xt appended to out (count in
-// *count).  Of those surely at the clip value only the ones below p_end[g] (of P
+// *count; cut: scratch, G).  Of those surely at the clip value only the ones below p_end[g] (of P
 // particles) are kept: enough for any k smallest, as ties are ordered by index.
 cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int64_t P, int64_t G, int64_t k,
-                          const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, int* p_end,
+                          const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, float2* cut,
                           Cand* out, unsigned long long* count, cudaStream_t s);
 // den[g][k] = (se^2 + 0.01 d^2) + eps_gk, the denominators of the error terms,
 // evaluated as in the per-term FP64 expression (bit-identical), and rden = 1/den

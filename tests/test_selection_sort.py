@@ -1,5 +1,5 @@
 """The per-gene sort at the list lengths where its path changes: counting over
-the whole list up to 512 entries, one window of bins up to 8,192, several
+the whole list up to 256 entries, one window of bins up to 8,192, several
 windows above; the bitonic networks for crowded bins (one far entry, or exact
 ties); ties at the clip value, binned by index.  eps = 10 accepts every
 particle, so that a list is as long as the particles are many."""
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape", ["spread", "crowded", "ties", "clipped", "all clipped"])
-@pytest.mark.parametrize("n", [1, 2, 33, 511, 512, 513, 4097, 8191, 8192, 8193, 16385, 40001])
+@pytest.mark.parametrize("n", [1, 2, 33, 255, 256, 257, 511, 512, 513, 4097, 8191, 8192, 8193, 16385, 40001])
 def test_lists_of_every_length(built, orc, n, shape):
     from abc_inference_transcription_gb300.host import Context
 
