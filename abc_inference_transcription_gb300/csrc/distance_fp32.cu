@@ -381,7 +381,6 @@ __global__ void __launch_bounds__(256) cand_filter_kernel(const Cand* cand, cons
   for (int64_t i0 = (int64_t)blockIdx.x * per; i0 < n; i0 += (int64_t)gridDim.x * per) {
     bool keep[kFilterItems], tie = false;
     Cand cd[kFilterItems];
-    float x[kFilterItems];
     unsigned m[kFilterItems];
 #pragma unroll
     for (int j = 0; j < kFilterItems; ++j) {
@@ -389,17 +388,19 @@ __global__ void __launch_bounds__(256) cand_filter_kernel(const Cand* cand, cons
       keep[j] = false;
       if (i < n) {
         cd[j] = cand[i];
-        x[j] = e[i];
-        keep[j] = (x[j] > 10.0f ? 10.0f : x[j]) <= Xt[cd[j].g];
-        tie = tie || (keep[j] && x[j] > 10.0f);
+        const float x = e[i], xt = Xt[cd[j].g];
+        const bool clip = x > 10.0f && xt >= 10.0f;
+        keep[j] = x <= xt || clip;
+        tie = tie || clip;
       }
     }
     if (tie) {
 #pragma unroll
       for (int j = 0; j < kFilterItems; ++j) {
-        if (keep[j] && x[j] > 10.0f) {
+        if (keep[j]) {
+          const float x = e[i0 + (int64_t)j * blockDim.x + threadIdx.x];
           const float2 c = cut[cd[j].g];
-          keep[j] = !surely_clipped(x[j], c.x) || cd[j].p < __float_as_int(c.y);
+          keep[j] = !surely_clipped(x, c.x) || cd[j].p < __float_as_int(c.y);
         }
       }
     }

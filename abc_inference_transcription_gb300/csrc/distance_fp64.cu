@@ -261,18 +261,21 @@ __global__ void ff_prep_genes_kernel(DistInputs in, float4* gt) {
 // recheck_grouped_kernel.  v[i] = the certified FP32 error (10 exactly when
 // it lies above 10 by more than its bound); pairs outside the derivation's
 // range get their position appended to pos (FP64 later).
-__global__ void __launch_bounds__(kRecheckWarps * 32) approx_grouped_kernel(DistInputs in, const int32_t* sp,
+// Blocks of four warps: a warp's share of shared memory is free again sooner (2.01 ms
+// for 10.9 million pairs of 72 statistics, 2.13 in blocks of eight).
+constexpr int kApproxWarps = 4;
+__global__ void __launch_bounds__(kApproxWarps * 32) approx_grouped_kernel(DistInputs in, const int32_t* sp,
                                                                             const int32_t* sg, int64_t n,
                                                                             const float4* gt, float rK, double* v,
                                                                             int32_t* pos,
                                                                             unsigned long long* count) {
-  __shared__ double rs_smem[kRecheckWarps * 32 * kRecheckLd];
+  __shared__ double rs_smem[kApproxWarps * 32 * kRecheckLd];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int K = in.K;
   double* S = rs_smem + warp * 32 * kRecheckLd;
   const int64_t n_chunks = (n + 31) >> 5;
-  const int64_t wstride = (int64_t)gridDim.x * kRecheckWarps;
-  for (int64_t ch = (int64_t)blockIdx.x * kRecheckWarps + warp; ch < n_chunks; ch += wstride) {
+  const int64_t wstride = (int64_t)gridDim.x * kApproxWarps;
+  for (int64_t ch = (int64_t)blockIdx.x * kApproxWarps + warp; ch < n_chunks; ch += wstride) {
     const int64_t i = ch * 32 + lane;
     const bool mine = i < n;
     const int32_t p = mine ? sp[i] : 0;
@@ -908,10 +911,10 @@ static cudaError_t launch_segsort(const int64_t* goff, int64_t G, int32_t* sp, d
   return cudaGetLastError();
 }
 
-static int grouped_blocks(int64_t n) {
+static int grouped_blocks(int64_t n, int warps) {
   const int64_t chunks = (n + 31) / 32;
-  const int64_t want = (chunks + kRecheckWarps - 1) / kRecheckWarps;
-  return (int)(want < 65536 ? want : 65536);
+  const int64_t want = (chunks + warps - 1) / warps;
+  return (int)(want < 131072 ? want : 131072);
 }
 
 static void launch_recheck_grouped(const DistInputs& in, const int32_t* sp, const int32_t* sg, int64_t n, double* se64,
@@ -920,7 +923,7 @@ static void launch_recheck_grouped(const DistInputs& in, const int32_t* sp, cons
   if (chunks <= 4 * 152)  // at most a warp per scheduler
     recheck_grouped_kernel<1><<<(unsigned)chunks, 32, 0, s>>>(in, sp, sg, n, se64);
   else
-    recheck_grouped_kernel<kRecheckWarps><<<grouped_blocks(n), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, se64);
+    recheck_grouped_kernel<kRecheckWarps><<<grouped_blocks(n, kRecheckWarps), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, se64);
 }
 
 cudaError_t launch_dist_group_recheck_sort(const DistInputs& in, Cand* cand, float* cand_e, int64_t n, int64_t* gcount,
@@ -947,8 +950,8 @@ cudaError_t launch_dist_group_certify_sort(const DistInputs& in, Cand* cand, flo
   const int64_t gk = in.G * in.K;
   ff_prep_genes_kernel<<<(unsigned)((gk + 255) / 256 < 4096 ? (gk + 255) / 256 : 4096), 256, 0, s>>>(in, gt);
   const float rK = (float)(1.0 / (double)in.K);
-  approx_grouped_kernel<<<grouped_blocks(n), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, gt, rK, se64, pos,
-                                                                         counts);
+  approx_grouped_kernel<<<grouped_blocks(n, kApproxWarps), kApproxWarps * 32, 0, s>>>(in, sp, sg, n, gt, rK, se64, pos,
+                                                                                     counts);
   const int list_blocks = 152 * 8;
   recheck_list_kernel<<<list_blocks, 128, 0, s>>>(in, sp, sg, pos, counts, se64);
   err = launch_segsort(goff, in.G, sp, se64, nullptr, cand, cand_e, s);
