@@ -1492,11 +1492,12 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   const size_t o_scr = w.add(scratch);
   const size_t o_mom = w.add(moments_out ? sizeof(double) * (size_t)P * J * A * 5 : 0);
   const size_t o_it = w.add(iters_out ? sizeof(int) * (size_t)P : 0);
+  const size_t o_status = w.add(sizeof(int));  // d_status belongs to the simulations until abc_synchronize reads it
   CK(w.allocate(c));
   CK(cudaMemcpyAsync(w.at<double>(o_theta), theta, sizeof(double) * P * npar, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(w.at<double>(o_bm), beta_mom, sizeof(double) * 2 * A * 3, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(w.at<double>(o_ad), age_dist, sizeof(double) * A * J, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemsetAsync(c->d_status.p, 0, sizeof(int), c->stream));
+  CK(cudaMemsetAsync(w.at<int>(o_status), 0, sizeof(int), c->stream));
   a.theta = w.at<double>(o_theta);
   a.beta_mom = w.at<double>(o_bm);
   a.age_dist = w.at<double>(o_ad);
@@ -1504,7 +1505,7 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
   a.moments = moments_out ? w.at<double>(o_mom) : nullptr;
   a.iters = iters_out ? w.at<int>(o_it) : nullptr;
   a.scratch = w.at<double>(o_scr);
-  a.status = c->d_status.p;
+  a.status = w.at<int>(o_status);
   if (c->prof && !c->sel_ev[0]) {
     CK(cudaEventCreate(&c->sel_ev[0]));
     CK(cudaEventCreate(&c->sel_ev[1]));
@@ -1519,7 +1520,7 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
     CK(cudaMemcpyAsync(moments_out, a.moments, sizeof(double) * P * J * A * 5, cudaMemcpyDeviceToHost, c->stream));
   if (iters_out) CK(cudaMemcpyAsync(iters_out, a.iters, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
   int hst = 0;
-  CK(cudaMemcpyAsync(&hst, c->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(&hst, a.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (c->prof) {
     float ms = 0.0f;
@@ -1548,6 +1549,7 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   const size_t o_out = w.add(sizeof(double) * (size_t)G * (n_boot + 1) * K);
   const size_t o_se = w.add(se_out ? sizeof(double) * (size_t)G * K : 0);
   const size_t o_sums = w.add(data_stats_scratch(c->dcfg, G, n_boot, C));
+  const size_t o_invalid = w.add(sizeof(int));  // not d_status, which belongs to the simulations
   CK(w.allocate(c));
   double* dout = w.at<double>(o_out);
   double* dse = se_out ? w.at<double>(o_se) : nullptr;
@@ -1568,7 +1570,7 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   a.seed = seed;
   a.out = dout;
   a.sums = w.at<unsigned long long>(o_sums);
-  a.invalid = c->d_status.p;
+  a.invalid = w.at<int>(o_invalid);
   if (c->prof && !c->sel_ev[0]) {
     CK(cudaEventCreate(&c->sel_ev[0]));
     CK(cudaEventCreate(&c->sel_ev[1]));
@@ -1581,7 +1583,7 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   // the counts are checked where they are read (a pass over them on the host
   // took a millisecond per 10^7): nothing is returned for invalid ones
   int invalid = 0;
-  CK(cudaMemcpyAsync(&invalid, c->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(&invalid, a.invalid, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (invalid) {
     trim_work(c);
