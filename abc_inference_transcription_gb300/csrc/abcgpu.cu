@@ -969,12 +969,15 @@ static int prof_end(abc_ctx* c) {
 
 // The arrays named by abc_select_output, made present behind the candidate pass:
 // the longest wait of a selection.
-static void present_outputs(abc_ctx* c) {
-  make_present(c->out_idx, sizeof(int64_t) * c->out_cap);
-  make_present(c->out_err, sizeof(double) * c->out_cap);
+static void forget_outputs(abc_ctx* c) {
   c->out_idx = nullptr;
   c->out_err = nullptr;
   c->out_cap = 0;
+}
+static void present_outputs(abc_ctx* c) {
+  make_present(c->out_idx, sizeof(int64_t) * c->out_cap);
+  make_present(c->out_err, sizeof(double) * c->out_cap);
+  forget_outputs(c);
 }
 
 // FP32 candidate pass on the CUDA cores; candidates and their FP32 errors in
@@ -1155,11 +1158,7 @@ static int select_impl(abc_ctx* c, const double* data, const double* se, int64_t
                        double eps_or_q, const double* thr, int64_t* n_accepted_total) {
   const int st = select_run(c, data, se, G, K, n_fam, fam, stats, stats_on_device, P, mode, eps_or_q, thr,
                             n_accepted_total);
-  if (c) {
-    c->out_idx = nullptr;
-    c->out_err = nullptr;
-    c->out_cap = 0;
-  }
+  if (c) forget_outputs(c);
   return st;
 }
 
@@ -1332,7 +1331,10 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
 int abc_errors_select(abc_ctx* c, const double* data, const double* se, int64_t G, int K, int n_fam,
                       const int32_t* fam, const double* stats, int64_t P, int mode, double eps_or_q,
                       int64_t* n_accepted_total) {
-  if (mode == 2) return fail(c, ABC_ERR_INVALID, "per-gene thresholds: use abc_errors_select_thr");
+  if (mode == 2) {
+    if (c) forget_outputs(c);
+    return fail(c, ABC_ERR_INVALID, "per-gene thresholds: use abc_errors_select_thr");
+  }
   return select_impl(c, data, se, G, K, n_fam, fam, stats, false, P, mode, eps_or_q, nullptr, n_accepted_total);
 }
 
