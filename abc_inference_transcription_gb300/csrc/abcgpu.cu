@@ -1238,6 +1238,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
     if (st) return st;
   }
   int64_t total = 0;
+  std::vector<float> hX;  // widened thresholds: outlives the copy from it, which the next pass's wait ends
   c->sel_rechecked = 0;
   c->sel_cands_emitted = 0;
   for (int round = 0; round < 4; ++round) {
@@ -1305,7 +1306,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
     if (round == 3) return fail(c, ABC_ERR_CAPACITY, "top-q selection did not converge");
     // the genes whose threshold was too narrow
     std::vector<int> hf((size_t)G);
-    std::vector<float> hX((size_t)G);
+    hX.resize((size_t)G);
     CK(cudaMemcpyAsync(hf.data(), c->d_fail.p + 1, sizeof(int) * G, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(hX.data(), c->d_X.p, sizeof(float) * G, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
