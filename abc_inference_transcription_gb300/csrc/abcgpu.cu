@@ -150,16 +150,27 @@ static int cuda_fail(abc_ctx* c, cudaError_t e, const char* where) {
               std::string(where) + ": " + cudaGetErrorString(e));
 }
 
-// Layout of a call's workspace: add() each piece, allocate() once, then at().
+// Layout of a call's workspace: add() each piece, allocate() once, then at().  At the
+// end of the call, on whichever path, a buffer above kKeepWork is given back.
 struct Work {
   size_t total = 0;
   uint8_t* base = nullptr;
+  abc_ctx* ctx = nullptr;
+  Work() = default;
+  Work(const Work&) = delete;
+  Work& operator=(const Work&) = delete;
+  ~Work() {
+    if (!ctx || ctx->d_work.cap <= kKeepWork) return;
+    cudaStreamSynchronize(ctx->stream);  // a call that fails may leave work on the stream
+    ctx->d_work.release();
+  }
   size_t add(size_t bytes) {
     const size_t off = total;
     total += (bytes + 255) & ~size_t(255);
     return off;
   }
   cudaError_t allocate(abc_ctx* c) {
+    ctx = c;
     const cudaError_t e = c->d_work.ensure(total);
     base = c->d_work.p;
     return e;
@@ -169,11 +180,6 @@ struct Work {
     return reinterpret_cast<T*>(base + off);
   }
 };
-
-// at the end of the call, after its stream has been waited for
-static void trim_work(abc_ctx* c) {
-  if (c->d_work.cap > kKeepWork) c->d_work.release();
-}
 
 #define CK(call)                                   \
   do {                                             \
@@ -941,7 +947,6 @@ int abc_errors(abc_ctx* c, const double* data, const double* se, int64_t G, int 
   make_present(err_out, sizeof(double) * P * G);
   CK(cudaMemcpyAsync(err_out, w.at<double>(o_out), sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  trim_work(c);
   return ABC_OK;
 }
 
@@ -1531,7 +1536,6 @@ int abc_moment_simulate(abc_ctx* c, int model, const double* theta, int64_t P, c
     c->sel_fast_ms = ms;
     c->sel_fast_passes = 1;
   }
-  trim_work(c);
   if (hst) return fail(c, ABC_ERR_NONFINITE, "abc_moment_simulate: non-finite rates for some particles (NaN rows)");
   return ABC_OK;
 }
@@ -1588,10 +1592,7 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   int invalid = 0;
   CK(cudaMemcpyAsync(&invalid, a.invalid, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (invalid) {
-    trim_work(c);
-    return fail(c, ABC_ERR_INVALID, "abc_data_stats: counts must lie in [0, 2^20]");
-  }
+  if (invalid) return fail(c, ABC_ERR_INVALID, "abc_data_stats: counts must lie in [0, 2^20]");
   // the estimate is resample 0 of each gene
   CK(cudaMemcpy2DAsync(stats_out, sizeof(double) * K, dout, sizeof(double) * K * (n_boot + 1), sizeof(double) * K,
                        (size_t)G, cudaMemcpyDeviceToHost, c->stream));
@@ -1603,7 +1604,6 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
     c->sel_fast_ms = ms;
     c->sel_fast_passes = 1;
   }
-  trim_work(c);
   return ABC_OK;
 }
 
@@ -1629,7 +1629,6 @@ int abc_model_probs(abc_ctx* c, const int64_t* counts, int64_t G, int M, int n_b
   CK(cudaMemcpyAsync(lb, out + n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(ub, out + 2 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  trim_work(c);
   return ABC_OK;
 }
 
@@ -1660,7 +1659,6 @@ int abc_posterior_summary(abc_ctx* c, const double* theta, int64_t ld, int npar,
   if (n_particles)
     CK(cudaMemcpyAsync(n_particles, w.at<int64_t>(o_n), sizeof(int64_t) * G, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  trim_work(c);
   return ABC_OK;
 }
 
