@@ -18,11 +18,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "distance.cuh"
 #include "kernels.h"
 #include "model.cuh"
+#include "smem_attr.h"
 
 namespace abc {
 namespace {
@@ -412,15 +414,14 @@ cudaError_t launch_data_stats(const DataStatsArgs& a, double* se, cudaStream_t s
   const bool copy = smem + (size_t)a.C * sizeof(int2) <= data_stats_smem_limit();
   if (copy) smem += (size_t)a.C * sizeof(int2);
   if (smem > data_stats_smem_limit()) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(data_phases_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<uint64_t> attr{0};  // the largest size sets the limit once per device, for all contexts
+  cudaError_t e = set_smem_once(attr, data_phases_kernel, (int)data_stats_smem_limit());
+  if (e != cudaSuccess) return e;
   int64_t per_gene = 0;
   const int64_t chunk = genes_at_a_time(a.cfg, a.G, a.n_boot, &per_gene);
   unsigned long long* S = a.sums;
   SizeTerms* terms = reinterpret_cast<SizeTerms*>(reinterpret_cast<char*>(S) + 2 * chunk * per_gene);
-  cudaError_t e = cudaMemsetAsync(a.invalid, 0, sizeof(int), s);
+  e = cudaMemsetAsync(a.invalid, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   DrawKeys keys;
   for (int r = 0; r < 10; ++r) {  // Weyl sequences of the Philox key
