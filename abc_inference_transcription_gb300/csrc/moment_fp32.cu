@@ -428,9 +428,8 @@ __global__ void __launch_bounds__(32) moment_path_kernel(MomArgs a, MomScratch w
     for (int r = 0; r < NA; ++r) y[e][r] = live[e] ? ws.start[((int64_t)(slot + e) * n + i) * NA + r] : 0.0f;
   }
   // substeps s0 .. s1 of the warp; the unlabelled propagators serve from un on, the labelled ones up to la
-  const int s0 = (int)__reduce_min_sync(0xffffffffu, first), s1 = (int)__reduce_max_sync(0xffffffffu, last);
-  // without a valid particle in the warp s0 is the largest int and s0 + t no substep: nothing is fetched
-  const bool walk = s0 < s1;
+  // (without a valid particle in the warp `first` is the largest int, beyond which nothing may be counted: s0 = s1 = 0)
+  const int s1 = (int)__reduce_max_sync(0xffffffffu, last), s0 = min((int)__reduce_min_sync(0xffffffffu, first), s1);
   un = __reduce_min_sync(0xffffffffu, un);
   la = __reduce_max_sync(0xffffffffu, la);
   const int64_t src0 = lane / kPathParticles * n + min(i, n - 1);
@@ -447,7 +446,7 @@ __global__ void __launch_bounds__(32) moment_path_kernel(MomArgs a, MomScratch w
     cp_async_commit();
   };
   int idx = s0 % nsub, ahead = idx;
-  for (int t = 0; walk && t < kPathStages - 1; ++t) {
+  for (int t = 0; t < kPathStages - 1; ++t) {
     fetch(s0 + t, ahead);
     if (++ahead == nsub) ahead = 0;
   }
