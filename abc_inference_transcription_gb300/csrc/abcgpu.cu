@@ -943,7 +943,7 @@ int abc_errors(abc_ctx* c, const double* data, const double* se, int64_t G, int 
   Work w;
   const size_t o_out = w.add(sizeof(double) * (size_t)P * G);
   CK(w.allocate(c));
-  CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, w.at<double>(o_out), c->stream));
+  CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, c->sms, w.at<double>(o_out), c->stream));
   make_present(err_out, sizeof(double) * P * G);
   CK(cudaMemcpyAsync(err_out, w.at<double>(o_out), sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

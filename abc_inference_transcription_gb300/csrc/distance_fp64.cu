@@ -420,33 +420,38 @@ __global__ void run_sort_kernel(const int32_t* sg, const int64_t* goff, const ui
 }
 
 // Full error matrix.  Errors are clipped at 10, and of a matrix over prior
-// draws most are: a block first evaluates its kFullRows x kFullTile pairs in
+// draws most are: a block first evaluates its ROWS x cols pairs in
 // FP32 (two FMAs per term, as dist_fast_kernel) and writes 10 where that is
 // certain; only the other pairs are computed in FP64, whose narrow pipe took
 // the whole 0.97 ms for 3,001 x 500 pairs of 53 statistics (0.08 with 0.4 %
-// of them below the clip; with all of them below it, as before).  32 particles
-// per block, so that such an input still fills the GPU evenly.
+// of them below the clip; with all of them below it, as before).  Particles and
+// genes per block: launch_dist_full.
 // Certain: K e32 > K sure.  With finite operands |e32 - e| <= B(e) =
 // 1.5 u (64 sqrt(e) + (K + 8) e) (distance.cuh), so e <= 10 implies e32 <= 10 + B(10), and
 // sure is 10 + 2 B(10).  An operand that is not finite in FP32 becomes
 // NaN, which no comparison holds for, so its pairs are computed in FP64.
-constexpr int kFullTile = 64, kFullRows = 32, kFullKc = 16;  // genes, particles, statistics
+constexpr int kFullRows = 32, kFullTile = 64, kFullKc = 16;  // particles and genes at most, statistics
 __device__ __forceinline__ float finite_or_nan(float x) { return fabsf(x) < INFINITY ? x : __int_as_float(0x7fc00000); }
 
+template <int ROWS>
 __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const float* __restrict__ sw,
-                                                        const float* __restrict__ dw, float sure, double* err) {
-  __shared__ float ss[kFullKc][kFullRows + 1], sa[kFullKc][kFullTile + 1], sd[kFullKc][kFullTile + 1];
-  __shared__ unsigned short todo[kFullRows * kFullTile];
+                                                        const float* __restrict__ dw, float sure, int even, double* err) {
+  const int cols = ROWS == kFullRows ? kFullTile : even;  // genes per tile
+  // threads: TY particles x TX genes, RI x GJ pairs each
+  constexpr int TY = ROWS < 16 ? ROWS : 16, TX = 256 / TY, RI = ROWS / TY, GJ = kFullTile / TX;
+  static_assert(ROWS <= kFullTile && TX <= kFullTile, "the tile's pairs fall to 256 threads");
+  __shared__ float ss[kFullKc][ROWS + 1], sa[kFullKc][kFullTile + 1], sd[kFullKc][kFullTile + 1];
+  __shared__ unsigned short todo[ROWS * kFullTile];
   __shared__ int n_todo;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31;
-  const int64_t g0 = (int64_t)blockIdx.x * kFullTile;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX, lane = threadIdx.x & 31;
+  const int64_t g0 = (int64_t)blockIdx.x * cols;
   if (threadIdx.x == 0) n_todo = 0;
-  for (int64_t p0 = (int64_t)blockIdx.y * kFullRows; p0 < in.P; p0 += (int64_t)gridDim.y * kFullRows) {
-    float acc[2][4];
+  for (int64_t p0 = (int64_t)blockIdx.y * ROWS; p0 < in.P; p0 += (int64_t)gridDim.y * ROWS) {
+    float acc[RI][GJ];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+      for (int j = 0; j < GJ; ++j) acc[i][j] = 0.0f;
     for (int k0 = 0; k0 < in.K; k0 += kFullKc) {
       __syncthreads();
       for (int q = threadIdx.x; q < kFullKc * kFullTile; q += 256) {
@@ -454,31 +459,31 @@ __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const flo
         const int64_t p = p0 + r, g = g0 + r;
         float s = 0.0f, a = 0.0f, d = 0.0f;
         if (k < in.K) {
-          if (r < kFullRows && p < in.P) s = finite_or_nan(rn32_bits(in.stats[p * in.K + k]));
+          if (r < ROWS && p < in.P) s = finite_or_nan(rn32_bits(in.stats[p * in.K + k]));
           if (g < in.G) {
             a = finite_or_nan(sw[g * in.K + k]);
             d = finite_or_nan(dw[g * in.K + k]);
           }
         }
-        if (r < kFullRows) ss[kk][r] = s;
+        if (r < ROWS) ss[kk][r] = s;
         sa[kk][r] = a;
         sd[kk][r] = d;
       }
       __syncthreads();
 #pragma unroll 4
       for (int kk = 0; kk < kFullKc; ++kk) {
-        float s[2], a[4], d[4];
+        float s[RI], a[GJ], d[GJ];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) s[i] = ss[kk][ty + 16 * i];
+        for (int i = 0; i < RI; ++i) s[i] = ss[kk][ty + TY * i];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          a[i] = sa[kk][tx + 16 * i];
-          d[i] = sd[kk][tx + 16 * i];
+        for (int j = 0; j < GJ; ++j) {
+          a[j] = sa[kk][tx + TX * j];
+          d[j] = sd[kk][tx + TX * j];
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < RI; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < GJ; ++j) {
             const float t = fmaf(-a[j], s[i], d[j]);
             acc[i][j] = fmaf(t, t, acc[i][j]);
           }
@@ -486,11 +491,11 @@ __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const flo
     }
     const float limit = sure * (float)in.K;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = ty + 16 * i, c = tx + 16 * j;
-        const bool real = p0 + r < in.P && g0 + c < in.G;
+      for (int j = 0; j < GJ; ++j) {
+        const int r = ty + TY * i, c = tx + TX * j;
+        const bool real = p0 + r < in.P && c < cols && g0 + c < in.G;
         const bool clip = acc[i][j] > limit;
         if (real && clip) err[(p0 + r) * in.G + g0 + c] = 10.0;
         const unsigned m = __ballot_sync(0xffffffffu, real && !clip);
@@ -510,13 +515,37 @@ __global__ void __launch_bounds__(256) dist_full_kernel(DistInputs in, const flo
   }
 }
 
-cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, double* err, cudaStream_t s) {
-  if (in.P <= 0 || in.G <= 0) return cudaSuccess;
+template <int ROWS>
+static cudaError_t launch_full(const DistInputs& in, const float* sw, const float* dw, int64_t tiles, double* err,
+                               cudaStream_t s) {
   const float sure = 10.0f + 2.0f * dist_bound_f(10.0f, in.K);
-  const int64_t py = (in.P + kFullRows - 1) / kFullRows;
-  dim3 grid((unsigned)((in.G + kFullTile - 1) / kFullTile), (unsigned)(py < 65535 ? py : 65535));
-  dist_full_kernel<<<grid, 256, 0, s>>>(in, sw, dw, sure, err);
+  const int64_t py = (in.P + ROWS - 1) / ROWS;
+  dim3 grid((unsigned)tiles, (unsigned)(py < 65535 ? py : 65535));
+  dist_full_kernel<ROWS><<<grid, 256, 0, s>>>(in, sw, dw, sure, (int)((in.G + tiles - 1) / tiles), err);
   return cudaGetLastError();
+}
+
+// 32 particles per tile read the genes' terms least often, but where few pairs are
+// clipped a thread computes eight of them one after the other, and with few blocks that
+// chain is the call: the most particles are taken for which every multiprocessor still
+// gets two blocks, and below 32 the genes are split evenly over the tiles.
+// Milliseconds of the whole call, 53 statistics, few pairs below the clip / all:
+//                a thread per pair   32 particles    by this rule
+//   64 x 64         0.088 / 0.088    0.055 / 0.277   0.045 / 0.080
+//   500 x 50        0.092 / 0.091    0.057 / 0.241   0.057 / 0.081
+//   700 x 100       0.120 / 0.120    0.073 / 0.308   0.073 / 0.134
+//   500 x 300       0.193 / 0.192    0.083 / 0.318   0.084 / 0.211
+//   200 x 2,000     0.561 / 0.562    0.114 / 0.483   0.112 / 0.387
+//   2,000 x 300     0.714 / 0.715    0.111 / 0.659   32 particles
+cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, int sms, double* err,
+                             cudaStream_t s) {
+  if (in.P <= 0 || in.G <= 0) return cudaSuccess;
+  const int64_t tiles = (in.G + kFullTile - 1) / kFullTile;
+  auto fills = [&](int rows) { return (in.P + rows - 1) / rows * tiles >= 2 * (int64_t)sms; };
+  if (fills(kFullRows)) return launch_full<kFullRows>(in, sw, dw, tiles, err, s);
+  if (fills(16)) return launch_full<16>(in, sw, dw, tiles, err, s);
+  if (fills(8)) return launch_full<8>(in, sw, dw, tiles, err, s);
+  return launch_full<4>(in, sw, dw, tiles, err, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -173,8 +173,9 @@ cudaError_t launch_scan(const int64_t* cnt, int64_t G, int64_t* off, cudaStream_
 // in.rden.  sp, sg: n scratch entries each.
 cudaError_t launch_accepted_errors(const DistInputs& in, const int64_t* aoff, const int64_t* idx, int64_t G,
                                    int64_t p_base, int64_t n, int32_t* sp, int32_t* sg, double* err, cudaStream_t s);
-// full FP64 error matrix [P][G]; sw, dw: G x K scratch values each
-cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, double* err, cudaStream_t s);
+// full FP64 error matrix [P][G]; sw, dw: the terms of launch_dist_den; sms: the device's multiprocessors
+cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, int sms, double* err,
+                             cudaStream_t s);
 
 // moment ODE (moment.cu)
 struct MomArgs {
