@@ -500,6 +500,7 @@ static int enqueue_simulate(abc_ctx* c, int model, const int32_t* d_models, cons
     sa.status = c->d_status.p;
     sa.fp32 = fp64 ? 0 : 1;
     CK(prof_mark(c));
+    sa.sms = c->sms;
     CK(launch_setup(sa, c->stream));
     CK(launch_work_order(c->d_rec.p, n, c->d_ohist.p, c->d_order.p, C, c->sms, std::max(1, bps), c->stream));
     SsaArgs ss;
@@ -554,6 +555,7 @@ static int enqueue_simulate(abc_ctx* c, int model, const int32_t* d_models, cons
     st.fp32 = fp64 ? 0 : 1;
     st.beta32 = c->d_beta32.p;
     st.max_group_cells = c->max_group_cells;
+    st.sms = c->sms;
     CK(launch_stats(st, c->stream));
     CK(prof_mark(c));
   }
@@ -896,6 +898,7 @@ static int load_dist_inputs(abc_ctx* c, const double* data, const double* se, in
   in.G = G;
   in.P = P;
   in.K = K;
+  in.sms = c->sms;
   if (n_fam <= 0 || !fam) {
     in.n_fam = 1;
     in.fam[0] = K;
@@ -943,7 +946,7 @@ int abc_errors(abc_ctx* c, const double* data, const double* se, int64_t G, int 
   Work w;
   const size_t o_out = w.add(sizeof(double) * (size_t)P * G);
   CK(w.allocate(c));
-  CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, c->sms, w.at<double>(o_out), c->stream));
+  CK(launch_dist_full(in, c->d_sw.p, c->d_dw.p, w.at<double>(o_out), c->stream));
   make_present(err_out, sizeof(double) * P * G);
   CK(cudaMemcpyAsync(err_out, w.at<double>(o_out), sizeof(double) * P * G, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1228,7 +1231,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
         }
         CK(launch_dist_fast(c->d_s32.p, c->d_sw.p, c->d_dw.p, P, G, K, nullptr, nullptr, nullptr, nullptr, 0,
                             c->d_esub.p, sub_stride, n_sub, c->stream));
-        CK(launch_dist_threshold(c->d_esub.p, n_sub, G, k_sub, c->d_b0.p, b1, c->d_X.p, c->stream));
+        CK(launch_dist_threshold(c->d_esub.p, n_sub, G, k_sub, c->d_b0.p, b1, c->d_X.p, c->sms, c->stream));
         if (dmode) {
           // about k_sub of every n_sub particles per gene pass X: size the per-CTA
           // segments for that (with room for imbalance) so one pass suffices
@@ -1261,7 +1264,7 @@ static int select_run(abc_ctx* c, const double* data, const double* se, int64_t 
       CK(c->d_cut.ensure((size_t)G));
       CK(c->d_cand2.ensure((size_t)std::max<int64_t>(ncand, 1)));
       CK(launch_refine(c->d_cand.p, c->d_cande.p, ncand, P, G, kq, c->d_X.p, c->d_b0.p, b1, c->d_hist.p, c->d_Xt.p,
-                       c->d_cut.p, c->d_cand2.p, c->d_ncand.p, c->stream));
+                       c->d_cut.p, c->d_cand2.p, c->d_ncand.p, c->sms, c->stream));
       unsigned long long* h = static_cast<unsigned long long*>(c->h_pin);
       CK(cudaMemcpyAsync(h, c->d_ncand.p, sizeof(*h), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
@@ -1564,6 +1567,7 @@ int abc_data_stats(abc_ctx* c, const int32_t* u, const int32_t* l, int64_t G, in
   CK(cudaMemcpyAsync(w.at<int32_t>(o_l), l, sizeof(int32_t) * G * C, cudaMemcpyHostToDevice, c->stream));
   DataStatsArgs a;
   a.cfg = c->dcfg;
+  a.sms = c->sms;
   a.u = w.at<int32_t>(o_u);
   a.l = w.at<int32_t>(o_l);
   a.G = G;

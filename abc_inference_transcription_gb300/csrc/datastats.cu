@@ -434,7 +434,7 @@ cudaError_t launch_data_stats(const DataStatsArgs& a, double* se, cudaStream_t s
     const int64_t ng = std::max<int64_t>(0, std::min<int64_t>(chunk, a.G - g0));
     const DataChunk now{g0, ng, S + (g0 / chunk % 2) * (chunk * per_gene / (int64_t)sizeof(unsigned long long))};
     // enough CTAs to fill the GPU several times over, resamples split among them
-    const int64_t want = (int64_t)4 * 152 * 5;
+    const int64_t want = (int64_t)4 * a.sms * 5;
     const int groups = ng ? (int)std::max<int64_t>(1, std::min<int64_t>(a.n_boot + 1, (want + ng - 1) / ng)) : 1;
     const int64_t items = before.n * (a.n_boot + 1) * (2 * A + J);
     const int64_t stats_blocks = (items + kThreads - 1) / kThreads;

@@ -226,11 +226,11 @@ __global__ void __launch_bounds__(1024) dist_threshold_kernel(const float* __res
 }
 
 cudaError_t launch_dist_threshold(const float* esub, int64_t n_sub, int64_t G, int64_t k_sub, const float* b0,
-                                  float b1, float* X, cudaStream_t s) {
+                                  float b1, float* X, int sms, cudaStream_t s) {
   if (G <= 0) return cudaSuccess;
   // as many genes per CTA as leave every multiprocessor one, at most 8 (128 KB of histograms)
   int lg = 0;
-  while (lg < 3 && (G >> (lg + 1)) >= 152) ++lg;
+  while (lg < 3 && (G >> (lg + 1)) >= sms) ++lg;
   const size_t smem = ((size_t)sizeof(unsigned int) * kHistBins) << lg;
   static std::atomic<uint64_t> attr{0};  // devices where the limit is set, shared by all contexts
   cudaError_t e = set_smem_once(attr, dist_threshold_kernel, (int)(sizeof(unsigned int) * kHistBins * 8));
@@ -441,7 +441,7 @@ cudaError_t launch_scatter_errors(const Cand* cand, const float* e, int64_t n, i
 
 cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int64_t P, int64_t G, int64_t k,
                           const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, float2* cut,
-                          Cand* out, unsigned long long* count, cudaStream_t s) {
+                          Cand* out, unsigned long long* count, int sms, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(unsigned int) * (size_t)G * kCandBins, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
@@ -451,7 +451,7 @@ cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int6
     static std::atomic<uint64_t> attr{0};
     e = set_smem_once(attr, cand_hist_smem_kernel, (int)(sizeof(unsigned int) * kCandBins * kSmemHistGenes));
     if (e != cudaSuccess) return e;
-    const int hb = (int)((n + 8191) / 8192 < 152 ? (n + 8191) / 8192 : 152);
+    const int hb = (int)((n + 8191) / 8192 < sms ? (n + 8191) / 8192 : sms);
     cand_hist_smem_kernel<<<hb, 1024, sizeof(unsigned int) * kCandBins * (size_t)G, s>>>(cand, cand_e, n, (int)G, b0, b1,
                                                                                         hist);
   } else if (n > 0) {

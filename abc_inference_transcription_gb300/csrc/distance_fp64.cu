@@ -537,11 +537,10 @@ static cudaError_t launch_full(const DistInputs& in, const float* sw, const floa
 //   500 x 300       0.193 / 0.192    0.083 / 0.318   0.084 / 0.211
 //   200 x 2,000     0.561 / 0.562    0.114 / 0.483   0.112 / 0.387
 //   2,000 x 300     0.714 / 0.715    0.111 / 0.659   32 particles
-cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, int sms, double* err,
-                             cudaStream_t s) {
+cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, double* err, cudaStream_t s) {
   if (in.P <= 0 || in.G <= 0) return cudaSuccess;
   const int64_t tiles = (in.G + kFullTile - 1) / kFullTile;
-  auto fills = [&](int rows) { return (in.P + rows - 1) / rows * tiles >= 2 * (int64_t)sms; };
+  auto fills = [&](int rows) { return (in.P + rows - 1) / rows * tiles >= 2 * (int64_t)in.sms; };
   if (fills(kFullRows)) return launch_full<kFullRows>(in, sw, dw, tiles, err, s);
   if (fills(16)) return launch_full<16>(in, sw, dw, tiles, err, s);
   if (fills(8)) return launch_full<8>(in, sw, dw, tiles, err, s);
@@ -949,7 +948,7 @@ static int grouped_blocks(int64_t n, int warps) {
 static void launch_recheck_grouped(const DistInputs& in, const int32_t* sp, const int32_t* sg, int64_t n, double* se64,
                                    cudaStream_t s) {
   const int64_t chunks = (n + 31) / 32;
-  if (chunks <= 4 * 152)  // at most a warp per scheduler
+  if (chunks <= 4 * (int64_t)in.sms)  // at most a warp per scheduler
     recheck_grouped_kernel<1><<<(unsigned)chunks, 32, 0, s>>>(in, sp, sg, n, se64);
   else
     recheck_grouped_kernel<kRecheckWarps><<<grouped_blocks(n, kRecheckWarps), kRecheckWarps * 32, 0, s>>>(in, sp, sg, n, se64);
@@ -981,7 +980,7 @@ cudaError_t launch_dist_group_certify_sort(const DistInputs& in, Cand* cand, flo
   const float rK = (float)(1.0 / (double)in.K);
   approx_grouped_kernel<<<grouped_blocks(n, kApproxWarps), kApproxWarps * 32, 0, s>>>(in, sp, sg, n, gt, rK, se64, pos,
                                                                                      counts);
-  const int list_blocks = 152 * 8;
+  const int list_blocks = in.sms * 8;
   recheck_list_kernel<<<list_blocks, 128, 0, s>>>(in, sp, sg, pos, counts, se64);
   err = launch_segsort(goff, in.G, sp, se64, nullptr, cand, cand_e, s);
   if (err) return err;

@@ -23,6 +23,7 @@ struct StatsArgs {
   int fp32 = 0;              // production mode: FP32 binomial capture (a different realisation)
   const float* beta32 = nullptr;  // [C] the capture efficiencies in FP32 (production mode)
   int64_t max_group_cells = INT64_MAX;  // cells of the largest (condition, age) group
+  int sms;                              // the device's multiprocessors
 };
 
 struct SetupArgs {
@@ -36,6 +37,7 @@ struct SetupArgs {
   PRecF* recf;
   int* status;
   int fp32 = 0;              // production mode: FP32 rates beyond its range are an error
+  int sms;                   // the device's multiprocessors
 };
 
 struct PriorArgs {
@@ -63,6 +65,7 @@ struct DistInputs {
   int K;
   int n_fam;
   int fam[16];          // family sizes (sum K)
+  int sms;              // the device's multiprocessors
 };
 
 struct Cand {
@@ -123,7 +126,7 @@ cudaError_t launch_dist_fast(const float* s32, const float* sw, const float* dw,
 // per gene: X[g] = upper edge of the histogram bin where the count of esub
 // reaches k_sub, plus the bound (+inf when fewer than k_sub finite values).
 cudaError_t launch_dist_threshold(const float* esub, int64_t n_sub, int64_t G, int64_t k_sub, const float* b0,
-                                  float b1, float* X, cudaStream_t s);
+                                  float b1, float* X, int sms, cudaStream_t s);
 cudaError_t launch_fill(float* x, int64_t n, float v, cudaStream_t s);
 // dense[p G + g] = e of candidate (p, g), clipped at 10
 cudaError_t launch_scatter_errors(const Cand* cand, const float* e, int64_t n, int64_t G, float* out, cudaStream_t s);
@@ -137,7 +140,7 @@ cudaError_t launch_x_from_thr(const double* thr, double eps, int64_t G, const fl
 // particles) are kept: enough for any k smallest, as ties are ordered by index.
 cudaError_t launch_refine(const Cand* cand, const float* cand_e, int64_t n, int64_t P, int64_t G, int64_t k,
                           const float* X, const float* b0, float b1, unsigned int* hist, float* Xt, float2* cut,
-                          Cand* out, unsigned long long* count, cudaStream_t s);
+                          Cand* out, unsigned long long* count, int sms, cudaStream_t s);
 // den[g][k] = (se^2 + 0.01 d^2) + eps_gk, the denominators of the error terms,
 // evaluated as in the per-term FP64 expression (bit-identical), and rden = 1/den
 // (both may be null); sw = sqrt(w), dw = sqrt(w) d in FP32, w = 1/den.
@@ -173,9 +176,8 @@ cudaError_t launch_scan(const int64_t* cnt, int64_t G, int64_t* off, cudaStream_
 // in.rden.  sp, sg: n scratch entries each.
 cudaError_t launch_accepted_errors(const DistInputs& in, const int64_t* aoff, const int64_t* idx, int64_t G,
                                    int64_t p_base, int64_t n, int32_t* sp, int32_t* sg, double* err, cudaStream_t s);
-// full FP64 error matrix [P][G]; sw, dw: the terms of launch_dist_den; sms: the device's multiprocessors
-cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, int sms, double* err,
-                             cudaStream_t s);
+// full FP64 error matrix [P][G]; sw, dw: the terms of launch_dist_den
+cudaError_t launch_dist_full(const DistInputs& in, const float* sw, const float* dw, double* err, cudaStream_t s);
 
 // moment ODE (moment.cu)
 struct MomArgs {
@@ -217,6 +219,7 @@ struct DataStatsArgs {
   double* out;                // [G][n_boot + 1][K]
   unsigned long long* sums;   // data_stats_scratch bytes
   int* invalid;               // set when a count lies outside [0, 2^20]
+  int sms;                    // the device's multiprocessors
 };
 // bytes of the group sums of the (gene, resample) pairs processed at a time,
 // and of the reciprocals of the sample sizes

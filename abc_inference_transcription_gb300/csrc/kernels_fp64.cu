@@ -75,8 +75,7 @@ cudaError_t launch_prior(const PriorArgs& a, cudaStream_t s) {
 // GPU.  One particle: 107 us with 8 lanes and sources inside the recurrences, 73 now; 10,000:
 // 455 us, 342 now.
 // ---------------------------------------------------------------------------
-constexpr int kSetupLanes = 8;  // 32 up to kSetupWide particles
-constexpr int64_t kSetupWide = 4 * 152;  // a warp per scheduler
+constexpr int kSetupLanes = 8;  // 32 up to a warp per scheduler
 static_assert(kSetupLanes >= kMaxSteps, "lane k holds age step k");
 constexpr int kMaxSub = kMaxSteps * kIcSub;
 
@@ -329,7 +328,7 @@ __global__ void __launch_bounds__(32) setup_kernel(SetupArgs A) {
 
 cudaError_t launch_setup(const SetupArgs& a, cudaStream_t s) {
   if (a.n_particles <= 0) return cudaSuccess;
-  if (a.n_particles <= kSetupWide) {
+  if (a.n_particles <= 4 * (int64_t)a.sms) {
     setup_kernel<32><<<(unsigned)a.n_particles, 32, 0, s>>>(a);
   } else {
     constexpr int per = 32 / kSetupLanes;
@@ -491,14 +490,11 @@ __device__ __forceinline__ __int128 shfl_xor_i128(__int128 v, int o) {
   return (__int128)(((unsigned __int128)(unsigned long long)hi << 64) | (unsigned __int128)lo);
 }
 
-// 1,024 threads per particle up to one particle per SM
-constexpr int kStatsWideParticles = 152;
-
 // NARROW: 64-bit sums of the squared counts (production mode: counts at most
 // 2^24, where FP32 increments stop, and at most 2^14 cells per group, so the
 // sums stay below 2^62); 128-bit otherwise.
 // THREADS: 256, or 1,024 where the launch has too few particles to fill the
-// GPU (the groups are then the parallelism: a particle alone with 55 groups
+// GPU, at most one per SM (the groups are then the parallelism: a particle alone with 55 groups
 // of 36 cells takes 90 us in 8 warps, 51 in 32).
 template <bool CAP32, bool NARROW, int THREADS>
 __global__ void __launch_bounds__(THREADS) stats_kernel(StatsArgs A) {
@@ -572,7 +568,7 @@ __global__ void __launch_bounds__(THREADS) stats_kernel(StatsArgs A) {
 cudaError_t launch_stats(const StatsArgs& a, cudaStream_t s) {
   if (a.n_particles <= 0) return cudaSuccess;
   int blocks = (int)(a.n_particles < 1048576 ? a.n_particles : 1048576);
-  if (a.fp32 && a.max_group_cells <= 16384 && blocks <= kStatsWideParticles)
+  if (a.fp32 && a.max_group_cells <= 16384 && blocks <= a.sms)
     stats_kernel<true, true, 1024><<<blocks, 1024, 0, s>>>(a);
   else if (a.fp32 && a.max_group_cells <= 16384)
     stats_kernel<true, true, 256><<<blocks, 256, 0, s>>>(a);

@@ -191,6 +191,9 @@ extern "C" int abc_simulate_noalloc(const abc_config* cfg, int model, int64_t n_
   d.npar = 5 + (model >= 3 ? cfg->n_steps - 1 : 0) + d.splicing + d.scaling_column;
   dcfg_set_grid(d);
 
+  int dev = 0, sms = 0;
+  NA_CK(cudaGetDevice(&dev));
+  NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   SetupArgs sa;
   sa.cfg = d;
   sa.model = model;
@@ -202,11 +205,9 @@ extern "C" int abc_simulate_noalloc(const abc_config* cfg, int model, int64_t n_
   sa.recf = d_recf;
   sa.status = status;
   sa.fp32 = cfg->precision == ABC_FP32 ? 1 : 0;
+  sa.sms = sms;
   NA_CK(launch_setup(sa, stream));
 
-  int dev = 0, sms = 0;
-  NA_CK(cudaGetDevice(&dev));
-  NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const bool fp64 = cfg->precision == ABC_FP64;
   const int bps = std::max(1, fp64 ? ssa_blocks_per_sm_fp64() : ssa_blocks_per_sm_fp32());
   SsaArgs ss;
@@ -250,6 +251,7 @@ extern "C" int abc_simulate_noalloc(const abc_config* cfg, int model, int64_t n_
   sta.fp32 = fp64 ? 0 : 1;
   sta.beta32 = d_beta32;
   sta.max_group_cells = *std::max_element(count.begin(), count.end());
+  sta.sms = sms;
   NA_CK(launch_stats(sta, stream));
 
   int hs = 0;

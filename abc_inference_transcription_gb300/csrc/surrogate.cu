@@ -243,7 +243,7 @@ __global__ void count_keep_kernel(const uint8_t* keep, int64_t N, unsigned long 
 }
 
 // of the kernels that keep the columns' terms per block
-int norm_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 152 * 8); }
+int norm_blocks(int64_t n, int sms) { return (int)std::min<int64_t>((n + 255) / 256, (int64_t)sms * 8); }
 int blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 65536); }
 
 // Survivor compaction in ascending row order: per-1024-row counts, one scan,
@@ -505,9 +505,9 @@ static int load_training(abc_surrogate* s, const double* theta, const double* st
   } else {
     asinh_apply_kernel<<<blocks(N * d.K), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->yscf.p);
   }
-  norm_x_kernel<<<norm_blocks(N * d.in_pad), 256, 0, s->stream>>>(s->th64.p, N, d.in_dim, d.in_dim, s->xm.p, s->xs.p,
+  norm_x_kernel<<<norm_blocks(N * d.in_pad, s->sms), 256, 0, s->stream>>>(s->th64.p, N, d.in_dim, d.in_dim, s->xm.p, s->xs.p,
                                                               d.in_pad, s->xn.p, nullptr);
-  norm_y_kernel<<<norm_blocks(N * d.K), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->ym.p, s->ys.p, s->yn.p);
+  norm_y_kernel<<<norm_blocks(N * d.K, s->sms), 256, 0, s->stream>>>(s->st64.p, N, d.K, s->ym.p, s->ys.p, s->yn.p);
   SK(cudaGetLastError());
   return ABC_OK;
 }
@@ -637,7 +637,7 @@ static int forward_chunk(abc_surrogate* s, const double* d_theta, int ld, int64_
   const int E = s->members;
   SK(s->X0.ensure((size_t)n * d.in_pad));
   SK(s->Y.ensure((size_t)E * n * d.out_pad));
-  norm_x_kernel<<<norm_blocks(n * d.in_pad), 256, 0, s->stream>>>(d_theta, n, d.in_dim, ld, s->xm.p, s->xs.p, d.in_pad,
+  norm_x_kernel<<<norm_blocks(n * d.in_pad, s->sms), 256, 0, s->stream>>>(d_theta, n, d.in_dim, ld, s->xm.p, s->xs.p, d.in_pad,
                                                               nullptr, s->X0.p);
   SK(cudaGetLastError());
   if (mlp_infer_fits(d)) {
@@ -733,6 +733,7 @@ int abc_surrogate_screen_device(abc_surrogate* s, const double* d_theta, int ld_
   in.K = K;
   in.n_fam = 1;
   in.fam[0] = K;
+  in.sms = s->sms;
   SK(launch_dist_den(in, nullptr, nullptr, s->sw.p, s->dw.p, s->stream));
   std::vector<float> hx((size_t)G);
   for (int64_t g = 0; g < G; ++g) hx[g] = (float)(thr[g] + margin);
