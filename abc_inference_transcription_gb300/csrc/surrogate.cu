@@ -371,11 +371,13 @@ static int ensure_batch(abc_surrogate* s, int B) {
   SK(s->X0.ensure(E * B * d.in_pad));
   SK(s->T.ensure(E * B * d.K));
   SK(s->Z.ensure(E * 3 * B * d.H));
-  SK(s->Ah.ensure(E * 3 * B * d.H));
   SK(s->Y.ensure(E * B * d.out_pad));
   SK(s->dY.ensure(E * B * d.out_pad));
-  SK(s->dZa.ensure(E * B * d.H));
-  SK(s->dZb.ensure(E * B * d.H));
+  if (!mlp_infer_fits(d)) {  // row-major activations and derivatives, which only the passes layer by layer keep
+    SK(s->Ah.ensure(E * 3 * B * d.H));
+    SK(s->dZa.ensure(E * B * d.H));
+    SK(s->dZb.ensure(E * B * d.H));
+  }
   s->ldT = (B + 7) / 8 * 8;   // 16-byte rows for the tensor maps
   const size_t lt = (size_t)s->ldT;
   SK(s->X0T.ensure(E * d.in_pad * lt));
