@@ -111,7 +111,8 @@ cudaError_t launch_tc_y(const float* X, const double* cg64, int64_t G, int K, fl
 // mode 1: TF32 one term, 2: TF32 hi/lo three terms, 3: BF16 hi/lo three terms
 cudaError_t launch_dist_tc(int mode, const void* A, const void* B, const TcArgs& args, int grid, cudaStream_t s);
 // concatenates the per-CTA segments; seg_e holds raw accumulators, out_e the
-// clipped FP32 errors min((acc + c_g) / K, 10)
+// FP32 errors (acc + c_g) / K, not clipped (launch_refine tells the surely clipped ones by
+// them; launch_scatter_errors clips); 10 where that is NaN
 cudaError_t launch_tc_gather(const Cand* seg, const float* seg_e, const unsigned* count, int n_seg, int64_t seg_cap,
                              const float* cg, int K, Cand* out, float* out_e, cudaStream_t s);
 

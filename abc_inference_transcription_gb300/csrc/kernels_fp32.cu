@@ -98,6 +98,13 @@ __global__ void order_hist_kernel(const PRec* rec, int64_t P, unsigned int* hist
 // five-model prior draws with 1, 2, 3, 4, 8 blocks: 101 particles x 1,437
 // cells 15, 17, 25, 27, 25; 2,000 x 2,000 (one block not measured) 74, 69, 76, 80; 10,000 x
 // 2,000 396, 360, 352, 363.  Blocks beyond the number leave at once.
+// The tables are those of the two-species kernel with a size exponent of 0 or 1 on the
+// integer grid.  The other kernels' iterations are longer, by much the same factor in
+// every row, which the choice does not depend on.  Milliseconds of the SSA kernel by this
+// rule / with all blocks, 2,000 cells, one model's prior draws, 64, 250 and 1,000 particles:
+// this kernel 13.9 / 29.0, 18.2 / 29.8, 43.0 / 45.3; splicing 21.3 / 35.2, 27.5 / 42.1,
+// 63.1 / 71.7; general exponent 21.4 / 33.1, 25.9 / 41.8, 59.0 / 66.9; both 45.1 / 56.8,
+// 46.4 / 83.0, 76.1 / 96.0.  Within 4 % of each other at 4 and 16 particles and at 4,000.
 __device__ __forceinline__ int planned_blocks(const WorkPlan* plan, int64_t n_cells, int sms, int most) {
   const float alone[8] = {76.f, 106.f, 155.f, 205.f, 251.f, 294.f, 340.f, 389.f};
   const float sum[8] = {110.f, 148.f, 201.f, 264.f, 319.f, 374.f, 433.f, 487.f};
