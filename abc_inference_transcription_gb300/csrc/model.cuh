@@ -275,6 +275,8 @@ ABC_HD void stats_from_moments_cond(const DevCfg& cfg, const double* m, const do
         st[off + a] = tot;
         st[off + A + a] = ((vu[a] + 2.0 * cv[a]) + vl[a]) / (tot + eps);
       }
+      if (off == 0 && j == cfg.chase_stat)  // one condition gives both families
+        for (int a = 0; a < 2 * A; ++a) st[2 * A + a] = st[a];
     }
   }
 }

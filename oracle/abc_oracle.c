@@ -844,8 +844,9 @@ int orc_stats_from_moments(const abc_config* cfg, const double* m, const double*
     double stds = sqrt(fabs(tvu * tvl));
     st[4 * A + J + j] = wsum(w, cv, A) / stds;
     st[4 * A + 2 * J + j] = wcov(mu, ml, w, A) / stds;
-    int off = (j == cfg->pulse_stat_cond) ? 0 : (j == cfg->chase_stat_cond) ? 2 * A : -1;
-    if (off >= 0) {
+    for (int f = 0; f < 2; ++f) {  /* both families where one condition gives them */
+      if (j != (f ? cfg->chase_stat_cond : cfg->pulse_stat_cond)) continue;
+      const int off = 2 * A * f;
       for (int a = 0; a < A; ++a) {
         double tot = mu[a] + ml[a];
         double eps = (tot == 0.0) ? 0.0001 : 0.0;
