@@ -128,7 +128,7 @@ __device__ __forceinline__ double div_whole(double t, double d, double y) {
 // Horner form and squaring back.
 __global__ void __launch_bounds__(kExpThreads) moment_exp_kernel(MomArgs a, MomScratch ws) {
   const int64_t i = (int64_t)blockIdx.x * kExpThreads + threadIdx.x, n = ws.n;
-  if (i >= n) return;
+  if (i >= n || ws.rates[kRateBad * n + i] != 0.0) return;
   const int lab = (int)blockIdx.y / a.nsub, idx = (int)blockIdx.y - lab * a.nsub, k = idx / a.per_step;
   const double* m = ws.rates + i;
   const double h = a.h;
@@ -260,6 +260,8 @@ __global__ void __launch_bounds__(32) moment_walk_kernel(MomArgs a, int64_t p0, 
   const int base = grp * NA;
   const int64_t i = (int64_t)blockIdx.x * kWalkGroup + grp, ic = min(i, n - 1);
   const bool live = lane < kWalkGroup * NA && i < n && ws.rates[kRateBad * n + ic] == 0.0;
+  // (an invalid particle beside a valid one has no propagators: its lanes feed only each other)
+  if (!__any_sync(0xffffffffu, live)) return;
   const int nsub = a.nsub;
   int col[kRow], len = 0;
 #pragma unroll
